@@ -472,7 +472,9 @@ cudaError_t launch_postamble(const dev::Inst* insts_d, const dev::WorkItem* work
  * every integer below 2^22 in magnitude: its float on the FP32 pipe; 2^32
  * doubles covering every high word: the integer-pipe narrowing toward zero
  * against the hardware conversion; 2^24 hashed operand sets: the packed
- * double-float accumulation against the scalar one. */
+ * double-float accumulation against the scalar one; 2^26 operand pairs: the
+ * integer-pipe division against the FP64 division; every float in [1, 2]: the
+ * reciprocal seed's error. */
 __global__ void f2d_selftest_kernel(unsigned long long* mismatches) {
   unsigned long long bad = 0;
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
@@ -512,6 +514,44 @@ __global__ void f2d_selftest_kernel(unsigned long long* mismatches) {
       if (__float_as_uint(g.x) != __float_as_uint(g1.x) || __float_as_uint(g.z) != __float_as_uint(g1.y) ||
           __float_as_uint(g.y) != __float_as_uint(g2.x) || __float_as_uint(g.w) != __float_as_uint(g2.y))
         ++bad;
+    }
+    /* the integer-pipe division against the FP64 division, on 2^26 hashed
+     * operand pairs: any bits, significands near a power of two, exact
+     * products, quotients near 1, small integers, zeros */
+    if ((i & 63u) == 0u) {
+      uint64_t h = i * 0x9E3779B97F4A7C15ull;
+      auto next = [&h]() {
+        h += 0x9E3779B97F4A7C15ull;
+        uint64_t z = h;
+        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+        z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+        return z ^ (z >> 31);
+      };
+      const uint64_t u = next(), v = next();
+      const uint64_t mask = (1ull << 52) - 1;
+      auto moderate = [](uint64_t w) { return dev::d_from_bits((w & 0x800fffffffffffffull) | ((923 + (w >> 52) % 200) << 52)); };
+      auto edge = [&](uint64_t w) {
+        const uint64_t m = (w & 1) ? mask - ((w >> 1) & 7) : ((w >> 1) & 7);
+        return dev::d_from_bits(((1000 + (w >> 8) % 46) << 52) | m);
+      };
+      double a, b;
+      switch ((i >> 6) & 7u) {
+        case 0: a = dev::d_from_bits(u); b = dev::d_from_bits(v); break;
+        case 1: a = edge(u); b = edge(v); break;
+        case 2: b = moderate(v); a = moderate(u) * b; break;
+        case 3: b = moderate(v); a = dev::d_from_bits(dev::d_bits(b) + (u & 15)); break;
+        case 4: a = double(u % 100000); b = double(1 + v % 1000); break;
+        case 5: a = (u & 1) ? 0.0 : -0.0; b = moderate(v); break;
+        default: a = moderate(u); b = moderate(v); break;
+      }
+      const uint64_t q = dev::d_bits(dev::ddiv_int(a, b)), want = dev::d_bits(a / b);
+      if (q != want && !(isnan(a / b) && isnan(dev::d_from_bits(q)))) ++bad;
+    }
+    /* the reciprocal seed never exceeds 2^24 / b and falls short by < 4.1 */
+    if (i <= 0x800000u) {
+      const double r = 16777216.0 / double(__uint_as_float(0x3f800000u + uint32_t(i)));
+      const double short_by = r - double(dev::rcp_seed(0x3f800000u + uint32_t(i)));
+      if (!(short_by >= 1.0 && short_by <= 3.0)) ++bad;
     }
   }
   if (bad) atomicAdd(mismatches, bad);

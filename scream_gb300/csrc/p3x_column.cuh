@@ -558,19 +558,19 @@ __device__ void p3_part12(const Inst& in, const int col, const KParams<TR>& kp, 
 
     double rho, inv_rho, qvsl, qvsi, qvssi, ccn_nc;
     TR rho_t, inv_rho_t;
-    const double exner = kF64 ? 1 / inv_exner : rcp_newton1(inv_exner);
+    const double exner = kF64 ? m_div(1.0, inv_exner) : rcp_newton1(inv_exner);
     double T = th * exner;
     qv = dmax0(qv);
     if constexpr (kF64) {
-      const double inv_cld_l = 1 / cld_l;
-      rho = dpres / dz / C::gravit;
-      inv_rho = 1 / rho;
+      const double inv_cld_l = m_div(1.0, cld_l);
+      rho = m_div(m_div(dpres, dz), C::gravit);
+      inv_rho = m_div(1.0, rho);
       rho_t = rho;
       inv_rho_t = inv_rho;
       qvsl = qv_sat_dry(T, pres, false, err);
       qvsi = qv_sat_dry(T, pres, true, err);
-      qvssi = qv / qvsi - 1;
-      ccn_nc = rt.spa_ccn_to_nc_factor * in.nccn[o] / inv_cld_l;
+      qvssi = m_div(qv, qvsi) - 1;
+      ccn_nc = m_div(rt.spa_ccn_to_nc_factor * in.nccn[o], inv_cld_l);
     } else {
       /* FP32-bulk: rho and 1/rho only feed rates, fall speeds and fluxes
        * (the sedimentation's FP64 coefficient is g / dpres), so they are
@@ -593,8 +593,8 @@ __device__ void p3_part12(const Inst& in, const int col, const KParams<TR>& kp, 
     }
     const TR rhofacr = m_pow(TR(C::RHO_1000MB) * inv_rho_t, TR(.54));
     const TR rhofaci = m_pow(TR(C::RHO_600MB) * inv_rho_t, TR(.54));
-    const TR dum = TR(1.496e-6) * m_pow(TR(T), TR(1.5)) / (TR(T) + TR(120));
-    const TR acn = TR(C::gravit) * TR(C::RHO_H2O) / (TR(18) * dum);
+    const TR dum = m_div(TR(1.496e-6) * m_pow(TR(T), TR(1.5)), TR(T) + TR(120));
+    const TR acn = m_div(TR(C::gravit) * TR(C::RHO_H2O), TR(18) * dum);
     if (dlt(T, C::T_zerodegc) && dge_neg(qvssi, -0.05)) nucl = true;
 
     /* A species below qsmall goes to vapour; a +0 moves nothing, so its FP64
@@ -703,11 +703,12 @@ __device__ void p3_part12(const Inst& in, const int col, const KParams<TR>& kp, 
     const double inv_exner = in.inv_exner[o];
     const double qvsl = SMA(A_QVSL, k), qvsi = SMA(A_QVSI, k);
     const double rho = SMA(A_RHO, k);
-    const double inv_rho = 1 / rho;
+    const double inv_rho = m_div(1.0, rho);
     const double rhofaci = SMA(A_RHOFACI, k);
     const double acn = SMA(A_ACN, k);
     Incld inc;
-    calc_incloud(s.qc, s.qr, s.qi, s.qm, s.nc, s.nr, s.ni, s.bm, 1 / cld_l, 1 / cld_i, 1 / cld_r, inc);
+    calc_incloud(s.qc, s.qr, s.qi, s.qm, s.nc, s.nr, s.ni, s.bm, m_div(1.0, cld_l), m_div(1.0, cld_i),
+                 m_div(1.0, cld_r), inc);
 
     Rates<TR> r;
     r.zero();
@@ -736,7 +737,7 @@ __device__ void p3_part12(const Inst& in, const int col, const KParams<TR>& kp, 
         get_rain_dsd2<TR>(TR(inc.qr), n_out, mu_r, lamr, rt);
         apply_n_adjust(inc.nr, n_in, n_out);
         if (dge(inc.qr, C::QSMALL)) {
-          cdistr = TR(inc.nr) / TR(rt.g_mur1);
+          cdistr = m_div(TR(inc.nr), TR(rt.g_mur1));
           logn0r = m_log10(cdistr) + (mu_r + TR(1)) * m_log10(lamr);
         }
         s.nr = inc.nr * cld_r;
@@ -771,7 +772,7 @@ __device__ void p3_part12(const Inst& in, const int col, const KParams<TR>& kp, 
       }
       const TR qi_r = inc.qi, qc_r = inc.qc, ni_r = inc.ni, nc_r = inc.nc, qr_r = inc.qr;
       const double dT0 = T - C::Tmelt;
-      const double dqv0 = C::ep_2 * esat0 / vmax(pres, 1.e-3) - s.qv;
+      const double dqv0 = m_div(C::ep_2 * esat0, vmax(pres, 1.e-3)) - s.qv;
       if (do_ice) {
         ice_cldliq_collection<TR>(rho, T, rhofaci, tv_qc2qi, qi_r, qc_r, ni_r, nc_r, r, rt);
         ice_rain_collection<TR>(rho, T, rhofaci, logn0r, tv_nr, tv_qr2qi, qi_r, ni_r, qr_r, r, rt);
@@ -783,7 +784,7 @@ __device__ void p3_part12(const Inst& in, const int col, const KParams<TR>& kp, 
       }
       /* ice_relaxation_timescale, p3_ice_relaxation_timescale_impl.hpp:9-37 */
       if (dge(inc.qi, C::QSMALL) && dlt(T, C::Tmelt)) {
-        epsi = ((tv_melt + tv_vent * m_cbrt(v.sc) * m_sqrt(rhofaci * rho / v.mu)) * TR(2.0) * TR(C::Pi) * rho *
+        epsi = ((tv_melt + tv_vent * m_cbrt(v.sc) * m_sqrt(m_div(rhofaci * rho, v.mu))) * TR(2.0) * TR(C::Pi) * rho *
                 v.dv) * ni_r;
         epsi_tot = epsi_tot + epsi;
       } else {
@@ -799,8 +800,8 @@ __device__ void p3_part12(const Inst& in, const int col, const KParams<TR>& kp, 
         Table3<TR> t3;
         lookup3<TR>(mu_r, lamr, rt, t3);
         epsr = TR(2) * TR(C::Pi) * cdistr * rho * v.dv *
-               (TR(C::f1r) * TR(rt.g_mur2) / lamr +
-                TR(C::f2r) * m_sqrt(rho / v.mu) * m_cbrt(v.sc) * apply_table3<TR>(tb, tb.revap, t3));
+               (m_div(TR(C::f1r) * TR(rt.g_mur2), lamr) +
+                TR(C::f2r) * m_sqrt(m_div(rho, v.mu)) * m_cbrt(v.sc) * apply_table3<TR>(tb, tb.revap, t3));
       }
       evaporate_rain(inc.qr, inc.qc, inc.nr, inc.qi, cld_l, cld_r, s.qv, in.qv_prev[o], qvsl, qvsi, v.ab, v.abi,
                      epsr, epsi_tot, T, in.t_prev[o], v.dqsdt, dt, r.qr2qv_evap_tend, r.nr_evap_tend);
@@ -820,7 +821,7 @@ __device__ void p3_part12(const Inst& in, const int col, const KParams<TR>& kp, 
 
     water_conservation<double>(s.qc, s.qr, s.qi, dt, r);
     number_conservation<double>(s.nc, s.nr, s.ni, dt, r);
-    ice_supersat_conservation(r, cld_i, s.qv, qvsi, s.th / inv_exner, dt);
+    ice_supersat_conservation(r, cld_i, s.qv, qvsi, m_div(s.th, inv_exner), dt);
     prevent_liq_supersaturation(pres, T, s.qv, dt, r, err);
     update_prognostics(r, inv_exner, predictNc, prescribedCCN, wet, dt, rho_qm_cloud, inv_rho, s);
 
@@ -833,7 +834,7 @@ __device__ void p3_part12(const Inst& in, const int col, const KParams<TR>& kp, 
                              r.qc2qi_berg_tend + r.qc2qi_collect_tend + r.qr2qi_collect_tend;
 
     hydro |= clip_to_vapour(s, inv_exner);
-    double ni_incld = s.ni / cld_i;
+    double ni_incld = m_div(s.ni, cld_i);
     impose_max_total_ni(ni_incld, rt.max_total_ni, inv_rho);
     s.ni = ni_incld * cld_i;
     in.qc[o] = s.qc; in.nc[o] = s.nc; in.qr[o] = s.qr; in.nr[o] = s.nr;
@@ -879,15 +880,15 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
   const int64_t co = int64_t(col) * in.ld;
   const int64_t ci = int64_t(col) * in.ld_int;
   const double dt = in.dt;
-  const double inv_dt = 1 / dt;
+  const double inv_dt = m_div(1.0, dt);
   const bool predictNc = in.predictNc != 0;
   const int kbot = nk - 1;
 #define SMA(a, k) sm[(a)*S + (k)]
   for (int k = lane; k < nk; k += LANES) {
     const double rho = scr_at(in, S_RHO, col)[k];
     SMA(B_RHO, k) = rho;
-    SMA(B_INVRHO, k) = 1 / rho;
-    SMA(B_INVDZ, k) = 1 / in.dz[co + k];
+    SMA(B_INVRHO, k) = m_div(1.0, rho);
+    SMA(B_INVDZ, k) = m_div(1.0, in.dz[co + k]);
   }
   double precip_liq_surf = 0, precip_ice_surf = 0;
 
@@ -961,7 +962,7 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
         if (sp == 0) {
           double qc_incld, nc_incld;
           if (first) {
-            const double inv_cld = 1 / cld;
+            const double inv_cld = m_div(1.0, cld);
             if (dge(R0[k], C::QSMALL)) {
               qc_incld = R0[k] * inv_cld;
               nc_incld = dmax0(R1[k] * inv_cld);
@@ -971,8 +972,8 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
             }
             qc_incld = dmin_c(qc_incld, C::incloud_limit);
           } else {
-            qc_incld = R0[k] / cld;
-            nc_incld = R1[k] / cld;
+            qc_incld = m_div(R0[k], cld);
+            nc_incld = m_div(R1[k], cld);
           }
           if (dgt(qc_incld, C::QSMALL)) {
             TR mu_c, lamc;
@@ -983,7 +984,7 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
             /* Stokes fall speeds, p3_cloud_sed_impl.hpp:99-103, with
              * Gamma(6+mu)/Gamma(4+mu) = (5+mu)(4+mu) and
              * Gamma(3+mu)/Gamma(1+mu) = (2+mu)(1+mu) (bcn = 2) */
-            const TR dum = TR(1) / (lamc * lamc);
+            const TR dum = m_div(TR(1), lamc * lamc);
             const TR acn = TR(FAC[k]);
             v1 = double(acn * ((TR(5) + mu_c) * (TR(4) + mu_c)) * dum);
             if (predictNc) v2 = double(acn * ((TR(2) + mu_c) * (TR(1) + mu_c)) * dum);
@@ -992,7 +993,7 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
         } else if (sp == 1) {
           double qr_incld, nr_incld;
           if (first) {
-            const double inv_cld = 1 / cld;
+            const double inv_cld = m_div(1.0, cld);
             if (dge(R0[k], C::QSMALL)) {
               qr_incld = R0[k] * inv_cld;
               nr_incld = dmax0(R1[k] * inv_cld);
@@ -1002,8 +1003,8 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
             }
             qr_incld = dmin_c(qr_incld, C::precip_limit);
           } else {
-            qr_incld = R0[k] / cld;
-            nr_incld = R1[k] / cld;
+            qr_incld = m_div(R0[k], cld);
+            nr_incld = m_div(R1[k], cld);
           }
           if (dgt(qr_incld, C::QSMALL)) {
             TR mu_r = 0, lamr;
@@ -1022,7 +1023,7 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
           {
             double qi_incld, ni_incld, qm_incld, bm_incld;
             if (first) {
-              const double inv_cld = 1 / cld;
+              const double inv_cld = m_div(1.0, cld);
               if (dge(R0[k], C::QSMALL)) {
                 qi_incld = R0[k] * inv_cld;
                 ni_incld = dmax0(R1[k] * inv_cld);
@@ -1032,7 +1033,7 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
               }
               if (dge(R0[k], C::QSMALL) && dge(R2[k], C::QSMALL)) {
                 qm_incld = R2[k] * inv_cld;
-                bm_incld = dmax0(R3[k] * (1 / in.cld_frac_l[co + k]));
+                bm_incld = dmax0(R3[k] * m_div(1.0, in.cld_frac_l[co + k]));
               } else {
                 qm_incld = 0;
                 bm_incld = 0;
@@ -1040,10 +1041,10 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
               qi_incld = dmin_c(qi_incld, C::incloud_limit);
               bm_incld = dmin_c(bm_incld, C::incloud_limit);
             } else {
-              qi_incld = R0[k] / cld;
-              ni_incld = R1[k] / cld;
-              qm_incld = R2[k] / cld;
-              bm_incld = R3[k] / cld;
+              qi_incld = m_div(R0[k], cld);
+              ni_incld = m_div(R1[k], cld);
+              qm_incld = m_div(R2[k], cld);
+              bm_incld = m_div(R3[k], cld);
             }
             if (dgt(qi_incld, C::QSMALL)) {
               ni_incld = dmax_c(ni_incld, C::NSMALL);
@@ -1081,7 +1082,7 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
        * fluxes from start-of-substep values, inflow from the level above by a
        * shuffle (carried across chunks), zero inflow at k_qxtop. */
       const int tmpint1 = static_cast<int>(Co_max + 1);
-      const double dt_sub = dt_left / tmpint1;
+      const double dt_sub = m_div(dt_left, double(tmpint1));
       const int k_temp = (k_qxbot == kbot) ? k_qxbot : k_qxbot + 1;
       double carry0 = 0, carry1 = 0, carry2 = 0, carry3 = 0, flux_bot = 0;
       for (int base = k_qxtop; base <= k_temp; base += LANES) {
@@ -1541,7 +1542,7 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
     float rho_f = 0.f, inv_rho_f = 0.f;
     if constexpr (kF64) {
       rho = scr_at(in, S_RHO, col)[k];
-      inv_rho = 1 / rho;
+      inv_rho = m_div(1.0, rho);
     } else {
       rho_f = scr_f(in, S_RHO, col)[k];
       inv_rho_f = 1.0f / rho_f;
@@ -1576,15 +1577,15 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
     if constexpr (sizeof(TR) == sizeof(double)) {
       /* part3: cloud */
       if (dge(s.qc, C::QSMALL)) {
-        const double qc_incld = s.qc / cld_l;
-        double nc_incld = s.nc / cld_l;
+        const double qc_incld = m_div(s.qc, cld_l);
+        double nc_incld = m_div(s.nc, cld_l);
         TR mu_c, lamc;
         const TR n_in = TR(nc_incld);
         TR n_out = n_in;
         get_cloud_dsd2<TR>(TR(qc_incld), n_out, mu_c, TR(rho), lamc);
         apply_n_adjust(nc_incld, n_in, n_out);
         s.nc = nc_incld * cld_l;
-        eff_qc = double(TR(0.5) * (mu_c + TR(3)) / lamc);
+        eff_qc = double(m_div(TR(0.5) * (mu_c + TR(3)), lamc));
       } else {
         if (dnz(s.qc)) {
           s.qv = s.qv + s.qc;
@@ -1596,15 +1597,15 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
       }
       /* part3: rain */
       if (dge(s.qr, C::QSMALL)) {
-        const double qr_incld = s.qr / cld_r;
-        double nr_incld = s.nr / cld_r;
+        const double qr_incld = m_div(s.qr, cld_r);
+        double nr_incld = m_div(s.nr, cld_r);
         TR mu_r = 0, lamr;
         const TR n_in = TR(nr_incld);
         TR n_out = n_in;
         get_rain_dsd2<TR>(TR(qr_incld), n_out, mu_r, lamr, rt);
         apply_n_adjust(nr_incld, n_in, n_out);
         s.nr = nr_incld * cld_r;
-        eff_qr = double(TR(1.5) / lamr);
+        eff_qr = double(m_div(TR(1.5), lamr));
       } else {
         if (dnz(s.qr)) {
           s.qv = s.qv + s.qr;
@@ -1618,10 +1619,10 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
       {
         const bool qi_gt_small = dge(s.qi, C::QSMALL);
         s.ni = dmax_c(s.ni, C::NSMALL);
-        const double qi_incld = s.qi / cld_i;
-        double ni_incld = s.ni / cld_i;
-        double qm_incld = s.qm / cld_i;
-        double bm_incld = s.bm / cld_i;
+        const double qi_incld = m_div(s.qi, cld_i);
+        double ni_incld = m_div(s.ni, cld_i);
+        double qm_incld = m_div(s.qm, cld_i);
+        double bm_incld = m_div(s.bm, cld_i);
         double rhop = 0;
         if (qi_gt_small) {
           rhop = calc_bulk_rho_rime(qi_incld, qm_incld, bm_incld, rt);
@@ -1746,7 +1747,7 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
        * p3_main_impl.hpp:316-323 with T = th exner): T must lie in
        * (173, 323) K and qv in (0, 0.04); the reference traps only on T, and
        * only when its debug abort is on.  Recorded, never trapped. */
-      const double T = s.th * (1 / inv_exner);
+      const double T = s.th * m_div(1.0, inv_exner);
       const unsigned long long key = check_key(inst_idx, col, k);
       if (!(dgt(T, 173.0) && dlt(T, 323.0))) {
         atomicAdd(&kp.check[kChkTCount], 1ull);

@@ -14,6 +14,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "p3x_intfp64.cuh"
+
 namespace p3x {
 namespace dev {
 
@@ -126,6 +128,14 @@ __device__ __forceinline__ float m_expm1(float x) { return expm1f(x); }
 static __device__ __noinline__ double m_tanh_nl(double x) { return tanh(x); }
 __device__ __forceinline__ double m_tanh(double x) { return m_tanh_nl(x); }
 __device__ __forceinline__ float m_tanh(float x) { return tanhf(x); }
+/* Division: the FP64 form through the integer pipes (p3x_intfp64.cuh), the
+ * same double as the FP64 division at a fifth of its pipe time.  One copy per
+ * kernel: part1+2 holds about a hundred divisions and waits on instruction
+ * fetch.  At 21,600 x 128: part1+2 10.0 -> 6.9 ms, sedimentation 27.3 -> 15.8
+ * ms, part3 1.64 -> 0.87 ms. */
+static __device__ __noinline__ double m_div_nl(double a, double b) { return ddiv_int(a, b); }
+__device__ __forceinline__ double m_div(double a, double b) { return m_div_nl(a, b); }
+__device__ __forceinline__ float m_div(float a, float b) { return a / b; }
 __device__ __forceinline__ double m_fabs(double x) { return fabs(x); }
 __device__ __forceinline__ float m_fabs(float x) { return fabsf(x); }
 
@@ -333,12 +343,12 @@ template <class TR>
 __device__ __forceinline__ TR murphy_koop_svp(TR t, bool ice, uint32_t& err) {
   if (!(t > TR(0))) err |= kErrNumeric;
   if (t < TR(C::Tmelt) && ice) {
-    return m_exp(TR(9.550426) - (TR(5723.265) / t) + (TR(3.53068) * m_log(t)) - (TR(0.00728332) * t));
+    return m_exp(TR(9.550426) - m_div(TR(5723.265), t) + (TR(3.53068) * m_log(t)) - (TR(0.00728332) * t));
   }
   const TR logt = m_log(t);
-  return m_exp(TR(54.842763) - (TR(6763.22) / t) - (TR(4.210) * logt) + (TR(0.000367) * t) +
+  return m_exp(TR(54.842763) - m_div(TR(6763.22), t) - (TR(4.210) * logt) + (TR(0.000367) * t) +
                (m_tanh(TR(0.0415) * (t - TR(218.8))) *
-                (TR(53.878) - (TR(1331.22) / t) - (TR(9.44523) * logt) + TR(0.014025) * t)));
+                (TR(53.878) - m_div(TR(1331.22), t) - (TR(9.44523) * logt) + TR(0.014025) * t)));
 }
 
 /* Murphy-Koop vapour pressure from the FP64 saturation table of the
@@ -381,7 +391,7 @@ __device__ __forceinline__ double svp_tabulated(const double* tab, double t, boo
  * plain form evaluates it (the FP32-bulk form reads svp_tabulated). */
 __device__ __forceinline__ double qv_sat_dry(double t, double p, bool ice, uint32_t& err) {
   const double e_pres = murphy_koop_svp<double>(t, ice, err);
-  return C::ep_2 * e_pres / vmax(p, 1.e-3);
+  return m_div(C::ep_2 * e_pres, vmax(p, 1.e-3));
 }
 
 /* ------------------------------------------------------------------ */
@@ -449,13 +459,13 @@ struct Table3 {
 /* lookup_ice, p3/impl/p3_table_ice_impl.hpp:80-138 */
 template <class TR>
 __device__ __forceinline__ void lookup_ice(TR qi, TR ni, TR qm, TR rhop, TableIce<TR>& tab) {
-  tab.dum1 = (m_log10(qi / ni) + TR(18)) * TR(C::lookup_table_1a_dum1_c) - TR(10);
+  tab.dum1 = (m_log10(m_div(qi, ni)) + TR(18)) * TR(C::lookup_table_1a_dum1_c) - TR(10);
   tab.dumi = table_index(tab.dum1, kIsize);
   tab.dum1 = vmin(tab.dum1, TR(kIsize));
   tab.dum1 = vmax(tab.dum1, TR(1.));
   tab.dumi = max(1, tab.dumi);
   tab.dumi = min(kIsize - 1, tab.dumi);
-  tab.dum4 = (qm / qi) * TR(3) + TR(1);
+  tab.dum4 = m_div(qm, qi) * TR(3) + TR(1);
   tab.dumii = table_index(tab.dum4, kRimsize);
   tab.dum4 = vmin(tab.dum4, TR(kRimsize));
   tab.dum4 = vmax(tab.dum4, TR(1.));
@@ -481,7 +491,7 @@ template <class TR>
 __device__ __forceinline__ void lookup_rain(TR qr, TR nr, TableRain<TR>& tab) {
   const bool gt_small = qr > TR(C::QSMALL) && nr > TR(0.0);
   TR dumlr = TR(1);
-  if (gt_small) dumlr = m_cbrt(qr / (TR(C::Pi) * TR(C::RHO_H2O) * nr));
+  if (gt_small) dumlr = m_cbrt(m_div(qr, TR(C::Pi) * TR(C::RHO_H2O) * nr));
   tab.dum3 = (m_log10(TR(1) * dumlr) + TR(5)) * TR(10.70415);
   tab.dumj = table_index(tab.dum3, kRcollsize);
   tab.dum3 = vmin(tab.dum3, TR(kRcollsize));
@@ -588,7 +598,7 @@ __device__ __forceinline__ TR apply_table_coll(int idx, const Tabs<TR>& t, const
  * constant rain shape parameter and precomputed (rt.t3_dumjj/t3_rdumjj). */
 template <class TR>
 __device__ __forceinline__ void lookup3(TR mu_r, TR lamr, const RuntimeDev& rt, Table3<TR>& tab) {
-  const TR dum1 = (mu_r + TR(1)) / lamr;
+  const TR dum1 = m_div(mu_r + TR(1), lamr);
   if (dum1 <= TR(195.e-6)) {
     const TR inv_dum3 = TR(0.1);
     TR rdumii = (dum1 * TR(1.e6) + TR(5)) * inv_dum3;
@@ -664,19 +674,19 @@ __device__ __forceinline__ void get_cloud_dsd2(TR qc, TR& nc, TR& mu_c, TR rho, 
   if (qc >= TR(C::QSMALL)) {
     nc = vmax(nc, TR(C::NSMALL));
     TR mu = TR(0.0005714) * (nc * TR(1.e-6) * rho) + TR(0.2714);
-    mu = TR(1) / (mu * mu) - TR(1);
+    mu = m_div(TR(1), mu * mu) - TR(1);
     mu = vmax(mu, TR(2.));
     mu = vmin(mu, TR(15.));
     mu_c = mu;
-    lamc = m_cbrt(TR(C::CONS1) * nc * (mu_c + TR(3)) * (mu_c + TR(2)) * (mu_c + TR(1)) / qc);
+    lamc = m_cbrt(m_div(TR(C::CONS1) * nc * (mu_c + TR(3)) * (mu_c + TR(2)) * (mu_c + TR(1)), qc));
     const TR lammin = (mu_c + TR(1)) * TR(2.5e+4);
     const TR lammax = (mu_c + TR(1)) * TR(1.e+6);
     const bool lt = lamc < lammin, gt = lamc > lammax;
     if (lt) lamc = lammin;
     if (gt) lamc = lammax;
     if (lt || gt) {
-      nc = TR(6) * (lamc * lamc * lamc) * qc /
-           (TR(C::Pi) * TR(C::RHO_H2O) * (mu_c + TR(3)) * (mu_c + TR(2)) * (mu_c + TR(1)));
+      nc = m_div(TR(6) * (lamc * lamc * lamc) * qc,
+                 TR(C::Pi) * TR(C::RHO_H2O) * (mu_c + TR(3)) * (mu_c + TR(2)) * (mu_c + TR(1)));
     }
   }
 }
@@ -689,7 +699,7 @@ __device__ __forceinline__ void get_rain_dsd2(TR qr, TR& nr, TR& mu_r, TR& lamr,
     const TR nr_lim = vmax(nr, TR(C::NSMALL));
     mu_r = P3X_RTP(TR, constant_mu_rain);
     const TR f = TR(C::CONS1) * (mu_r + TR(3)) * (mu_r + TR(2)) * (mu_r + TR(1));
-    lamr = m_cbrt(f * nr_lim / qr);
+    lamr = m_cbrt(m_div(f * nr_lim, qr));
     const TR lammax = (mu_r + TR(1.)) * TR(1.e+5);
     const TR lammin = (mu_r + TR(1.)) * TR(500);
     const bool lt = lamr < lammin, gt = lamr > lammax;
@@ -697,7 +707,7 @@ __device__ __forceinline__ void get_rain_dsd2(TR qr, TR& nr, TR& mu_r, TR& lamr,
     if (lt || gt) {
       if (lt) lamr = lammin;
       if (gt) lamr = lammax;
-      nr = lamr * lamr * lamr * qr / f;
+      nr = m_div(lamr * lamr * lamr * qr, f);
     }
   }
 }
@@ -705,7 +715,7 @@ __device__ __forceinline__ void get_rain_dsd2(TR qr, TR& nr, TR& mu_r, TR& lamr,
 /* impose_max_total_ni, p3_impose_max_total_ni_impl.hpp:9-27 */
 template <class T>
 __device__ __forceinline__ void impose_max_total_ni(T& ni_local, T max_total_ni, T inv_rho_local) {
-  if (ni_local >= T(1e-20)) ni_local = ni_local * vmin(max_total_ni * inv_rho_local / ni_local, T(1.));
+  if (ni_local >= T(1e-20)) ni_local = ni_local * vmin(m_div(max_total_ni * inv_rho_local, ni_local), T(1.));
 }
 
 /* calc_bulk_rho_rime, p3/impl/p3_ice_sed_impl.hpp:14-64 */
@@ -714,14 +724,14 @@ __device__ __forceinline__ T calc_bulk_rho_rime(T qi_tot, T& qi_rim, T& bi_rim, 
   T rho_rime = 0;
   const bool gt = bi_rim >= T(C::BSMALL);
   const bool lt = bi_rim < T(C::BSMALL);
-  if (gt) rho_rime = qi_rim / bi_rim;
+  if (gt) rho_rime = m_div(qi_rim, bi_rim);
   const bool rr_lt_min = rho_rime < P3X_RTP(T, min_rime_rho);
   const bool rr_gt_max = rho_rime > P3X_RTP(T, max_rime_rho);
   if (gt && rr_lt_min) rho_rime = P3X_RTP(T, min_rime_rho);
   if (gt && rr_gt_max) rho_rime = P3X_RTP(T, max_rime_rho);
-  if (gt && (rr_gt_max || rr_lt_min)) bi_rim = qi_rim / rho_rime;
+  if (gt && (rr_gt_max || rr_lt_min)) bi_rim = m_div(qi_rim, rho_rime);
   if (lt) { qi_rim = 0; bi_rim = 0; rho_rime = 0; }
-  if (qi_rim > qi_tot && rho_rime > T(0)) { qi_rim = qi_tot; bi_rim = qi_rim / rho_rime; }
+  if (qi_rim > qi_tot && rho_rime > T(0)) { qi_rim = qi_tot; bi_rim = m_div(qi_rim, rho_rime); }
   if (qi_rim < T(C::QSMALL)) { qi_rim = 0; bi_rim = 0; }
   return rho_rime;
 }
@@ -757,10 +767,10 @@ struct PhysVars {
 template <class TR>
 __device__ __forceinline__ void get_time_space_phys_variables(TR T_atm, TR pres, TR rho, TR qv_sat_l,
                                                               TR qv_sat_i, PhysVars<TR>& v) {
-  v.mu = TR(1.496e-6) * m_pow(T_atm, TR(1.5)) / (T_atm + TR(120));
-  v.dv = TR(8.794e-5) * m_pow(T_atm, TR(1.81)) / pres;
-  v.sc = v.mu / (rho * v.dv);
-  const TR dum = TR(1) / (TR(C::RV) * sq(T_atm));
+  v.mu = m_div(TR(1.496e-6) * m_pow(T_atm, TR(1.5)), T_atm + TR(120));
+  v.dv = m_div(TR(8.794e-5) * m_pow(T_atm, TR(1.81)), pres);
+  v.sc = m_div(v.mu, rho * v.dv);
+  const TR dum = m_div(TR(1), TR(C::RV) * sq(T_atm));
   v.dqsdt = TR(C::LatVap) * qv_sat_l * dum;
   v.dqsidt = TR(C::LatVap + C::LatIce) * qv_sat_i * dum;
   v.ab = TR(1) + v.dqsdt * TR(C::LatVap) * TR(C::INV_CP);
@@ -769,7 +779,7 @@ __device__ __forceinline__ void get_time_space_phys_variables(TR T_atm, TR pres,
   if (T_atm < TR(253.15)) {
     v.eii = TR(0.001);
   } else if (T_atm < TR(273.15)) {
-    v.eii = TR(0.001) + (T_atm - TR(253.15)) * (TR(0.3) - TR(0.001)) / TR(20);
+    v.eii = TR(0.001) + m_div((T_atm - TR(253.15)) * (TR(0.3) - TR(0.001)), TR(20));
   } else {
     v.eii = TR(0.3);
   }
@@ -814,10 +824,10 @@ __device__ __forceinline__ void ice_self_collection(TR rho, TR rhofaci, TR tv, T
   const bool qm_pos = qm_incld > TR(0);
   if (qi_incld >= TR(C::QSMALL)) {
     TR tmp1 = 0;
-    if (qm_pos) tmp1 = qm_incld / qi_incld;
+    if (qm_pos) tmp1 = m_div(qm_incld, qi_incld);
     TR Eii_fact = 0;
     if (tmp1 < TR(0.6) && qm_pos) Eii_fact = TR(1);
-    if (tmp1 >= TR(0.6) && tmp1 < TR(0.9) && qm_pos) Eii_fact = TR(1) - (tmp1 - TR(0.6)) / TR(0.3);
+    if (tmp1 >= TR(0.6) && tmp1 < TR(0.9) && qm_pos) Eii_fact = TR(1) - m_div(tmp1 - TR(0.6), TR(0.3));
     if (tmp1 >= TR(0.9) && qm_pos) Eii_fact = TR(0);
     if (!qm_pos) Eii_fact = TR(1);
     r.ni_selfcollect_tend = tv * rho * eii * Eii_fact * rhofaci * ni_incld * ni_incld;
@@ -832,13 +842,13 @@ __device__ __forceinline__ void ice_melting(TR rho, double dT0, double dqv0, TR 
                                             TR tv_vent, const PhysVars<TR>& v, TR qi_incld,
                                             TR ni_incld, Rates<TR>& r) {
   if (qi_incld >= TR(C::QSMALL) && dpos(dT0)) {
-    TR t = ((tv_melt + tv_vent * m_cbrt(v.sc) * m_sqrt(rhofaci * rho / v.mu)) *
-            (TR(dT0) * v.kap - rho * TR(C::LatVap) * v.dv * TR(dqv0)) * TR(2) *
-            TR(C::Pi) / TR(C::LatIce)) *
+    TR t = m_div((tv_melt + tv_vent * m_cbrt(v.sc) * m_sqrt(m_div(rhofaci * rho, v.mu))) *
+                     (TR(dT0) * v.kap - rho * TR(C::LatVap) * v.dv * TR(dqv0)) * TR(2) * TR(C::Pi),
+                 TR(C::LatIce)) *
            ni_incld;
     t = vmax(t, TR(0.));
     r.qi2qr_melt_tend = t;
-    r.ni2nr_melt_tend = t * (ni_incld / qi_incld);
+    r.ni2nr_melt_tend = t * m_div(ni_incld, qi_incld);
   }
 }
 
@@ -853,9 +863,9 @@ __device__ __forceinline__ bool ice_cldliq_wet_growth(TR rho, double dT0, double
   const bool any_if_col = any_if && (r.qc2qi_collect_tend + r.qr2qi_collect_tend) >= TR(1.0e-10);
   bool wet = false;
   if (any_if) {
-    TR g = ((tv_melt + tv_vent * m_cbrt(v.sc) * m_sqrt(rhofaci * rho / v.mu)) * TR(C::Pi * 2) *
-            (rho * TR(C::LatVap) * v.dv * TR(dqv0) - TR(dT0) * v.kap) /
-            (TR(C::LatIce) + TR(C::CpLiq) * TR(dT0))) *
+    TR g = m_div((tv_melt + tv_vent * m_cbrt(v.sc) * m_sqrt(m_div(rhofaci * rho, v.mu))) * TR(C::Pi * 2) *
+                     (rho * TR(C::LatVap) * v.dv * TR(dqv0) - TR(dT0) * v.kap),
+                 TR(C::LatIce) + TR(C::CpLiq) * TR(dT0)) *
            ni_incld;
     g = vmax(g, TR(0.));
     /* The shed excess dum = collection - g and the collection that remains,
@@ -888,10 +898,10 @@ __device__ __forceinline__ TR calc_rime_density(TR T_atm, TR rhofaci, TR tv_fall
     const TR vtrmi1 = tv_fallspd * rhofaci;
     if (qc_incld >= TR(C::QSMALL)) {
       /* Gamma(4+bcn+mu_c)/Gamma(4+mu_c) = (5+mu_c)(4+mu_c) for bcn = 2 */
-      const TR Vt_qc = acn * ((TR(5) + mu_c) * (TR(4) + mu_c)) / (lamc * lamc);
-      const TR D_c = (TR(4) + mu_c) / lamc;
+      const TR Vt_qc = m_div(acn * ((TR(5) + mu_c) * (TR(4) + mu_c)), lamc * lamc);
+      const TR D_c = m_div(TR(4) + mu_c, lamc);
       const TR V_impact = m_fabs(vtrmi1 - Vt_qc);
-      const TR inv_Tc = TR(1) / vmin(TR(-0.001), T_atm - TR(C::T_zerodegc));
+      const TR inv_Tc = m_div(TR(1), vmin(TR(-0.001), T_atm - TR(C::T_zerodegc)));
       const TR Ri = vmax(TR(1.), vmin(TR(-0.5e+6) * D_c * V_impact * inv_Tc, TR(12.)));
       if (Ri <= TR(8.0)) {
         rho_qm_cloud = (TR(0.051) + TR(0.114) * Ri - TR(0.0055) * sq(Ri)) * TR(1000);
@@ -912,7 +922,7 @@ __device__ __forceinline__ void cldliq_immersion_freezing(TR T_atm, TR lamc, TR 
                                                           Rates<TR>& r, const RuntimeDev& rt) {
   if (qc_incld >= TR(C::QSMALL) && T_atm <= TR(C::T_rainfrz)) {
     const TR expAimmDt = m_exp(P3X_RTP(TR, immersion_freezing_exponent) * (TR(C::T_zerodegc) - T_atm));
-    const TR inv_lamc = TR(1) / lamc;
+    const TR inv_lamc = m_div(TR(1), lamc);
     const TR inv_lamc3 = inv_lamc * inv_lamc * inv_lamc;
     const TR p3 = (TR(1) + mu_c) * (TR(2) + mu_c) * (TR(3) + mu_c);
     const TR p6 = p3 * ((TR(4) + mu_c) * (TR(5) + mu_c) * (TR(6) + mu_c));
@@ -973,7 +983,7 @@ __device__ __forceinline__ void cloud_water_autoconversion(TR rho, TR qc_incld, 
     r.qc2qr_autoconv_tend = P3X_RTP(TR, autoconversion_prefactor) * m_pow(qc_incld, P3X_RTP(TR, autoconversion_qc_exponent)) *
                             m_pow(nc_incld * TR(1.e-6) * rho, (-P3X_RTP(TR, autoconversion_nc_exponent)));
     r.ncautr = r.qc2qr_autoconv_tend * P3X_RTP(TR, cons3);
-    r.nc2nr_autoconv_tend = r.qc2qr_autoconv_tend * nc_incld / qc_incld;
+    r.nc2nr_autoconv_tend = m_div(r.qc2qr_autoconv_tend * nc_incld, qc_incld);
   }
   if (r.qc2qr_autoconv_tend == TR(0)) r.nc2nr_autoconv_tend = 0;
   if (r.nc2nr_autoconv_tend == TR(0)) r.qc2qr_autoconv_tend = 0;
@@ -990,7 +1000,7 @@ __device__ __forceinline__ void cloud_rain_accretion(TR qc_incld, TR nc_incld, T
       r.qc2qr_accret_tend = P3X_RTP(TR, accretion_prefactor) * m_pow(qc_incld, P3X_RTP(TR, accretion_qc_exponent)) *
                             m_pow(qr_incld, P3X_RTP(TR, accretion_qr_exponent));
     }
-    r.nc_accret_tend = r.qc2qr_accret_tend * nc_incld / qc_incld;
+    r.nc_accret_tend = m_div(r.qc2qr_accret_tend * nc_incld, qc_incld);
     if (r.nc_accret_tend == TR(0)) r.qc2qr_accret_tend = 0;
     if (r.qc2qr_accret_tend == TR(0)) r.nc_accret_tend = 0;
   }
@@ -1001,7 +1011,7 @@ template <class TR>
 __device__ __forceinline__ void rain_self_collection(TR rho, TR qr_incld, TR nr_incld, Rates<TR>& r,
                                                      const RuntimeDev& rt) {
   if (qr_incld >= TR(C::QSMALL)) {
-    const TR dum2 = m_cbrt((qr_incld) / (TR(C::Pi) * TR(C::RHO_H2O) * nr_incld));
+    const TR dum2 = m_cbrt(m_div(qr_incld, TR(C::Pi) * TR(C::RHO_H2O) * nr_incld));
     const TR dbr = P3X_RTP(TR, rain_selfcollection_breakup_diameter);
     const TR dum = (dum2 < dbr) ? TR(1) : TR(2) - m_exp(TR(2300) * (dum2 - dbr));
     r.nr_selfcollect_tend = dum * P3X_RTP(TR, rain_selfcollection_prefactor) * nr_incld * qr_incld * rho;
@@ -1057,37 +1067,38 @@ __device__ __forceinline__ void evaporate_rain(double qr_incld, double qc_incld,
                                                double& qr2qv_evap_tend, double& nr_evap_tend) {
   qr2qv_evap_tend = 0;
   nr_evap_tend = 0;
-  const double inv_dt = 1 / dt;
+  const double inv_dt = m_div(1.0, dt);
   const double inv_cp = 1 / C::Cpair;
   const double ssat_r = qv - qv_sat_l;
   const double cld_frac = ((qc_incld + qi_incld) < 1.e-6) ? 0.0 : cld_frac_l;
   if (qr_incld >= C::QSMALL && ssat_r < 0 && cld_frac_r > cld_frac) {
-    const double tau_r = 1 / epsr;
+    const double tau_r = m_div(1.0, epsr);
     double eps_eff, A_c;
     if (t_atm < C::Tmelt) {
-      eps_eff = epsr + epsi_tot * (1 + (C::LatVap + C::LatIce) * inv_cp * dqsdt) / abi;
+      eps_eff = epsr + m_div(epsi_tot * (1 + (C::LatVap + C::LatIce) * inv_cp * dqsdt), abi);
       A_c = (qv - qv_prev) * inv_dt - dqsdt * (t_atm - t_atm_prev) * inv_dt -
-            (qv_sat_l - qv_sat_i) * (1 + (C::LatVap + C::LatIce) * inv_cp * dqsdt) / abi * epsi_tot;
+            m_div((qv_sat_l - qv_sat_i) * (1 + (C::LatVap + C::LatIce) * inv_cp * dqsdt), abi) * epsi_tot;
     } else {
       eps_eff = epsr;
       A_c = (qv - qv_prev) * inv_dt - dqsdt * (t_atm - t_atm_prev) * inv_dt;
     }
     if (eps_eff < 1e-20) eps_eff = 1e-20;
-    const double tau_eff = 1 / eps_eff;
-    if (qr_incld < 1e-12 && qv / qv_sat_l < 0.999) {
+    const double tau_eff = m_div(1.0, eps_eff);
+    if (qr_incld < 1e-12 && m_div(qv, qv_sat_l) < 0.999) {
       qr2qv_evap_tend = qr_incld * inv_dt;
     } else {
-      const double dt_over_tau = dt / tau_eff;
-      const double w = -expm1(-dt_over_tau) / dt_over_tau;
-      const double equilib = -A_c / ab * tau_eff / tau_r;
-      const double instant = -ssat_r / (ab * tau_r);
+      const double dt_over_tau = m_div(dt, tau_eff);
+      const double w = m_div(-expm1(-dt_over_tau), dt_over_tau);
+      const double equilib = m_div(m_div(-A_c, ab) * tau_eff, tau_r);
+      const double instant = m_div(-ssat_r, ab * tau_r);
       qr2qv_evap_tend = instant * w + equilib * (1 - w);
     }
-    if (qr2qv_evap_tend > -ssat_r * inv_dt / ab) qr2qv_evap_tend = -ssat_r * inv_dt / ab;
+    const double ssat_lim = m_div(-ssat_r * inv_dt, ab);
+    if (qr2qv_evap_tend > ssat_lim) qr2qv_evap_tend = ssat_lim;
     if (qr2qv_evap_tend < 0) qr2qv_evap_tend = 0;
     if (qr2qv_evap_tend > qr_incld * inv_dt) qr2qv_evap_tend = qr_incld * inv_dt;
-    qr2qv_evap_tend = qr2qv_evap_tend * (cld_frac_r - cld_frac) / cld_frac_r;
-    nr_evap_tend = qr2qv_evap_tend * (nr_incld / qr_incld);
+    qr2qv_evap_tend = m_div(qr2qv_evap_tend * (cld_frac_r - cld_frac), cld_frac_r);
+    nr_evap_tend = qr2qv_evap_tend * m_div(nr_incld, qr_incld);
   }
 }
 
@@ -1176,15 +1187,15 @@ __device__ __forceinline__ void ice_deposition_sublimation(double qi_incld, doub
                                                            double& berg) {
   berg = 0; vapdep = 0; sublim = 0; ni_sublim = 0;
   if (dgt(qi_incld, C::QSMALL)) {
-    const double qi_tend = vmin(epsi / abi, inv_dt) * (qv - qv_sat_i);
+    const double qi_tend = vmin(m_div(epsi, abi), inv_dt) * (qv - qv_sat_i);
     const bool neg = dneg(qi_tend);
     if (neg) {
       sublim = -qi_tend;
-      ni_sublim = sublim * (ni_incld / qi_incld);
+      ni_sublim = sublim * m_div(ni_incld, qi_incld);
     }
     const bool T_lt_frz = dlt(T_atm, C::T_zerodegc);
     if (T_lt_frz && !neg) vapdep = qi_tend;
-    if (T_lt_frz) berg = dmax0(epsi / abi * (qv_sat_l - qv_sat_i));
+    if (T_lt_frz) berg = dmax0(m_div(epsi, abi) * (qv_sat_l - qv_sat_i));
   }
 }
 
@@ -1201,7 +1212,7 @@ __device__ __forceinline__ int water_conservation(T qc, T qr, T qi, T dt, Rates<
     T ratio;
     if (sinks > sources && sinks >= T(C::QTENDSMALL)) {
       limited |= 1;
-      ratio = sources / sinks;
+      ratio = m_div(sources, sinks);
       r.qc2qr_autoconv_tend *= ratio;
       r.qc2qr_accret_tend *= ratio;
       r.qc2qi_collect_tend *= ratio;
@@ -1222,7 +1233,7 @@ __device__ __forceinline__ int water_conservation(T qc, T qr, T qi, T dt, Rates<
                                  r.qc2qr_ice_shed_tend) * dt;
     if (sinks > sources && sinks >= T(C::QTENDSMALL)) {
       limited |= 2;
-      const T ratio = sources / sinks;
+      const T ratio = m_div(sources, sinks);
       r.qr2qv_evap_tend *= ratio;
       r.qr2qi_collect_tend *= ratio;
       r.qr2qi_immers_freeze_tend *= ratio;
@@ -1235,7 +1246,7 @@ __device__ __forceinline__ int water_conservation(T qc, T qr, T qi, T dt, Rates<
                                  r.qc2qi_hetero_freeze_tend + r.qc2qi_berg_tend) * dt;
     if (sinks > sources && sinks >= T(C::QTENDSMALL)) {
       limited |= 4;
-      const T ratio = sources / sinks;
+      const T ratio = m_div(sources, sinks);
       r.qi2qv_sublim_tend *= ratio;
       r.qi2qr_melt_tend *= ratio;
     }
@@ -1252,7 +1263,7 @@ __device__ __forceinline__ int number_conservation(T nc, T nr, T ni, T dt, Rates
     const T source = nc + r.nc_selfcollect_tend * dt;
     if (sink > source) {
       limited |= 1;
-      const T ratio = source / sink;
+      const T ratio = m_div(source, sink);
       r.nc_collect_tend *= ratio;
       r.nc2ni_immers_freeze_tend *= ratio;
       r.nc_accret_tend *= ratio;
@@ -1264,7 +1275,7 @@ __device__ __forceinline__ int number_conservation(T nc, T nr, T ni, T dt, Rates
     const T source = nr + (r.ni2nr_melt_tend * T(C::nmltratio) + r.nr_ice_shed_tend + r.ncshdc + r.nc2nr_autoconv_tend) * dt;
     if (sink > source) {
       limited |= 2;
-      const T ratio = source / sink;
+      const T ratio = m_div(source, sink);
       r.nr_collect_tend *= ratio;
       r.nr2ni_immers_freeze_tend *= ratio;
       r.nr_selfcollect_tend *= ratio;
@@ -1276,7 +1287,7 @@ __device__ __forceinline__ int number_conservation(T nc, T nr, T ni, T dt, Rates
     const T source = ni + (r.ni_nucleat_tend + r.nr2ni_immers_freeze_tend + r.nc2ni_immers_freeze_tend) * dt;
     if (sink > source) {
       limited |= 4;
-      const T ratio = source / sink;
+      const T ratio = m_div(source, sink);
       r.ni2nr_melt_tend *= ratio;
       r.ni_sublim_tend *= ratio;
       r.ni_selfcollect_tend *= ratio;
@@ -1291,11 +1302,12 @@ __device__ __forceinline__ void ice_supersat_conservation(Rates<double>& r, doub
   const double latsublim2 = (C::LatVap + C::LatIce) * (C::LatVap + C::LatIce);
   const double qv_sink = r.qv2qi_vapdep_tend + r.qv2qi_nucleat_tend;
   if (dgt(qv_sink, C::QSMALL) && dgt(cld_frac_i, 1e-20)) {
-    double qv_avail = (qv + (r.qi2qv_sublim_tend + r.qr2qv_evap_tend) * dt - qv_sat_i) /
-                      (1 + latsublim2 * qv_sat_i / (C::CP * C::RH2O * sq(t_atm))) / dt;
+    double qv_avail = m_div(m_div(qv + (r.qi2qv_sublim_tend + r.qr2qv_evap_tend) * dt - qv_sat_i,
+                                  1 + m_div(latsublim2 * qv_sat_i, C::CP * C::RH2O * sq(t_atm))),
+                            dt);
     qv_avail = dmax0(qv_avail);
     if (qv_sink > qv_avail) {
-      const double fract = qv_avail / qv_sink;
+      const double fract = m_div(qv_avail, qv_sink);
       r.qv2qi_nucleat_tend *= fract;
       r.qv2qi_vapdep_tend *= fract;
     }
@@ -1311,9 +1323,9 @@ __device__ __forceinline__ void prevent_liq_supersaturation(double pres, double 
   const double T_endstep = t_atm + ((qv_sinks - r.qi2qv_sublim_tend) * (C::LatVap + C::LatIce) * C::INV_CP -
                                     r.qr2qv_evap_tend * C::LatVap * C::INV_CP) * dt;
   const double qsl = qv_sat_dry(T_endstep, pres, false, err);
-  const double A = C::LatVap * qsl * dt * C::INV_CP / (C::RV * T_endstep * T_endstep) *
+  const double A = m_div(C::LatVap * qsl * dt * C::INV_CP, C::RV * T_endstep * T_endstep) *
                    ((C::LatVap + C::LatIce) * r.qi2qv_sublim_tend + C::LatVap * r.qr2qv_evap_tend);
-  double frac = (qsl - qv + qv_sinks * dt + A) / (qv_sources * dt + A);
+  double frac = m_div(qsl - qv + qv_sinks * dt + A, qv_sources * dt + A);
   frac = dmax_0x(frac);
   frac = dlt(frac, 1.) ? frac : 1.;
   r.qi2qv_sublim_tend = frac * r.qi2qv_sublim_tend;
@@ -1375,15 +1387,15 @@ __device__ __forceinline__ void update_prognostics(const Rates<double>& r, doubl
   s.nr = s.nr + (-r.nr_collect_tend - r.nr2ni_immers_freeze_tend + C::nmltratio * r.ni2nr_melt_tend +
                  r.nr_ice_shed_tend + r.ncshdc) * dt;
   if (dge(s.qi, C::QSMALL)) {
-    s.bm = s.bm - ((r.qi2qv_sublim_tend + r.qi2qr_melt_tend) / s.qi) * dt * s.bm;
-    s.qm = s.qm - ((r.qi2qv_sublim_tend + r.qi2qr_melt_tend) * s.qm / s.qi) * dt;
+    s.bm = s.bm - m_div(r.qi2qv_sublim_tend + r.qi2qr_melt_tend, s.qi) * dt * s.bm;
+    s.qm = s.qm - m_div((r.qi2qv_sublim_tend + r.qi2qr_melt_tend) * s.qm, s.qi) * dt;
     s.qi = s.qi - (r.qi2qv_sublim_tend + r.qi2qr_melt_tend) * dt;
   }
   const double dum = (r.qr2qi_collect_tend + r.qc2qi_collect_tend + r.qr2qi_immers_freeze_tend +
                       r.qc2qi_hetero_freeze_tend) * dt;
   s.qi = s.qi + (r.qv2qi_vapdep_tend + r.qv2qi_nucleat_tend + r.qc2qi_berg_tend) * dt + dum;
   s.qm = s.qm + dum;
-  s.bm = s.bm + (r.qr2qi_collect_tend * C::INV_RHO_RIMEMAX + r.qc2qi_collect_tend / rho_qm_cloud +
+  s.bm = s.bm + (r.qr2qi_collect_tend * C::INV_RHO_RIMEMAX + m_div(r.qc2qi_collect_tend, rho_qm_cloud) +
                  (r.qr2qi_immers_freeze_tend + r.qc2qi_hetero_freeze_tend) * C::INV_RHO_RIMEMAX) * dt;
   s.ni = s.ni + (r.ni_nucleat_tend - r.ni2nr_melt_tend - r.ni_sublim_tend - r.ni_selfcollect_tend +
                  r.nr2ni_immers_freeze_tend + r.nc2ni_immers_freeze_tend) * dt;
