@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "p3x.h"
+#include "p3x_fixtables.hpp"
 #include "p3x_internal.hpp"
 #include "p3x_launch.hpp"
 
@@ -33,6 +34,12 @@ struct p3x_context {
   double* d_t3slices = nullptr;
   float* f_t3slices = nullptr;
   double* d_svp = nullptr; /* FP32-bulk saturation table */
+  /* FP64 form: fixed-point tables (p3x_intfp64.cuh), ice-table cells and
+   * their powers of two of sedimentation and part3, Table3 fall speeds */
+  p3x::dev::FixTables* d_fix = nullptr;
+  int64_t *d_cell_sed = nullptr, *d_cell_part3 = nullptr;
+  int32_t *d_shift_sed = nullptr, *d_shift_part3 = nullptr;
+  double* d_t3sed = nullptr;
   uint32_t* d_err = nullptr;
   /* check_values words (dev::kCheckWords) and mode (P3X_CHECK_*) */
   unsigned long long* d_check = nullptr;
@@ -103,8 +110,8 @@ const HostTables& generated_tables() {
   return *g_generated;
 }
 
-template <class T>
-int upload(T** dst, const std::vector<double>& src) {
+template <class T, class U>
+int upload(T** dst, const std::vector<U>& src) {
   std::vector<T> tmp(src.begin(), src.end());
   P3X_CUDA(cudaMalloc(reinterpret_cast<void**>(dst), sizeof(T) * tmp.size()));
   P3X_CUDA(cudaMemcpy(*dst, tmp.data(), sizeof(T) * tmp.size(), cudaMemcpyHostToDevice));
@@ -153,6 +160,17 @@ dev::RuntimeDev make_runtime(const p3x_runtime& r) {
   d.g_mur2 = std::tgamma(mu_r + 2.0);
   d.lg_mur4 = std::log(std::tgamma(mu_r + 4.0));
   d.lg_mur7 = std::log(std::tgamma(mu_r + 7.0));
+  {
+    const double f = dev::C::CONS1 * (mu_r + 3) * (mu_r + 2) * (mu_r + 1);
+    const double lam_hi = (mu_r + 1.) * 1.e+5, lam_lo = (mu_r + 1.) * 500;
+    d.rain_fix = mu_r > -0.99 && mu_r < 1.0e4 ? 1 : 0;
+    d.rain_kd = d.rain_fix ? std::llroundl((std::log2(static_cast<long double>(mu_r) + 1) -
+                                            std::log2(static_cast<long double>(f)) / 3) * 0x1p57L)
+                           : 0;
+    d.rain_n_hi = lam_hi * lam_hi * lam_hi / f;
+    d.rain_n_lo = lam_lo * lam_lo * lam_lo / f;
+    d.t3_wj = d.t3_rdumjj - d.t3_dumjj;
+  }
   d.accretion_same_exponent = r.accretion_qc_exponent == r.accretion_qr_exponent ? 1 : 0;
   /* float copies for the FP32-bulk rates (round to nearest, as a device
    * conversion gives) */
@@ -234,6 +252,12 @@ dev::KParams<double> make_kparams<double>(p3x_context* ctx, const dev::RuntimeDe
   kp.revap = ctx->d_revap;
   kp.t3slice = ctx->d_t3slices + size_t(rtd.t3_dumjj - 1) * dev::kT3SliceElems;
   kp.rt.svp_tab = ctx->d_svp;
+  kp.fix = ctx->d_fix;
+  kp.cell_sed = ctx->d_cell_sed;
+  kp.cell_part3 = ctx->d_cell_part3;
+  kp.cell_sed_shift = ctx->d_shift_sed;
+  kp.cell_part3_shift = ctx->d_shift_part3;
+  kp.t3sed = reinterpret_cast<const double4*>(ctx->d_t3sed);
   kp.err = ctx->d_err;
   kp.check = ctx->check_mode ? ctx->d_check : nullptr;
   kp.check_fail = ctx->check_mode == P3X_CHECK_FAIL ? 1 : 0;
@@ -591,9 +615,29 @@ int p3x_context_create(const char* table_file, p3x_context** out, int* info) {
       for (int i = 0; i < kVT0; ++i)
         for (int c = 0; c < 2; ++c) s[t * 600 + i * 2 + c] = (*tabs[t])[size_t(i) * kVT1 + (j - 1 + c)];
   }
+  std::vector<double> t3sed(size_t(kVT1) * dev::kT3SedRows * 4);
+  for (int j = 0; j < kVT1; ++j)
+    for (int i = 0; i < kVT0; ++i) {
+      const size_t a = size_t(i) * kVT1 + j, b = size_t(i + 1 < kVT0 ? i + 1 : i) * kVT1 + j;
+      double* row = &t3sed[(size_t(j) * dev::kT3SedRows + i) * 4];
+      row[0] = H.vm[a];
+      row[1] = H.vm[b] - H.vm[a];
+      row[2] = H.vn[a];
+      row[3] = H.vn[b] - H.vn[a];
+    }
+  static const int kSedCols[dev::kCellCols] = {0, 1, 6, 7}, kPart3Cols[dev::kCellCols] = {6, 7, 5, 11};
+  std::vector<int64_t> cell_sed, cell_part3;
+  std::vector<int32_t> shift_sed, shift_part3;
+  build_ice_cells(H.ice.data(), kSedCols, cell_sed, shift_sed);
+  build_ice_cells(H.ice.data(), kPart3Cols, cell_part3, shift_part3);
+  std::vector<dev::FixTables> fix(1);
+  build_fix_tables(fix[0]);
   std::vector<double> svp;
   build_svp_table(svp);
-  if ((st = upload(&ctx->d_t3slices, sl)) || (st = upload(&ctx->f_t3slices, sl)) || (st = upload(&ctx->d_svp, svp))) {
+  if ((st = upload(&ctx->d_t3slices, sl)) || (st = upload(&ctx->f_t3slices, sl)) || (st = upload(&ctx->d_svp, svp)) ||
+      (st = upload(&ctx->d_t3sed, t3sed)) || (st = upload(&ctx->d_cell_sed, cell_sed)) ||
+      (st = upload(&ctx->d_cell_part3, cell_part3)) || (st = upload(&ctx->d_shift_sed, shift_sed)) ||
+      (st = upload(&ctx->d_shift_part3, shift_part3)) || (st = upload(&ctx->d_fix, fix))) {
     if (info) *info = st;
     p3x_context_destroy(ctx.release());
     return st;
@@ -645,6 +689,7 @@ int p3x_context_destroy(p3x_context* ctx) {
   if (!ctx) return P3X_EINVAL;
   void* ptrs[] = {ctx->d_ice, ctx->d_coll, ctx->d_vn, ctx->d_vm, ctx->d_revap, ctx->f_ice, ctx->f_ice_sed, ctx->f_coll,
                   ctx->f_vn, ctx->f_vm, ctx->f_revap, ctx->d_t3slices, ctx->f_t3slices, ctx->d_svp, ctx->d_err,
+                  ctx->d_fix, ctx->d_cell_sed, ctx->d_cell_part3, ctx->d_shift_sed, ctx->d_shift_part3, ctx->d_t3sed,
                   ctx->d_check, ctx->d_maxloc, ctx->fstage};
   for (void* p : ptrs)
     if (p) cudaFree(p);

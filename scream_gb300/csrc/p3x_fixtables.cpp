@@ -1,0 +1,64 @@
+/*
+ * Host side of p3x_intfp64.cuh: the logarithm / exponential tables and the
+ * fixed-point ice-table cells, in extended precision.
+ */
+#include "p3x_fixtables.hpp"
+
+#include <cmath>
+
+namespace p3x {
+
+void build_fix_tables(dev::FixTables& t) {
+  for (int j = 0; j < 128; ++j) {
+    const long double c = 1.0L + (j + 0.5L) / 128.0L;
+    const uint32_t r = uint32_t(std::llroundl(4294967296.0L / c));
+    t.log2[j].r = r;
+    t.log2[j].pad = 0;
+    t.log2[j].nlog2 = std::llroundl(-std::log2(static_cast<long double>(r) / 4294967296.0L) * 0x1p62L);
+    t.exp2[j] = std::llroundl(std::exp2((j + 0.5L) / 128.0L) * 0x1p62L);
+  }
+}
+
+void build_ice_cells(const double* ice, const int cols[dev::kCellCols], std::vector<int64_t>& coef,
+                     std::vector<int32_t>& shift) {
+  coef.assign(size_t(dev::kIceCells) * dev::kCellCols * dev::kCellCoefs, 0);
+  shift.assign(size_t(dev::kIceCells) * dev::kCellCols, 0);
+  auto at = [&](int jj, int ii, int i, int c) {
+    return static_cast<long double>(ice[size_t((jj * kRimsize + ii) * kIsize + i) * kIceCols + cols[c]]);
+  };
+  /* the power of two each coefficient is stored with: one per weight */
+  static const int kWeights[dev::kCellCoefs] = {0, 1, 1, 2, 1, 2, 2, 3};
+  for (int jj = 0; jj < dev::kCellD; ++jj)
+    for (int ii = 0; ii < dev::kCellR; ++ii)
+      for (int i = 0; i < dev::kCellI; ++i)
+        for (int c = 0; c < dev::kCellCols; ++c) {
+          long double v[2][2][2];
+          for (int a = 0; a < 2; ++a)
+            for (int b = 0; b < 2; ++b)
+              for (int d = 0; d < 2; ++d) v[a][b][d] = at(jj + a, ii + b, i + d, c);
+          long double k[dev::kCellCoefs];
+          for (int a = 0; a < 2; ++a)
+            for (int b = 0; b < 2; ++b) {
+              k[4 * a + 2 * b] = v[a][b][0];
+              k[4 * a + 2 * b + 1] = v[a][b][1] - v[a][b][0];
+            }
+          for (int a = 0; a < 2; ++a)
+            for (int d = 0; d < 2; ++d) k[4 * a + 2 + d] -= k[4 * a + d];
+          for (int m = 0; m < 4; ++m) k[4 + m] -= k[m];
+          long double most = 0;
+          for (int m = 0; m < dev::kCellCoefs; ++m)
+            most = std::fmax(most, std::fabs(std::ldexp(k[m], kWeights[m])));
+          const size_t cell = size_t((jj * dev::kCellR + ii) * dev::kCellI + i) * dev::kCellCols + c;
+          /* the largest stored coefficient lies in [2^59, 2^60), so that no
+           * partial sum reaches 2^63; a cell of (near) zeros stays zero */
+          if (!(most > 0x1p-900L) || !std::isfinite(most)) continue;
+          int e = 0;
+          std::frexp(most, &e);
+          const int s = 60 - e;
+          shift[cell] = s;
+          for (int m = 0; m < dev::kCellCoefs; ++m)
+            coef[cell * dev::kCellCoefs + m] = std::llroundl(std::ldexp(k[m], kWeights[m] + s));
+        }
+}
+
+}  // namespace p3x

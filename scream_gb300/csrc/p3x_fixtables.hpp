@@ -1,0 +1,23 @@
+/* Tables of the fixed-point FP64 operations (p3x_intfp64.cuh). */
+#ifndef P3X_FIXTABLES_HPP
+#define P3X_FIXTABLES_HPP
+
+#include <cstdint>
+#include <vector>
+
+#include "p3x_intfp64.cuh"
+#include "p3x_internal.hpp"
+
+namespace p3x {
+
+void build_fix_tables(dev::FixTables& t);
+
+/* Fixed-point coefficients of four ice-table columns for every cell
+ * [kIceCells][kCellCols][kCellCoefs] and the power of two of each cell and
+ * column [kIceCells][kCellCols]: value = fix_trilinear(...) 2^-shift. */
+void build_ice_cells(const double* ice, const int cols[dev::kCellCols], std::vector<int64_t>& coef,
+                     std::vector<int32_t>& shift);
+
+}  // namespace p3x
+
+#endif

@@ -7,9 +7,15 @@
  * nearly idle.  A composite FP64 operation is therefore cheaper as integer
  * arithmetic on the significands.  Measured on one GB300 (SM cycles per warp
  * instruction with the SM full of warps; latency of a lone warp in cycles):
- *   FP64 add, multiply, FMA, conversion   15.5-18    ~100
- *   FP64 division                         131        564
- *   ddiv_int inlined / called             22 / 28    192 / 287
+ *   FP64 add, multiply, FMA, conversion      15.5-18    ~100
+ *   FP64 division                            131        564
+ *   ddiv_int inlined / called                22 / 28    192 / 287
+ *   64-bit integer high product              5.2        29
+ *   log10 / log2_q57                         553 / 49
+ *   cbrt / cbrt_int                          227 / 98
+ *   pow / pow_int                            1499 / 101
+ *   one ice-table column, 14 FP64 operations / ice_cell_value and its double
+ *                                            224 / 67
  */
 #pragma once
 
@@ -46,6 +52,28 @@ P3X_HD double d_from_bits(uint64_t u) {
   double x;
   std::memcpy(&x, &u, 8);
   return x;
+#endif
+}
+P3X_HD int64_t mulhi_s64(int64_t a, int64_t b) {
+#ifdef __CUDA_ARCH__
+  return __mul64hi(a, b);
+#else
+  return int64_t((__int128(a) * b) >> 64);
+#endif
+}
+P3X_HD uint64_t mulhi_u64(uint64_t a, uint64_t b) {
+#ifdef __CUDA_ARCH__
+  return __umul64hi(a, b);
+#else
+  return uint64_t((static_cast<unsigned __int128>(a) * b) >> 64);
+#endif
+}
+P3X_HD int32_t mulhi_s32(int32_t a, int32_t b) { return int32_t((int64_t(a) * b) >> 32); }
+P3X_HD int clz_u64(uint64_t x) {
+#ifdef __CUDA_ARCH__
+  return __clzll(static_cast<long long>(x));
+#else
+  return x ? __builtin_clzll(x) : 64;
 #endif
 }
 P3X_HD uint32_t mulhi_u32(uint32_t a, uint32_t b) { return uint32_t((uint64_t(a) * b) >> 32); }
@@ -116,6 +144,242 @@ P3X_HD double ddiv_int(double a, double b) {
   if (ea - 1u < 2046u && eb - 1u < 2046u && er - 1u < 2043u && !open) return res;
   if ((ua << 1) == 0 && eb - 1u < 2046u) return d_from_bits(uint64_t(sign) << 32); /* 0 / b */
   return ddiv_general(a, b);
+}
+
+/* ------------------------------------------------------------------ */
+/* logarithm, exponential, powers in 64-bit fixed point                */
+/* ------------------------------------------------------------------ */
+/* Fixed-point values are written Qn: an integer in units of 2^-n. */
+
+/* Tables of the functions below, 128 intervals each (built on the host in
+ * extended precision): r is 2^32 / c for the interval's midpoint c, rounded,
+ * and nlog2 = -log2(r / 2^32) in Q62; exp2 holds 2^((j + 1/2) / 128) in Q62. */
+struct alignas(16) Log2Entry {
+  uint32_t r, pad;
+  int64_t nlog2;
+};
+struct FixTables {
+  Log2Entry log2[128];
+  int64_t exp2[128];
+};
+
+/* log2 of M / 2^52 for a 53-bit significand M, in Q62.  With r ~ 1 / c the
+ * table leaves z = r M / 2^52 - 1, |z| < 2^-8, exact to 2^-63, and
+ * ln(1 + z) = z - z^2 (1/2 - z (1/3 - z (1/4 - z (1/5 - z / 6)))) is cut off
+ * below 2^-58; the inner terms need 32 bits only.  Error below 2^-57. */
+P3X_HD int64_t log2_sig(uint64_t M, const FixTables* t) {
+  const Log2Entry* en = &t->log2[uint32_t(M >> 45) & 127u];
+#ifdef __CUDA_ARCH__
+  const uint4 ev = __ldg(reinterpret_cast<const uint4*>(en));
+  const uint32_t r = ev.x;
+  const int64_t nl = int64_t((uint64_t(ev.w) << 32) | ev.z);
+#else
+  const uint32_t r = en->r;
+  const int64_t nl = en->nlog2;
+#endif
+  const uint64_t M63 = M << 11;
+  const uint64_t P = (M63 >> 32) * r + ((uint64_t(uint32_t(M63)) * r) >> 32);
+  const int64_t z = int64_t(P - (1ull << 63)); /* Q63 */
+  const int64_t z8 = z << 8;                    /* Q71 */
+  const int32_t zs = int32_t(z >> 24);          /* Q39 */
+  constexpr int32_t k6 = int32_t((1ll << 31) / 6), k5 = int32_t((1ll << 31) / 5), k4 = 1 << 29;
+  constexpr int64_t k3 = (1ll << 62) / 3, k2 = 1ll << 61, kLog2e = 6653256548922161245ll; /* log2(e) Q62 */
+  const int32_t t4 = k5 - (mulhi_s32(zs, k6) >> 7);
+  const int32_t t3 = k4 - (mulhi_s32(zs, t4) >> 7);
+  const int64_t t2 = k3 - ((int64_t(zs) * t3) >> 8);
+  const int64_t t1 = k2 - (mulhi_s64(z8, t2) >> 7);
+  const int64_t u = mulhi_s64(z8, t1);         /* z t1, Q69 */
+  const int64_t v = mulhi_s64(z8, u << 3);     /* z^2 t1, Q79 */
+  const int64_t ln = z8 - (v >> 8);            /* Q71 */
+  return nl + (mulhi_s64(ln, kLog2e) >> 7);
+}
+
+/* 2^F for F in [0, 1) given in Q64: the significand in Q62, error below
+ * 2^-60.  2^(1/256 + j/128) from the table times e^g, |g| < 2^-8.5, with
+ * e^g - 1 = g + g^2 (1/2 + g (1/6 + g (1/24 + g (1/120 + g / 720)))). */
+P3X_HD int64_t exp2_sig(uint64_t F, const FixTables* t) {
+#ifdef __CUDA_ARCH__
+  const int64_t T = __ldg(reinterpret_cast<const long long*>(&t->exp2[uint32_t(F >> 57)]));
+#else
+  const int64_t T = t->exp2[uint32_t(F >> 57)];
+#endif
+  const int64_t f = int64_t((F << 7) ^ (1ull << 63)); /* (F mod 2^-7) - 2^-8, Q71 */
+  constexpr int64_t kLn2 = 6393154322601327829ll;     /* ln 2, Q63 */
+  const int64_t g2 = mulhi_s64(f, kLn2) << 1;         /* g, Q71 */
+  const int32_t gs = int32_t(g2 >> 32);               /* Q39 */
+  constexpr int32_t k720 = int32_t((1ll << 31) / 720), k120 = int32_t((1ll << 31) / 120), k24 = int32_t((1ll << 31) / 24);
+  constexpr int64_t k6 = (1ll << 62) / 6, k2 = 1ll << 61;
+  const int32_t q5 = k120 + (mulhi_s32(gs, k720) >> 7);
+  const int32_t q4 = k24 + (mulhi_s32(gs, q5) >> 7);
+  const int64_t q3 = k6 + ((int64_t(gs) * q4) >> 8);
+  const int64_t q2 = k2 + (mulhi_s64(g2, q3) >> 7);
+  const int64_t w = mulhi_s64(g2, q2);      /* g q2, Q69 */
+  const int64_t gw = mulhi_s64(g2, w << 3); /* g^2 q2, Q79 */
+  const int64_t em1 = g2 + (gw >> 8);       /* Q71 */
+  return T + (mulhi_s64(T, em1) >> 7);
+}
+
+/* the double nearest to S 2^(E - 62) for S in [2^62 - 2^8, 2^63) and a result
+ * in the normal range */
+P3X_HD double d_from_q62(int64_t S, int E) {
+  return d_from_bits((uint64_t(uint32_t(E + 1022)) << 52) + uint64_t(S >> 10) + uint64_t((S >> 9) & 1));
+}
+
+/* biased exponent field of a positive double, and its 53-bit significand */
+P3X_HD uint32_t d_expo(uint64_t u) { return uint32_t(u >> 52) & 0x7ffu; }
+P3X_HD uint64_t d_sig(uint64_t u) { return (u & 0xfffffffffffffull) | 0x10000000000000ull; }
+/* x is positive and normal */
+P3X_HD bool d_normal_pos(uint64_t u) { return uint32_t(u >> 32) - 0x00100000u < 0x7fe00000u; }
+
+/* log2(x) in Q57 for a positive normal x in [2^-63, 2^63) */
+P3X_HD int64_t log2_q57(uint64_t u, const FixTables* t) {
+  return (int64_t(int32_t(d_expo(u)) - 1023) << 57) + (log2_sig(d_sig(u), t) >> 5);
+}
+/* log2(x) in Q57 with the exponent limited to [-63, 62] */
+P3X_HD int64_t log2_q57_clamped(uint64_t u, const FixTables* t) {
+  int e = int32_t(d_expo(u)) - 1023;
+  e = e < -63 ? -63 : (e > 62 ? 62 : e);
+  return (int64_t(e) << 57) + (log2_sig(d_sig(u), t) >> 5);
+}
+/* 2^y for y in Q57 */
+P3X_HD double exp2_q57(int64_t y, const FixTables* t) {
+  return d_from_q62(exp2_sig(uint64_t(y) << 7, t), int(y >> 57));
+}
+
+/* cube root of a positive normal x: 2^((e + log2 m) / 3), relative error
+ * below 2^-58 before the rounding to a double */
+P3X_HD double cbrt_int(double x, const FixTables* t) {
+  const uint64_t u = d_bits(x);
+  const uint32_t eb = d_expo(u), k = mulhi_u32(eb, 0x55555556u), rem = eb - 3 * k; /* 1023 = 3 * 341 */
+  const uint64_t X = (uint64_t(rem) << 62) + uint64_t(log2_sig(d_sig(u), t));       /* Q62, < 3 */
+  const uint64_t F = X + mulhi_u64(X, 0x5555555555555555ull);                        /* X / 3, Q64 */
+  return d_from_q62(exp2_sig(F, t), int(k) - 341);
+}
+
+/* x^c for a positive normal x in [2^-63, 2^63) and 0 < c < 1 in Q63,
+ * relative error below 2^-56 before the rounding to a double */
+P3X_HD double pow_int(double x, int64_t c, const FixTables* t) {
+  const int64_t y = mulhi_s64(log2_q57(d_bits(x), t), c); /* Q56 */
+  return d_from_q62(exp2_sig(uint64_t(y) << 8, t), int(y >> 56));
+}
+
+/* the double nearest to V 2^-s */
+P3X_HD double d_from_fix(int64_t V, int s) {
+  const uint64_t neg = uint64_t(V) & (1ull << 63);
+  const uint64_t a = neg ? uint64_t(0) - uint64_t(V) : uint64_t(V);
+  const int lz = clz_u64(a);
+  const uint64_t n = a << (lz & 63);
+  const uint64_t r = (uint64_t(uint32_t(1085 - lz - s)) << 52) + (n >> 11) + ((n >> 10) & 1);
+  return V == 0 ? 0.0 : d_from_bits(r | neg);
+}
+
+/* Coordinate of a table axis in 64-bit fixed point: the interval [0, n - 1]
+ * of a value in Qq already limited to [0, n], and the position in it as a Q63
+ * weight (1 as 1 - 2^-63). */
+struct FixAxis {
+  int i;
+  int64_t w;
+};
+P3X_HD FixAxis fix_axis(int64_t x, int q, int n) {
+  FixAxis a;
+  a.i = int(x >> q);
+  a.i = a.i < n ? a.i : n - 1;
+  const uint64_t w = uint64_t(x - (int64_t(a.i) << q)) << (63 - q);
+  a.w = int64_t(w >> 63 ? (1ull << 63) - 1 : w);
+  return a;
+}
+P3X_HD int64_t fix_clamp(int64_t x, int64_t lo, int64_t hi) { return x < lo ? lo : (x > hi ? hi : x); }
+
+/* Trilinear interpolation of one ice-table column inside one cell from the
+ * cell's eight coefficients c[0..7] in fixed point:
+ *   c0 + w1 c1 + w4 (c2 + w1 c3) + w5 (c4 + w1 c5 + w4 (c6 + w1 c7)),
+ * each coefficient stored times 2 per weight it is multiplied with (a Q63
+ * weight halves the product's high word). */
+constexpr int kCellCoefs = 8, kCellCols = 4;
+P3X_HD int64_t fix_trilinear(const int64_t c[kCellCoefs], int64_t w1, int64_t w4, int64_t w5) {
+  const int64_t e = c[0] + mulhi_s64(w1, c[1]), d = c[2] + mulhi_s64(w1, c[3]);
+  const int64_t b = c[4] + mulhi_s64(w1, c[5]), a = c[6] + mulhi_s64(w1, c[7]);
+  return e + mulhi_s64(w4, d) + mulhi_s64(w5, b + mulhi_s64(w4, a));
+}
+
+/* Position of an ice category in the ice table (lookup_ice,
+ * p3/impl/p3_table_ice_impl.hpp:80-138): the size axis
+ * (log10(qi / ni) + 18) 4.135985... - 10, the rime axis 3 qm / qi + 1 and the
+ * density axis, each limited as the reference limits it, 0-based. */
+struct IceCell {
+  int cell;
+  bool odd; /* an argument is infinite, NaN or (qi / ni) not a positive normal number */
+  int64_t w1, w4, w5;
+};
+constexpr int kCellI = 49, kCellR = 3, kCellD = 4, kIceCells = kCellI * kCellR * kCellD;
+/* rhop: 0 or positive; ratio_qm = qm / qi >= 0; qi_ni = qi / ni positive */
+P3X_HD IceCell ice_cell(double qi_ni, double ratio_qm, double rhop, const FixTables* t) {
+  /* d log2(x) + c of the size axis less one, Q55 */
+  constexpr int64_t kd = 5741805296813221454ll; /* 4.135985029041767 log10(2), Q62 */
+  constexpr int64_t kc = 2285945404318149440ll;  /* 18 * 4.135985029041767 - 11, Q55 */
+  const uint64_t ux = d_bits(qi_ni);
+  const int64_t x1 = mulhi_s64(log2_q57_clamped(ux, t), kd) + kc;
+  const FixAxis a1 = fix_axis(fix_clamp(x1, 0, 49ll << 55), 55, kCellI);
+  /* 3 ratio, Q60 */
+  const uint64_t ur = d_bits(ratio_qm);
+  const int er = 1023 - int(d_expo(ur));
+  const uint64_t q60 = er <= 0 ? (1ull << 60) : ((d_sig(ur) << 8) >> (er < 63 ? er : 63));
+  const FixAxis a4 = fix_axis(int64_t(3 * q60), 60, kCellR);
+  /* density, Q52, then Q58: (rho - 50) 0.005 up to 650, 3 + (rho - 650) 0.004
+   * above; beyond 900 the axis ends */
+  const uint64_t up = d_bits(rhop);
+  const int ep = int(d_expo(up)) - 1023;
+  const uint64_t p52 = ep > 9 ? (1023ull << 52) : (ep >= 0 ? d_sig(up) << ep : 0);
+  const bool low = up <= 0x4084500000000000ull; /* rho <= 650 */
+  const int64_t k = low ? 5902958103587056517ll : 4722366482869645213ll; /* 0.005, 0.004 in Q70 */
+  const int64_t x5 = mulhi_s64(int64_t(p52) - (int64_t(low ? 50 : 650) << 52), k) + (low ? 0 : (3ll << 58));
+  const FixAxis a5 = fix_axis(fix_clamp(x5, 0, 4ll << 58), 58, kCellD);
+  const bool odd = !d_normal_pos(ux) || er == -1024 || ep == 1024;
+  return IceCell{(a5.i * kCellR + a4.i) * kCellI + a1.i, odd, a1.w, a4.w, a5.w};
+}
+
+/* value of one column in a cell: c points to its eight coefficients */
+P3X_HD int64_t ice_cell_value(const int64_t* c, const IceCell& p) {
+  int64_t k[kCellCoefs];
+#ifdef __CUDA_ARCH__
+#pragma unroll
+  for (int j = 0; j < kCellCoefs; j += 2) {
+    const longlong2 v = __ldg(reinterpret_cast<const longlong2*>(c + j));
+    k[j] = v.x;
+    k[j + 1] = v.y;
+  }
+#else
+  for (int j = 0; j < kCellCoefs; ++j) k[j] = c[j];
+#endif
+  return fix_trilinear(k, p.w1, p.w4, p.w5);
+}
+/* V 2^-s < 1 for V >= 0 */
+P3X_HD bool fix_below_one(int64_t V, int s) { return s >= 0 && (V >> (s < 63 ? s : 63)) == 0; }
+
+/* Rain drop size D = (mu + 1) / lambda with lambda^3 = f n / q, limited to
+ * [1e-5, 2e-3] (the reference's limits on lambda, p3_dsd2_impl.hpp:76-126),
+ * and its Table3 row coordinate (lookup, p3_table3_impl.hpp:14-64).  In base-2
+ * logarithms log2 D = kd - log2(n / q) / 3 with kd = log2(mu + 1) - log2(f) / 3
+ * in Q57, so neither lambda nor a division is formed. */
+struct RainRow {
+  int side;    /* -1: D was below the limits (n too large), 1: above, 0: inside */
+  int row;     /* 1-based row of Table3 */
+  double frac; /* position between row and row + 1 */
+};
+P3X_HD RainRow rain_row(double n_q, int64_t kd, const FixTables* t) {
+  constexpr int64_t kLogMin = -2393701460845809080ll; /* log2(1e-5), Q57 */
+  constexpr int64_t kLogMax = -1292105688431629576ll; /* log2(2e-3), Q57 */
+  int64_t y = kd - mulhi_s64(log2_q57_clamped(d_bits(n_q), t), 6148914691236517205ll);
+  RainRow r;
+  r.side = y < kLogMin ? -1 : (y > kLogMax ? 1 : 0);
+  y = fix_clamp(y, kLogMin, kLogMax);
+  const int64_t D = exp2_sig(uint64_t(y) << 7, t) >> (-9 - int(y >> 57)); /* Q71 */
+  const bool fine = D <= 460430732079790408ll;                             /* 195e-6 */
+  /* (1e6 D + 5) / 10 below 195 microns, 20 + (1e6 D - 195) / 30 above, Q53 */
+  const int64_t c = mulhi_s64(D, fine ? 7036874417766400000ll : 2345624805922133333ll) + (fine ? 1ll << 52 : 27ll << 52);
+  r.row = int(c >> 53);
+  r.frac = d_from_bits(0x3ff0000000000000ull | ((uint64_t(c) >> 1) & 0xfffffffffffffull)) - 1.0;
+  return r;
 }
 
 }  // namespace dev

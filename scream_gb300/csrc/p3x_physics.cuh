@@ -66,6 +66,13 @@ struct RuntimeDev {
   double g_mur2;      /* Gamma(mu_r + 2)       */
   double lg_mur4;     /* log Gamma(mu_r + 4)   */
   double lg_mur7;     /* log Gamma(mu_r + 7)   */
+  /* rain drop size in the FP64 sedimentation (rain_row): log2(mu_r + 1) -
+   * log2(f) / 3 in Q57 with f = CONS1 (mu_r+3)(mu_r+2)(mu_r+1), the number per
+   * mass at the two lambda limits, and the weight of Table3's second mu
+   * column; rain_fix is 0 when mu_r has no such form (the general path) */
+  int rain_fix;
+  int64_t rain_kd;
+  double rain_n_hi, rain_n_lo, t3_wj;
   /* FP32-bulk saturation table (layout of build_svp_table) */
   const double* svp_tab;
   /* accretion_qc_exponent == accretion_qr_exponent (the single-power form) */
@@ -131,11 +138,15 @@ __device__ __forceinline__ float m_tanh(float x) { return tanhf(x); }
 /* Division: the FP64 form through the integer pipes (p3x_intfp64.cuh), the
  * same double as the FP64 division at a fifth of its pipe time.  One copy per
  * kernel: part1+2 holds about a hundred divisions and waits on instruction
- * fetch.  At 21,600 x 128: part1+2 10.0 -> 6.9 ms, sedimentation 27.3 -> 15.8
- * ms, part3 1.64 -> 0.87 ms. */
+ * fetch.  At 21,600 x 128: part1+2 10.0 -> 6.9 ms. */
 static __device__ __noinline__ double m_div_nl(double a, double b) { return ddiv_int(a, b); }
 __device__ __forceinline__ double m_div(double a, double b) { return m_div_nl(a, b); }
 __device__ __forceinline__ float m_div(float a, float b) { return a / b; }
+/* cube root on the integer pipes (98 cycles of an SM against 227); zero, infinities, NaN, subnormals and
+ * negative arguments by the library function */
+static __device__ __noinline__ double cbrt_fix(double x, const FixTables* t) {
+  return d_normal_pos(d_bits(x)) ? cbrt_int(x, t) : cbrt(x);
+}
 __device__ __forceinline__ double m_fabs(double x) { return fabs(x); }
 __device__ __forceinline__ float m_fabs(float x) { return fabsf(x); }
 
@@ -668,8 +679,8 @@ __device__ __forceinline__ void calc_incloud(double qc, double qr, double qi, do
  * spectral moments cdist (used only by the inactive cloud relaxation time
  * epsc) and cdist1 = nc/Gamma(mu_c+1) (immersion freezing, evaluated there
  * with the Gamma recurrence) are not needed by any output. */
-template <class TR>
-__device__ __forceinline__ void get_cloud_dsd2(TR qc, TR& nc, TR& mu_c, TR rho, TR& lamc) {
+template <class TR, class Cbrt>
+__device__ __forceinline__ void get_cloud_dsd2(TR qc, TR& nc, TR& mu_c, TR rho, TR& lamc, Cbrt&& cube_root) {
   lamc = 0; mu_c = 0;
   if (qc >= TR(C::QSMALL)) {
     nc = vmax(nc, TR(C::NSMALL));
@@ -678,7 +689,7 @@ __device__ __forceinline__ void get_cloud_dsd2(TR qc, TR& nc, TR& mu_c, TR rho, 
     mu = vmax(mu, TR(2.));
     mu = vmin(mu, TR(15.));
     mu_c = mu;
-    lamc = m_cbrt(m_div(TR(C::CONS1) * nc * (mu_c + TR(3)) * (mu_c + TR(2)) * (mu_c + TR(1)), qc));
+    lamc = cube_root(m_div(TR(C::CONS1) * nc * (mu_c + TR(3)) * (mu_c + TR(2)) * (mu_c + TR(1)), qc));
     const TR lammin = (mu_c + TR(1)) * TR(2.5e+4);
     const TR lammax = (mu_c + TR(1)) * TR(1.e+6);
     const bool lt = lamc < lammin, gt = lamc > lammax;
@@ -691,15 +702,21 @@ __device__ __forceinline__ void get_cloud_dsd2(TR qc, TR& nc, TR& mu_c, TR rho, 
   }
 }
 
-/* get_rain_dsd2, p3_dsd2_impl.hpp:76-126 */
 template <class TR>
-__device__ __forceinline__ void get_rain_dsd2(TR qr, TR& nr, TR& mu_r, TR& lamr, const RuntimeDev& rt) {
+__device__ __forceinline__ void get_cloud_dsd2(TR qc, TR& nc, TR& mu_c, TR rho, TR& lamc) {
+  get_cloud_dsd2<TR>(qc, nc, mu_c, rho, lamc, [](TR x) { return m_cbrt(x); });
+}
+
+/* get_rain_dsd2, p3_dsd2_impl.hpp:76-126 */
+template <class TR, class Cbrt>
+__device__ __forceinline__ void get_rain_dsd2(TR qr, TR& nr, TR& mu_r, TR& lamr, const RuntimeDev& rt,
+                                              Cbrt&& cube_root) {
   lamr = 0;
   if (qr >= TR(C::QSMALL)) {
     const TR nr_lim = vmax(nr, TR(C::NSMALL));
     mu_r = P3X_RTP(TR, constant_mu_rain);
     const TR f = TR(C::CONS1) * (mu_r + TR(3)) * (mu_r + TR(2)) * (mu_r + TR(1));
-    lamr = m_cbrt(m_div(f * nr_lim, qr));
+    lamr = cube_root(m_div(f * nr_lim, qr));
     const TR lammax = (mu_r + TR(1.)) * TR(1.e+5);
     const TR lammin = (mu_r + TR(1.)) * TR(500);
     const bool lt = lamr < lammin, gt = lamr > lammax;
@@ -710,6 +727,11 @@ __device__ __forceinline__ void get_rain_dsd2(TR qr, TR& nr, TR& mu_r, TR& lamr,
       nr = m_div(lamr * lamr * lamr * qr, f);
     }
   }
+}
+
+template <class TR>
+__device__ __forceinline__ void get_rain_dsd2(TR qr, TR& nr, TR& mu_r, TR& lamr, const RuntimeDev& rt) {
+  get_rain_dsd2<TR>(qr, nr, mu_r, lamr, rt, [](TR x) { return m_cbrt(x); });
 }
 
 /* impose_max_total_ni, p3_impose_max_total_ni_impl.hpp:9-27 */
