@@ -40,6 +40,9 @@ struct p3x_context {
   int64_t *d_cell_sed = nullptr, *d_cell_part3 = nullptr;
   int32_t *d_shift_sed = nullptr, *d_shift_part3 = nullptr;
   double* d_t3sed = nullptr;
+  /* liquid saturation vapour pressure at 0 C, as the device evaluates it (it
+   * took every launch of part1+2 a chain of log, tanh and exp, 5 us) */
+  double esat0 = 0;
   uint32_t* d_err = nullptr;
   /* check_values words (dev::kCheckWords) and mode (P3X_CHECK_*) */
   unsigned long long* d_check = nullptr;
@@ -259,6 +262,7 @@ dev::KParams<double> make_kparams<double>(p3x_context* ctx, const dev::RuntimeDe
   kp.cell_part3_shift = ctx->d_shift_part3;
   kp.t3sed = reinterpret_cast<const double4*>(ctx->d_t3sed);
   kp.err = ctx->d_err;
+  kp.esat0 = ctx->esat0;
   kp.check = ctx->check_mode ? ctx->d_check : nullptr;
   kp.check_fail = ctx->check_mode == P3X_CHECK_FAIL ? 1 : 0;
   return kp;
@@ -276,6 +280,7 @@ dev::KParams<float> make_kparams<float>(p3x_context* ctx, const dev::RuntimeDev&
   kp.t3slice = ctx->f_t3slices + size_t(rtd.t3_dumjj - 1) * dev::kT3SliceElems;
   kp.rt.svp_tab = ctx->d_svp;
   kp.err = ctx->d_err;
+  kp.esat0 = ctx->esat0;
   kp.check = ctx->check_mode ? ctx->d_check : nullptr;
   kp.check_fail = ctx->check_mode == P3X_CHECK_FAIL ? 1 : 0;
   return kp;
@@ -650,6 +655,11 @@ int p3x_context_create(const char* table_file, p3x_context** out, int* info) {
     if (info) *info = P3X_ENOMEM;
     p3x_context_destroy(ctx.release());
     return P3X_ENOMEM;
+  }
+  if ((st = cuda_status(saturation_at_melting(&ctx->esat0)))) {
+    if (info) *info = st;
+    p3x_context_destroy(ctx.release());
+    return st;
   }
   {
     cudaMemPoolProps props{};

@@ -557,6 +557,22 @@ __global__ void f2d_selftest_kernel(unsigned long long* mismatches) {
   if (bad) atomicAdd(mismatches, bad);
 }
 
+__global__ void saturation_at_melting_kernel(double* out) {
+  uint32_t err = 0;
+  *out = dev::murphy_koop_svp<double>(dev::C::Tmelt, false, err);
+}
+
+cudaError_t saturation_at_melting(double* out) {
+  double* d = nullptr;
+  cudaError_t e = cudaMalloc(&d, sizeof(*d));
+  if (e != cudaSuccess) return e;
+  saturation_at_melting_kernel<<<1, 1>>>(d);
+  e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpy(out, d, sizeof(*d), cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e;
+}
+
 cudaError_t launch_selftest(unsigned long long* mismatches_d, cudaStream_t st) {
   f2d_selftest_kernel<<<4096, 256, 0, st>>>(mismatches_d);
   return cudaGetLastError();

@@ -85,6 +85,7 @@ struct KParams {
   const WorkItem* work;
   const Inst* insts;
   uint32_t* err;
+  double esat0; /* liquid saturation vapour pressure at 0 C (ice_melting, ice_cldliq_wet_growth) */
   /* kWorkCounters zeroed counters: groups take work items from them as they
    * finish the last ones.  Null: groups stride the list statically. */
   uint32_t* wctr;
@@ -105,6 +106,8 @@ __host__ __device__ inline unsigned long long check_key(int inst, int col, int k
 constexpr int kIceTableElems = kDensize * kRimsize * kIsize * kIceCols; /* 12000 */
 constexpr int kT3SliceElems = 3 * 300 * 2;
 constexpr int kT3SedRows = 300;
+/* (RHO_600MB / RHO_1000MB)^0.54 */
+constexpr double kRhofaciOverR = 0.790740972875368752906;
 constexpr long long kInfBits = 0x7ff0000000000000ll;
 constexpr uint64_t kNaNBits = 0x7ff8000000000000ull;
 constexpr int kMaxSubsteps = 100000;
@@ -113,6 +116,7 @@ constexpr uint64_t kWaitNanosLimit = 2000000000ull; /* 2 s */
 
 /* shared arrays of one column group in K1 */
 enum { A_TATM = 0, A_RHO, A_RHOFACR, A_RHOFACI, A_ACN, A_QVSL, A_QVSI, A_QVSSI, A_EPINVP, A_NARR };
+constexpr int A_LIST = A_EPINVP; /* FP64 form: the level lists (16-bit entries) */
 /* shared arrays of one column group in K2 (FP64 form, p3_sed); the rain flux
  * accumulator re-uses R2 (rain has two fields) */
 enum { B_FR = 0, B_CF, B_QS, B_V1, B_V2, B_R0, B_R1, B_R2, B_R3, B_NARR };
@@ -307,7 +311,7 @@ __device__ __forceinline__ bool clip_to_vapour(State& s, double inv_exner) {
  * FP64 state and its shadow.  sm / S: the K1 shared arrays of the column. */
 __device__ __forceinline__ void part2_level_bulk(const Inst& in, const int64_t o, const int k,
                                                  double* __restrict__ sm, const int S, const KParams<float>& kp,
-                                                 const Tabs<float>& tb, const double esat0, const float dtf,
+                                                 const Tabs<float>& tb, const float dtf,
                                                  const float inv_dtf, bool& hydro, uint32_t& err) {
   const RuntimeDev& rt = kp.rt;
   const bool predictNc = in.predictNc != 0, prescribedCCN = in.prescribedCCN != 0;
@@ -374,6 +378,7 @@ __device__ __forceinline__ void part2_level_bulk(const Inst& in, const int64_t o
   float epsi = 0, epsr = 0, epsi_tot = 0;
   float rho_qm_cloud = 400.0f;
   bool wet = false;
+  const auto rain_size = [&] { return m_cbrt(qr_in / (float(C::Pi) * float(C::RHO_H2O) * nr_in)); };
 
   if (qc_in >= QS || qr_in >= QS || qi_in >= QS) {
     get_time_space_phys_variables<float>(T_r, float(in.pres[o]), rho, float(qvsl), qvsi_r, v);
@@ -419,7 +424,7 @@ __device__ __forceinline__ void part2_level_bulk(const Inst& in, const int64_t o
       TableIce<float> ti;
       lookup_ice<float>(qi_in, ni_in, qm_in, rhop, ti);
       TableRain<float> trn;
-      lookup_rain<float>(qr_in, nr_in, trn);
+      lookup_rain<float>(qr_in, nr_in, trn, rain_size);
       float ta[4], tc[4];
       apply_table_ice4<float>(tb, ti, 0, ta); /* columns 0, 1, 6, 7 */
       apply_table_ice4<float>(tb, ti, 4, tc); /* columns 2, 3, 4, 9 */
@@ -438,16 +443,17 @@ __device__ __forceinline__ void part2_level_bulk(const Inst& in, const int64_t o
       ni_in = vmax(ni_in, tv_lammin * ni_in);
     }
     const double dT0 = T - C::Tmelt;
-    const double dqv0 = esat0 * ep_inv_p - s.qv;
+    const double dqv0 = kp.esat0 * ep_inv_p - s.qv;
+    const auto vent = [&] { return tv_melt + tv_vent * m_cbrt(v.sc) * m_sqrt(rhofaci * rho / v.mu); };
+    const auto imm = [&] { return m_exp(rt.f.immersion_freezing_exponent * (float(C::T_zerodegc) - T_r)); };
     if (do_ice) {
       ice_cldliq_collection<float>(rho, T, rhofaci, tv_qc2qi, qi_in, qc_in, ni_in, nc_in, r, rt);
       ice_rain_collection<float>(rho, T, rhofaci, logn0r, tv_nr, tv_qr2qi, qi_in, ni_in, qr_in, r, rt);
       ice_self_collection<float>(rho, rhofaci, tv_selfcol, v.eii, qm_in, qi_in, ni_in, r);
     }
-    ice_melting<float>(rho, dT0, dqv0, rhofaci, tv_melt, tv_vent, v, qi_in, ni_in, r);
+    ice_melting<float>(rho, dT0, dqv0, v, qi_in, ni_in, r, vent);
     if (do_ice) {
-      wet = ice_cldliq_wet_growth<float>(rho, dT0, dqv0, rhofaci, tv_melt, tv_vent, v, qc_in, qi_in, ni_in, qr_in,
-                                         r);
+      wet = ice_cldliq_wet_growth<float>(rho, dT0, dqv0, v, qc_in, qi_in, ni_in, qr_in, r, vent);
     }
     /* ice_relaxation_timescale, p3_ice_relaxation_timescale_impl.hpp:9-37 */
     if (qi_in >= QS && dlt(T, C::Tmelt)) {
@@ -458,8 +464,8 @@ __device__ __forceinline__ void part2_level_bulk(const Inst& in, const int64_t o
     rho_qm_cloud = calc_rime_density<float>(T_r, rhofaci, tv_fallspd, acn, lamc, mu_c, qc_in,
                                             r.qc2qi_collect_tend);
     if (do_ice) {
-      cldliq_immersion_freezing<float>(T_r, lamc, mu_c, nc_in, qc_in, r, rt);
-      rain_immersion_freezing<float>(T_r, lamr, mu_r, cdistr, qr_in, r, rt);
+      cldliq_immersion_freezing<float>(T_r, lamc, mu_c, nc_in, qc_in, r, rt, imm);
+      rain_immersion_freezing<float>(T_r, lamr, mu_r, cdistr, qr_in, r, rt, imm);
     }
     /* calc_liq_relaxation_timescale, p3_calc_liq_relaxation_timescale_impl.hpp:13-43 */
     if (qr_in >= QS) {
@@ -484,7 +490,7 @@ __device__ __forceinline__ void part2_level_bulk(const Inst& in, const int64_t o
   cloud_water_autoconversion<float>(rho, qc_in, nc_in, r, rt);
   if (qc_in >= QS) r.nc_selfcollect_tend = 0.0f;
   cloud_rain_accretion<float>(qc_in, nc_in, qr_in, r, rt);
-  rain_self_collection<float>(rho, qr_in, nr_in, r, rt);
+  rain_self_collection<float>(rho, qr_in, nr_in, r, rt, rain_size);
   back_to_cell_average<float>(cl, cr, ci, r);
 
   /* limiters on the FP32 rates (FP64 vapour residuals), one FP64
@@ -520,11 +526,505 @@ __device__ __forceinline__ void part2_level_bulk(const Inst& in, const int64_t o
 /* ------------------------------------------------------------------ */
 /* one column                                                          */
 /* ------------------------------------------------------------------ */
-/* K1: p3_main_init, p3_main_part1, p3_main_part2 of one column. */
-template <class TR, int LANES>
-__device__ void p3_part12(const Inst& in, const int col, const KParams<TR>& kp, const Tabs<TR>& tb,
-                          double* __restrict__ sm, const double esat0, uint32_t& err) {
-  constexpr bool kF64 = sizeof(TR) == sizeof(double);
+/* Saturation vapour pressure (murphy_koop_svp) of the FP64 part1+2 with the
+ * logarithm of the temperature shared by its liquid and ice forms. */
+__device__ __forceinline__ double svp_liquid(double t, double logt) {
+  return m_exp(54.842763 - m_div(6763.22, t) - (4.210 * logt) + (0.000367 * t) +
+               (m_tanh(0.0415 * (t - 218.8)) * (53.878 - m_div(1331.22, t) - (9.44523 * logt) + 0.014025 * t)));
+}
+__device__ __forceinline__ double svp_ice(double t, double logt) {
+  return m_exp(9.550426 - m_div(5723.265, t) + (3.53068 * logt) - (0.00728332 * t));
+}
+/* x^0.54 and x^0.5 in fixed point, the library function outside its range */
+static __device__ __noinline__ double pow_fix(double x, int64_t c, double cd, const FixTables* t) {
+  return uint32_t(d_bits(x) >> 52) - (1023u - 62u) < 124u ? pow_int(x, c, t) : pow(x, cd);
+}
+
+/* p3_main_part2 of one level with a hydrometeor in the FP64 form
+ * (p3_main_part2_impl.hpp, same order of processes).  Each library function
+ * (a pow holds the FP64 pipe for 1,500 cycles) is evaluated once and only
+ * where a process reads it: the cube root of the Schmidt number and the
+ * ventilation term serve melting, wet growth, relaxation and rain
+ * evaporation; the viscosity terms need rain or ice, rhofaci ice, acn cloud
+ * and ice, and logn0r rain and ice. */
+__device__ __forceinline__ void part2_level_f64(const Inst& in, const int64_t o, const int k, double* __restrict__ sm,
+                                                const int S, const KParams<double>& kp, const Tabs<double>& tb,
+                                                const double dt, const double inv_dt, bool& hydro, uint32_t& err) {
+  const RuntimeDev& rt = kp.rt;
+  const bool predictNc = in.predictNc != 0, prescribedCCN = in.prescribedCCN != 0;
+  const bool do_ice = rt.do_ice_production != 0;
+  State s;
+  s.qc = in.qc[o]; s.nc = in.nc[o]; s.qr = in.qr[o]; s.nr = in.nr[o];
+  s.qi = in.qi[o]; s.qm = in.qm[o]; s.ni = in.ni[o]; s.bm = in.bm[o];
+  s.qv = in.qv[o]; s.th = in.th[o];
+  const double T = sm[A_TATM * S + k];
+  const double qvssi = sm[A_QVSSI * S + k];
+  if (dlt(s.qc, C::QSMALL) && dlt(s.qr, C::QSMALL) && dlt(s.qi, C::QSMALL) && dlt(T, C::T_zerodegc) &&
+      dlt_neg(qvssi, -0.05))
+    return;
+
+  const double pres = in.pres[o];
+  const double cld_i = in.cld_frac_i[o], cld_l = in.cld_frac_l[o], cld_r = in.cld_frac_r[o];
+  const double inv_exner = in.inv_exner[o];
+  const double qvsl = sm[A_QVSL * S + k], qvsi = sm[A_QVSI * S + k];
+  const double rho = sm[A_RHO * S + k];
+  const double inv_rho = m_div(1.0, rho);
+  Incld inc;
+  calc_incloud(s.qc, s.qr, s.qi, s.qm, s.nc, s.nr, s.ni, s.bm, m_div(1.0, cld_l), m_div(1.0, cld_i),
+               m_div(1.0, cld_r), inc);
+
+  Rates<double> r;
+  r.zero();
+  PhysVars<double> v;
+  v.mu = v.dv = v.sc = v.dqsdt = v.dqsidt = v.ab = v.abi = v.kap = v.eii = 0.0;
+  double tv_fallspd = 0, tv_selfcol = 0, tv_qc2qi = 0, tv_melt = 0, tv_nr = 0, tv_qr2qi = 0, tv_lammax = 0,
+         tv_lammin = 0, tv_vent = 0;
+  double mu_c = 0, lamc = 0, mu_r = 0, lamr = 0, cdistr = 0, logn0r = 0;
+  double epsi = 0, epsr = 0, epsi_tot = 0;
+  double rho_qm_cloud = 400.0;
+  double rain_size = 0; /* (qr / (pi rho_w nr))^(1/3) */
+  bool wet = false;
+
+  const bool has_c = dge(inc.qc, C::QSMALL), has_r = dge(inc.qr, C::QSMALL), has_i = dge(inc.qi, C::QSMALL);
+  if (has_c || has_r || has_i) {
+    double cbrt_sc = 0;
+    if (has_r || has_i) {
+      get_time_space_phys_variables<double>(T, pres, rho, qvsl, qvsi, v);
+      cbrt_sc = m_cbrt(v.sc);
+    }
+    {
+      const double n_in = inc.nc;
+      double n_out = n_in;
+      get_cloud_dsd2<double>(inc.qc, n_out, mu_c, rho, lamc);
+      apply_n_adjust(inc.nc, n_in, n_out);
+      s.nc = inc.nc * cld_l;
+    }
+    {
+      const double n_in = inc.nr;
+      double n_out = n_in;
+      get_rain_dsd2<double>(inc.qr, n_out, mu_r, lamr, rt);
+      apply_n_adjust(inc.nr, n_in, n_out);
+      if (has_r) {
+        cdistr = m_div(inc.nr, rt.g_mur1);
+        if (has_i) logn0r = m_log10(cdistr) + (mu_r + 1.0) * m_log10(lamr);
+      }
+      s.nr = inc.nr * cld_r;
+    }
+    impose_max_total_ni(inc.ni, rt.max_total_ni, inv_rho);
+    if (has_i) {
+      inc.ni = dmax_c(inc.ni, C::NSMALL);
+      inc.nr = dmax_c(inc.nr, C::NSMALL);
+    }
+    if (has_r) rain_size = m_cbrt(m_div(inc.qr, C::Pi * C::RHO_H2O * inc.nr));
+    double rhofaci = 0, vent = 0;
+    if (has_i) {
+      rhofaci = m_pow(C::RHO_600MB * inv_rho, .54);
+      const double rhop = calc_bulk_rho_rime(inc.qi, inc.qm, inc.bm, rt);
+      s.qm = inc.qm * cld_i;
+      s.bm = inc.bm * cld_i;
+      TableIce<double> ti;
+      lookup_ice<double>(inc.qi, inc.ni, inc.qm, rhop, ti);
+      TableRain<double> trn;
+      lookup_rain<double>(inc.qr, inc.nr, trn, [&] { return rain_size; });
+      double ta[4], tc[4];
+      apply_table_ice4<double>(tb, ti, 0, ta); /* columns 0, 1, 6, 7 */
+      apply_table_ice4<double>(tb, ti, 4, tc); /* columns 2, 3, 4, 9 */
+      tv_fallspd = ta[1];
+      tv_selfcol = tc[0];
+      tv_qc2qi = tc[1];
+      tv_melt = tc[2];
+      tv_lammax = ta[2];
+      tv_lammin = ta[3];
+      tv_vent = tc[3];
+      if (has_r) {
+        tv_nr = apply_table_coll<double>(0, tb, ti, trn);
+        tv_qr2qi = apply_table_coll<double>(1, tb, ti, trn);
+      }
+      inc.ni = vmin(inc.ni, tv_lammax * inc.ni);
+      inc.ni = vmax(inc.ni, tv_lammin * inc.ni);
+      vent = tv_melt + tv_vent * cbrt_sc * m_sqrt(m_div(rhofaci * rho, v.mu));
+    }
+    const double qi_r = inc.qi, qc_r = inc.qc, ni_r = inc.ni, nc_r = inc.nc, qr_r = inc.qr;
+    const double dT0 = T - C::Tmelt;
+    const double dqv0 = m_div(C::ep_2 * kp.esat0, vmax(pres, 1.e-3)) - s.qv;
+    if (do_ice) {
+      ice_cldliq_collection<double>(rho, T, rhofaci, tv_qc2qi, qi_r, qc_r, ni_r, nc_r, r, rt);
+      ice_rain_collection<double>(rho, T, rhofaci, logn0r, tv_nr, tv_qr2qi, qi_r, ni_r, qr_r, r, rt);
+      ice_self_collection<double>(rho, rhofaci, tv_selfcol, v.eii, inc.qm, qi_r, ni_r, r);
+    }
+    ice_melting<double>(rho, dT0, dqv0, v, qi_r, ni_r, r, [&] { return vent; });
+    if (do_ice) wet = ice_cldliq_wet_growth<double>(rho, dT0, dqv0, v, qc_r, qi_r, ni_r, qr_r, r, [&] { return vent; });
+    /* ice_relaxation_timescale, p3_ice_relaxation_timescale_impl.hpp:9-37 */
+    if (has_i && dlt(T, C::Tmelt)) {
+      epsi = (vent * 2.0 * C::Pi * rho * v.dv) * ni_r;
+      epsi_tot = epsi_tot + epsi;
+    }
+    if (has_c && has_i) {
+      /* acn from the viscosity, which is part1's unless part1 changed the
+       * temperature (it then left acn with the sign bit set) */
+      const double a = sm[A_ACN * S + k];
+      const double acn = dneg(a) ? -a : m_div(C::gravit * C::RHO_H2O, 18.0 * v.mu);
+      rho_qm_cloud = calc_rime_density<double>(T, rhofaci, tv_fallspd, acn, lamc, mu_c, qc_r, r.qc2qi_collect_tend);
+    }
+    if (do_ice && (has_c || has_r) && T <= C::T_rainfrz) {
+      const double e = m_exp(rt.immersion_freezing_exponent * (C::T_zerodegc - T));
+      cldliq_immersion_freezing<double>(T, lamc, mu_c, nc_r, qc_r, r, rt, [&] { return e; });
+      rain_immersion_freezing<double>(T, lamr, mu_r, cdistr, qr_r, r, rt, [&] { return e; });
+    }
+    /* calc_liq_relaxation_timescale, p3_calc_liq_relaxation_timescale_impl.hpp:13-43 */
+    if (has_r) {
+      Table3<double> t3;
+      lookup3<double>(mu_r, lamr, rt, t3);
+      epsr = 2.0 * C::Pi * cdistr * rho * v.dv *
+             (m_div(C::f1r * rt.g_mur2, lamr) +
+              C::f2r * m_sqrt(m_div(rho, v.mu)) * cbrt_sc * apply_table3<double>(tb, tb.revap, t3));
+    }
+    evaporate_rain(inc.qr, inc.qc, inc.nr, inc.qi, cld_l, cld_r, s.qv, in.qv_prev[o], qvsl, qvsi, v.ab, v.abi, epsr,
+                   epsi_tot, T, in.t_prev[o], v.dqsdt, dt, r.qr2qv_evap_tend, r.nr_evap_tend);
+    if (do_ice) {
+      ice_deposition_sublimation(inc.qi, inc.ni, T, qvsl, qvsi, epsi, v.abi, s.qv, inv_dt, r.qv2qi_vapdep_tend,
+                                 r.qi2qv_sublim_tend, r.ni_sublim_tend, r.qc2qi_berg_tend);
+    }
+  }
+  if (do_ice) {
+    ice_nucleation<double>(T, inv_rho, s.ni, in.ni_activated[o], qvssi, inv_dt, predictNc, prescribedCCN, r, rt);
+  }
+  cloud_water_autoconversion<double>(rho, inc.qc, inc.nc, r, rt);
+  if (has_c) r.nc_selfcollect_tend = 0.0;
+  cloud_rain_accretion<double>(inc.qc, inc.nc, inc.qr, r, rt);
+  rain_self_collection<double>(rho, inc.qr, inc.nr, r, rt, [&] { return rain_size; });
+  back_to_cell_average<double>(cld_l, cld_r, cld_i, r);
+
+  water_conservation<double>(s.qc, s.qr, s.qi, dt, r);
+  number_conservation<double>(s.nc, s.nr, s.ni, dt, r);
+  ice_supersat_conservation(r, cld_i, s.qv, qvsi, m_div(s.th, inv_exner), dt);
+  prevent_liq_supersaturation(pres, T, s.qv, dt, r, err);
+  update_prognostics(r, inv_exner, predictNc, prescribedCCN, wet, dt, rho_qm_cloud, inv_rho, s);
+
+  in.qv2qi_depos_tend[o] = r.qv2qi_vapdep_tend - r.qi2qv_sublim_tend + r.qv2qi_nucleat_tend;
+  in.precip_total_tend[o] = r.qc2qr_accret_tend + r.qc2qr_autoconv_tend + r.qc2qr_ice_shed_tend + r.qc2qi_collect_tend;
+  in.nevapr[o] = r.qi2qv_sublim_tend + r.qr2qv_evap_tend;
+  in.vap_ice_exchange[o] = r.qv2qi_vapdep_tend - r.qi2qv_sublim_tend + r.qv2qi_nucleat_tend;
+  in.vap_liq_exchange[o] = -r.qr2qv_evap_tend;
+  in.liq_ice_exchange[o] = r.qc2qi_hetero_freeze_tend + r.qr2qi_immers_freeze_tend - r.qi2qr_melt_tend +
+                           r.qc2qi_berg_tend + r.qc2qi_collect_tend + r.qr2qi_collect_tend;
+
+  hydro |= clip_to_vapour(s, inv_exner);
+  double ni_incld = m_div(s.ni, cld_i);
+  impose_max_total_ni(ni_incld, rt.max_total_ni, inv_rho);
+  s.ni = ni_incld * cld_i;
+  in.qc[o] = s.qc; in.nc[o] = s.nc; in.qr[o] = s.qr; in.nr[o] = s.nr;
+  in.qi[o] = s.qi; in.qm[o] = s.qm; in.ni[o] = s.ni; in.bm[o] = s.bm;
+  in.qv[o] = s.qv; in.th[o] = s.th;
+}
+
+/* p3_main_part2 of one level without hydrometeors, where ice nucleation is
+ * the only process that can have a rate: the same operations that
+ * part2_level_f64 leaves once every other rate is +0 (its limiters do not
+ * engage, its sums add zeros). */
+__device__ __forceinline__ void part2_nucleation_f64(const Inst& in, const int64_t o, const int k,
+                                                     const double* __restrict__ sm, const int S,
+                                                     const KParams<double>& kp, const double dt, const double inv_dt,
+                                                     bool& hydro) {
+  const RuntimeDev& rt = kp.rt;
+  const double T = sm[A_TATM * S + k], qvssi = sm[A_QVSSI * S + k], qvsi = sm[A_QVSI * S + k];
+  const double inv_rho = m_div(1.0, sm[A_RHO * S + k]);
+  Rates<double> r;
+  r.zero();
+  ice_nucleation<double>(T, inv_rho, 0.0, in.ni_activated[o], qvssi, inv_dt, in.predictNc != 0, in.prescribedCCN != 0,
+                         r, rt);
+  if (!dnz(r.ni_nucleat_tend) && !dnz(r.qv2qi_nucleat_tend)) return;
+  State s;
+  s.qc = s.nc = s.qr = s.nr = s.qm = s.bm = 0.0;
+  s.qv = in.qv[o];
+  s.th = in.th[o];
+  const double cld_i = in.cld_frac_i[o], inv_exner = in.inv_exner[o];
+  ice_supersat_conservation(r, cld_i, s.qv, qvsi, m_div(s.th, inv_exner), dt);
+  const double q = r.qv2qi_nucleat_tend;
+  s.qi = q * dt;
+  s.ni = r.ni_nucleat_tend * dt;
+  s.qv = fma(-q, dt, s.qv);
+  s.th = fma(inv_exner * (q * (C::LatVap + C::LatIce) * C::INV_CP), dt, s.th);
+  in.qv2qi_depos_tend[o] = q;
+  in.vap_ice_exchange[o] = q;
+  hydro |= clip_to_vapour(s, inv_exner);
+  double ni_incld = m_div(s.ni, cld_i);
+  impose_max_total_ni(ni_incld, rt.max_total_ni, inv_rho);
+  in.qi[o] = s.qi;
+  in.ni[o] = ni_incld * cld_i;
+  in.qv[o] = s.qv;
+  in.th[o] = s.th;
+}
+
+/* K1 of one column in the FP64 form: p3_main_init, p3_main_part1,
+ * p3_main_part2.
+ *
+ * What bounds it: the FP64 pipe, through the library functions (pow 1,499
+ * cycles of an SM, log 516, tanh 429, exp 274), whose bits ice sedimentation
+ * carries into every later result, so they stay the library's.  They are
+ * therefore evaluated only on the levels whose processes read them.  A first
+ * pass over all levels does what part1 does without saturation (the fall-speed
+ * factors, which only sedimentation reads on these levels, in fixed point)
+ * and sorts the levels into three classes:
+ *   - with a hydrometeor: saturation, the rest of part1 and part2, on a list,
+ *     so that a group's lanes hold LANES such levels and not the few of them
+ *     among LANES consecutive ones;
+ *   - without, cold, where the supersaturation over ice (in FP32, good to
+ *     1e-4) is near the nucleation threshold or above, or so near the -0.05 of
+ *     the early exit that FP32 cannot decide it: exact saturation over ice and
+ *     nucleation, on a second list;
+ *   - the rest: no process has a rate there.
+ * At 21,600 x 128: 6.9 -> 3.4 ms, at 64 x 72: 325 -> 127 us, the state bit for
+ * bit the same.  Of the 3.4 ms the FP64 pipe is busy 68 %; instruction fetch is
+ * the largest stall besides it. */
+template <int LANES>
+__device__ void p3_part12_f64(const Inst& in, const int col, const KParams<double>& kp, const Tabs<double>& tb,
+                              double* __restrict__ sm, uint32_t& err) {
+  const RuntimeDev& rt = kp.rt;
+  const FixTables* const ft = kp.fix;
+  const unsigned mask = group_mask<LANES>();
+  const int lane = threadIdx.x & (LANES - 1);
+  const int nk = in.nlev;
+  const int S = kp.sm_stride;
+  const int64_t co = int64_t(col) * in.ld;
+  const int64_t ci = int64_t(col) * in.ld_int;
+  const double dt = in.dt;
+  const double inv_dt = m_div(1.0, dt);
+  const bool predictNc = in.predictNc != 0, prescribedCCN = in.prescribedCCN != 0;
+  const bool do_ice = rt.do_ice_production != 0;
+#define SMA(a, k) sm[(a)*S + (k)]
+  /* level lists: hydrometeor levels from the front, nucleation levels from
+   * position nk (2 nk 16-bit entries in one slot of S doubles) */
+  uint16_t* const list = reinterpret_cast<uint16_t*>(&SMA(A_LIST, 0));
+  __syncwarp(mask); /* every lane is done with the last column's arrays */
+  int n_hyd = 0, n_nuc = 0;
+  const unsigned below = (1u << (threadIdx.x & 31u)) - 1u;
+
+  /* ---------------- p3_main_init, part1 without saturation ---------------- */
+  bool nucl = false, hydro = false;
+  for (int base = 0; base < nk; base += LANES) {
+    const int k = base + lane;
+    bool is_hyd = false, is_nuc = false;
+    if (k < nk) {
+      const int64_t o = co + k;
+      const double inv_exner = in.inv_exner[o];
+      double th = in.th[o];
+      const double dz = in.dz[o];
+      double qv = dmax0(in.qv[o]);
+      const double pres = in.pres[o];
+      const double dpres = in.dpres[o];
+      const double qc = in.qc[o], qr = in.qr[o], qi = in.qi[o];
+
+      in.diag_eff_radius_qc[o] = 10.e-6;
+      in.diag_eff_radius_qi[o] = 25.e-6;
+      in.diag_eff_radius_qr[o] = 500.e-6;
+      in.rho_qi[o] = 0;
+      in.qv2qi_depos_tend[o] = 0;
+      in.precip_total_tend[o] = 0;
+      in.nevapr[o] = 0;
+      in.liq_ice_exchange[o] = 0;
+      in.vap_liq_exchange[o] = 0;
+      in.vap_ice_exchange[o] = 0;
+
+      const double exner = m_div(1.0, inv_exner);
+      double T = th * exner;
+      if (dbits(T) <= 0 || dbits(T) > kInfBits) err |= kErrNumeric;
+      const double rho = m_div(m_div(dpres, dz), C::gravit);
+      const double inv_rho = m_div(1.0, rho);
+      /* fall-speed factors; rhofaci is rhofacr times a constant */
+      constexpr int64_t k54 = 4980620899901579264ll; /* 0.54, Q63 */
+      constexpr int64_t k50 = 1ll << 62;
+      const double rhofacr = pow_fix(C::RHO_1000MB * inv_rho, k54, .54, ft);
+      const double visc = m_div(1.496e-6 * (T * pow_fix(T, k50, .5, ft)), T + 120.0);
+      SMA(A_RHO, k) = rho;
+      SMA(A_RHOFACR, k) = rhofacr;
+      SMA(A_RHOFACI, k) = rhofacr * kRhofaciOverR;
+      SMA(A_ACN, k) = m_div(C::gravit * C::RHO_H2O, 18.0 * visc);
+
+      is_hyd = dge(qc, C::QSMALL) || dge(qr, C::QSMALL) || dge(qi, C::QSMALL);
+      if (is_hyd) {
+        in.qv[o] = qv;
+        SMA(A_TATM, k) = T;
+      } else {
+        if (dlt(T, C::T_zerodegc)) {
+          /* supersaturation over ice in FP32 */
+          const float tf = float(T);
+          const float e = __expf(9.550426f - 5723.265f / tf + 3.53068f * __logf(tf) - 0.00728332f * tf);
+          const float ss = float(qv) * float(dmax_c(pres, 1.e-3)) / (float(C::ep_2) * e) - 1.0f;
+          const bool known = dgt(T, 150.0) && (ss < -0.051f || (ss > -0.049f && (ss < 0.049f || dgt(T, C::Tmelt - 14.9))));
+          is_nuc = !known;
+          nucl = nucl || (known && ss > -0.05f);
+          SMA(A_QVSSI, k) = qv; /* the vapour that the exact supersaturation is formed with */
+        }
+        /* a species below qsmall goes to vapour; a +0 moves nothing */
+        bool th_changed = false;
+        if (dnz(qc)) {
+          qv = qv + qc;
+          th = th - inv_exner * qc * C::LatVap * C::INV_CP;
+          th_changed = true;
+        }
+        if (dnz(qr)) {
+          qv = qv + qr;
+          th = th - inv_exner * qr * C::LatVap * C::INV_CP;
+          th_changed = true;
+        }
+        if (dnz(qi)) {
+          qv = qv + qi;
+          th = th - inv_exner * qi * (C::LatVap + C::LatIce) * C::INV_CP;
+          th_changed = true;
+        }
+        if (is_nuc) SMA(A_QVSI, k) = T; /* and the temperature */
+        if (th_changed) T = th * exner;
+        in.qc[o] = 0; in.nc[o] = 0; in.qr[o] = 0; in.nr[o] = 0;
+        in.qi[o] = 0; in.ni[o] = 0; in.qm[o] = 0; in.bm[o] = 0;
+        in.qv[o] = qv; in.th[o] = th;
+        SMA(A_TATM, k) = T;
+      }
+    }
+    const unsigned b_hyd = __ballot_sync(mask, is_hyd), b_nuc = __ballot_sync(mask, is_nuc);
+    if (is_hyd) list[n_hyd + __popc(b_hyd & below & mask)] = uint16_t(k);
+    if (is_nuc) list[nk + n_nuc + __popc(b_nuc & below & mask)] = uint16_t(k);
+    n_hyd += __popc(b_hyd & mask);
+    n_nuc += __popc(b_nuc & mask);
+  }
+  for (int k = lane; k <= nk; k += LANES) {
+    in.precip_liq_flux[ci + k] = 0;
+    in.precip_ice_flux[ci + k] = 0;
+  }
+  if (lane == 0) {
+    in.precip_liq_surf[col] = 0;
+    in.precip_ice_surf[col] = 0;
+  }
+  __syncwarp(mask);
+
+  /* ---------------- saturation over ice of the nucleation levels ---------------- */
+  for (int j = lane; j < n_nuc; j += LANES) {
+    const int k = list[nk + j];
+    const double T = SMA(A_QVSI, k);
+    const double qvsi = m_div(C::ep_2 * svp_ice(T, m_log(T)), vmax(in.pres[co + k], 1.e-3));
+    const double qvssi = m_div(SMA(A_QVSSI, k), qvsi) - 1;
+    SMA(A_QVSI, k) = qvsi;
+    SMA(A_QVSSI, k) = qvssi;
+    if (dge_neg(qvssi, -0.05)) nucl = true;
+  }
+  /* ---------------- the rest of part1 on the hydrometeor levels ---------------- */
+  for (int j = lane; j < n_hyd; j += LANES) {
+    const int k = list[j];
+    const int64_t o = co + k;
+    const double inv_exner = in.inv_exner[o];
+    const double exner = m_div(1.0, inv_exner);
+    double th = in.th[o], qv = in.qv[o], T = SMA(A_TATM, k);
+    double qc = in.qc[o], nc = in.nc[o], qr = in.qr[o], nr = in.nr[o];
+    double qi = in.qi[o], ni = in.ni[o], qm = in.qm[o], bm = in.bm[o];
+    const double p = vmax(in.pres[o], 1.e-3);
+    const bool cold = T < C::Tmelt;
+    const double logt = m_log(T);
+    const double qvsl = m_div(C::ep_2 * svp_liquid(T, logt), p);
+    const double qvsi = cold ? m_div(C::ep_2 * svp_ice(T, logt), p) : qvsl;
+    const double qvssi = m_div(qv, qvsi) - 1;
+    if (dlt(T, C::T_zerodegc) && dge_neg(qvssi, -0.05)) nucl = true;
+
+    /* A species below qsmall goes to vapour; a +0 moves nothing, so its FP64
+     * updates are skipped (bitwise the same result). */
+    const double T_before = T;
+    bool th_changed = false;
+    if (dlt(qc, C::QSMALL)) {
+      if (dnz(qc)) {
+        qv = qv + qc;
+        th = th - inv_exner * qc * C::LatVap * C::INV_CP;
+        th_changed = true;
+      }
+      qc = 0;
+      nc = 0;
+    } else {
+      hydro = true;
+      if (prescribedCCN) {
+        nc = vmax(nc, m_div(rt.spa_ccn_to_nc_factor * in.nccn[o], m_div(1.0, in.cld_frac_l[o])));
+      } else if (predictNc) {
+        nc = dmax0(nc + in.nc_nuceat_tend[o] * dt);
+      } else {
+        nc = C::NCCNST * m_div(1.0, SMA(A_RHO, k));
+      }
+    }
+    if (dlt(qr, C::QSMALL)) {
+      if (dnz(qr)) {
+        qv = qv + qr;
+        th = th - inv_exner * qr * C::LatVap * C::INV_CP;
+        th_changed = true;
+      }
+      qr = 0;
+      nr = 0;
+    } else {
+      hydro = true;
+    }
+    if (dlt(qi, C::QSMALL) || (dlt(qi, 1.e-8) && dlt_neg(qvssi, -0.1))) {
+      if (dnz(qi)) {
+        qv = qv + qi;
+        th = th - inv_exner * qi * (C::LatVap + C::LatIce) * C::INV_CP;
+        th_changed = true;
+      }
+      qi = 0; ni = 0; qm = 0; bm = 0;
+    } else {
+      hydro = true;
+    }
+    if (dge(qi, C::QSMALL) && dlt(qi, 1.e-8) && dge(T, C::T_zerodegc)) {
+      qr = qr + qi;
+      th = th - inv_exner * qi * C::LatIce * C::INV_CP;
+      th_changed = true;
+      qi = 0; ni = 0; qm = 0; bm = 0;
+    }
+    if (th_changed) {
+      T = th * exner;
+      if (dge(qc, C::QSMALL) && dge(qi, C::QSMALL)) {
+        /* part2 reads acn at the temperature before these changes */
+        const double dum = m_div(1.496e-6 * m_pow(T_before, 1.5), T_before + 120.0);
+        SMA(A_ACN, k) = -m_div(C::gravit * C::RHO_H2O, 18.0 * dum);
+      }
+    }
+    in.qc[o] = qc; in.nc[o] = nc; in.qr[o] = qr; in.nr[o] = nr;
+    in.qi[o] = qi; in.ni[o] = ni; in.qm[o] = qm; in.bm[o] = bm;
+    in.qv[o] = qv; in.th[o] = th;
+    SMA(A_TATM, k) = T;
+    SMA(A_QVSL, k) = qvsl;
+    SMA(A_QVSI, k) = qvsi;
+    SMA(A_QVSSI, k) = qvssi;
+  }
+  if (!group_any<LANES>(mask, nucl || hydro)) {
+    if (lane == 0) in.cflag[col] = 0;
+    return;
+  }
+
+  /* ---------------- p3_main_part2 ---------------- */
+  /* a lane owns the list positions it had above, so only its own stores are
+   * read back */
+  hydro = false;
+  for (int j = lane; j < n_hyd; j += LANES)
+    part2_level_f64(in, co + list[j], list[j], sm, S, kp, tb, dt, inv_dt, hydro, err);
+  if (do_ice) {
+    for (int j = lane; j < n_nuc; j += LANES)
+      part2_nucleation_f64(in, co + list[nk + j], list[nk + j], sm, S, kp, dt, inv_dt, hydro);
+  }
+  if (!group_any<LANES>(mask, hydro)) {
+    if (lane == 0) in.cflag[col] = 0;
+    return;
+  }
+  __syncwarp(mask);
+  for (int k = lane; k < nk; k += LANES) {
+    scr_at(in, S_TATM, col)[k] = SMA(A_TATM, k);
+    scr_at(in, S_RHO, col)[k] = SMA(A_RHO, k);
+    scr_at(in, S_RHOFACR, col)[k] = SMA(A_RHOFACR, k);
+    scr_at(in, S_RHOFACI, col)[k] = SMA(A_RHOFACI, k);
+    scr_at(in, S_ACN, col)[k] = m_fabs(SMA(A_ACN, k));
+  }
+  if (lane == 0) in.cflag[col] = 1;
+#undef SMA
+}
+
+/* K1 of one column in the FP32-bulk form: p3_main_init, p3_main_part1,
+ * p3_main_part2. */
+template <int LANES>
+__device__ void p3_part12_bulk(const Inst& in, const int col, const KParams<float>& kp, const Tabs<float>& tb,
+                               double* __restrict__ sm, uint32_t& err) {
   const RuntimeDev& rt = kp.rt;
   const unsigned mask = group_mask<LANES>();
   const int lane = threadIdx.x & (LANES - 1);
@@ -535,7 +1035,6 @@ __device__ void p3_part12(const Inst& in, const int col, const KParams<TR>& kp, 
   const double dt = in.dt;
   const double inv_dt = 1 / dt;
   const bool predictNc = in.predictNc != 0, prescribedCCN = in.prescribedCCN != 0;
-  const bool do_ice = rt.do_ice_production != 0;
 #define SMA(a, k) sm[(a)*S + (k)]
   /* FP32-bulk: the float-valued slots (rho, fall-speed factors, acn) hold
    * floats in the first half of their slot */
@@ -566,45 +1065,28 @@ __device__ void p3_part12(const Inst& in, const int col, const KParams<TR>& kp, 
     in.vap_liq_exchange[o] = 0;
     in.vap_ice_exchange[o] = 0;
 
-    double rho, inv_rho, qvsl, qvsi, qvssi, ccn_nc;
-    TR rho_t, inv_rho_t;
-    const double exner = kF64 ? m_div(1.0, inv_exner) : rcp_newton1(inv_exner);
+    const double exner = rcp_newton1(inv_exner);
     double T = th * exner;
     qv = dmax0(qv);
-    if constexpr (kF64) {
-      const double inv_cld_l = m_div(1.0, cld_l);
-      rho = m_div(m_div(dpres, dz), C::gravit);
-      inv_rho = m_div(1.0, rho);
-      rho_t = rho;
-      inv_rho_t = inv_rho;
-      qvsl = qv_sat_dry(T, pres, false, err);
-      qvsi = qv_sat_dry(T, pres, true, err);
-      qvssi = m_div(qv, qvsi) - 1;
-      ccn_nc = m_div(rt.spa_ccn_to_nc_factor * in.nccn[o], inv_cld_l);
-    } else {
-      /* FP32-bulk: rho and 1/rho only feed rates, fall speeds and fluxes
-       * (the sedimentation's FP64 coefficient is g / dpres), so they are
-       * FP32 and kept as floats in the shared slots and the hand-over; one
-       * Newton reciprocal of the pressure, times ep_2, shared by both
-       * saturation ratios (and kept for part2's melting departure and
-       * supersaturation limiter); the supersaturation ratio (threshold and
-       * rate input) in FP32 */
-      const float rho_f = float(dpres) / (float(dz) * float(C::gravit));
-      rho_t = rho_f;
-      rho = f2d(rho_f);
-      inv_rho_t = 1.0f / rho_f;
-      inv_rho = f2d(inv_rho_t);
-      const double ep_inv_p = C::ep_2 * rcp_newton1(dmax_c(pres, 1.e-3));
-      SMA(A_EPINVP, k) = ep_inv_p;
-      qvsl = svp_tabulated(rt.svp_tab, T, false, err) * ep_inv_p;
-      qvsi = svp_tabulated(rt.svp_tab, T, true, err) * ep_inv_p;
-      qvssi = f2d(float(qv) / float(qvsi) - 1.0f);
-      ccn_nc = rt.spa_ccn_to_nc_factor * in.nccn[o] * cld_l;
-    }
-    const TR rhofacr = m_pow(TR(C::RHO_1000MB) * inv_rho_t, TR(.54));
-    const TR rhofaci = m_pow(TR(C::RHO_600MB) * inv_rho_t, TR(.54));
-    const TR dum = m_div(TR(1.496e-6) * m_pow(TR(T), TR(1.5)), TR(T) + TR(120));
-    const TR acn = m_div(TR(C::gravit) * TR(C::RHO_H2O), TR(18) * dum);
+    /* rho and 1/rho only feed rates, fall speeds and fluxes (the
+     * sedimentation's FP64 coefficient is g / dpres), so they are FP32 and
+     * kept as floats in the shared slots and the hand-over; one Newton
+     * reciprocal of the pressure, times ep_2, shared by both saturation ratios
+     * (and kept for part2's melting departure and supersaturation limiter);
+     * the supersaturation ratio (threshold and rate input) in FP32 */
+    const float rho_t = float(dpres) / (float(dz) * float(C::gravit));
+    const float inv_rho_t = 1.0f / rho_t;
+    const double inv_rho = f2d(inv_rho_t);
+    const double ep_inv_p = C::ep_2 * rcp_newton1(dmax_c(pres, 1.e-3));
+    SMA(A_EPINVP, k) = ep_inv_p;
+    const double qvsl = svp_tabulated(rt.svp_tab, T, false, err) * ep_inv_p;
+    const double qvsi = svp_tabulated(rt.svp_tab, T, true, err) * ep_inv_p;
+    const double qvssi = f2d(float(qv) / float(qvsi) - 1.0f);
+    const double ccn_nc = rt.spa_ccn_to_nc_factor * in.nccn[o] * cld_l;
+    const float rhofacr = m_pow(float(C::RHO_1000MB) * inv_rho_t, float(.54));
+    const float rhofaci = m_pow(float(C::RHO_600MB) * inv_rho_t, float(.54));
+    const float dum = float(1.496e-6) * m_pow(float(T), float(1.5)) / (float(T) + float(120));
+    const float acn = float(C::gravit) * float(C::RHO_H2O) / (float(18) * dum);
     if (dlt(T, C::T_zerodegc) && dge_neg(qvssi, -0.05)) nucl = true;
 
     /* A species below qsmall goes to vapour; a +0 moves nothing, so its FP64
@@ -661,17 +1143,10 @@ __device__ void p3_part12(const Inst& in, const int col, const KParams<TR>& kp, 
     in.qi[o] = qi; in.ni[o] = ni; in.qm[o] = qm; in.bm[o] = bm;
     in.qv[o] = qv; in.th[o] = th;
     SMA(A_TATM, k) = T;
-    if constexpr (kF64) {
-      SMA(A_RHO, k) = rho;
-      SMA(A_RHOFACR, k) = rhofacr;
-      SMA(A_RHOFACI, k) = rhofaci;
-      SMA(A_ACN, k) = acn;
-    } else {
-      SMF(A_RHO)[k] = rho_t;
-      SMF(A_RHOFACR)[k] = rhofacr;
-      SMF(A_RHOFACI)[k] = rhofaci;
-      SMF(A_ACN)[k] = acn;
-    }
+    SMF(A_RHO)[k] = rho_t;
+    SMF(A_RHOFACR)[k] = rhofacr;
+    SMF(A_RHOFACI)[k] = rhofaci;
+    SMF(A_ACN)[k] = acn;
     SMA(A_QVSL, k) = qvsl;
     SMA(A_QVSI, k) = qvsi;
     SMA(A_QVSSI, k) = qvssi;
@@ -691,184 +1166,19 @@ __device__ void p3_part12(const Inst& in, const int col, const KParams<TR>& kp, 
 
   /* ---------------- phase 2: p3_main_part2 ---------------- */
   hydro = false;
-  if constexpr (!kF64) {
-    const float dtf = float(dt), inv_dtf = float(inv_dt);
-    for (int k = lane; k < nk; k += LANES)
-      part2_level_bulk(in, co + k, k, sm, S, kp, tb, esat0, dtf, inv_dtf, hydro, err);
-  } else {
-  for (int k = lane; k < nk; k += LANES) {
-    const int64_t o = co + k;
-    State s;
-    s.qc = in.qc[o]; s.nc = in.nc[o]; s.qr = in.qr[o]; s.nr = in.nr[o];
-    s.qi = in.qi[o]; s.qm = in.qm[o]; s.ni = in.ni[o]; s.bm = in.bm[o];
-    s.qv = in.qv[o]; s.th = in.th[o];
-    const double T = SMA(A_TATM, k);
-    const double qvssi = SMA(A_QVSSI, k);
-    if (dlt(s.qc, C::QSMALL) && dlt(s.qr, C::QSMALL) && dlt(s.qi, C::QSMALL) && dlt(T, C::T_zerodegc) &&
-        dlt_neg(qvssi, -0.05))
-      continue;
-
-    const double pres = in.pres[o];
-    const double cld_i = in.cld_frac_i[o], cld_l = in.cld_frac_l[o], cld_r = in.cld_frac_r[o];
-    const double inv_exner = in.inv_exner[o];
-    const double qvsl = SMA(A_QVSL, k), qvsi = SMA(A_QVSI, k);
-    const double rho = SMA(A_RHO, k);
-    const double inv_rho = m_div(1.0, rho);
-    const double rhofaci = SMA(A_RHOFACI, k);
-    const double acn = SMA(A_ACN, k);
-    Incld inc;
-    calc_incloud(s.qc, s.qr, s.qi, s.qm, s.nc, s.nr, s.ni, s.bm, m_div(1.0, cld_l), m_div(1.0, cld_i),
-                 m_div(1.0, cld_r), inc);
-
-    Rates<TR> r;
-    r.zero();
-    PhysVars<TR> v;
-    v.mu = v.dv = v.sc = v.dqsdt = v.dqsidt = v.ab = v.abi = v.kap = v.eii = TR(0);
-    TR tv_fallspd = 0, tv_selfcol = 0, tv_qc2qi = 0, tv_melt = 0, tv_nr = 0, tv_qr2qi = 0,
-       tv_lammax = 0, tv_lammin = 0, tv_vent = 0;
-    TR mu_c = 0, lamc = 0, mu_r = 0, lamr = 0, cdistr = 0, logn0r = 0;
-    TR epsi = 0, epsr = 0, epsi_tot = 0;
-    TR rho_qm_cloud = TR(400);
-    bool wet = false;
-
-    const bool skip_micro = !(dge(inc.qc, C::QSMALL) || dge(inc.qr, C::QSMALL) || dge(inc.qi, C::QSMALL));
-    if (!skip_micro) {
-      get_time_space_phys_variables<TR>(T, pres, rho, qvsl, qvsi, v);
-      {
-        const TR n_in = TR(inc.nc);
-        TR n_out = n_in;
-        get_cloud_dsd2<TR>(TR(inc.qc), n_out, mu_c, rho, lamc);
-        apply_n_adjust(inc.nc, n_in, n_out);
-        s.nc = inc.nc * cld_l;
-      }
-      {
-        const TR n_in = TR(inc.nr);
-        TR n_out = n_in;
-        get_rain_dsd2<TR>(TR(inc.qr), n_out, mu_r, lamr, rt);
-        apply_n_adjust(inc.nr, n_in, n_out);
-        if (dge(inc.qr, C::QSMALL)) {
-          cdistr = m_div(TR(inc.nr), TR(rt.g_mur1));
-          logn0r = m_log10(cdistr) + (mu_r + TR(1)) * m_log10(lamr);
-        }
-        s.nr = inc.nr * cld_r;
-      }
-      impose_max_total_ni(inc.ni, rt.max_total_ni, inv_rho);
-      if (dge(inc.qi, C::QSMALL)) {
-        inc.ni = dmax_c(inc.ni, C::NSMALL);
-        inc.nr = dmax_c(inc.nr, C::NSMALL);
-        const TR rhop = calc_bulk_rho_rime(inc.qi, inc.qm, inc.bm, rt);
-        s.qm = inc.qm * cld_i;
-        s.bm = inc.bm * cld_i;
-        TableIce<TR> ti;
-        lookup_ice<TR>(TR(inc.qi), TR(inc.ni), TR(inc.qm), rhop, ti);
-        TableRain<TR> trn;
-        lookup_rain<TR>(TR(inc.qr), TR(inc.nr), trn);
-        TR ta[4], tc[4];
-        apply_table_ice4<TR>(tb, ti, 0, ta); /* columns 0, 1, 6, 7 */
-        apply_table_ice4<TR>(tb, ti, 4, tc); /* columns 2, 3, 4, 9 */
-        tv_fallspd = ta[1];
-        tv_selfcol = tc[0];
-        tv_qc2qi = tc[1];
-        tv_melt = tc[2];
-        tv_lammax = ta[2];
-        tv_lammin = ta[3];
-        tv_vent = tc[3];
-        if (dge(inc.qr, C::QSMALL)) {
-          tv_nr = apply_table_coll<TR>(0, tb, ti, trn);
-          tv_qr2qi = apply_table_coll<TR>(1, tb, ti, trn);
-        }
-        inc.ni = vmin(inc.ni, tv_lammax * inc.ni);
-        inc.ni = vmax(inc.ni, tv_lammin * inc.ni);
-      }
-      const TR qi_r = inc.qi, qc_r = inc.qc, ni_r = inc.ni, nc_r = inc.nc, qr_r = inc.qr;
-      const double dT0 = T - C::Tmelt;
-      const double dqv0 = m_div(C::ep_2 * esat0, vmax(pres, 1.e-3)) - s.qv;
-      if (do_ice) {
-        ice_cldliq_collection<TR>(rho, T, rhofaci, tv_qc2qi, qi_r, qc_r, ni_r, nc_r, r, rt);
-        ice_rain_collection<TR>(rho, T, rhofaci, logn0r, tv_nr, tv_qr2qi, qi_r, ni_r, qr_r, r, rt);
-        ice_self_collection<TR>(rho, rhofaci, tv_selfcol, v.eii, TR(inc.qm), qi_r, ni_r, r);
-      }
-      ice_melting<TR>(rho, dT0, dqv0, rhofaci, tv_melt, tv_vent, v, qi_r, ni_r, r);
-      if (do_ice) {
-        wet = ice_cldliq_wet_growth<TR>(rho, dT0, dqv0, rhofaci, tv_melt, tv_vent, v, qc_r, qi_r, ni_r, qr_r, r);
-      }
-      /* ice_relaxation_timescale, p3_ice_relaxation_timescale_impl.hpp:9-37 */
-      if (dge(inc.qi, C::QSMALL) && dlt(T, C::Tmelt)) {
-        epsi = ((tv_melt + tv_vent * m_cbrt(v.sc) * m_sqrt(m_div(rhofaci * rho, v.mu))) * TR(2.0) * TR(C::Pi) * rho *
-                v.dv) * ni_r;
-        epsi_tot = epsi_tot + epsi;
-      } else {
-        epsi = TR(0);
-      }
-      rho_qm_cloud = calc_rime_density<TR>(T, rhofaci, tv_fallspd, acn, lamc, mu_c, qc_r, r.qc2qi_collect_tend);
-      if (do_ice) {
-        cldliq_immersion_freezing<TR>(T, lamc, mu_c, nc_r, qc_r, r, rt);
-        rain_immersion_freezing<TR>(T, lamr, mu_r, cdistr, qr_r, r, rt);
-      }
-      /* calc_liq_relaxation_timescale, p3_calc_liq_relaxation_timescale_impl.hpp:13-43 */
-      if (dge(inc.qr, C::QSMALL)) {
-        Table3<TR> t3;
-        lookup3<TR>(mu_r, lamr, rt, t3);
-        epsr = TR(2) * TR(C::Pi) * cdistr * rho * v.dv *
-               (m_div(TR(C::f1r) * TR(rt.g_mur2), lamr) +
-                TR(C::f2r) * m_sqrt(m_div(rho, v.mu)) * m_cbrt(v.sc) * apply_table3<TR>(tb, tb.revap, t3));
-      }
-      evaporate_rain(inc.qr, inc.qc, inc.nr, inc.qi, cld_l, cld_r, s.qv, in.qv_prev[o], qvsl, qvsi, v.ab, v.abi,
-                     epsr, epsi_tot, T, in.t_prev[o], v.dqsdt, dt, r.qr2qv_evap_tend, r.nr_evap_tend);
-      if (do_ice) {
-        ice_deposition_sublimation(inc.qi, inc.ni, T, qvsl, qvsi, epsi, v.abi, s.qv, inv_dt, r.qv2qi_vapdep_tend,
-                                   r.qi2qv_sublim_tend, r.ni_sublim_tend, r.qc2qi_berg_tend);
-      }
-    }
-    if (do_ice) {
-      ice_nucleation<TR>(T, inv_rho, s.ni, in.ni_activated[o], qvssi, inv_dt, predictNc, prescribedCCN, r, rt);
-    }
-    cloud_water_autoconversion<TR>(rho, inc.qc, inc.nc, r, rt);
-    if (dge(inc.qc, C::QSMALL)) r.nc_selfcollect_tend = TR(0);
-    cloud_rain_accretion<TR>(inc.qc, inc.nc, inc.qr, r, rt);
-    rain_self_collection<TR>(rho, inc.qr, inc.nr, r, rt);
-    back_to_cell_average<TR>(cld_l, cld_r, cld_i, r);
-
-    water_conservation<double>(s.qc, s.qr, s.qi, dt, r);
-    number_conservation<double>(s.nc, s.nr, s.ni, dt, r);
-    ice_supersat_conservation(r, cld_i, s.qv, qvsi, m_div(s.th, inv_exner), dt);
-    prevent_liq_supersaturation(pres, T, s.qv, dt, r, err);
-    update_prognostics(r, inv_exner, predictNc, prescribedCCN, wet, dt, rho_qm_cloud, inv_rho, s);
-
-    in.qv2qi_depos_tend[o] = r.qv2qi_vapdep_tend - r.qi2qv_sublim_tend + r.qv2qi_nucleat_tend;
-    in.precip_total_tend[o] = r.qc2qr_accret_tend + r.qc2qr_autoconv_tend + r.qc2qr_ice_shed_tend + r.qc2qi_collect_tend;
-    in.nevapr[o] = r.qi2qv_sublim_tend + r.qr2qv_evap_tend;
-    in.vap_ice_exchange[o] = r.qv2qi_vapdep_tend - r.qi2qv_sublim_tend + r.qv2qi_nucleat_tend;
-    in.vap_liq_exchange[o] = -r.qr2qv_evap_tend;
-    in.liq_ice_exchange[o] = r.qc2qi_hetero_freeze_tend + r.qr2qi_immers_freeze_tend - r.qi2qr_melt_tend +
-                             r.qc2qi_berg_tend + r.qc2qi_collect_tend + r.qr2qi_collect_tend;
-
-    hydro |= clip_to_vapour(s, inv_exner);
-    double ni_incld = m_div(s.ni, cld_i);
-    impose_max_total_ni(ni_incld, rt.max_total_ni, inv_rho);
-    s.ni = ni_incld * cld_i;
-    in.qc[o] = s.qc; in.nc[o] = s.nc; in.qr[o] = s.qr; in.nr[o] = s.nr;
-    in.qi[o] = s.qi; in.qm[o] = s.qm; in.ni[o] = s.ni; in.bm[o] = s.bm;
-    in.qv[o] = s.qv; in.th[o] = s.th;
-  }
-  }
+  const float dtf = float(dt), inv_dtf = float(inv_dt);
+  for (int k = lane; k < nk; k += LANES)
+    part2_level_bulk(in, co + k, k, sm, S, kp, tb, dtf, inv_dtf, hydro, err);
   if (!group_any<LANES>(mask, hydro)) {
     if (lane == 0) in.cflag[col] = 0;
     return;
   }
   for (int k = lane; k < nk; k += LANES) {
     scr_at(in, S_TATM, col)[k] = SMA(A_TATM, k);
-    if constexpr (kF64) {
-      scr_at(in, S_RHO, col)[k] = SMA(A_RHO, k);
-      scr_at(in, S_RHOFACR, col)[k] = SMA(A_RHOFACR, k);
-      scr_at(in, S_RHOFACI, col)[k] = SMA(A_RHOFACI, k);
-      scr_at(in, S_ACN, col)[k] = SMA(A_ACN, k);
-    } else {
-      scr_f(in, S_RHO, col)[k] = SMF(A_RHO)[k];
-      scr_f(in, S_RHOFACR, col)[k] = SMF(A_RHOFACR)[k];
-      scr_f(in, S_RHOFACI, col)[k] = SMF(A_RHOFACI)[k];
-      scr_f(in, S_ACN, col)[k] = SMF(A_ACN)[k];
-    }
+    scr_f(in, S_RHO, col)[k] = SMF(A_RHO)[k];
+    scr_f(in, S_RHOFACR, col)[k] = SMF(A_RHOFACR)[k];
+    scr_f(in, S_RHOFACI, col)[k] = SMF(A_RHOFACI)[k];
+    scr_f(in, S_ACN, col)[k] = SMF(A_ACN)[k];
   }
   if (lane == 0) in.cflag[col] = 1;
 #undef SMA
@@ -1876,13 +2186,14 @@ __global__ void __launch_bounds__(256, sizeof(TR) == sizeof(float) ? 2 : 1)
   }
   const int g_in_block = threadIdx.x / LANES;
   double* sm = reinterpret_cast<double*>(base) + size_t(g_in_block) * A_NARR * kp.sm_stride;
-  /* liquid saturation vapour pressure at 0 C (qsat0 of ice_melting and
-   * ice_cldliq_wet_growth), evaluated once */
-  const double esat0 = murphy_koop_svp<double>(C::Tmelt, false, err);
   for_each_work<LANES>(kp.wctr ? kp.wctr + 0 : nullptr, kp.nwork, kp.groups_per_block, [&](int w) {
     int col;
     const Inst& in = work_inst(inst0, kp, w, col);
-    p3_part12<TR, LANES>(in, col, kp, tb, sm, esat0, err);
+    if constexpr (sizeof(TR) == sizeof(double)) {
+      p3_part12_f64<LANES>(in, col, kp, tb, sm, err);
+    } else {
+      p3_part12_bulk<LANES>(in, col, kp, tb, sm, err);
+    }
   });
   if (err) atomicOr(kp.err, err);
 }

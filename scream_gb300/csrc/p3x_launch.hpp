@@ -153,6 +153,10 @@ struct EamPtrs {
 cudaError_t launch_eam(const EamPtrs& p, int ncol, int nlev, int64_t ld, int64_t ld_int, bool post, double dt,
                        cudaStream_t st);
 
+/* Murphy-Koop vapour pressure over liquid at 0 C, evaluated on the device
+ * (synchronous). */
+cudaError_t saturation_at_melting(double* out);
+
 cudaError_t launch_selftest(unsigned long long* mismatches_d, cudaStream_t st);
 
 /* Fields of the column mass / energy conservation check (device pointers;

@@ -498,11 +498,12 @@ __device__ __forceinline__ void lookup_ice(TR qi, TR ni, TR qm, TR rhop, TableIc
 }
 
 /* lookup_rain, p3_table_ice_impl.hpp:140-173 */
-template <class TR>
-__device__ __forceinline__ void lookup_rain(TR qr, TR nr, TableRain<TR>& tab) {
+/* size: (qr / (pi rho_w nr))^(1/3), evaluated where it is read */
+template <class TR, class Size>
+__device__ __forceinline__ void lookup_rain(TR qr, TR nr, TableRain<TR>& tab, Size&& size) {
   const bool gt_small = qr > TR(C::QSMALL) && nr > TR(0.0);
   TR dumlr = TR(1);
-  if (gt_small) dumlr = m_cbrt(m_div(qr, TR(C::Pi) * TR(C::RHO_H2O) * nr));
+  if (gt_small) dumlr = size();
   tab.dum3 = (m_log10(TR(1) * dumlr) + TR(5)) * TR(10.70415);
   tab.dumj = table_index(tab.dum3, kRcollsize);
   tab.dum3 = vmin(tab.dum3, TR(kRcollsize));
@@ -859,12 +860,13 @@ __device__ __forceinline__ void ice_self_collection(TR rho, TR rhofaci, TR tv, T
 /* ice_melting, p3/impl/p3_ice_melting_impl.hpp:10-53 (max(...,0) inside the branch) */
 /* The departures dT0 = T - T_0C and dqv0 = qsat(T_0C) - qv are formed in FP64
  * by the caller (small differences of large numbers near the melting point). */
-template <class TR>
-__device__ __forceinline__ void ice_melting(TR rho, double dT0, double dqv0, TR rhofaci, TR tv_melt,
-                                            TR tv_vent, const PhysVars<TR>& v, TR qi_incld,
-                                            TR ni_incld, Rates<TR>& r) {
+/* vent: tv_melt + tv_vent Sc^(1/3) (rhofaci rho / mu)^(1/2), evaluated where
+ * it is read */
+template <class TR, class Vent>
+__device__ __forceinline__ void ice_melting(TR rho, double dT0, double dqv0, const PhysVars<TR>& v, TR qi_incld,
+                                            TR ni_incld, Rates<TR>& r, Vent&& vent) {
   if (qi_incld >= TR(C::QSMALL) && dpos(dT0)) {
-    TR t = m_div((tv_melt + tv_vent * m_cbrt(v.sc) * m_sqrt(m_div(rhofaci * rho, v.mu))) *
+    TR t = m_div(vent() *
                      (TR(dT0) * v.kap - rho * TR(C::LatVap) * v.dv * TR(dqv0)) * TR(2) * TR(C::Pi),
                  TR(C::LatIce)) *
            ni_incld;
@@ -875,17 +877,16 @@ __device__ __forceinline__ void ice_melting(TR rho, double dT0, double dqv0, TR 
 }
 
 /* ice_cldliq_wet_growth, p3/impl/p3_ice_cldliq_wet_growth_impl.hpp:12-80 */
-template <class TR>
-__device__ __forceinline__ bool ice_cldliq_wet_growth(TR rho, double dT0, double dqv0, TR rhofaci, TR tv_melt,
-                                                      TR tv_vent, const PhysVars<TR>& v,
+template <class TR, class Vent>
+__device__ __forceinline__ bool ice_cldliq_wet_growth(TR rho, double dT0, double dqv0, const PhysVars<TR>& v,
                                                       TR qc_incld, TR qi_incld, TR ni_incld, TR qr_incld,
-                                                      Rates<TR>& r) {
+                                                      Rates<TR>& r, Vent&& vent) {
   const bool t_neg = dneg(dT0);
   const bool any_if = qi_incld >= TR(C::QSMALL) && (qc_incld + qr_incld) >= TR(1.0e-6) && t_neg;
   const bool any_if_col = any_if && (r.qc2qi_collect_tend + r.qr2qi_collect_tend) >= TR(1.0e-10);
   bool wet = false;
   if (any_if) {
-    TR g = m_div((tv_melt + tv_vent * m_cbrt(v.sc) * m_sqrt(m_div(rhofaci * rho, v.mu))) * TR(C::Pi * 2) *
+    TR g = m_div(vent() * TR(C::Pi * 2) *
                      (rho * TR(C::LatVap) * v.dv * TR(dqv0) - TR(dT0) * v.kap),
                  TR(C::LatIce) + TR(C::CpLiq) * TR(dT0)) *
            ni_incld;
@@ -939,11 +940,12 @@ __device__ __forceinline__ TR calc_rime_density(TR T_atm, TR rhofaci, TR tv_fall
  * cdist1 * Gamma(7+mu_c) and cdist1 * Gamma(4+mu_c), with cdist1 =
  * nc/Gamma(mu_c+1) (p3_dsd2_impl.hpp:72), are evaluated as nc times the
  * rising products (1+mu)...(6+mu) and (1+mu)(2+mu)(3+mu). */
-template <class TR>
+/* imm: exp(immersion_freezing_exponent (T_0C - T)), evaluated where it is read */
+template <class TR, class Imm>
 __device__ __forceinline__ void cldliq_immersion_freezing(TR T_atm, TR lamc, TR mu_c, TR nc_incld, TR qc_incld,
-                                                          Rates<TR>& r, const RuntimeDev& rt) {
+                                                          Rates<TR>& r, const RuntimeDev& rt, Imm&& imm) {
   if (qc_incld >= TR(C::QSMALL) && T_atm <= TR(C::T_rainfrz)) {
-    const TR expAimmDt = m_exp(P3X_RTP(TR, immersion_freezing_exponent) * (TR(C::T_zerodegc) - T_atm));
+    const TR expAimmDt = imm();
     const TR inv_lamc = m_div(TR(1), lamc);
     const TR inv_lamc3 = inv_lamc * inv_lamc * inv_lamc;
     const TR p3 = (TR(1) + mu_c) * (TR(2) + mu_c) * (TR(3) + mu_c);
@@ -959,18 +961,19 @@ __device__ __forceinline__ void cldliq_immersion_freezing(TR T_atm, TR lamc, TR 
 }
 
 /* rain_immersion_freezing, p3/impl/p3_rain_imm_freezing_impl.hpp:13-44 */
-template <class TR>
+template <class TR, class Imm>
 __device__ __forceinline__ void rain_immersion_freezing(TR T_atm, TR lamr, TR mu_r, TR cdistr, TR qr_incld,
-                                                        Rates<TR>& r, const RuntimeDev& rt) {
+                                                        Rates<TR>& r, const RuntimeDev& rt, Imm&& imm) {
   if (qr_incld >= TR(C::QSMALL) && T_atm <= TR(C::T_rainfrz)) {
-    const TR e = m_exp(P3X_RTP(TR, immersion_freezing_exponent) * (TR(C::T_zerodegc) - T_atm));
+    const TR e = imm();
     /* mu_r is the runtime constant here: log(Gamma(7+mu_r)) and
      * log(Gamma(4+mu_r)) are precomputed on the host */
     (void)mu_r;
+    const TR log_cdistr = m_log(cdistr), log_lamr = m_log(lamr);
     r.qr2qi_immers_freeze_tend =
-        TR(C::CONS6) * m_exp(m_log(cdistr) + P3X_RTP(TR, lg_mur7) - TR(6.) * m_log(lamr)) * e;
+        TR(C::CONS6) * m_exp(log_cdistr + P3X_RTP(TR, lg_mur7) - TR(6.) * log_lamr) * e;
     r.nr2ni_immers_freeze_tend =
-        TR(C::CONS5) * m_exp(m_log(cdistr) + P3X_RTP(TR, lg_mur4) - TR(3.) * m_log(lamr)) * e;
+        TR(C::CONS5) * m_exp(log_cdistr + P3X_RTP(TR, lg_mur4) - TR(3.) * log_lamr) * e;
   }
 }
 
@@ -1029,11 +1032,12 @@ __device__ __forceinline__ void cloud_rain_accretion(TR qc_incld, TR nc_incld, T
 }
 
 /* rain_self_collection, p3/impl/p3_rain_self_collection_impl.hpp:9-56 */
-template <class TR>
+/* size as in lookup_rain */
+template <class TR, class Size>
 __device__ __forceinline__ void rain_self_collection(TR rho, TR qr_incld, TR nr_incld, Rates<TR>& r,
-                                                     const RuntimeDev& rt) {
+                                                     const RuntimeDev& rt, Size&& size) {
   if (qr_incld >= TR(C::QSMALL)) {
-    const TR dum2 = m_cbrt(m_div(qr_incld, TR(C::Pi) * TR(C::RHO_H2O) * nr_incld));
+    const TR dum2 = size();
     const TR dbr = P3X_RTP(TR, rain_selfcollection_breakup_diameter);
     const TR dum = (dum2 < dbr) ? TR(1) : TR(2) - m_exp(TR(2300) * (dum2 - dbr));
     r.nr_selfcollect_tend = dum * P3X_RTP(TR, rain_selfcollection_prefactor) * nr_incld * qr_incld * rho;
@@ -1111,7 +1115,7 @@ __device__ __forceinline__ void evaporate_rain(double qr_incld, double qc_incld,
     } else {
       const double dt_over_tau = m_div(dt, tau_eff);
       const double w = m_div(-expm1(-dt_over_tau), dt_over_tau);
-      const double equilib = m_div(m_div(-A_c, ab) * tau_eff, tau_r);
+      const double equilib = -m_div(m_div(A_c, ab) * tau_eff, tau_r);
       const double instant = m_div(-ssat_r, ab * tau_r);
       qr2qv_evap_tend = instant * w + equilib * (1 - w);
     }
