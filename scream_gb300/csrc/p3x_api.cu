@@ -34,9 +34,8 @@ struct p3x_context {
   double* d_t3slices = nullptr;
   float* f_t3slices = nullptr;
   double* d_svp = nullptr; /* FP32-bulk saturation table */
-  /* FP64 form: fixed-point tables (p3x_intfp64.cuh), ice-table cells and
-   * their powers of two of sedimentation and part3, Table3 fall speeds */
-  p3x::dev::FixTables* d_fix = nullptr;
+  /* FP64 form: fixed-point ice-table cells and their powers of two of
+   * sedimentation and part3, Table3 fall speeds */
   int64_t *d_cell_sed = nullptr, *d_cell_part3 = nullptr;
   int32_t *d_shift_sed = nullptr, *d_shift_part3 = nullptr;
   double* d_t3sed = nullptr;
@@ -255,7 +254,6 @@ dev::KParams<double> make_kparams<double>(p3x_context* ctx, const dev::RuntimeDe
   kp.revap = ctx->d_revap;
   kp.t3slice = ctx->d_t3slices + size_t(rtd.t3_dumjj - 1) * dev::kT3SliceElems;
   kp.rt.svp_tab = ctx->d_svp;
-  kp.fix = ctx->d_fix;
   kp.cell_sed = ctx->d_cell_sed;
   kp.cell_part3 = ctx->d_cell_part3;
   kp.cell_sed_shift = ctx->d_shift_sed;
@@ -635,14 +633,12 @@ int p3x_context_create(const char* table_file, p3x_context** out, int* info) {
   std::vector<int32_t> shift_sed, shift_part3;
   build_ice_cells(H.ice.data(), kSedCols, cell_sed, shift_sed);
   build_ice_cells(H.ice.data(), kPart3Cols, cell_part3, shift_part3);
-  std::vector<dev::FixTables> fix(1);
-  build_fix_tables(fix[0]);
   std::vector<double> svp;
   build_svp_table(svp);
   if ((st = upload(&ctx->d_t3slices, sl)) || (st = upload(&ctx->f_t3slices, sl)) || (st = upload(&ctx->d_svp, svp)) ||
       (st = upload(&ctx->d_t3sed, t3sed)) || (st = upload(&ctx->d_cell_sed, cell_sed)) ||
       (st = upload(&ctx->d_cell_part3, cell_part3)) || (st = upload(&ctx->d_shift_sed, shift_sed)) ||
-      (st = upload(&ctx->d_shift_part3, shift_part3)) || (st = upload(&ctx->d_fix, fix))) {
+      (st = upload(&ctx->d_shift_part3, shift_part3))) {
     if (info) *info = st;
     p3x_context_destroy(ctx.release());
     return st;
@@ -699,7 +695,7 @@ int p3x_context_destroy(p3x_context* ctx) {
   if (!ctx) return P3X_EINVAL;
   void* ptrs[] = {ctx->d_ice, ctx->d_coll, ctx->d_vn, ctx->d_vm, ctx->d_revap, ctx->f_ice, ctx->f_ice_sed, ctx->f_coll,
                   ctx->f_vn, ctx->f_vm, ctx->f_revap, ctx->d_t3slices, ctx->f_t3slices, ctx->d_svp, ctx->d_err,
-                  ctx->d_fix, ctx->d_cell_sed, ctx->d_cell_part3, ctx->d_shift_sed, ctx->d_shift_part3, ctx->d_t3sed,
+                  ctx->d_cell_sed, ctx->d_cell_part3, ctx->d_shift_sed, ctx->d_shift_part3, ctx->d_t3sed,
                   ctx->d_check, ctx->d_maxloc, ctx->fstage};
   for (void* p : ptrs)
     if (p) cudaFree(p);

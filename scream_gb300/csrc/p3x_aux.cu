@@ -55,9 +55,9 @@ __global__ void column_budgets(const double* __restrict__ qv, const double* __re
   double w = 0, e = 0;
   for (int k = lane; k < nlev; k += 32) {
     const double dp = dpres[o + k];
-    const double T = th[o + k] / inv_exner[o + k];
-    w += (qv[o + k] + qc[o + k] + qi[o + k] + qr[o + k]) * dp / g;
-    e += (T * cp + (Lv + Lf) * qv[o + k] + Lf * (qc[o + k] + qr[o + k])) * dp / g;
+    const double T = dev::ddiv_int(th[o + k], inv_exner[o + k]);
+    w += dev::ddiv_int((qv[o + k] + qc[o + k] + qi[o + k] + qr[o + k]) * dp, g);
+    e += dev::ddiv_int((T * cp + (Lv + Lf) * qv[o + k] + Lf * (qc[o + k] + qr[o + k])) * dp, g);
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
@@ -86,13 +86,13 @@ __global__ void conservation_kernel(ConsPtrs p, int ncol, int nlev, int64_t ld, 
   double m = 0, e = 0;
   for (int k = lane; k < nlev; k += 32) {
     const double pd = p.pd[o + k];
-    m += (p.qv[o + k] + p.qc[o + k] + p.qi[o + k] + p.qr[o + k]) * pd / g;
+    m += dev::ddiv_int((p.qv[o + k] + p.qc[o + k] + p.qi[o + k] + p.qr[o + k]) * pd, g);
     double ke = 0;
     if (p.winds) {
       const double u = p.winds[int64_t(warp) * 2 * ld + k], v = p.winds[int64_t(warp) * 2 * ld + ld + k];
       ke = 0.5 * (u * u + v * v);
     }
-    e += (p.T[o + k] * cp + ke + (Lv + Lf) * p.qv[o + k] + Lf * (p.qc[o + k] + p.qr[o + k])) * pd / g;
+    e += dev::ddiv_int((p.T[o + k] * cp + ke + (Lv + Lf) * p.qv[o + k] + Lf * (p.qc[o + k] + p.qr[o + k])) * pd, g);
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
@@ -176,7 +176,7 @@ __global__ void postamble_kernel(const dev::Inst* __restrict__ insts, const dev:
     double* t_prev = const_cast<double*>(in.t_prev);
     for (int k = lane; k < in.nlev; k += 32) {
       qv_prev[co + k] = in.qv[co + k];
-      t_prev[co + k] = in.th[co + k] / in.inv_exner[co + k];
+      t_prev[co + k] = dev::ddiv_int(in.th[co + k], in.inv_exner[co + k]);
     }
   }
 }
@@ -188,8 +188,12 @@ __global__ void postamble_kernel(const dev::Inst* __restrict__ insts, const dev:
  * wet <-> dry factor pseudo_density / pseudo_density_dry (or its inverse) is
  * formed once per level and multiplies the ten mixing ratios, where the
  * reference divides each of them (x * pd / pdd): one rounding apart, at most
- * ~2 ulp, for a tenth of the FP64 divisions, which set this kernel's cost
- * on a part whose FP64 pipe issues a warp instruction every 16 cycles. */
+ * ~2 ulp.  Divisions are ddiv_int (IEEE's result); the postamble's Exner
+ * function is the fixed-point power, which nothing but its own outputs reads,
+ * while the preamble's stays the library's pow (82 % of its time): th and
+ * inv_exner start the step, and ice sedimentation would carry a last-bit
+ * difference far.  At 65,536 x 128: preamble 2.1 -> 1.6 ms, postamble 1.8 ->
+ * 0.43 ms, against 0.31 and 0.32 ms for their bytes. */
 __global__ void interface_preamble_kernel(InterfacePtrs p, int ncol, int nlev, int64_t ld) {
   const int col = int((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
@@ -202,14 +206,14 @@ __global__ void interface_preamble_kernel(InterfacePtrs p, int ncol, int nlev, i
     const double qv_wet = p.q[8][o];
     /* calculate_dz with the virtual temperature of the wet state */
     const double Tv = T * (1.0 + c1 * qv_wet);
-    p.dz[o] = (dev::C::RD / dev::C::gravit) * pd * Tv / pmid;
-    const double wet_to_dry = pd / pdd;
+    p.dz[o] = dev::ddiv_int((dev::C::RD / dev::C::gravit) * pd * Tv, pmid);
+    const double wet_to_dry = dev::ddiv_int(pd, pdd);
 #pragma unroll
     for (int s = 0; s < 9; ++s) p.q[s][o] = p.q[s][o] * wet_to_dry;
     p.qv_prev[o] = p.qv_prev[o] * wet_to_dry;
-    const double exner = pow(pmid / dev::C::P0, dev::C::RD * dev::C::INV_CP);
-    p.inv_exner[o] = 1.0 / exner;
-    p.th[o] = T / exner;
+    const double exner = pow(dev::ddiv_int(pmid, dev::C::P0), dev::C::RD * dev::C::INV_CP);
+    p.inv_exner[o] = dev::ddiv_int(1.0, exner);
+    p.th[o] = dev::ddiv_int(T, exner);
     const double ct = p.cld_t[o];
     const double cl = ct > mincld ? ct : mincld;
     p.cld_l[o] = cl;
@@ -230,9 +234,9 @@ __global__ void interface_postamble_kernel(InterfacePtrs p, int ncol, int nlev, 
   for (int k = lane; k < nlev; k += 32) {
     const int64_t o = int64_t(col) * ld + k;
     const double pd = p.pd[o], pdd = p.pdd[o], pmid = p.pmid[o];
-    const double dry_to_wet = pdd / pd;
+    const double dry_to_wet = dev::ddiv_int(pdd, pd);
     const double T_before = p.T[o];
-    const double exner = pow(pmid / dev::C::P0, dev::C::RD * dev::C::INV_CP);
+    const double exner = dev::pow_fix(dev::ddiv_int(pmid, dev::C::P0), dev::C::RD * dev::C::INV_CP);
     double T = (p.th[o] * exner - T_before) * dry_to_wet;
     T += T_before;
     p.T[o] = T;
@@ -290,11 +294,11 @@ __global__ void eam_pre_kernel(EamPtrs p, int ncol, int nlev, int64_t ld, int64_
     bool reset = true;
     if (act) {
       const int64_t o = int64_t(col) * ld + k;
-      const double ratio = p.pdel[o] / p.pdeldry[o];
+      const double ratio = dev::ddiv_int(p.pdel[o], p.pdeldry[o]);
 #pragma unroll
       for (int s = 0; s < 9; ++s) p.w[s][o] = p.q[s][o] * ratio;
       p.qv_prev_dry[o] = p.qv_prev[o] * ratio;
-      const double inv_exner = 1.0 / pow(p.pmid[o] * 1.e-5, kappa);
+      const double inv_exner = dev::ddiv_int(1.0, pow(p.pmid[o] * 1.e-5, kappa));
       p.inv_exner[o] = inv_exner;
       const int64_t oi = int64_t(col) * ld_int + k;
       p.dz[o] = p.zi[oi] - p.zi[oi + 1];
@@ -310,8 +314,9 @@ __global__ void eam_pre_kernel(EamPtrs p, int ncol, int nlev, int64_t ld, int64_
         if (k > 0) {
           if (p.method == P3X_PRECIP_FRAC_MAX_OVERLAP) {
             /* rain or ice mass in the level above (dry mixing ratios) */
-            const double qr_up = p.q[3][o - 1] * (p.pdel[o - 1] / p.pdeldry[o - 1]);
-            const double qi_up = p.q[5][o - 1] * (p.pdel[o - 1] / p.pdeldry[o - 1]);
+            const double ratio_up = dev::ddiv_int(p.pdel[o - 1], p.pdeldry[o - 1]);
+            const double qr_up = p.q[3][o - 1] * ratio_up;
+            const double qi_up = p.q[5][o - 1] * ratio_up;
             reset = !(qr_up >= eam::kQsmall || qi_up >= eam::kQsmall);
           } else {
             reset = !(p.w[1][o] < eam::kQsmall && p.w[5][o] < eam::kQsmall);
@@ -344,7 +349,12 @@ __global__ void eam_pre_kernel(EamPtrs p, int ncol, int nlev, int64_t ld, int64_
   }
 }
 
-/* Use of the P3 results (micro_p3_interface.F90:1182-1431). */
+/* Use of the P3 results (micro_p3_interface.F90:1182-1431).  The driver's
+ * twenty divisions per level run on the integer pipes (ddiv_int, the same
+ * doubles; the ten over dt share one reciprocal seed) and its threshold tests
+ * compare bit patterns: 6.6 -> 1.3 ms at 65,536 x 128, where the ~4.7 GB it
+ * moves take 0.7 ms; the FP64 multiplications and differences of its formulas
+ * make up most of the rest. */
 __global__ void eam_post_kernel(EamPtrs p, int ncol, int nlev, int64_t ld, int64_t ld_int, double dt) {
   const int col = int((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
@@ -352,36 +362,37 @@ __global__ void eam_post_kernel(EamPtrs p, int ncol, int nlev, int64_t ld, int64
   double cdnumc = 0.0;
   for (int k = lane; k < nlev; k += 32) {
     const int64_t o = int64_t(col) * ld + k;
-    const double ratio = p.pdeldry[o] / p.pdel[o];
+    const double ratio = dev::ddiv_int(p.pdeldry[o], p.pdel[o]);
     double w[9];
 #pragma unroll
     for (int s = 0; s < 9; ++s) w[s] = p.w[s][o] * ratio;
     const double t = p.t[o];
-    double dtemp = p.th[o] / p.inv_exner[o] - t;
+    double dtemp = dev::ddiv_int(p.th[o], p.inv_exner[o]) - t;
     dtemp = __dmul_rn(dtemp, ratio); /* rounded before the sum, as the driver writes it (no fused multiply-add) */
     const double temp = dtemp + t;
-    p.ptend_s[o] = eam::kCpair * (temp - t) / dt;
+    p.ptend_s[o] = dev::ddiv_int(eam::kCpair * (temp - t), dt);
 #pragma unroll
-    for (int s = 0; s < 9; ++s) p.ptend_q[s][o] = (eam::fmax_(0.0, w[s]) - p.q[s][o]) / dt;
+    for (int s = 0; s < 9; ++s) p.ptend_q[s][o] = dev::ddiv_int(dev::dmax0(w[s]) - p.q[s][o], dt);
     p.t_prev[o] = temp;
     p.qv_prev[o] = w[0];
     const double cme = p.cmeliq[o];
     if (p.qme) p.qme[o] = cme + p.depos[o];
     p.vap_liq[o] = p.vap_liq[o] + cme;
     const double pmid = p.pmid[o];
-    if (p.rho) p.rho[o] = pmid / (eam::kRair * temp);
+    if (p.rho) p.rho[o] = dev::ddiv_int(pmid, eam::kRair * temp);
     const double cl = p.cld_l[o], ci = p.cld_i[o], cr = p.cld_r[o];
-    const double icimr = eam::fmin_(p.q[5][o] / eam::fmax_(eam::kMincld, ci), 0.005);
-    const double icwmr = eam::fmin_(p.q[1][o] / eam::fmax_(eam::kMincld, cl), 0.005);
-    const double icin = p.q[6][o] / eam::fmax_(eam::kMincld, ci) * pmid / (287.15 * t);
-    const double icwn = p.q[2][o] / eam::fmax_(eam::kMincld, cl) * pmid / (287.15 * t);
+    const double ci_d = dev::dmax_c(ci, eam::kMincld), cl_d = dev::dmax_c(cl, eam::kMincld), rt = 287.15 * t;
+    const double icimr = dev::dmin_c(dev::ddiv_int(p.q[5][o], ci_d), 0.005);
+    const double icwmr = dev::dmin_c(dev::ddiv_int(p.q[1][o], cl_d), 0.005);
+    const double icin = dev::ddiv_int(dev::ddiv_int(p.q[6][o], ci_d) * pmid, rt);
+    const double icwn = dev::ddiv_int(dev::ddiv_int(p.q[2][o], cl_d) * pmid, rt);
     if (p.icimrst) p.icimrst[o] = icimr;
     if (p.icwmrst) p.icwmrst[o] = icwmr;
     if (p.icinc) p.icinc[o] = icin;
     if (p.icwnc) p.icwnc[o] = icwn;
     const double rel = p.eff_qc[o] * 1e6, rei = p.eff_qi[o] * 1e6;
     double dei = rei * 2.0, mu = 0.0, lambdac = 0.0;
-    if (p.ast[o] < 1.e-4) {
+    if (dev::dlt(p.ast[o], 1.e-4)) {
       mu = eam::kMucon;
       lambdac = (eam::kMucon + 1.0) / eam::kDcon;
       dei = eam::kDeicon;
@@ -393,9 +404,9 @@ __global__ void eam_post_kernel(EamPtrs p, int ncol, int nlev, int64_t ld, int64
     if (p.lambdac) p.lambdac[o] = lambdac;
     /* w: 1 cldliq, 2 numliq, 3 rain, 4 numrain, 5 cldice */
     const double tot = w[3] + w[5] + w[1];
-    if (p.nfice) p.nfice[o] = (w[5] > eam::kQsmall && tot > eam::kQsmall) ? eam::fmin_(w[5] / tot, 1.0) : 0.0;
-    cdnumc = cdnumc + w[2] * p.pdel[o] / eam::kGravit;
-    const bool liq = cl > 0.01 && icwmr > 5.e-5, ice = ci > 0.01 && icimr > 1.e-6;
+    if (p.nfice) p.nfice[o] = (dev::dgt(w[5], eam::kQsmall) && dev::dgt(tot, eam::kQsmall)) ? dev::dmin_c(dev::ddiv_int(w[5], tot), 1.0) : 0.0;
+    cdnumc = cdnumc + dev::ddiv_int(w[2] * p.pdel[o], eam::kGravit);
+    const bool liq = dev::dgt(cl, 0.01) && dev::dgt(icwmr, 5.e-5), ice = dev::dgt(ci, 0.01) && dev::dgt(icimr, 1.e-6);
     if (p.efcout) p.efcout[o] = liq ? rel * cl : 0.0;
     if (p.ncout) p.ncout[o] = liq ? icwn * cl : 0.0;
     if (p.freql) p.freql[o] = liq ? cl : 0.0;
@@ -404,7 +415,7 @@ __global__ void eam_post_kernel(EamPtrs p, int ncol, int nlev, int64_t ld, int64
     if (p.freqi) p.freqi[o] = ice ? ci : 0.0;
     const double reff = p.eff_qr[o];
     if (p.deff_rain) p.deff_rain[o] = reff * 2.0 * 1.e6;
-    const bool rain = w[3] >= 1.e-7;
+    const bool rain = dev::dge(w[3], 1.e-7);
     if (p.aqrain) p.aqrain[o] = rain ? w[3] * cr : 0.0;
     if (p.anrain) p.anrain[o] = rain ? w[4] * cr : 0.0;
     if (p.freqr) p.freqr[o] = rain ? cr : 0.0;

@@ -69,11 +69,9 @@ struct KParams {
   const TR* vn;
   const TR* vm;
   const TR* revap;
-  /* FP64 form: tables of the fixed-point arithmetic (p3x_intfp64.cuh), the
-   * fixed-point ice-table cells of sedimentation (columns 0, 1, 6, 7) and
+  /* FP64 form: the fixed-point ice-table cells of sedimentation (columns 0, 1, 6, 7) and
    * part3 (6, 7, 5, 11) with their powers of two, and Table3's fall speeds as
    * {vm, vm step, vn, vn step} per row for each of the 10 mu columns */
-  const FixTables* fix;
   const int64_t *cell_sed, *cell_part3;
   const int32_t *cell_sed_shift, *cell_part3_shift;
   const double4* t3sed;
@@ -535,11 +533,6 @@ __device__ __forceinline__ double svp_liquid(double t, double logt) {
 __device__ __forceinline__ double svp_ice(double t, double logt) {
   return m_exp(9.550426 - m_div(5723.265, t) + (3.53068 * logt) - (0.00728332 * t));
 }
-/* x^0.54 and x^0.5 in fixed point, the library function outside its range */
-static __device__ __noinline__ double pow_fix(double x, int64_t c, double cd, const FixTables* t) {
-  return uint32_t(d_bits(x) >> 52) - (1023u - 62u) < 124u ? pow_int(x, c, t) : pow(x, cd);
-}
-
 /* p3_main_part2 of one level with a hydrometeor in the FP64 form
  * (p3_main_part2_impl.hpp, same order of processes).  Each library function
  * (a pow holds the FP64 pipe for 1,500 cycles) is evaluated once and only
@@ -781,7 +774,6 @@ template <int LANES>
 __device__ void p3_part12_f64(const Inst& in, const int col, const KParams<double>& kp, const Tabs<double>& tb,
                               double* __restrict__ sm, uint32_t& err) {
   const RuntimeDev& rt = kp.rt;
-  const FixTables* const ft = kp.fix;
   const unsigned mask = group_mask<LANES>();
   const int lane = threadIdx.x & (LANES - 1);
   const int nk = in.nlev;
@@ -832,10 +824,8 @@ __device__ void p3_part12_f64(const Inst& in, const int col, const KParams<doubl
       const double rho = m_div(m_div(dpres, dz), C::gravit);
       const double inv_rho = m_div(1.0, rho);
       /* fall-speed factors; rhofaci is rhofacr times a constant */
-      constexpr int64_t k54 = 4980620899901579264ll; /* 0.54, Q63 */
-      constexpr int64_t k50 = 1ll << 62;
-      const double rhofacr = pow_fix(C::RHO_1000MB * inv_rho, k54, .54, ft);
-      const double visc = m_div(1.496e-6 * (T * pow_fix(T, k50, .5, ft)), T + 120.0);
+      const double rhofacr = pow_fix(C::RHO_1000MB * inv_rho, .54);
+      const double visc = m_div(1.496e-6 * (T * pow_fix(T, .5)), T + 120.0);
       SMA(A_RHO, k) = rho;
       SMA(A_RHOFACR, k) = rhofacr;
       SMA(A_RHOFACI, k) = rhofacr * kRhofaciOverR;
@@ -1207,7 +1197,7 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
   static_assert(sizeof(TR) == sizeof(double), "the FP32-bulk sedimentation is p3_sed_bulk");
   if (in.cflag[col] == 0) return;
   const RuntimeDev& rt = kp.rt;
-  const FixTables* const ft = kp.fix;
+  const FixTables* const ft = &kFixTables;
   const unsigned mask = group_mask<LANES>();
   const int lane = threadIdx.x & (LANES - 1);
   const int nk = in.nlev;
@@ -1919,7 +1909,7 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
         TR mu_c, lamc;
         const TR n_in = TR(nc_incld);
         TR n_out = n_in;
-        get_cloud_dsd2<TR>(TR(qc_incld), n_out, mu_c, TR(rho), lamc, [&kp](TR x) { return cbrt_fix(x, kp.fix); });
+        get_cloud_dsd2<TR>(TR(qc_incld), n_out, mu_c, TR(rho), lamc, [](TR x) { return cbrt_fix(x, &kFixTables); });
         apply_n_adjust(nc_incld, n_in, n_out);
         s.nc = nc_incld * cld_l;
         eff_qc = double(m_div(TR(0.5) * (mu_c + TR(3)), lamc));
@@ -1939,7 +1929,7 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
         TR mu_r = 0, lamr;
         const TR n_in = TR(nr_incld);
         TR n_out = n_in;
-        get_rain_dsd2<TR>(TR(qr_incld), n_out, mu_r, lamr, rt, [&kp](TR x) { return cbrt_fix(x, kp.fix); });
+        get_rain_dsd2<TR>(TR(qr_incld), n_out, mu_r, lamr, rt, [](TR x) { return cbrt_fix(x, &kFixTables); });
         apply_n_adjust(nr_incld, n_in, n_out);
         s.nr = nr_incld * cld_r;
         eff_qr = double(m_div(TR(1.5), lamr));
@@ -1970,7 +1960,7 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
         if (qi_gt_small) {
           /* table position, limits and values in fixed point (part3 0.87 ->
            * 0.37 ms at 21,600 x 128) */
-          const IceCell cell = ice_cell(m_div(qi_incld, ni_incld), m_div(qm_incld, qi_incld), rhop, kp.fix);
+          const IceCell cell = ice_cell(m_div(qi_incld, ni_incld), m_div(qm_incld, qi_incld), rhop, &kFixTables);
           const int64_t* const cf = kp.cell_part3 + size_t(cell.cell) * (kCellCols * kCellCoefs);
           const int4 sh = __ldg(reinterpret_cast<const int4*>(kp.cell_part3_shift) + cell.cell);
           const int64_t hi = ice_cell_value(cf, cell), lo = ice_cell_value(cf + kCellCoefs, cell);

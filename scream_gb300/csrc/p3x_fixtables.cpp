@@ -1,23 +1,12 @@
 /*
- * Host side of p3x_intfp64.cuh: the logarithm / exponential tables and the
- * fixed-point ice-table cells, in extended precision.
+ * Host side of p3x_intfp64.cuh: the fixed-point ice-table cells, in extended
+ * precision.
  */
 #include "p3x_fixtables.hpp"
 
 #include <cmath>
 
 namespace p3x {
-
-void build_fix_tables(dev::FixTables& t) {
-  for (int j = 0; j < 128; ++j) {
-    const long double c = 1.0L + (j + 0.5L) / 128.0L;
-    const uint32_t r = uint32_t(std::llroundl(4294967296.0L / c));
-    t.log2[j].r = r;
-    t.log2[j].pad = 0;
-    t.log2[j].nlog2 = std::llroundl(-std::log2(static_cast<long double>(r) / 4294967296.0L) * 0x1p62L);
-    t.exp2[j] = std::llroundl(std::exp2((j + 0.5L) / 128.0L) * 0x1p62L);
-  }
-}
 
 void build_ice_cells(const double* ice, const int cols[dev::kCellCols], std::vector<int64_t>& coef,
                      std::vector<int32_t>& shift) {

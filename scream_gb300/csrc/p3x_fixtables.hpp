@@ -1,4 +1,4 @@
-/* Tables of the fixed-point FP64 operations (p3x_intfp64.cuh). */
+/* Ice-table cells of the fixed-point FP64 operations (p3x_intfp64.cuh). */
 #ifndef P3X_FIXTABLES_HPP
 #define P3X_FIXTABLES_HPP
 
@@ -9,8 +9,6 @@
 #include "p3x_internal.hpp"
 
 namespace p3x {
-
-void build_fix_tables(dev::FixTables& t);
 
 /* Fixed-point coefficients of four ice-table columns for every cell
  * [kIceCells][kCellCols][kCellCoefs] and the power of two of each cell and

@@ -151,9 +151,10 @@ P3X_HD double ddiv_int(double a, double b) {
 /* ------------------------------------------------------------------ */
 /* Fixed-point values are written Qn: an integer in units of 2^-n. */
 
-/* Tables of the functions below, 128 intervals each (built on the host in
- * extended precision): r is 2^32 / c for the interval's midpoint c, rounded,
- * and nlog2 = -log2(r / 2^32) in Q62; exp2 holds 2^((j + 1/2) / 128) in Q62. */
+/* Tables of the functions below, 128 intervals each: r is 2^32 / c for the
+ * interval's midpoint c, rounded, and nlog2 = -log2(r / 2^32) in Q62; exp2
+ * holds 2^((j + 1/2) / 128) in Q62.  They are static data of the module (3 KB
+ * per translation unit), so no launch depends on a context or an upload. */
 struct alignas(16) Log2Entry {
   uint32_t r, pad;
   int64_t nlog2;
@@ -162,6 +163,15 @@ struct FixTables {
   Log2Entry log2[128];
   int64_t exp2[128];
 };
+#ifdef __CUDACC__
+static __device__ const FixTables kFixTables =
+#include "p3x_fixtables.inc"
+    ;
+#else
+static const FixTables kFixTables =
+#include "p3x_fixtables.inc"
+    ;
+#endif
 
 /* log2 of M / 2^52 for a 53-bit significand M, in Q62.  With r ~ 1 / c the
  * table leaves z = r M / 2^52 - 1, |z| < 2^-8, exact to 2^-63, and

@@ -147,6 +147,14 @@ __device__ __forceinline__ float m_div(float a, float b) { return a / b; }
 static __device__ __noinline__ double cbrt_fix(double x, const FixTables* t) {
   return d_normal_pos(d_bits(x)) ? cbrt_int(x, t) : cbrt(x);
 }
+/* x^c for a constant 0 < c < 1 on the integer pipes (101 cycles against pow's
+ * 1,499), the library function outside pow_int's range */
+static __device__ __noinline__ double pow_fix_nl(double x, int64_t c, double cd) {
+  return uint32_t(d_bits(x) >> 52) - (1023u - 62u) < 124u ? pow_int(x, c, &kFixTables) : pow(x, cd);
+}
+__device__ __forceinline__ double pow_fix(double x, double c) {
+  return pow_fix_nl(x, int64_t(c * 9223372036854775808.0), c); /* a double below 1 is exact in Q63 */
+}
 __device__ __forceinline__ double m_fabs(double x) { return fabs(x); }
 __device__ __forceinline__ float m_fabs(float x) { return fabsf(x); }
 

@@ -133,8 +133,7 @@ int main(int argc, char** argv) {
     std::printf("%ld\n", check_div(family, n));
     return 0;
   }
-  static FixTables t;
-  p3x::build_fix_tables(t);
+  const FixTables& t = kFixTables;
   if (what == "ice" || what == "rain") {
     std::printf("%.6Le\n", what == "ice" ? check_ice(family, n, t) : check_rain(family, n, t));
     return 0;
