@@ -53,8 +53,17 @@ cudaError_t launch_p3_part(const dev::Inst& inst0, const dev::KParams<TR>& kp_in
   } else if (part == kPartK2) {
     if constexpr (LANES == 32) {
       if constexpr (sizeof(TR) == sizeof(float)) {
-        e = launch_persistent<TR>(dev::p3_sed_bulk_kernel<LANES>, inst0, kp, threads,
-                                  sed_smem_bytes<TR>(ls, kp.sm_stride), 0, num_sms, stream, ls.grid_frac);
+        const int per_sm = sed_staged_columns(kp.sm_stride);
+        if (kp.wctr && per_sm > 0 && kp.nwork >= per_sm * num_sms) {
+          kp.groups_per_block = per_sm;
+          const size_t smem = dev::sed_table_bytes() +
+                              size_t(per_sm) * dev::kSedBulkSlots * size_t(kp.sm_stride) * sizeof(double);
+          e = launch_persistent<TR>(dev::p3_sed_bulk_kernel<LANES, true>, inst0, kp, per_sm * LANES, smem, 0, num_sms,
+                                    stream, ls.grid_frac);
+        } else {
+          e = launch_persistent<TR>(dev::p3_sed_bulk_kernel<LANES, false>, inst0, kp, threads,
+                                    sed_smem_bytes<TR>(ls, kp.sm_stride), 0, num_sms, stream, ls.grid_frac);
+        }
       } else {
         e = launch_persistent<TR>(dev::p3_sed_kernel<TR, LANES>, inst0, kp, threads,
                                   sed_smem_bytes<TR>(ls, kp.sm_stride), 0, num_sms, stream, ls.grid_frac);

@@ -46,6 +46,15 @@ inline LaunchSpec sed_spec(const LaunchSpec& ls) {
   return s;
 }
 
+/* Columns of one CTA of the FP32-bulk sedimentation that keeps its tables in
+ * shared memory, one CTA per SM: as many as fit beside the 20.8 KB of tables, 20
+ * at most (96 registers a thread).  0 where that is fewer than 16. */
+inline int sed_staged_columns(int sm_stride) {
+  const size_t col = dev::kSedBulkSlots * size_t(sm_stride) * sizeof(double);
+  const size_t n = (size_t(227 * 1024) - dev::sed_table_bytes()) / col;
+  return n >= 20 ? 20 : (n >= 16 ? int(n) : 0);
+}
+
 /* CTAs of kernel `func` that fit on one SM with `threads` threads and `smem`
  * bytes of dynamic shared memory on the current device.  The first query of
  * a (device, kernel, threads, smem) shape raises the kernel's
