@@ -1321,13 +1321,14 @@ __device__ void p3_part12_bulk(const Inst& in, const int col, const KParams<floa
  * ~3,300 cycles of an SM and a rain level for ~1,400 (a warp instruction every
  * 16 cycles; a division takes 131, cbrt 227, log10 553).  Here the divisions,
  * the logarithm, the cube root and the table interpolation are 64-bit integer
- * arithmetic (22, ~50, ~95 and ~50 cycles), the in-cloud values are never
+ * arithmetic (16, 35, 73 and 42 cycles), the in-cloud values are never
  * formed (every quantity that the fall speeds need is a ratio of two fields of
  * one level, so the cloud fraction cancels; the in-cloud thresholds become
  * thresholds times the cloud fraction), and what stays FP64 is the flux:
  * one product, one difference and one multiply-add per field, with 1 / (dz rho)
  * formed once per level and V rho kept instead of V.  At 21,600 x 128: 15.8 ms
- * with integer divisions alone, 3.6 ms in this form; the results differ from
+ * with integer divisions alone, 2.7 ms in this form (3.6 ms with exact 64-bit
+ * high products, rounded quotients and 100 registers); the results differ from
  * the reference's order of operations by rounding (1e-14 of a field's norm). */
 template <class TR, int LANES>
 __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, const Tabs<TR>& tb,
@@ -1451,8 +1452,7 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
             if (number) v2 = w * ((2.0 + mu_c) * (1.0 + mu_c));
           } else if (sp == 1) {
             if (rt.rain_fix) {
-              const double n_q = ddiv_int(n, q);
-              const RainRow rr = rain_row(n_q, rt.rain_kd, ft);
+              const RainRow rr = rain_row(log2_of(raw_quotient(n, q), ft), rt.rain_kd, ft);
               if (rr.side != 0) n = (rr.side < 0 ? rt.rain_n_hi : rt.rain_n_lo) * q;
               const double4 t = kp.t3sed[(rt.t3_dumjj - 1) * kT3SedRows + rr.row - 1];
               v1 = fma(rr.frac, t.y, t.x);
@@ -1462,7 +1462,7 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
                 v1 = fma(rt.t3_wj, fma(rr.frac, t1.y, t1.x) - v1, v1);
                 v2 = fma(rt.t3_wj, fma(rr.frac, t1.w, t1.z) - v2, v2);
               }
-              if (!d_normal_pos(d_bits(n_q))) v1 = d_from_bits(kNaNBits);
+              if (!(dbits(q) < kInfBits && dbits(n) < kInfBits)) v1 = d_from_bits(kNaNBits);
             } else {
               const double cld = cldp[k];
               double mu_r = 0, lamr, n_out = m_div(n, cld);
@@ -1489,16 +1489,22 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
                 b = 0;
               }
             }
-            /* calc_bulk_rho_rime, p3/impl/p3_ice_sed_impl.hpp:14-64 */
-            double rho_rime = 0;
+            /* calc_bulk_rho_rime, p3/impl/p3_ice_sed_impl.hpp:14-64; the rime
+             * density itself is only needed in fixed point */
+            uint64_t rho52 = 0;
             const bool rimed = dbits(b) >= dbits(qs) || dbits(b) >= dbits(qs * (C::BSMALL / C::QSMALL));
             if (rimed && dbits(b) <= kInfBits) {
-              rho_rime = ddiv_int(m, b);
-              const bool lt = dlt(rho_rime, rt.min_rime_rho), gt = dgt(rho_rime, rt.max_rime_rho);
-              if (lt) rho_rime = rt.min_rime_rho;
-              if (gt) rho_rime = rt.max_rime_rho;
-              if (dbits(m) > dbits(q)) m = q;
-              if (lt || gt || dbits(m) != dbits(R2[k])) b = ddiv_int(m, rho_rime);
+              const bool lt = dbits(m) < dbits(rt.min_rime_rho * b), gt = dbits(m) > dbits(rt.max_rime_rho * b);
+              double rho_lim = lt ? rt.min_rime_rho : rt.max_rime_rho;
+              if (!lt && !gt) {
+                rho52 = rho_q52(raw_quotient(m, b));
+                if (dbits(m) > dbits(q)) rho_lim = ddiv_int(m, b);
+              } else {
+                rho52 = rho_q52(rho_lim);
+              }
+              const bool over = dbits(m) > dbits(q);
+              if (over) m = q;
+              if (lt || gt || over) b = ddiv_int(m, rho_lim);
             } else if (!rimed) {
               m = 0;
               b = 0;
@@ -1509,7 +1515,8 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
             }
             R2[k] = m;
             R3[k] = b;
-            const IceCell cell = ice_cell(ddiv_int(q, n), ddiv_int(m, q), rho_rime, ft);
+            const IceCell cell = ice_cell_at(log2_of(raw_quotient(q, n), ft), dnz(m) ? fix_of(raw_quotient(m, q), 60) : 0, rho52);
+            const bool odd = !(dbits(q) < kInfBits && dbits(n) < kInfBits && dbits(m) < kInfBits);
             const int64_t* const cf = kp.cell_sed + size_t(cell.cell) * (kCellCols * kCellCoefs);
             const int4 sh = __ldg(reinterpret_cast<const int4*>(kp.cell_sed_shift) + cell.cell);
             /* columns 6 and 7: the limits of the number */
@@ -1519,7 +1526,7 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
             R1[k] = n;
             v1 = d_from_fix(ice_cell_value(cf + kCellCoefs, cell), sh.y) * FR[k];
             v2 = d_from_fix(ice_cell_value(cf, cell), sh.x) * FR[k];
-            if (cell.odd) v1 = d_from_bits(kNaNBits);
+            if (odd) v1 = d_from_bits(kNaNBits);
           }
           if (!dpos(qs)) v1 = d_from_bits(kNaNBits); /* no cloud fraction: reported below */
           lmax = dmax_nn(lmax, v1 * CF[k]);
@@ -2370,8 +2377,10 @@ __global__ void __launch_bounds__(256, sizeof(TR) == sizeof(float) ? 2 : 1)
   if (err) atomicOr(kp.err, err);
 }
 
+/* 96 registers (a few dozen bytes spill): five 4-column CTAs per SM instead of
+ * four, 3.61 -> 3.48 ms at 21,600 x 128 (80 registers: no faster). */
 template <class TR, int LANES>
-__global__ void __launch_bounds__(256) p3_sed_kernel(const Inst inst0, const KParams<TR> kp) {
+__global__ void __maxnreg__(96) p3_sed_kernel(const Inst inst0, const KParams<TR> kp) {
   static_assert(sizeof(TR) == sizeof(double), "the FP32-bulk sedimentation kernel is p3_sed_bulk_kernel");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint32_t err = 0;

@@ -38,12 +38,12 @@ void build_ice_cells(const double* ice, const int cols[dev::kCellCols], std::vec
           for (int m = 0; m < dev::kCellCoefs; ++m)
             most = std::fmax(most, std::fabs(std::ldexp(k[m], kWeights[m])));
           const size_t cell = size_t((jj * dev::kCellR + ii) * dev::kCellI + i) * dev::kCellCols + c;
-          /* the largest stored coefficient lies in [2^59, 2^60), so that no
+          /* the largest stored coefficient lies in [2^60, 2^61), so that no
            * partial sum reaches 2^63; a cell of (near) zeros stays zero */
           if (!(most > 0x1p-900L) || !std::isfinite(most)) continue;
           int e = 0;
           std::frexp(most, &e);
-          const int s = 60 - e;
+          const int s = 61 - e;
           shift[cell] = s;
           for (int m = 0; m < dev::kCellCoefs; ++m)
             coef[cell * dev::kCellCoefs + m] = std::llroundl(std::ldexp(k[m], kWeights[m] + s));

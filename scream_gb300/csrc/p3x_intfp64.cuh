@@ -10,12 +10,13 @@
  *   FP64 add, multiply, FMA, conversion      15.5-18    ~100
  *   FP64 division                            131        564
  *   ddiv_int inlined / called                22 / 28    192 / 287
- *   64-bit integer high product              5.2        29
- *   log10 / log2_q57                         553 / 49
- *   cbrt / cbrt_int                          227 / 98
- *   pow / pow_int                            1499 / 101
- *   one ice-table column, 14 FP64 operations / ice_cell_value and its double
- *                                            224 / 67
+ *   raw_quotient (not rounded)               16
+ *   64-bit high product, exact / mulhi_add   8.9 / 5.8  29
+ *   log10 / log2 in Q57                      553 / 35
+ *   cbrt / cbrt_int                          227 / 73
+ *   pow / pow_int                            1499 / 76
+ *   ice-table position / one column of it and its double (14 FP64 operations)
+ *                                            17 / 42 (224)
  */
 #pragma once
 
@@ -69,6 +70,25 @@ P3X_HD uint64_t mulhi_u64(uint64_t a, uint64_t b) {
 #endif
 }
 P3X_HD int32_t mulhi_s32(int32_t a, int32_t b) { return int32_t((int64_t(a) * b) >> 32); }
+/* acc + (a b >> 64), good to 4 units: the product of the low words is left
+ * out, and the cross products lose the low word's last bit, which makes that
+ * word a positive signed one.  Five instructions of the multiplier pipe, where
+ * the exact high product takes a dozen, half of them on the adder pipe.  For
+ * products with bits to spare below the last one that counts. */
+P3X_HD int64_t mulhi_add(int64_t acc, int64_t a, int64_t b) {
+  const int32_t ah = int32_t(a >> 32), bh = int32_t(b >> 32);
+  const int32_t al = int32_t(uint32_t(a) >> 1), bl = int32_t(uint32_t(b) >> 1);
+#ifdef __CUDA_ARCH__
+  int32_t x;
+  asm("mul.hi.s32 %0, %1, %2;" : "=r"(x) : "r"(ah), "r"(bl));
+  asm("mad.hi.s32 %0, %1, %2, %3;" : "=r"(x) : "r"(bh), "r"(al), "r"(x));
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(acc) : "r"(ah), "r"(bh), "l"(acc));
+  asm("mad.wide.s32 %0, %1, 2, %2;" : "=l"(acc) : "r"(x), "l"(acc));
+  return acc;
+#else
+  return acc + int64_t(ah) * bh + 2 * int64_t(mulhi_s32(ah, bl) + mulhi_s32(bh, al));
+#endif
+}
 P3X_HD int clz_u64(uint64_t x) {
 #ifdef __CUDA_ARCH__
   return __clzll(static_cast<long long>(x));
@@ -105,35 +125,40 @@ P3X_HD uint32_t rcp_seed(uint32_t fbits) {
  * bits leave the rounding open). */
 P3X_HD_NOINLINE double ddiv_general(double a, double b) { return a / b; }
 
-/* a / b on the integer pipes, the same double as the FP64 division.
+/* The quotient A / B of two 53-bit significands (bit 52 set), in units of
+ * 2^-63, less under 2 units: S in [2^62, 2^64).
  *
- * The 53-bit significands A and B give Q = A / B in (1/2, 2) by long division
- * in three digits from one FP32 reciprocal seed R <= 2^24 / (B / 2^52): each
- * digit is the high word of (leading remainder bits) x R, never above the
- * true one, and its exact remainder feeds the next.
+ * Long division in three digits from one FP32 reciprocal seed R <= 2^24 /
+ * (B / 2^52): each digit is the high word of (leading remainder bits) x R,
+ * never above the true one, and its exact remainder feeds the next.
  *   q1 ~ Q 2^30,              rem1 = A 2^30 - q1 B        in [0, 2^63)
  *   q2 ~ (rem1 / B) 2^19,     rem2 = rem1 2^19 - q2 B     in [0, 2^61)
  *   q3 ~ (rem2 / B) 2^19
- * S = q1 2^33 + q2 2^14 + (q3 >> 5) is then Q 2^63 less under 2 units (the
- * cube of the seed's error, 2^-63.6, and the truncations), and a quotient of
- * doubles is never half way between two doubles, so the nearest double follows
- * from S except where its bits below the last place are the ones just under
- * one half: one quotient in 1024, which takes the FP64 division. */
-P3X_HD double ddiv_int(double a, double b) {
-  const uint64_t ua = d_bits(a), ub = d_bits(b);
-  const uint32_t ah = uint32_t(ua >> 32), al = uint32_t(ua), bh = uint32_t(ub >> 32), bl = uint32_t(ub);
-  const uint32_t ea = (ah >> 20) & 0x7ffu, eb = (bh >> 20) & 0x7ffu;
-  const uint32_t sign = (ah ^ bh) & 0x80000000u;
-  const uint32_t mah = (ah & 0xfffffu) | 0x100000u, mbh = (bh & 0xfffffu) | 0x100000u;
-  const uint64_t A = (uint64_t(mah) << 32) | al, B = (uint64_t(mbh) << 32) | bl;
+ * S = q1 2^33 + q2 2^14 + (q3 >> 5): the cube of the seed's error, 2^-63.6, and
+ * the truncations stay below 2 units. */
+P3X_HD uint64_t sig_quotient(uint64_t A, uint64_t B) {
   /* B / 2^52 rounded to the nearest float */
-  const uint32_t R7 = rcp_seed((uint32_t((ub << 12) >> 40) + 0x7f000001u) >> 1) << 7;
+  const uint32_t R7 = rcp_seed((uint32_t((B << 12) >> 40) + 0x7f000001u) >> 1) << 7;
   const uint32_t q1 = mulhi_u32(uint32_t(A >> 21), R7);
   const uint64_t rem1 = (A << 30) - B * q1;
   const uint32_t q2 = mulhi_u32(uint32_t(rem1 >> 32), R7);
   const uint64_t rem2 = (rem1 << 19) - B * q2;
   const uint32_t q3 = mulhi_u32(uint32_t(rem2 >> 32), R7);
-  uint64_t S = (uint64_t(q1) << 33) + (uint64_t(q2) << 14) + (q3 >> 5);
+  return (uint64_t(q1) << 33) + (uint64_t(q2) << 14) + (q3 >> 5);
+}
+
+/* a / b on the integer pipes, the same double as the FP64 division.  A
+ * quotient of doubles is never half way between two doubles, so the nearest
+ * double follows from sig_quotient except where its bits below the last place
+ * are the ones just under one half: one quotient in 1024, which takes the FP64
+ * division. */
+P3X_HD double ddiv_int(double a, double b) {
+  const uint64_t ua = d_bits(a), ub = d_bits(b);
+  const uint32_t ah = uint32_t(ua >> 32), bh = uint32_t(ub >> 32);
+  const uint32_t ea = (ah >> 20) & 0x7ffu, eb = (bh >> 20) & 0x7ffu;
+  const uint32_t sign = (ah ^ bh) & 0x80000000u;
+  uint64_t S = sig_quotient((uint64_t((ah & 0xfffffu) | 0x100000u) << 32) | uint32_t(ua),
+                            (uint64_t((bh & 0xfffffu) | 0x100000u) << 32) | uint32_t(ub));
   const uint32_t low = uint32_t(S >> 63) ^ 1u; /* 1: Q < 1 */
   S <<= low;
   const uint32_t er = ea - eb + 1022u - low; /* the result's exponent field less one */
@@ -173,12 +198,12 @@ static const FixTables kFixTables =
     ;
 #endif
 
-/* log2 of M / 2^52 for a 53-bit significand M, in Q62.  With r ~ 1 / c the
- * table leaves z = r M / 2^52 - 1, |z| < 2^-8, exact to 2^-63, and
+/* log2 of M63 / 2^63 for a significand with bit 63 set, in Q62.  With r ~ 1 / c
+ * the table leaves z = r M63 / 2^63 - 1, |z| < 2^-8, exact to 2^-63, and
  * ln(1 + z) = z - z^2 (1/2 - z (1/3 - z (1/4 - z (1/5 - z / 6)))) is cut off
  * below 2^-58; the inner terms need 32 bits only.  Error below 2^-57. */
-P3X_HD int64_t log2_sig(uint64_t M, const FixTables* t) {
-  const Log2Entry* en = &t->log2[uint32_t(M >> 45) & 127u];
+P3X_HD int64_t log2_sig(uint64_t M63, const FixTables* t) {
+  const Log2Entry* en = &t->log2[uint32_t(M63 >> 56) & 127u];
 #ifdef __CUDA_ARCH__
   const uint4 ev = __ldg(reinterpret_cast<const uint4*>(en));
   const uint32_t r = ev.x;
@@ -187,7 +212,6 @@ P3X_HD int64_t log2_sig(uint64_t M, const FixTables* t) {
   const uint32_t r = en->r;
   const int64_t nl = en->nlog2;
 #endif
-  const uint64_t M63 = M << 11;
   const uint64_t P = (M63 >> 32) * r + ((uint64_t(uint32_t(M63)) * r) >> 32);
   const int64_t z = int64_t(P - (1ull << 63)); /* Q63 */
   const int64_t z8 = z << 8;                    /* Q71 */
@@ -197,11 +221,11 @@ P3X_HD int64_t log2_sig(uint64_t M, const FixTables* t) {
   const int32_t t4 = k5 - (mulhi_s32(zs, k6) >> 7);
   const int32_t t3 = k4 - (mulhi_s32(zs, t4) >> 7);
   const int64_t t2 = k3 - ((int64_t(zs) * t3) >> 8);
-  const int64_t t1 = k2 - (mulhi_s64(z8, t2) >> 7);
-  const int64_t u = mulhi_s64(z8, t1);         /* z t1, Q69 */
-  const int64_t v = mulhi_s64(z8, u << 3);     /* z^2 t1, Q79 */
+  const int64_t t1 = k2 - (mulhi_add(0, z8, t2) >> 7);
+  const int64_t u = mulhi_add(0, z8, t1);      /* z t1, Q69 */
+  const int64_t v = mulhi_add(0, z8, u << 3);  /* z^2 t1, Q79 */
   const int64_t ln = z8 - (v >> 8);            /* Q71 */
-  return nl + (mulhi_s64(ln, kLog2e) >> 7);
+  return nl + (mulhi_add(0, ln, kLog2e) >> 7);
 }
 
 /* 2^F for F in [0, 1) given in Q64: the significand in Q62, error below
@@ -215,18 +239,18 @@ P3X_HD int64_t exp2_sig(uint64_t F, const FixTables* t) {
 #endif
   const int64_t f = int64_t((F << 7) ^ (1ull << 63)); /* (F mod 2^-7) - 2^-8, Q71 */
   constexpr int64_t kLn2 = 6393154322601327829ll;     /* ln 2, Q63 */
-  const int64_t g2 = mulhi_s64(f, kLn2) << 1;         /* g, Q71 */
+  const int64_t g2 = mulhi_add(0, f, kLn2) << 1;      /* g, Q71 */
   const int32_t gs = int32_t(g2 >> 32);               /* Q39 */
   constexpr int32_t k720 = int32_t((1ll << 31) / 720), k120 = int32_t((1ll << 31) / 120), k24 = int32_t((1ll << 31) / 24);
   constexpr int64_t k6 = (1ll << 62) / 6, k2 = 1ll << 61;
   const int32_t q5 = k120 + (mulhi_s32(gs, k720) >> 7);
   const int32_t q4 = k24 + (mulhi_s32(gs, q5) >> 7);
   const int64_t q3 = k6 + ((int64_t(gs) * q4) >> 8);
-  const int64_t q2 = k2 + (mulhi_s64(g2, q3) >> 7);
-  const int64_t w = mulhi_s64(g2, q2);      /* g q2, Q69 */
-  const int64_t gw = mulhi_s64(g2, w << 3); /* g^2 q2, Q79 */
-  const int64_t em1 = g2 + (gw >> 8);       /* Q71 */
-  return T + (mulhi_s64(T, em1) >> 7);
+  const int64_t q2 = k2 + (mulhi_add(0, g2, q3) >> 7);
+  const int64_t w = mulhi_add(0, g2, q2);      /* g q2, Q69 */
+  const int64_t gw = mulhi_add(0, g2, w << 3); /* g^2 q2, Q79 */
+  const int64_t em1 = g2 + (gw >> 8);          /* Q71 */
+  return T + (mulhi_add(0, T, em1) >> 7);
 }
 
 /* the double nearest to S 2^(E - 62) for S in [2^62 - 2^8, 2^63) and a result
@@ -243,13 +267,13 @@ P3X_HD bool d_normal_pos(uint64_t u) { return uint32_t(u >> 32) - 0x00100000u < 
 
 /* log2(x) in Q57 for a positive normal x in [2^-63, 2^63) */
 P3X_HD int64_t log2_q57(uint64_t u, const FixTables* t) {
-  return (int64_t(int32_t(d_expo(u)) - 1023) << 57) + (log2_sig(d_sig(u), t) >> 5);
+  return (int64_t(int32_t(d_expo(u)) - 1023) << 57) + (log2_sig(d_sig(u) << 11, t) >> 5);
 }
 /* log2(x) in Q57 with the exponent limited to [-63, 62] */
 P3X_HD int64_t log2_q57_clamped(uint64_t u, const FixTables* t) {
   int e = int32_t(d_expo(u)) - 1023;
   e = e < -63 ? -63 : (e > 62 ? 62 : e);
-  return (int64_t(e) << 57) + (log2_sig(d_sig(u), t) >> 5);
+  return (int64_t(e) << 57) + (log2_sig(d_sig(u) << 11, t) >> 5);
 }
 /* 2^y for y in Q57 */
 P3X_HD double exp2_q57(int64_t y, const FixTables* t) {
@@ -261,7 +285,7 @@ P3X_HD double exp2_q57(int64_t y, const FixTables* t) {
 P3X_HD double cbrt_int(double x, const FixTables* t) {
   const uint64_t u = d_bits(x);
   const uint32_t eb = d_expo(u), k = mulhi_u32(eb, 0x55555556u), rem = eb - 3 * k; /* 1023 = 3 * 341 */
-  const uint64_t X = (uint64_t(rem) << 62) + uint64_t(log2_sig(d_sig(u), t));       /* Q62, < 3 */
+  const uint64_t X = (uint64_t(rem) << 62) + uint64_t(log2_sig(d_sig(u) << 11, t));       /* Q62, < 3 */
   const uint64_t F = X + mulhi_u64(X, 0x5555555555555555ull);                        /* X / 3, Q64 */
   return d_from_q62(exp2_sig(F, t), int(k) - 341);
 }
@@ -307,9 +331,9 @@ P3X_HD int64_t fix_clamp(int64_t x, int64_t lo, int64_t hi) { return x < lo ? lo
  * weight halves the product's high word). */
 constexpr int kCellCoefs = 8, kCellCols = 4;
 P3X_HD int64_t fix_trilinear(const int64_t c[kCellCoefs], int64_t w1, int64_t w4, int64_t w5) {
-  const int64_t e = c[0] + mulhi_s64(w1, c[1]), d = c[2] + mulhi_s64(w1, c[3]);
-  const int64_t b = c[4] + mulhi_s64(w1, c[5]), a = c[6] + mulhi_s64(w1, c[7]);
-  return e + mulhi_s64(w4, d) + mulhi_s64(w5, b + mulhi_s64(w4, a));
+  const int64_t e = mulhi_add(c[0], w1, c[1]), d = mulhi_add(c[2], w1, c[3]);
+  const int64_t b = mulhi_add(c[4], w1, c[5]), a = mulhi_add(c[6], w1, c[7]);
+  return mulhi_add(mulhi_add(e, w4, d), w5, mulhi_add(b, w4, a));
 }
 
 /* Position of an ice category in the ice table (lookup_ice,
@@ -322,31 +346,62 @@ struct IceCell {
   int64_t w1, w4, w5;
 };
 constexpr int kCellI = 49, kCellR = 3, kCellD = 4, kIceCells = kCellI * kCellR * kCellD;
-/* rhop: 0 or positive; ratio_qm = qm / qi >= 0; qi_ni = qi / ni positive */
-P3X_HD IceCell ice_cell(double qi_ni, double ratio_qm, double rhop, const FixTables* t) {
+/* log2_qn: log2(qi / ni), Q57; ratio: qm / qi in Q60, at most 1; rho52: rime
+ * density in Q52, at most 1023 (beyond 900 the axis ends) */
+P3X_HD IceCell ice_cell_at(int64_t log2_qn, uint64_t ratio, uint64_t rho52) {
   /* d log2(x) + c of the size axis less one, Q55 */
   constexpr int64_t kd = 5741805296813221454ll; /* 4.135985029041767 log10(2), Q62 */
   constexpr int64_t kc = 2285945404318149440ll;  /* 18 * 4.135985029041767 - 11, Q55 */
-  const uint64_t ux = d_bits(qi_ni);
-  const int64_t x1 = mulhi_s64(log2_q57_clamped(ux, t), kd) + kc;
+  const int64_t x1 = mulhi_s64(log2_qn, kd) + kc;
   const FixAxis a1 = fix_axis(fix_clamp(x1, 0, 49ll << 55), 55, kCellI);
-  /* 3 ratio, Q60 */
-  const uint64_t ur = d_bits(ratio_qm);
-  const int er = 1023 - int(d_expo(ur));
-  const uint64_t q60 = er <= 0 ? (1ull << 60) : ((d_sig(ur) << 8) >> (er < 63 ? er : 63));
-  const FixAxis a4 = fix_axis(int64_t(3 * q60), 60, kCellR);
-  /* density, Q52, then Q58: (rho - 50) 0.005 up to 650, 3 + (rho - 650) 0.004
-   * above; beyond 900 the axis ends */
+  const FixAxis a4 = fix_axis(int64_t(3 * ratio), 60, kCellR);
+  /* (rho - 50) 0.005 up to 650, 3 + (rho - 650) 0.004 above, Q58 */
+  const bool low = rho52 <= (650ull << 52);
+  const int64_t k = low ? 5902958103587056517ll : 4722366482869645213ll; /* 0.005, 0.004 in Q70 */
+  const int64_t x5 = mulhi_add(low ? 0 : (3ll << 58), int64_t(rho52) - (int64_t(low ? 50 : 650) << 52), k);
+  const FixAxis a5 = fix_axis(fix_clamp(x5, 0, 4ll << 58), 58, kCellD);
+  return IceCell{(a5.i * kCellR + a4.i) * kCellI + a1.i, false, a1.w, a4.w, a5.w};
+}
+/* The same from doubles.  rhop: 0 or positive; ratio_qm = qm / qi >= 0; qi_ni =
+ * qi / ni positive. */
+P3X_HD uint64_t rho_q52(double rhop) {
   const uint64_t up = d_bits(rhop);
   const int ep = int(d_expo(up)) - 1023;
-  const uint64_t p52 = ep > 9 ? (1023ull << 52) : (ep >= 0 ? d_sig(up) << ep : 0);
-  const bool low = up <= 0x4084500000000000ull; /* rho <= 650 */
-  const int64_t k = low ? 5902958103587056517ll : 4722366482869645213ll; /* 0.005, 0.004 in Q70 */
-  const int64_t x5 = mulhi_s64(int64_t(p52) - (int64_t(low ? 50 : 650) << 52), k) + (low ? 0 : (3ll << 58));
-  const FixAxis a5 = fix_axis(fix_clamp(x5, 0, 4ll << 58), 58, kCellD);
-  const bool odd = !d_normal_pos(ux) || er == -1024 || ep == 1024;
-  return IceCell{(a5.i * kCellR + a4.i) * kCellI + a1.i, odd, a1.w, a4.w, a5.w};
+  return ep > 9 ? (1023ull << 52) : (ep >= 0 ? d_sig(up) << ep : 0);
 }
+P3X_HD IceCell ice_cell(double qi_ni, double ratio_qm, double rhop, const FixTables* t) {
+  const uint64_t ux = d_bits(qi_ni), ur = d_bits(ratio_qm);
+  const int er = 1023 - int(d_expo(ur));
+  const uint64_t q60 = er <= 0 ? (1ull << 60) : ((d_sig(ur) << 8) >> (er < 63 ? er : 63));
+  IceCell c = ice_cell_at(log2_q57_clamped(ux, t), q60, rho_q52(rhop));
+  c.odd = !d_normal_pos(ux) || er == -1024 || d_expo(d_bits(rhop)) == 2047u;
+  return c;
+}
+/* The quotient a / b of two positive normal doubles, unrounded: S 2^(e - 63)
+ * with S in [2^62, 2^64). */
+struct RawQuotient {
+  uint64_t S;
+  int e;
+};
+P3X_HD RawQuotient raw_quotient(double a, double b) {
+  const uint64_t ua = d_bits(a), ub = d_bits(b);
+  return RawQuotient{sig_quotient(d_sig(ua), d_sig(ub)), int(d_expo(ua)) - int(d_expo(ub))};
+}
+/* its log2 in Q57, the exponent limited to [-63, 62] */
+P3X_HD int64_t log2_of(const RawQuotient& q, const FixTables* t) {
+  const int low = int(q.S >> 63) ^ 1;
+  int e = q.e - low;
+  e = e < -63 ? -63 : (e > 62 ? 62 : e);
+  return (int64_t(e) << 57) + (log2_sig(q.S << low, t) >> 5);
+}
+/* its value in Qn for a value below 2^(63 - n) */
+P3X_HD uint64_t fix_of(const RawQuotient& q, int n) {
+  const int sh = 63 - n - q.e;
+  return q.S >> (sh < 63 ? (sh > 0 ? sh : 0) : 63);
+}
+/* a rime density m / b in Q52 for ice_cell_at (512 to 1023 comes with e = 10
+ * where the quotient of the significands is below one) */
+P3X_HD uint64_t rho_q52(const RawQuotient& q) { return q.e > 10 ? (1023ull << 52) : fix_of(q, 52); }
 
 /* value of one column in a cell: c points to its eight coefficients */
 P3X_HD int64_t ice_cell_value(const int64_t* c, const IceCell& p) {
@@ -376,10 +431,10 @@ struct RainRow {
   int row;     /* 1-based row of Table3 */
   double frac; /* position between row and row + 1 */
 };
-P3X_HD RainRow rain_row(double n_q, int64_t kd, const FixTables* t) {
+P3X_HD RainRow rain_row(int64_t log2_nq, int64_t kd, const FixTables* t) {
   constexpr int64_t kLogMin = -2393701460845809080ll; /* log2(1e-5), Q57 */
   constexpr int64_t kLogMax = -1292105688431629576ll; /* log2(2e-3), Q57 */
-  int64_t y = kd - mulhi_s64(log2_q57_clamped(d_bits(n_q), t), 6148914691236517205ll);
+  int64_t y = kd - mulhi_s64(log2_nq, 6148914691236517205ll); /* 2^64 / 3 */
   RainRow r;
   r.side = y < kLogMin ? -1 : (y > kLogMax ? 1 : 0);
   y = fix_clamp(y, kLogMin, kLogMax);

@@ -142,12 +142,12 @@ __device__ __forceinline__ float m_tanh(float x) { return tanhf(x); }
 static __device__ __noinline__ double m_div_nl(double a, double b) { return ddiv_int(a, b); }
 __device__ __forceinline__ double m_div(double a, double b) { return m_div_nl(a, b); }
 __device__ __forceinline__ float m_div(float a, float b) { return a / b; }
-/* cube root on the integer pipes (98 cycles of an SM against 227); zero, infinities, NaN, subnormals and
+/* cube root on the integer pipes (73 cycles of an SM against 227); zero, infinities, NaN, subnormals and
  * negative arguments by the library function */
 static __device__ __noinline__ double cbrt_fix(double x, const FixTables* t) {
   return d_normal_pos(d_bits(x)) ? cbrt_int(x, t) : cbrt(x);
 }
-/* x^c for a constant 0 < c < 1 on the integer pipes (101 cycles against pow's
+/* x^c for a constant 0 < c < 1 on the integer pipes (76 cycles against pow's
  * 1,499), the library function outside pow_int's range */
 static __device__ __noinline__ double pow_fix_nl(double x, int64_t c, double cd) {
   return uint32_t(d_bits(x) >> 52) - (1023u - 62u) < 124u ? pow_int(x, c, &kFixTables) : pow(x, cd);

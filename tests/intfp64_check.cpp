@@ -72,7 +72,16 @@ static long double check_ice(int family, long n, const FixTables& t) {
     } else if (family == 2) {
       rho = 650.0 + (double(g() % 5) - 2) * 0x1p-42;
     }
-    const IceCell c = ice_cell(q_n, rat, rho, &t);
+    IceCell c = ice_cell(q_n, rat, rho, &t);
+    if (i & 1) { /* from unrounded quotients, as sedimentation forms them */
+      const double n = 1.0 + double(g() % 1000) / 7.0, q = q_n * n; /* q_n below: what the doubles give */
+      const double b = std::ldexp(1.0, int(g() % 40) - 30); /* rho b is exact */
+      const RawQuotient rq = raw_quotient(q, n);
+      q_n = q / n;
+      if (rat <= 1) c = ice_cell_at(log2_of(rq, &t), rat > 0 ? fix_of(raw_quotient(rat, 1.0), 60) : 0,
+                                    rho > 0 ? rho_q52(raw_quotient(rho * b, b)) : 0);
+      else c = ice_cell(q_n, rat, rho, &t);
+    }
     const long double d1 = clampl((std::log10((long double)q_n) + 18) * (long double)4.135985029041767 - 10, 1, 50);
     const long double d4 = clampl(3 * (long double)rat + 1, 1, 4);
     const long double d5 = clampl(rho <= 650 ? ((long double)rho - 50) * 0.005L + 1 : ((long double)rho - 650) * 0.004L + 4, 1, 5);
@@ -106,7 +115,7 @@ static long double check_rain(int family, long n, const FixTables& t) {
     if (family == 1) D = ((g() & 1) ? 1e-5L : 2e-3L) * (1 + ((long double)(g() % 2001) - 1000) * 1e-12L);
     if (family == 2) D = 195e-6L * (1 + ((long double)(g() % 2001) - 1000) * 1e-12L);
     const double n_q = double(std::pow((mu + 1) / D, 3) / f);
-    const RainRow r = rain_row(n_q, kd, &t);
+    const RainRow r = rain_row(log2_q57_clamped(d_bits(n_q), &t), kd, &t);
     const long double Dx = clampl((mu + 1) / std::cbrt((long double)f * n_q), 1e-5L, 2e-3L);
     const long double c = Dx <= 195e-6L ? (Dx * 1e6L + 5) / 10 : (Dx * 1e6L - 195) / 30 + 20;
     worst = std::fmax(worst, std::fabs((long double)r.row + r.frac - c));

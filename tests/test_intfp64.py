@@ -9,7 +9,8 @@ through the power 0.54 (0.04, and its Q56 product 2^-56 ln 2 = 0.05) or the
 cube root and the exponential (2^-58 and 2^-60), plus the check's own extended
 precision; a log2 in Q57 is off by its last unit and 2^-57.  Ice table: the
 coordinates' error, 2^-54, times the table's slope (neighbouring entries
-within a factor of 8, three axes) and one rounding.  Rain table: the
+within a factor of 8, three axes), the products' 28 units of a stored
+coefficient's last place (2^-60 of the cell's largest), and one rounding.  Rain table: the
 coordinate is at most 80 with a relative error of 2^-57, in Q53."""
 import subprocess
 from pathlib import Path
