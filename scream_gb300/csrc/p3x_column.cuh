@@ -80,6 +80,7 @@ struct KParams {
   int sm_stride;     /* doubles per per-level shared array (>= nlev_max + 1, even) */
   int groups_per_block;
   int nwork;         /* number of columns (single) or work items (batched) */
+  int part3_split;   /* K3: groups that share a work item's levels */
   const WorkItem* work;
   const Inst* insts;
   uint32_t* err;
@@ -2031,11 +2032,11 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
 #undef SMA
 }
 
-/* K3: homogeneous freezing and p3_main_part3 of one column that went on past
- * part2. */
+/* K3: homogeneous freezing and p3_main_part3 of the levels first + lane, first
+ * + step + lane, ... of one column that went on past part2. */
 template <class TR, int LANES>
 __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, const Tabs<TR>& tb, const int inst_idx,
-                         uint32_t& err) {
+                         const int first, const int step, uint32_t& err) {
   if (in.cflag[col] == 0) return;
   const RuntimeDev& rt = kp.rt;
   const int lane = threadIdx.x & (LANES - 1);
@@ -2045,7 +2046,7 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
   const double* const t_start = scr_at(in, S_TATM, col);
   constexpr bool kF64 = sizeof(TR) == sizeof(double);
   /* ---------------- phase 4: homogeneous freezing + p3_main_part3 ---------------- */
-  for (int k = lane; k < nk; k += LANES) {
+  for (int k = first + lane; k < nk; k += step) {
     const int64_t o = co + k;
     State s;
     s.qc = in.qc[o]; s.nc = in.nc[o]; s.qr = in.qr[o]; s.nr = in.nr[o];
@@ -2452,10 +2453,13 @@ __global__ void __launch_bounds__(256) p3_part3_kernel(const Inst inst0, const K
   uint32_t err = 0;
   Tabs<TR> tb;
   setup_tables<TR>(kp, false, smem_raw, tb, err);
-  for_each_work<LANES>(kp.wctr ? kp.wctr + 2 : nullptr, kp.nwork, kp.groups_per_block, [&](int w) {
+  const int split = kp.part3_split;
+  for_each_work<LANES>(kp.wctr ? kp.wctr + 2 : nullptr, kp.nwork * split, kp.groups_per_block, [&](int w) {
+    const int item = split == 1 ? w : w / split;
     int col;
-    const Inst& in = work_inst(inst0, kp, w, col);
-    p3_part3<TR, LANES>(in, col, kp, tb, kp.work ? kp.work[w].inst : 0, err);
+    const Inst& in = work_inst(inst0, kp, item, col);
+    p3_part3<TR, LANES>(in, col, kp, tb, kp.work ? kp.work[item].inst : 0, (w - item * split) * LANES, split * LANES,
+                        err);
   });
   if (err) atomicOr(kp.err, err);
 }

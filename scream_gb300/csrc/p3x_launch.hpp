@@ -32,11 +32,12 @@ inline size_t sed_smem_bytes(const LaunchSpec& ls, int sm_stride) {
   return size_t(ls.groups_per_block) * dev::sed_slots<TR>() * size_t(sm_stride) * sizeof(double);
 }
 
-/* Launch shape of K2.  Sedimentation always runs 32 lanes per column,
- * whatever lane count K1 and K3 use: its substeps walk the levels chunk by
- * chunk, so a narrower group only lengthens the walk (measured at 65,536 x
- * 128 with 16 lanes: FP64 K2 +17 %, FP32-bulk K2 +95 %), while K1 in the
- * FP64 form runs 7 % faster at 16 lanes.  Columns per CTA as configured, at
+/* Launch shape of K2 and K3.  Sedimentation always runs 32 lanes per column,
+ * whatever lane count K1 uses: its substeps walk the levels chunk by chunk, so a
+ * narrower group only lengthens the walk (measured at 65,536 x 128 with 16
+ * lanes: FP64 K2 +17 %, FP32-bulk K2 +95 %).  Part3 too: FP64 at 21,600 x 128
+ * 344 us against 369 at 16 lanes, 1,537 x 97 39 against 55, 64 x 72 31 against
+ * 43.  Columns per CTA as configured, at
  * most 8 (256 threads). */
 inline LaunchSpec sed_spec(const LaunchSpec& ls) {
   LaunchSpec s = ls;
@@ -68,7 +69,8 @@ cudaError_t kernel_occupancy(const void* func, int threads, size_t smem, int* pe
 enum : int { kPartK1 = 1, kPartK2 = 2, kPartK3 = 4 };
 
 /* Persistent launch of one part for one lane count (defined in
- * p3x_kernels_impl.cuh, instantiated in p3x_k_*.cu; K2 only for 32 lanes).
+ * p3x_kernels_impl.cuh, instantiated in p3x_k_*.cu; K2 and K3 only for 32
+ * lanes).
  * kp.nwork, kp.work, kp.insts and kp.sm_stride are set by the caller, and
  * every instance's scratch (Inst::scr, Inst::cflag) is bound. */
 template <class TR, int LANES>
@@ -104,7 +106,7 @@ inline cudaError_t launch_p3(const dev::Inst& inst0, const dev::KParams<TR>& kp,
     e = launch_p3_part<TR, 32>(inst0, kp, sed_spec(ls), kPartK2, num_sms, stream);
     if (e != cudaSuccess) return e;
   }
-  if (parts & kPartK3) e = launch_p3_part_lanes<TR>(inst0, kp, ls, kPartK3, num_sms, stream);
+  if (parts & kPartK3) e = launch_p3_part<TR, 32>(inst0, kp, sed_spec(ls), kPartK3, num_sms, stream);
   return e;
 }
 

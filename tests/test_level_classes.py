@@ -1,7 +1,8 @@
 """Part1+2 sorts the levels of a column (with a hydrometeor, near ice
-nucleation, neither) and evaluates saturation only where it is read; the
-FP32-bulk sedimentation has a launch with its tables in shared memory for
-calls that fill the GPU.  Both are checked where the choice changes."""
+nucleation, neither) and evaluates saturation only where it is read; and
+the kernels have launch shapes of their own for calls that fill the GPU and
+for calls that leave most of it idle.  Both are checked where the choice
+changes."""
 import numpy as np
 import pytest
 
@@ -74,22 +75,25 @@ def test_dry_levels_at_the_class_limits(gpu_ctx, tables, ccn, qi):
                 assert rel_l2(g_rows[h][on], rows[h][on]) <= 1e-12, h
 
 
-@pytest.mark.parametrize("nlev", [1, 33, 72, 128, 129, 164, 170])
-def test_sedimentation_with_staged_tables_equals_the_other_launch(gpu_ctx, nlev):
-    """A call that fills every SM with columns (tables in shared memory, where
-    the columns leave room) against the same columns in calls too small for
-    that: columns are independent, so every field is bitwise the same."""
+@pytest.mark.parametrize("precision", ["fp64", "bulk"])
+@pytest.mark.parametrize("nlev", [1, 31, 32, 33, 72, 128, 129, 164, 170, 257])
+def test_launch_shapes_agree(gpu_ctx, nlev, precision):
+    """A call that fills every SM with columns (FP32-bulk sedimentation: tables
+    in shared memory, where the columns leave room) against the same columns
+    in smaller calls, the smallest of which share a column's levels among
+    warps: columns are independent, so every field is bitwise the same."""
     import torch
     import scream_gb300 as p3
+    prec = p3.P3X_FP64 if precision == "fp64" else p3.P3X_FP32_BULK
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     n = 20 * sms + 3
     half = 10 * sms
     inp = p3.generate_inputs(0, 77, n, nlev)
     whole = p3.P3Fields.from_inputs(inp)
-    gpu_ctx.p3_main(whole, DT, p3.P3X_FP32_BULK)
+    gpu_ctx.p3_main(whole, DT, prec)
     whole = whole.to_host()
-    for a, b in ((0, half), (half, n)):
+    for a, b in ((0, 1), (1, 8), (8, 2 * sms), (2 * sms, half), (half, n)):
         part = p3.P3Fields.from_inputs({k: np.ascontiguousarray(v[a:b]) for k, v in inp.items()})
-        gpu_ctx.p3_main(part, DT, p3.P3X_FP32_BULK)
+        gpu_ctx.p3_main(part, DT, prec)
         for k, v in part.to_host().items():
             np.testing.assert_array_equal(v, whole[k][a:b], err_msg=f"{k} {a}:{b}")
