@@ -351,6 +351,7 @@ int launch_kernels(p3x_context* ctx, const p3x_runtime* rt, const dev::Inst& in,
   if (in.precision == P3X_FP32_BULK) {
     dev::KParams<float> kp = make_kparams<float>(ctx, rtd);
     kp.sm_stride = stride;
+    kp.nlev_max = in.nlev;
     kp.nwork = in.ncol;
     kp.work = nullptr;
     kp.insts = nullptr;
@@ -359,6 +360,7 @@ int launch_kernels(p3x_context* ctx, const p3x_runtime* rt, const dev::Inst& in,
   } else {
     dev::KParams<double> kp = make_kparams<double>(ctx, rtd);
     kp.sm_stride = stride;
+    kp.nlev_max = in.nlev;
     kp.nwork = in.ncol;
     kp.work = nullptr;
     kp.insts = nullptr;
@@ -1412,6 +1414,7 @@ int launch_work_t(p3x_context* ctx, const dev::RuntimeDev& rtd, const LaunchSpec
   if (!spec_fits(prec, ls, stride)) return P3X_EINVAL;
   dev::KParams<TR> kp = make_kparams<TR>(ctx, rtd);
   kp.sm_stride = stride;
+  kp.nlev_max = nlev_max;
   kp.nwork = nwork;
   kp.work = work_d;
   kp.insts = insts_d;

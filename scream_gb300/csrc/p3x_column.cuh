@@ -80,6 +80,7 @@ struct KParams {
   int sm_stride;     /* doubles per per-level shared array (>= nlev_max + 1, even) */
   int groups_per_block;
   int nwork;         /* number of columns (single) or work items (batched) */
+  int nlev_max;      /* levels of the deepest column */
   int part3_split;   /* K3: groups that share a work item's levels */
   const WorkItem* work;
   const Inst* insts;
@@ -166,7 +167,7 @@ __host__ __device__ constexpr size_t table_smem_bytes() {
 /* ------------------------------------------------------------------ */
 template <int LANES>
 __device__ __forceinline__ unsigned group_mask() {
-  if (LANES == 32) return 0xffffffffu;
+  if (LANES >= 32) return 0xffffffffu;
   const unsigned lw = threadIdx.x & 31u;
   return (0xffffffffu >> (32 - LANES)) << (lw & ~unsigned(LANES - 1));
 }
@@ -200,6 +201,81 @@ __device__ __forceinline__ int group_min_int(unsigned mask, int v) {
 template <int LANES>
 __device__ __forceinline__ int group_max_int(unsigned mask, int v) {
   return __reduce_max_sync(mask, v);
+}
+
+/* Sedimentation also runs groups of several warps, LANES > 32 threads (at least
+ * as many as the column has levels): the warps of a group exchange through this
+ * shared scratch and meet at a barrier.  SPLIT: a CTA has three such groups,
+ * one per species, each with its own scratch and barrier (named 1 to 3);
+ * otherwise the group is the CTA. */
+struct GroupScratch {
+  double max_d[8];
+  float max_f[8];
+  int lo[3][8], hi[3][8]; /* tops and bottoms of the species */
+  double edge[8][4];      /* fluxes of each warp's last level */
+  double prt[4];          /* surface precipitation of the species */
+};
+static_assert(sizeof(GroupScratch) % 16 == 0, "the arrays behind it are 16-byte aligned");
+template <int LANES, bool SPLIT = false>
+__device__ __forceinline__ void group_sync(unsigned mask) {
+  if constexpr (SPLIT) {
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + int(threadIdx.x) / LANES), "n"(LANES) : "memory");
+  } else if constexpr (LANES > 32) {
+    __syncthreads();
+  } else {
+    __syncwarp(mask);
+  }
+}
+template <int LANES>
+__device__ __forceinline__ int group_warp() {
+  return int(threadIdx.x & (LANES - 1)) >> 5;
+}
+/* Tops (minima) and bottoms (maxima) of the three species over the group. */
+template <int LANES, bool SPLIT>
+__device__ __forceinline__ void group_bounds(unsigned mask, GroupScratch* gs, int lo[3], int hi[3]) {
+  constexpr int kWarp = LANES < 32 ? LANES : 32;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    lo[i] = group_min_int<kWarp>(mask, lo[i]);
+    hi[i] = group_max_int<kWarp>(mask, hi[i]);
+  }
+  if constexpr (LANES > 32) {
+    const int w = group_warp<LANES>();
+    if ((threadIdx.x & 31) == 0) {
+      for (int i = 0; i < 3; ++i) {
+        gs->lo[i][w] = lo[i];
+        gs->hi[i][w] = hi[i];
+      }
+    }
+    group_sync<LANES, SPLIT>(mask);
+    for (int i = 0; i < 3; ++i)
+      for (int j = 0; j < LANES / 32; ++j) {
+        lo[i] = min(lo[i], gs->lo[i][j]);
+        hi[i] = max(hi[i], gs->hi[i][j]);
+      }
+  }
+}
+/* maximum of non-negative values over the group */
+template <int LANES, bool SPLIT>
+__device__ __forceinline__ double group_max_wide(unsigned mask, GroupScratch* gs, double v) {
+  v = group_max_nn<LANES < 32 ? LANES : 32>(mask, v);
+  if constexpr (LANES > 32) {
+    if ((threadIdx.x & 31) == 0) gs->max_d[group_warp<LANES>()] = v;
+    group_sync<LANES, SPLIT>(mask);
+    for (int j = 0; j < LANES / 32; ++j) v = dmax_nn(v, gs->max_d[j]);
+  }
+  return v;
+}
+template <int LANES, bool SPLIT>
+__device__ __forceinline__ float group_max_wide(unsigned mask, GroupScratch* gs, float v) {
+  v = group_max_nn<LANES < 32 ? LANES : 32>(mask, v);
+  if constexpr (LANES > 32) {
+    if ((threadIdx.x & 31) == 0) gs->max_f[group_warp<LANES>()] = v;
+    group_sync<LANES, SPLIT>(mask);
+    for (int j = 0; j < LANES / 32; ++j)
+      v = __float_as_uint(v) < __float_as_uint(gs->max_f[j]) ? gs->max_f[j] : v;
+  }
+  return v;
 }
 
 /* ------------------------------------------------------------------ */
@@ -1331,9 +1407,9 @@ __device__ void p3_part12_bulk(const Inst& in, const int col, const KParams<floa
  * with integer divisions alone, 2.7 ms in this form (3.6 ms with exact 64-bit
  * high products, rounded quotients and 100 registers); the results differ from
  * the reference's order of operations by rounding (1e-14 of a field's norm). */
-template <class TR, int LANES>
+template <class TR, int LANES, bool SPLIT = false>
 __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, const Tabs<TR>& tb,
-                       double* __restrict__ sm, uint32_t& err) {
+                       double* __restrict__ sm, GroupScratch* gs, uint32_t& err) {
   static_assert(sizeof(TR) == sizeof(double), "the FP32-bulk sedimentation is p3_sed_bulk");
   if (in.cflag[col] == 0) return;
   const RuntimeDev& rt = kp.rt;
@@ -1348,6 +1424,7 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
   const double inv_dt = m_div(1.0, dt);
   const bool predictNc = in.predictNc != 0;
   const int kbot = nk - 1;
+  constexpr int kWarp = LANES < 32 ? LANES : 32; /* lanes that shuffle with one another */
   double* const FR = sm + B_FR * S;   /* fall-speed factor of the species times rho */
   double* const CF = sm + B_CF * S;   /* 1 / (dz rho) */
   double* const QS = sm + B_QS * S;   /* QSMALL times the species' cloud fraction */
@@ -1363,19 +1440,15 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
   /* Top and bottom of the three species (p3_find_impl.hpp) in one pass.  A
    * species only changes the levels from its top down to its final leading
    * edge; the others keep their values. */
-  int top_c = 1 << 30, top_r = 1 << 30, top_i = 1 << 30, bot_c = -1, bot_r = -1, bot_i = -1;
+  int top[3] = {1 << 30, 1 << 30, 1 << 30}, bot[3] = {-1, -1, -1};
   for (int k = lane; k < nk; k += LANES) {
-    if (dge(in.qc[co + k], C::QSMALL)) { top_c = min(top_c, k); bot_c = k; }
-    if (dge(in.qr[co + k], C::QSMALL)) { top_r = min(top_r, k); bot_r = k; }
-    if (dge(in.qi[co + k], C::QSMALL)) { top_i = min(top_i, k); bot_i = k; }
+    if (dge(in.qc[co + k], C::QSMALL)) { top[0] = min(top[0], k); bot[0] = k; }
+    if (dge(in.qr[co + k], C::QSMALL)) { top[1] = min(top[1], k); bot[1] = k; }
+    if (dge(in.qi[co + k], C::QSMALL)) { top[2] = min(top[2], k); bot[2] = k; }
   }
-  top_c = group_min_int<LANES>(mask, top_c);
-  top_r = group_min_int<LANES>(mask, top_r);
-  top_i = group_min_int<LANES>(mask, top_i);
-  bot_c = group_max_int<LANES>(mask, bot_c);
-  bot_r = group_max_int<LANES>(mask, bot_r);
-  bot_i = group_max_int<LANES>(mask, bot_i);
-  for (int k = min(top_c, min(top_r, top_i)) + lane; k < nk; k += LANES)
+  if (LANES > 32 && lane < 3) gs->prt[lane] = 0;
+  group_bounds<LANES, SPLIT>(mask, gs, top, bot);
+  for (int k = min(top[0], min(top[1], top[2])) + lane; k < nk; k += LANES)
     CF[k] = ddiv_int(1.0, in.dz[co + k] * rho_row[k]);
   double precip_liq_surf = 0, precip_ice_surf = 0;
 
@@ -1386,8 +1459,8 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
     const double* const cldp = (sp == 0 ? in.cld_frac_l : (sp == 1 ? in.cld_frac_r : in.cld_frac_i)) + co;
     const double* const facp = scr_at(in, sp == 0 ? S_ACN : (sp == 1 ? S_RHOFACR : S_RHOFACI), col);
     const bool number = sp != 0 || predictNc; /* the number falls too */
-    const int k_qxtop = sp == 0 ? top_c : (sp == 1 ? top_r : top_i);
-    int k_qxbot = sp == 0 ? bot_c : (sp == 1 ? bot_r : bot_i);
+    const int k_qxtop = top[sp];
+    int k_qxbot = bot[sp];
     if (k_qxbot < 0) return; /* species absent (group-uniform) */
 
     for (int k = k_qxtop + lane; k < nk; k += LANES) {
@@ -1404,7 +1477,7 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
     if (sp == 1) {
       for (int k = k_qxtop + lane; k <= nk; k += LANES) PF[k] = 0;
     }
-    __syncwarp(mask);
+    group_sync<LANES, SPLIT>(mask);
 
     /* From here on lane l owns levels k_qxtop + l + j*LANES in both the
      * fall-speed pass and the flux walk, so only shuffles cross lanes. */
@@ -1539,7 +1612,7 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
         V1[k_qxbot + 1] = 0; /* the cell receiving the leading edge has no fall speed */
         V2[k_qxbot + 1] = 0;
       }
-      const double Co_max = group_max_nn<LANES>(mask, lmax) * dt_left;
+      const double Co_max = group_max_wide<LANES, SPLIT>(mask, gs, lmax) * dt_left;
       if (!(Co_max >= 0) || Co_max > 2.0e9) {
         err |= kErrNumeric;
         break;
@@ -1569,11 +1642,21 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
             f3 = v1 * r3;
           }
         }
-        double u0 = __shfl_up_sync(mask, f0, 1, LANES), u1 = 0, u2 = 0, u3 = 0;
-        if (number) u1 = __shfl_up_sync(mask, f1, 1, LANES);
+        double u0 = __shfl_up_sync(mask, f0, 1, kWarp), u1 = 0, u2 = 0, u3 = 0;
+        if (number) u1 = __shfl_up_sync(mask, f1, 1, kWarp);
         if (sp == 2) {
-          u2 = __shfl_up_sync(mask, f2, 1, LANES);
-          u3 = __shfl_up_sync(mask, f3, 1, LANES);
+          u2 = __shfl_up_sync(mask, f2, 1, kWarp);
+          u3 = __shfl_up_sync(mask, f3, 1, kWarp);
+        }
+        if constexpr (LANES > 32) {
+          double* const edge = gs->edge[group_warp<LANES>()];
+          if ((lane & 31) == 31) {
+            edge[0] = f0; edge[1] = f1; edge[2] = f2; edge[3] = f3;
+          }
+          group_sync<LANES, SPLIT>(mask);
+          if ((lane & 31) == 0 && lane > 0) {
+            u0 = edge[-4]; u1 = edge[-3]; u2 = edge[-2]; u3 = edge[-1];
+          }
         }
         if (lane == 0) {
           u0 = carry0; u1 = carry1; u2 = carry2; u3 = carry3;
@@ -1590,28 +1673,34 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
           if (k == kbot) flux_bot = f0;
         }
         if (base + LANES <= k_temp) {
-          carry0 = __shfl_sync(mask, f0, LANES - 1, LANES);
-          if (number) carry1 = __shfl_sync(mask, f1, LANES - 1, LANES);
+          carry0 = __shfl_sync(mask, f0, kWarp - 1, kWarp);
+          if (number) carry1 = __shfl_sync(mask, f1, kWarp - 1, kWarp);
           if (sp == 2) {
-            carry2 = __shfl_sync(mask, f2, LANES - 1, LANES);
-            carry3 = __shfl_sync(mask, f3, LANES - 1, LANES);
+            carry2 = __shfl_sync(mask, f2, kWarp - 1, kWarp);
+            carry3 = __shfl_sync(mask, f3, kWarp - 1, kWarp);
           }
         }
       }
       if (k_qxbot == kbot) {
-        const int owner = (kbot - k_qxtop) % LANES;
-        prt_accum += __shfl_sync(mask, flux_bot, owner, LANES) * dt_sub;
+        /* a group of several warps: the lane that owns the bottom level sums */
+        if constexpr (LANES <= 32) flux_bot = __shfl_sync(mask, flux_bot, (kbot - k_qxtop) % LANES, LANES);
+        prt_accum += flux_bot * dt_sub;
       } else {
         k_qxbot += 1;
       }
       dt_left -= dt_sub;
       first = false;
     }
+    if constexpr (LANES > 32) {
+      if (lane == kbot - k_qxtop) gs->prt[sp] = prt_accum;
+      group_sync<LANES, SPLIT>(mask);
+      prt_accum = gs->prt[sp];
+    }
     if (sp == 0) precip_liq_surf = prt_accum * C::INV_RHO_H2O * inv_dt;
     else if (sp == 1) precip_liq_surf += prt_accum * C::INV_RHO_H2O * inv_dt;
     else precip_ice_surf += prt_accum * C::INV_RHO_H2O * inv_dt;
 
-    __syncwarp(mask);
+    group_sync<LANES, SPLIT>(mask);
     for (int k = k_qxtop + lane; k <= k_qxbot; k += LANES) {
       g0[co + k] = R0[k];
       g1[co + k] = R1[k];
@@ -1624,12 +1713,26 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
       /* interfaces above the top stay at part1's zero */
       for (int k = k_qxtop + 1 + lane; k <= nk; k += LANES) in.precip_liq_flux[ci + k] = PF[k];
     }
-    __syncwarp(mask);
+    group_sync<LANES, SPLIT>(mask);
   };
-  species(std::integral_constant<int, 0>{});
-  species(std::integral_constant<int, 1>{});
-  species(std::integral_constant<int, 2>{});
-  if (lane == 0) {
+  if constexpr (SPLIT) {
+    const int sp = int(threadIdx.x) / LANES;
+    if (sp == 0) species(std::integral_constant<int, 0>{});
+    else if (sp == 1) species(std::integral_constant<int, 1>{});
+    else species(std::integral_constant<int, 2>{});
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      /* thread 0 belongs to the first group: gs[0], gs[1], gs[2] are the three */
+      precip_liq_surf = gs[0].prt[0] * C::INV_RHO_H2O * inv_dt;
+      precip_liq_surf += gs[1].prt[1] * C::INV_RHO_H2O * inv_dt;
+      precip_ice_surf = gs[2].prt[2] * C::INV_RHO_H2O * inv_dt;
+    }
+  } else {
+    species(std::integral_constant<int, 0>{});
+    species(std::integral_constant<int, 1>{});
+    species(std::integral_constant<int, 2>{});
+  }
+  if (SPLIT ? threadIdx.x == 0 : lane == 0) {
     in.precip_liq_surf[col] = precip_liq_surf;
     in.precip_ice_surf[col] = precip_ice_surf;
   }
@@ -1650,9 +1753,9 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
  * column's mass telescopes exactly, and the surface precipitation is the
  * bottom face's G.  Where a limiter rewrites a level's state to x during the
  * walk, B_k is reset so that R_k = x at that moment. */
-template <int LANES>
+template <int LANES, bool SPLIT = false>
 __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>& kp, const Tabs<float>& tb,
-                            double* __restrict__ sm, uint32_t& err) {
+                            double* __restrict__ sm, GroupScratch* gs, uint32_t& err) {
   if (in.cflag[col] == 0) return;
   const RuntimeDev& rt = kp.rt;
   const unsigned mask = group_mask<LANES>();
@@ -1665,6 +1768,7 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
   const double inv_dt = 1 / dt;
   const bool predictNc = in.predictNc != 0;
   const int kbot = nk - 1;
+  constexpr int kWarp = LANES < 32 ? LANES : 32; /* lanes that shuffle with one another */
 #define SMA(a, k) sm[(a)*S + (k)]
   /* kSedBulkSlots slots of S doubles; two float arrays share a slot.  The
    * density is read from the hand-over row (a float per level, L1-resident
@@ -1703,19 +1807,15 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
    * down to its final leading edge, so conversions, flux coefficients and the
    * FP64 state rebuild are limited to those levels; the levels above the top
    * and below the leading edge keep their values. */
-  int top_c = 1 << 30, top_r = 1 << 30, top_i = 1 << 30, bot_c = -1, bot_r = -1, bot_i = -1;
+  int top[3] = {1 << 30, 1 << 30, 1 << 30}, bot[3] = {-1, -1, -1};
   for (int k = lane; k < nk; k += LANES) {
-    if (dge(in.qc[co + k], C::QSMALL)) { top_c = min(top_c, k); bot_c = k; }
-    if (dge(in.qr[co + k], C::QSMALL)) { top_r = min(top_r, k); bot_r = k; }
-    if (dge(in.qi[co + k], C::QSMALL)) { top_i = min(top_i, k); bot_i = k; }
+    if (dge(in.qc[co + k], C::QSMALL)) { top[0] = min(top[0], k); bot[0] = k; }
+    if (dge(in.qr[co + k], C::QSMALL)) { top[1] = min(top[1], k); bot[1] = k; }
+    if (dge(in.qi[co + k], C::QSMALL)) { top[2] = min(top[2], k); bot[2] = k; }
   }
-  top_c = group_min_int<LANES>(mask, top_c);
-  top_r = group_min_int<LANES>(mask, top_r);
-  top_i = group_min_int<LANES>(mask, top_i);
-  bot_c = group_max_int<LANES>(mask, bot_c);
-  bot_r = group_max_int<LANES>(mask, bot_r);
-  bot_i = group_max_int<LANES>(mask, bot_i);
-  const int k_first = min(top_c, min(top_r, top_i));
+  if (SPLIT && lane < 3) gs->prt[lane] = 0;
+  group_bounds<LANES, SPLIT>(mask, gs, top, bot);
+  const int k_first = min(top[0], min(top[1], top[2]));
   for (int k = k_first + lane; k < nk; k += LANES) {
     const double coef = C::gravit * rcp_newton(in.dpres[co + k]);
     INVDZf[k] = 1.0f / float(in.dz[co + k]);
@@ -1738,6 +1838,8 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
     const float* const facp = scr_f(in, sfac, col);
     const int nfield = sp == 0 ? (predictNc ? 2 : 1) : (sp == 1 ? 2 : 4);
     const int nstate = sp == 2 ? 4 : 2; /* fields that limiters may rewrite */
+    /* (the species of a split group run at once: the rows are the ice's) */
+    constexpr bool kDefer = sp == 2 || (sp == 1 && !SPLIT);
     float* const late_vn = scr_f(in, S_RHO, col) + in.ld;
     float* const late_gh = scr_f(in, S_RHOFACR, col) + in.ld;
     float* const late_gl = scr_f(in, S_RHOFACI, col) + in.ld;
@@ -1777,8 +1879,8 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
       r_set(f, k, __fmul_rn(v, cldf));
     };
 
-    const int k_qxtop = sp == 0 ? top_c : (sp == 1 ? top_r : top_i);
-    int k_qxbot = sp == 0 ? bot_c : (sp == 1 ? bot_r : bot_i);
+    const int k_qxtop = top[sp];
+    int k_qxbot = bot[sp];
     if (k_qxbot < 0) return; /* species absent (group-uniform) */
     /* the walk and the rebuild read G one level above the top */
     for (int k = max(k_qxtop - 1, 0) + lane; k < nk; k += LANES) {
@@ -1788,7 +1890,7 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
         R01[k] = make_float2(float(B0[co + k]), float(B1[co + k]));
         CLDf[k] = float(cldp[co + k]);
         FACf[k] = facp[k];
-        if (sp != 0) late_vn[k] = kNotLate;
+        if (kDefer) late_vn[k] = kNotLate;
         if (sp == 2) {
           R23[k] = make_float2(float(B2[co + k]), float(B3[co + k]));
           late_vb[k] = kNotLate;
@@ -1798,7 +1900,7 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
     if (sp == 1) {
       for (int k = k_qxtop + 1 + lane; k <= nk; k += LANES) PF[k] = make_float2(0.f, 0.f);
     }
-    __syncwarp(mask);
+    group_sync<LANES, SPLIT>(mask);
 
     /* The substep schedule is FP32 scalar work: one dt_sub scales every face
      * flux of a substep alike, so its rounding only changes that substep's
@@ -1865,7 +1967,13 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
             lookup3<float>(mu_r, lamr, rt, t3);
             v1 = apply_table3<float>(tb, tb.vm, t3) * FACf[k];
             v2 = apply_table3<float>(tb, tb.vn, t3) * FACf[k];
-            if (n_out != n_plain) defer_state(1, k, n_out, cldf);
+            if (n_out != n_plain) {
+              if constexpr (kDefer) {
+                defer_state(1, k, n_out, cldf);
+              } else {
+                set_state(1, k, n_out, cldf);
+              }
+            }
             fall = true;
           }
         } else {
@@ -1912,7 +2020,7 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
       if (k_qxbot < kbot && lane == (k_qxbot + 1 - k_qxtop) % LANES) {
         V12[k_qxbot + 1] = make_float2(0.f, 0.f); /* the cell receiving the leading edge has no fall speed */
       }
-      const float Co_max = group_max_nn<LANES>(mask, lmax) * dt_left;
+      const float Co_max = group_max_wide<LANES, SPLIT>(mask, gs, lmax) * dt_left;
       if (!(Co_max >= 0.0f) || Co_max > 2.0e9f) {
         err |= kErrNumeric;
         break;
@@ -1937,11 +2045,21 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
           if (nfield > 2) f23 = __fmul2_rn(__fmul2_rn(f2splat(v.x), R23[k]), rho2);
         }
         float2 u01, u23 = make_float2(0.f, 0.f);
-        u01.x = __shfl_up_sync(mask, f01.x, 1, LANES);
-        u01.y = nfield > 1 ? __shfl_up_sync(mask, f01.y, 1, LANES) : 0.f;
+        u01.x = __shfl_up_sync(mask, f01.x, 1, kWarp);
+        u01.y = nfield > 1 ? __shfl_up_sync(mask, f01.y, 1, kWarp) : 0.f;
         if (nfield > 2) {
-          u23.x = __shfl_up_sync(mask, f23.x, 1, LANES);
-          u23.y = __shfl_up_sync(mask, f23.y, 1, LANES);
+          u23.x = __shfl_up_sync(mask, f23.x, 1, kWarp);
+          u23.y = __shfl_up_sync(mask, f23.y, 1, kWarp);
+        }
+        if constexpr (LANES > 32) {
+          float4* const edge = reinterpret_cast<float4*>(gs->edge[group_warp<LANES>()]);
+          if ((lane & 31) == 31) *edge = make_float4(f01.x, f01.y, f23.x, f23.y);
+          group_sync<LANES, SPLIT>(mask);
+          if ((lane & 31) == 0 && lane > 0) {
+            const float4 u = *reinterpret_cast<const float4*>(gs->edge[group_warp<LANES>() - 1]);
+            u01 = make_float2(u.x, u.y);
+            u23 = make_float2(u.z, u.w);
+          }
         }
         if (lane == 0) {
           u01 = c01;
@@ -1958,24 +2076,25 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
           if (sp == 1) dfloat_add(PF[k + 1], f01.x);
         }
         if (base + LANES <= k_temp) {
-          c01.x = __shfl_sync(mask, f01.x, LANES - 1, LANES);
-          c01.y = nfield > 1 ? __shfl_sync(mask, f01.y, LANES - 1, LANES) : 0.f;
+          c01.x = __shfl_sync(mask, f01.x, kWarp - 1, kWarp);
+          c01.y = nfield > 1 ? __shfl_sync(mask, f01.y, kWarp - 1, kWarp) : 0.f;
           if (nfield > 2) {
-            c23.x = __shfl_sync(mask, f23.x, LANES - 1, LANES);
-            c23.y = __shfl_sync(mask, f23.y, LANES - 1, LANES);
+            c23.x = __shfl_sync(mask, f23.x, kWarp - 1, kWarp);
+            c23.y = __shfl_sync(mask, f23.y, kWarp - 1, kWarp);
           }
         }
       }
       if (k_qxbot < kbot) k_qxbot += 1;
       dt_left -= dt_sub;
       first = false;
-      __syncwarp(mask); /* G of the level above is read by set_state */
+      group_sync<LANES, SPLIT>(mask); /* G of the level above is read by set_state */
     }
-    __syncwarp(mask);
+    group_sync<LANES, SPLIT>(mask);
     /* the bottom face's integral is what left the column: V is zero at the
      * leading edge, so G_kbot gains only in substeps where the species
      * reaches the surface */
     const double prt_accum = g_value(0, kbot);
+    if (SPLIT && lane == 0) gs->prt[sp] = prt_accum;
     if (sp == 0) precip_liq_surf = prt_accum * C::INV_RHO_H2O * inv_dt;
     else if (sp == 1) precip_liq_surf += prt_accum * C::INV_RHO_H2O * inv_dt;
     else precip_ice_surf += prt_accum * C::INV_RHO_H2O * inv_dt;
@@ -1992,11 +2111,12 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
       for (int f = 0; f < 4; ++f) {
         if (f < nstate) {
           const double g = act ? g_value(f, k) : 0.0;
-          double gin = __shfl_up_sync(mask, g, 1, LANES);
+          double gin = __shfl_up_sync(mask, g, 1, kWarp);
           if (lane == 0) gin = g_in[f];
+          if (LANES > 32 && (lane & 31) == 0 && lane > 0 && act) gin = g_value(f, k - 1);
           if (act) {
             double B = Bf[f][co + k];
-            if (sp != 0 && (f == 1 || f == 3)) {
+            if (kDefer && (f == 1 || f == 3)) {
               const float v = f == 1 ? late_vn[k] : late_vb[k];
               if (__float_as_uint(v) != 0xffc0deadu) {
                 const float2 g0 = make_float2(__int_as_float(__double2loint(B)), __int_as_float(__double2hiint(B)));
@@ -2012,7 +2132,7 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
             }
             Bf[f][co + k] = B + COEF[k] * (gin - g);
           }
-          g_in[f] = __shfl_sync(mask, g, LANES - 1, LANES);
+          g_in[f] = __shfl_sync(mask, g, kWarp - 1, kWarp);
         }
       }
     }
@@ -2020,12 +2140,26 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
       /* interfaces above the top stay at part1's zero */
       for (int k = k_qxtop + 1 + lane; k <= nk; k += LANES) in.precip_liq_flux[ci + k] = dfloat_value(PF[k]);
     }
-    __syncwarp(mask);
+    group_sync<LANES, SPLIT>(mask);
   };
-  species(std::integral_constant<int, 0>{});
-  species(std::integral_constant<int, 1>{});
-  species(std::integral_constant<int, 2>{});
-  if (lane == 0) {
+  if constexpr (SPLIT) {
+    const int sp = int(threadIdx.x) / LANES;
+    if (sp == 0) species(std::integral_constant<int, 0>{});
+    else if (sp == 1) species(std::integral_constant<int, 1>{});
+    else species(std::integral_constant<int, 2>{});
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      /* thread 0 belongs to the first group: gs[0], gs[1], gs[2] are the three */
+      precip_liq_surf = gs[0].prt[0] * C::INV_RHO_H2O * inv_dt;
+      precip_liq_surf += gs[1].prt[1] * C::INV_RHO_H2O * inv_dt;
+      precip_ice_surf = gs[2].prt[2] * C::INV_RHO_H2O * inv_dt;
+    }
+  } else {
+    species(std::integral_constant<int, 0>{});
+    species(std::integral_constant<int, 1>{});
+    species(std::integral_constant<int, 2>{});
+  }
+  if (SPLIT ? threadIdx.x == 0 : lane == 0) {
     in.precip_liq_surf[col] = precip_liq_surf;
     in.precip_ice_surf[col] = precip_ice_surf;
   }
@@ -2392,9 +2526,48 @@ __global__ void __maxnreg__(96) p3_sed_kernel(const Inst inst0, const KParams<TR
   for_each_work<LANES>(kp.wctr ? kp.wctr + 1 : nullptr, kp.nwork, kp.groups_per_block, [&](int w) {
     int col;
     const Inst& in = work_inst(inst0, kp, w, col);
-    p3_sed<TR, LANES>(in, col, kp, tb, sm, err);
+    p3_sed<TR, LANES>(in, col, kp, tb, sm, nullptr, err);
   });
   if (err) atomicOr(kp.err, err);
+}
+
+/* K2 with a CTA per column, for calls whose columns leave most warps idle
+ * (sed_wide_lanes): every level has its own thread of LANES, so a substep costs
+ * one fall-speed pass and one flux pass instead of one of each per 32 levels,
+ * and with SPLIT the three species, which are independent, run at once.  The
+ * calls it is for are bound by the latency of the slowest column's substeps:
+ * 64 x 72 FP64 152 -> 109 us, with SPLIT 70 us; FP32-bulk 70 -> 50 -> 33 us. */
+template <int LANES, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 3 * LANES : LANES)
+    p3_sed_wide_kernel(const Inst inst0, const KParams<double> kp) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  uint32_t err = 0;
+  Tabs<double> tb;
+  setup_tables<double>(kp, false, smem_raw, tb, err);
+  constexpr int kGroups = SPLIT ? 3 : 1;
+  const int g = SPLIT ? int(threadIdx.x) / LANES : 0;
+  GroupScratch* const gs = reinterpret_cast<GroupScratch*>(smem_raw);
+  double* const sm = reinterpret_cast<double*>(smem_raw + kGroups * sizeof(GroupScratch)) +
+                     size_t(g) * sed_slots<double>() * kp.sm_stride;
+  int col;
+  const Inst& in = work_inst(inst0, kp, int(blockIdx.x), col);
+  p3_sed<double, LANES, SPLIT>(in, col, kp, tb, sm, gs + g, err);
+  if (err) atomicOr(kp.err, err);
+}
+
+/* Tables of the FP32-bulk sedimentation: compact copies, so that the lookups
+ * of the substep walk stay in the L1 data cache beside the CTAs' shared memory:
+ * the four ice-table columns of sedimentation (16 KB) and the two-column
+ * Table3 slices of the rain shape (2.4 KB each) rather than the full tables
+ * (48 KB and 12 KB). */
+__device__ __forceinline__ void sed_tables(const KParams<float>& kp, Tabs<float>& tb) {
+  tb.collect = kp.collect;
+  tb.ice = kp.ice_sed;
+  tb.vn = kp.t3slice;
+  tb.vm = kp.t3slice + kT3SliceElems / 3;
+  tb.revap = kp.t3slice + 2 * (kT3SliceElems / 3);
+  tb.t3_stride = 2;
+  tb.t3_j0 = kp.rt.t3_dumjj - 1;
 }
 
 /* K2 of the FP32-bulk form.  STAGED: one CTA of up to 20 columns per SM with
@@ -2410,18 +2583,8 @@ template <int LANES, bool STAGED>
 __global__ void __maxnreg__(96) p3_sed_bulk_kernel(const Inst inst0, const KParams<float> kp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint32_t err = 0;
-  /* Compact tables, so that the lookups of the substep walk stay in the L1
-   * data cache beside the CTAs' shared memory: the four ice-table columns of
-   * sedimentation (16 KB) and the two-column Table3 slices of the rain
-   * shape (2.4 KB each) rather than the full tables (48 KB and 12 KB). */
   Tabs<float> tb;
-  tb.collect = kp.collect;
-  tb.ice = kp.ice_sed;
-  tb.vn = kp.t3slice;
-  tb.vm = kp.t3slice + kT3SliceElems / 3;
-  tb.revap = kp.t3slice + 2 * (kT3SliceElems / 3);
-  tb.t3_stride = 2;
-  tb.t3_j0 = kp.rt.t3_dumjj - 1;
+  sed_tables(kp, tb);
   unsigned char* columns = smem_raw;
   if constexpr (STAGED) {
     /* ice table, then vn and vm (sed_table_bytes) */
@@ -2442,8 +2605,27 @@ __global__ void __maxnreg__(96) p3_sed_bulk_kernel(const Inst inst0, const KPara
   for_each_work<LANES>(kp.wctr ? kp.wctr + 1 : nullptr, kp.nwork, kp.groups_per_block, [&](int w) {
     int col;
     const Inst& in = work_inst(inst0, kp, w, col);
-    p3_sed_bulk<LANES>(in, col, kp, tb, sm, err);
+    p3_sed_bulk<LANES>(in, col, kp, tb, sm, nullptr, err);
   });
+  if (err) atomicOr(kp.err, err);
+}
+
+/* p3_sed_wide_kernel of the FP32-bulk form */
+template <int LANES, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 3 * LANES : LANES)
+    p3_sed_bulk_wide_kernel(const Inst inst0, const KParams<float> kp) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  uint32_t err = 0;
+  Tabs<float> tb;
+  sed_tables(kp, tb);
+  constexpr int kGroups = SPLIT ? 3 : 1;
+  const int g = SPLIT ? int(threadIdx.x) / LANES : 0;
+  GroupScratch* const gs = reinterpret_cast<GroupScratch*>(smem_raw);
+  double* const sm = reinterpret_cast<double*>(smem_raw + kGroups * sizeof(GroupScratch)) +
+                     size_t(g) * sed_slots<float>() * kp.sm_stride;
+  int col;
+  const Inst& in = work_inst(inst0, kp, int(blockIdx.x), col);
+  p3_sed_bulk<LANES, SPLIT>(in, col, kp, tb, sm, gs + g, err);
   if (err) atomicOr(kp.err, err);
 }
 

@@ -52,7 +52,10 @@ cudaError_t launch_p3_part(const dev::Inst& inst0, const dev::KParams<TR>& kp_in
     if (e == cudaSuccess && ls.marks) cudaEventRecord(ls.marks[1], stream);
   } else if (part == kPartK2) {
     if constexpr (LANES == 32) {
-      if constexpr (sizeof(TR) == sizeof(float)) {
+      const int wide = kp.wctr ? sed_wide_lanes(kp.nwork, kp.nlev_max, num_sms) : 0;
+      if (wide) {
+        e = launch_sed_wide<TR>(inst0, kp, wide, num_sms, stream);
+      } else if constexpr (sizeof(TR) == sizeof(float)) {
         const int per_sm = sed_staged_columns(kp.sm_stride);
         if (kp.wctr && per_sm > 0 && kp.nwork >= per_sm * num_sms) {
           kp.groups_per_block = per_sm;

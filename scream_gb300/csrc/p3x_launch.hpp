@@ -47,6 +47,20 @@ inline LaunchSpec sed_spec(const LaunchSpec& ls) {
   return s;
 }
 
+/* Threads per column of K2 where a call leaves most warps idle: a CTA of 128
+ * or 256 threads (at least the column's levels) per column while at most 32
+ * warps an SM result; 0: 32 lanes per column.  Measured, CTA per column against
+ * 32 lanes: 608 x 128 FP64 220 / 351 us, FP32-bulk 82 / 140; 1,216 x 128 330 /
+ * 388 and 109 / 156; 1,520 x 72 213 / 180 and 85 / 75. */
+inline int sed_wide_lanes(int nwork, int nlev_max, int num_sms) {
+  const int lanes = nlev_max <= 128 ? 128 : (nlev_max <= 256 ? 256 : 0);
+  return lanes && nlev_max > 32 && (long long)nwork * (lanes / 32) <= (long long)num_sms * 32 ? lanes : 0;
+}
+/* Launch of K2 with a CTA per column (p3x_k_dwide.cu, p3x_k_fwide.cu). */
+template <class TR>
+cudaError_t launch_sed_wide(const dev::Inst& inst0, const dev::KParams<TR>& kp, int lanes, int num_sms,
+                            cudaStream_t stream);
+
 /* Columns of one CTA of the FP32-bulk sedimentation that keeps its tables in
  * shared memory, one CTA per SM: as many as fit beside the 20.8 KB of tables, 20
  * at most (96 registers a thread).  0 where that is fewer than 16. */
