@@ -225,7 +225,7 @@ bool spec_fits(int precision, const LaunchSpec& ls, int stride) {
   if (ls.lanes != 8 && ls.lanes != 16 && ls.lanes != 32) return false;
   if (ls.groups_per_block <= 0 || ls.groups_per_block * ls.lanes > 256) return false;
   const bool f32 = precision == P3X_FP32_BULK;
-  const size_t k1 = f32 ? p3_smem_bytes<float>(ls, stride) : p3_smem_bytes<double>(ls, stride);
+  const size_t k1 = f32 ? p3_smem_bytes<float>(ls, stride - 1) : p3_smem_bytes<double>(ls, stride - 1);
   const LaunchSpec ls2 = sed_spec(ls);
   const size_t k2 = f32 ? sed_smem_bytes<float>(ls2, stride) : sed_smem_bytes<double>(ls2, stride);
   return k1 <= size_t(227 * 1024) && k2 <= size_t(227 * 1024);
@@ -672,12 +672,9 @@ int p3x_context_create(const char* table_file, p3x_context** out, int* info) {
       return P3X_ECUDA;
     }
   }
-  /* 4 columns per CTA with the tables read through L1: part1+part2 then fits
-   * two CTAs per SM (staging the tables in shared memory leaves room for one),
-   * measured faster in both forms; staging remains a launch option.  The FP64
-   * part1+part2 (254 registers) keeps twice the columns in flight at 16 lanes
-   * per column and ran 7 % faster there (sedimentation stays at 32). */
-  ctx->cfg[P3X_FP64] = p3x_launch_config{16, 4, 0, 0};
+  /* CTAs of 4 warps with the tables read through L1: staging them in shared
+   * memory measured slower in both forms and remains a launch option. */
+  ctx->cfg[P3X_FP64] = p3x_launch_config{32, 4, 0, 0};
   ctx->cfg[P3X_FP32_BULK] = p3x_launch_config{32, 4, 0, 0};
   /* reserve the fixed hand-over scratch of p3x_main_fixed_scratch on this
    * device now (see g_step_scratch) */
@@ -1563,8 +1560,8 @@ int p3x_batch_destroy(p3x_batch* b) {
 }
 
 /* Times every candidate configuration on the batch and keeps the fastest.
- * The sweep covers threads per column (8, 16, 32 lanes, i.e. nlev/8 .. nlev/32
- * levels per thread), columns per CTA and staging of the ice / Table3 tables
+ * The sweep covers lanes per column (8, 16, 32: the pool size of part1+2),
+ * columns per CTA and staging of the ice / Table3 tables
  * into shared memory.  Each timed run advances the batch's instances by one
  * step. */
 int p3x_autotune_batch(p3x_batch* b, void* stream, int32_t reps, p3x_launch_config* best, double* ms_best) {

@@ -1,30 +1,31 @@
 /*
  * The P3 step as three column kernels.
  *
- * One group of LANES threads (8, 16 or 32; a warp or part of one) owns one
- * column at a time; lane l owns levels l, l+LANES, l+2*LANES, ...  Inputs
- * are level-contiguous (EAMxx layout), so a group's loads of one field are
- * coalesced.  The reference's stage order (p3/impl/p3_main_impl.hpp:108-325)
- * is kept across three launches on one stream:
+ * Inputs are level-contiguous (EAMxx layout): the lanes of a warp take
+ * neighbouring levels, so loads of one field are coalesced.  The reference's
+ * stage order (p3/impl/p3_main_impl.hpp:108-325) is kept across three launches
+ * on one stream:
  *
  *   K1 p3_part12_kernel: p3_main_init + p3_main_part1 and p3_main_part2
- *      (level-parallel), with the two column-wide early exits of
- *      p3_main_impl.hpp:237-239 and :260 as group ballots.  It hands the
- *      per-level start-of-step temperature, density and fall-speed factors
- *      to K2/K3 through a scratch array and marks each column that goes on.
- *   K2 p3_sed_kernel: cloud, rain and ice sedimentation: CFL substeps with
- *      the Courant maximum as a group shuffle reduction and the upwind flux
- *      divergence walked down the levels chunk by chunk with a shuffle-up and
- *      a carry (p3_upwind_impl.hpp:14-116).  Substep loops are capped.
+ *      (level-parallel; a warp takes a pool of columns, a CTA one column where
+ *      a call is small), with the two column-wide early exits of
+ *      p3_main_impl.hpp:237-239 and :260.  It hands the per-level
+ *      start-of-step temperature, density and fall-speed factors to K2/K3
+ *      through a scratch array and marks each column that goes on.
+ *   K2 p3_sed_kernel: cloud, rain and ice sedimentation, a column to a warp or,
+ *      where a call is small, to a CTA: CFL substeps with the Courant maximum
+ *      as a group reduction and the upwind flux divergence walked down the
+ *      levels chunk by chunk with a shuffle-up and a carry
+ *      (p3_upwind_impl.hpp:14-116).  Substep loops are capped.
  *   K3 p3_part3_kernel: homogeneous freezing + p3_main_part3.
  *
  * Splitting lets each kernel keep its own register and shared-memory
  * footprint: part2's ~45 rates no longer limit the occupancy of the
- * latency-bound sedimentation walk.  Per-level temporaries of a phase live
- * in shared memory (9 FP64 arrays per column in K1, 11 in K2).  Lookup
- * tables are read from global memory (L1/L2) or, in K1, staged into shared
- * memory once per CTA with cp.async.bulk + mbarrier (Table3 slices for the
- * runtime's constant rain shape parameter, plus the whole ice table).
+ * latency-bound sedimentation walk.  K1 keeps only its level lists in shared
+ * memory, K2 its per-level arrays (9 or 10 slots of FP64 width per column).
+ * Lookup tables are read from global memory (L1/L2) or, in K1, staged into
+ * shared memory once per CTA with cp.async.bulk + mbarrier (Table3 slices for
+ * the runtime's constant rain shape parameter, plus the whole ice table).
  */
 #pragma once
 
@@ -59,6 +60,21 @@ struct WorkItem {
   int32_t inst, col;
 };
 
+/* K1: level lists of a pool of columns, entries (column of the pool, level) */
+constexpr int kPoolTiers = 5; /* pools of 16, 8, 4, 2, 1 columns */
+constexpr int kPoolMaxCols = 1 << (kPoolTiers - 1);
+constexpr int kPoolLevelBits = 12;
+constexpr int kPart12WideThreads = 128;
+/* what the warps of a CTA share where they work on one column */
+struct PoolScratch {
+  uint32_t n_hyd, n_nuc, active;
+};
+/* deeper columns than that do not fit K2's shared memory either */
+static_assert(kPoolMaxCols << kPoolLevelBits == 1 << 16, "16-bit entries");
+__host__ __device__ constexpr size_t pool_list_entries(int cols, int nlev_max) {
+  return (size_t(cols) * size_t(nlev_max) + 7) / 8 * 8;
+}
+
 template <class TR>
 struct KParams {
   RuntimeDev rt;
@@ -82,6 +98,9 @@ struct KParams {
   int nwork;         /* number of columns (single) or work items (batched) */
   int nlev_max;      /* levels of the deepest column */
   int part3_split;   /* K3: groups that share a work item's levels */
+  int pool_cols;     /* K1: columns of the largest pool */
+  int npools;        /* K1: pools */
+  int pool_end[kPoolTiers - 1]; /* K1: pools of pool_cols columns, of those and half that, ... (running totals) */
   const WorkItem* work;
   const Inst* insts;
   uint32_t* err;
@@ -119,9 +138,6 @@ constexpr int kMaxSubsteps = 100000;
 constexpr long long kWaitSpinLimit = 1ll << 26;
 constexpr uint64_t kWaitNanosLimit = 2000000000ull; /* 2 s */
 
-/* shared arrays of one column group in K1 */
-enum { A_TATM = 0, A_RHO, A_RHOFACR, A_RHOFACI, A_ACN, A_QVSL, A_QVSI, A_QVSSI, A_EPINVP, A_NARR };
-constexpr int A_LIST = A_EPINVP; /* FP64 form: the level lists (16-bit entries) */
 /* shared arrays of one column group in K2 (FP64 form, p3_sed); the rain flux
  * accumulator re-uses R2 (rain has two fields) */
 enum { B_FR = 0, B_CF, B_QS, B_V1, B_V2, B_R0, B_R1, B_R2, B_R3, B_NARR };
@@ -165,24 +181,13 @@ __host__ __device__ constexpr size_t table_smem_bytes() {
 /* ------------------------------------------------------------------ */
 /* group primitives                                                    */
 /* ------------------------------------------------------------------ */
-template <int LANES>
-__device__ __forceinline__ unsigned group_mask() {
-  if (LANES >= 32) return 0xffffffffu;
-  const unsigned lw = threadIdx.x & 31u;
-  return (0xffffffffu >> (32 - LANES)) << (lw & ~unsigned(LANES - 1));
-}
-template <int LANES>
-__device__ __forceinline__ bool group_any(unsigned mask, bool p) {
-  return __ballot_sync(mask, p) != 0u;
-}
 /* Maxima and minima over the group with the warp-reduction instruction
- * (redux.sync), one instruction instead of log2(LANES) dependent shuffles.
+ * (redux.sync), one instruction instead of five dependent shuffles.
  * Non-negative floats and doubles order as their bit patterns (as unsigned
  * integers), so their maximum is the maximum of the patterns; a NaN (a
  * pattern above +inf) wins and reaches the caller's Courant check. */
 /* maximum over the group of non-negative doubles (dmax_nn): the largest high
  * word, then the largest low word among the lanes holding it */
-template <int LANES>
 __device__ __forceinline__ double group_max_nn(unsigned mask, double v) {
   const unsigned hi = unsigned(__double2hiint(v)), lo = unsigned(__double2loint(v));
   const unsigned mhi = __reduce_max_sync(mask, hi);
@@ -190,20 +195,17 @@ __device__ __forceinline__ double group_max_nn(unsigned mask, double v) {
   return __hiloint2double(int(mhi), int(mlo));
 }
 /* maximum over the group of non-negative floats (Courant numbers) */
-template <int LANES>
 __device__ __forceinline__ float group_max_nn(unsigned mask, float v) {
   return __uint_as_float(__reduce_max_sync(mask, __float_as_uint(v)));
 }
-template <int LANES>
 __device__ __forceinline__ int group_min_int(unsigned mask, int v) {
   return __reduce_min_sync(mask, v);
 }
-template <int LANES>
 __device__ __forceinline__ int group_max_int(unsigned mask, int v) {
   return __reduce_max_sync(mask, v);
 }
 
-/* Sedimentation also runs groups of several warps, LANES > 32 threads (at least
+/* A sedimentation group is a warp or several, LANES > 32 threads (at least
  * as many as the column has levels): the warps of a group exchange through this
  * shared scratch and meet at a barrier.  SPLIT: a CTA has three such groups,
  * one per species, each with its own scratch and barrier (named 1 to 3);
@@ -233,11 +235,10 @@ __device__ __forceinline__ int group_warp() {
 /* Tops (minima) and bottoms (maxima) of the three species over the group. */
 template <int LANES, bool SPLIT>
 __device__ __forceinline__ void group_bounds(unsigned mask, GroupScratch* gs, int lo[3], int hi[3]) {
-  constexpr int kWarp = LANES < 32 ? LANES : 32;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    lo[i] = group_min_int<kWarp>(mask, lo[i]);
-    hi[i] = group_max_int<kWarp>(mask, hi[i]);
+    lo[i] = group_min_int(mask, lo[i]);
+    hi[i] = group_max_int(mask, hi[i]);
   }
   if constexpr (LANES > 32) {
     const int w = group_warp<LANES>();
@@ -258,7 +259,7 @@ __device__ __forceinline__ void group_bounds(unsigned mask, GroupScratch* gs, in
 /* maximum of non-negative values over the group */
 template <int LANES, bool SPLIT>
 __device__ __forceinline__ double group_max_wide(unsigned mask, GroupScratch* gs, double v) {
-  v = group_max_nn<LANES < 32 ? LANES : 32>(mask, v);
+  v = group_max_nn(mask, v);
   if constexpr (LANES > 32) {
     if ((threadIdx.x & 31) == 0) gs->max_d[group_warp<LANES>()] = v;
     group_sync<LANES, SPLIT>(mask);
@@ -268,7 +269,7 @@ __device__ __forceinline__ double group_max_wide(unsigned mask, GroupScratch* gs
 }
 template <int LANES, bool SPLIT>
 __device__ __forceinline__ float group_max_wide(unsigned mask, GroupScratch* gs, float v) {
-  v = group_max_nn<LANES < 32 ? LANES : 32>(mask, v);
+  v = group_max_nn(mask, v);
   if constexpr (LANES > 32) {
     if ((threadIdx.x & 31) == 0) gs->max_f[group_warp<LANES>()] = v;
     group_sync<LANES, SPLIT>(mask);
@@ -382,63 +383,123 @@ __device__ __forceinline__ bool clip_to_vapour(State& s, double inv_exner) {
   return hydro;
 }
 
-/* What part1 and part2 need to know of a level without hydrometeors below
- * freezing, where FP32 can tell: `counts`, whether its supersaturation over
- * ice is at least -0.05 (the column then goes on to part2), and that ice does
- * not nucleate there (that takes T < Tmelt - 15 and a supersaturation of 0.05).
- * The FP32 Murphy-Koop formula is good to 1e-4 of the ratio, the margins are
- * ten times that; false: the exact value has to decide. */
-__device__ __forceinline__ bool dry_level_known(double T, float tf, float qv, float p, bool& counts) {
+/* Whether a level without hydrometeors below freezing may nucleate ice, which
+ * takes T < Tmelt - 15 and a supersaturation over ice of 0.05.  The FP32
+ * Murphy-Koop formula is good to 1e-4 of the ratio and the margin is ten times
+ * that; true wherever FP32 cannot exclude it (also below 150 K and for NaN). */
+__device__ __forceinline__ bool may_nucleate(double T, float tf, float qv, float p) {
+  if (dgt(T, C::Tmelt - 14.9)) return false;
   const float e = __expf(9.550426f - 5723.265f / tf + 3.53068f * __logf(tf) - 0.00728332f * tf);
-  const float ss = qv * p / (float(C::ep_2) * e) - 1.0f;
-  const bool high = ss > -0.049f;
-  const bool known = dgt(T, 150.0) && (ss < -0.051f || (high && (ss < 0.049f || dgt(T, C::Tmelt - 14.9))));
-  counts = known && high;
-  return known;
+  return !(dgt(T, 150.0) && qv * p / (float(C::ep_2) * e) - 1.0f < 0.049f);
 }
 
-/* p3_main_part2 of one level in the FP32-bulk form (p3_main_part2_impl.hpp,
+__device__ __forceinline__ void store_state(const Inst& in, const int64_t o, const State& s) {
+  in.qc[o] = s.qc; in.nc[o] = s.nc; in.qr[o] = s.qr; in.nr[o] = s.nr;
+  in.qi[o] = s.qi; in.qm[o] = s.qm; in.ni[o] = s.ni; in.bm[o] = s.bm;
+  in.qv[o] = s.qv; in.th[o] = s.th;
+}
+__device__ __forceinline__ void load_state(const Inst& in, const int64_t o, State& s) {
+  s.qc = in.qc[o]; s.nc = in.nc[o]; s.qr = in.qr[o]; s.nr = in.nr[o];
+  s.qi = in.qi[o]; s.qm = in.qm[o]; s.ni = in.ni[o]; s.bm = in.bm[o];
+  s.qv = in.qv[o]; s.th = in.th[o];
+}
+
+/* The species below their thresholds at the start of a level's part1: to
+ * vapour (or, small ice above freezing, to rain), and the droplet number of a
+ * level that keeps its cloud (`activated`).  A +0 moves nothing, so its FP64
+ * updates are skipped (bitwise the same result).  Returns whether the potential
+ * temperature changed. */
+template <class F>
+__device__ __forceinline__ bool part1_thresholds(State& s, double T, double inv_exner, double qvssi, F&& activated) {
+  bool th_changed = false;
+  if (dlt(s.qc, C::QSMALL)) {
+    if (dnz(s.qc)) {
+      s.qv = s.qv + s.qc;
+      s.th = s.th - inv_exner * s.qc * C::LatVap * C::INV_CP;
+      th_changed = true;
+    }
+    s.qc = 0;
+    s.nc = 0;
+  } else {
+    s.nc = activated(s.nc);
+  }
+  if (dlt(s.qr, C::QSMALL)) {
+    if (dnz(s.qr)) {
+      s.qv = s.qv + s.qr;
+      s.th = s.th - inv_exner * s.qr * C::LatVap * C::INV_CP;
+      th_changed = true;
+    }
+    s.qr = 0;
+    s.nr = 0;
+  }
+  if (dlt(s.qi, C::QSMALL) || (dlt(s.qi, 1.e-8) && dlt_neg(qvssi, -0.1))) {
+    if (dnz(s.qi)) {
+      s.qv = s.qv + s.qi;
+      s.th = s.th - inv_exner * s.qi * (C::LatVap + C::LatIce) * C::INV_CP;
+      th_changed = true;
+    }
+    s.qi = 0; s.ni = 0; s.qm = 0; s.bm = 0;
+  }
+  if (dge(s.qi, C::QSMALL) && dlt(s.qi, 1.e-8) && dge(T, C::T_zerodegc)) {
+    s.qr = s.qr + s.qi;
+    s.th = s.th - inv_exner * s.qi * C::LatIce * C::INV_CP;
+    th_changed = true;
+    s.qi = 0; s.ni = 0; s.qm = 0; s.bm = 0;
+  }
+  return th_changed;
+}
+
+/* Saturation, the rest of p3_main_part1 and p3_main_part2 of one level with a
+ * hydrometeor in the FP32-bulk form (p3_main_part2_impl.hpp,
  * same order of processes).  The FP64 state is read once and shadowed in
  * FP32; the in-cloud values, DSDs, table lookups, process rates and limiter
  * ratios are FP32, while the thresholds test the FP64 state.  The vapour
  * residuals, the melting / wet-growth departures and the state update are
  * FP64.  A DSD or rime limiter that changes an in-cloud value rewrites the
- * FP64 state and its shadow.  sm / S: the K1 shared arrays of the column. */
-__device__ __forceinline__ void part2_level_bulk(const Inst& in, const int64_t o, const int k,
-                                                 double* __restrict__ sm, const int S, const KParams<float>& kp,
-                                                 const Tabs<float>& tb, const float dtf,
-                                                 const float inv_dtf, bool& hydro, uint32_t& err) {
+ * FP64 state and its shadow. */
+__device__ __forceinline__ void hydro_level_bulk(const Inst& in, const int col, const int k, const KParams<float>& kp,
+                                                 const Tabs<float>& tb, const float dtf, const float inv_dtf,
+                                                 bool& hydro, uint32_t& err) {
   const RuntimeDev& rt = kp.rt;
   const bool predictNc = in.predictNc != 0, prescribedCCN = in.prescribedCCN != 0;
   const bool do_ice = rt.do_ice_production != 0;
   const double inv_dt_d = f2d(inv_dtf);
-  const float* const smf_rho = reinterpret_cast<const float*>(&sm[A_RHO * S]);
-  const float* const smf_rhofaci = reinterpret_cast<const float*>(&sm[A_RHOFACI * S]);
-  const float* const smf_acn = reinterpret_cast<const float*>(&sm[A_ACN * S]);
+  const int64_t o = int64_t(col) * in.ld + k;
+  const float rho = scr_f(in, S_RHO, col)[k], rhofaci = scr_f(in, S_RHOFACI, col)[k], acn = scr_f(in, S_ACN, col)[k];
+  double T = scr_at(in, S_TATM, col)[k];
   State s;
-  s.qc = in.qc[o]; s.nc = in.nc[o]; s.qr = in.qr[o]; s.nr = in.nr[o];
-  s.qi = in.qi[o]; s.qm = in.qm[o]; s.ni = in.ni[o]; s.bm = in.bm[o];
-  s.qv = in.qv[o]; s.th = in.th[o];
-  const double T = sm[A_TATM * S + k];
-  const double qvssi = sm[A_QVSSI * S + k];
-  const bool dry = dlt(s.qc, C::QSMALL) && dlt(s.qr, C::QSMALL) && dlt(s.qi, C::QSMALL);
-  if (dry && dlt(T, C::T_zerodegc) && dlt_neg(qvssi, -0.05)) return;
-  /* A level without hydrometeors where ice cannot nucleate (nucleation
-   * needs T < Tmelt - 15 and qv_supersat_i >= 0.05; the test below leaves a
-   * margin for the float temperature) has no process rate, so the level keeps
-   * its state and every tendency output is the +0 that part1 wrote, except
-   * vap_liq_exchange = -(+0).  With nc diagnosed (neither predicted nor
-   * prescribed) the update resets nc, so that case goes the whole way. */
-  if (dry && (predictNc || prescribedCCN) && !(dlt(T, C::Tmelt - 14.0) && dge(qvssi, 0.04))) {
-    in.vap_liq_exchange[o] = -0.0;
-    return;
+  load_state(in, o, s);
+  const double inv_exner = in.inv_exner[o];
+  /* one Newton reciprocal of the pressure, times ep_2, shared by both
+   * saturation ratios, the melting departure and the supersaturation limiter;
+   * the supersaturation ratio (threshold and rate input) in FP32 */
+  const double ep_inv_p = C::ep_2 * rcp_newton1(dmax_c(in.pres[o], 1.e-3));
+  const double qvsi = __dmul_rn(svp_tabulated(rt.svp_tab, T, true, err), ep_inv_p);
+  const double qvssi = f2d(float(s.qv) / float(qvsi) - 1.0f);
+  const double qvsl = __dmul_rn(svp_tabulated(rt.svp_tab, T, false, err), ep_inv_p);
+  if (part1_thresholds(s, T, inv_exner, qvssi, [&](double nc) {
+        if (prescribedCCN) return vmax(nc, rt.spa_ccn_to_nc_factor * in.nccn[o] * in.cld_frac_l[o]);
+        if (predictNc) return dmax0(nc + in.nc_nuceat_tend[o] * double(in.dt));
+        return __dmul_rn(C::NCCNST, f2d(1.0f / rho));
+      })) {
+    T = __dmul_rn(s.th, rcp_newton1(inv_exner));
+    scr_at(in, S_TATM, col)[k] = T;
+  }
+  if (dlt(s.qc, C::QSMALL) && dlt(s.qr, C::QSMALL) && dlt(s.qi, C::QSMALL)) {
+    /* Without a hydrometeor left and where ice cannot nucleate (that needs
+     * T < Tmelt - 15 and a supersaturation of 0.05; the test leaves a margin for
+     * the float temperature) the level has no process rate: every tendency
+     * output is the +0 of the first pass, except vap_liq_exchange = -(+0). */
+    const bool dry_cold = dlt(T, C::T_zerodegc) && dlt_neg(qvssi, -0.05);
+    if (dry_cold || ((predictNc || prescribedCCN) && !(dlt(T, C::Tmelt - 14.0) && dge(qvssi, 0.04)))) {
+      if (!dry_cold) in.vap_liq_exchange[o] = -0.0;
+      store_state(in, o, s);
+      return;
+    }
   }
 
   const double cld_i = in.cld_frac_i[o], cld_l = in.cld_frac_l[o], cld_r = in.cld_frac_r[o];
-  const double inv_exner = in.inv_exner[o];
-  const double qvsl = sm[A_QVSL * S + k], qvsi = sm[A_QVSI * S + k];
-  const double ep_inv_p = sm[A_EPINVP * S + k]; /* ep_2 / max(p, 1e-3) */
-  const float rho = smf_rho[k], inv_rho = 1.0f / rho, rhofaci = smf_rhofaci[k], acn = smf_acn[k];
+  const float inv_rho = 1.0f / rho;
   const float T_r = float(T), qvsi_r = float(qvsi);
   const float cl = float(cld_l), ci = float(cld_i), cr = float(cld_r);
   const float icl = 1.0f / cl, ici = 1.0f / ci, icr = 1.0f / cr;
@@ -613,36 +674,36 @@ __device__ __forceinline__ void part2_level_bulk(const Inst& in, const int64_t o
     const float f = vmin(rt.f.max_total_ni * inv_rho * ci / float(s.ni), 1.0f);
     if (f < 1.0f) s.ni = s.ni * f2d(f);
   }
-  in.qc[o] = s.qc; in.nc[o] = s.nc; in.qr[o] = s.qr; in.nr[o] = s.nr;
-  in.qi[o] = s.qi; in.qm[o] = s.qm; in.ni[o] = s.ni; in.bm[o] = s.bm;
-  in.qv[o] = s.qv; in.th[o] = s.th;
+  store_state(in, o, s);
 }
 
-/* p3_main_part2 of one level without hydrometeors in the FP32-bulk form,
- * where ice nucleation is the only process that can have a rate: the same
- * operations that part2_level_bulk leaves once every other rate is +0 (a
- * fifth of its FP64 instructions, which it spends on converting and updating
- * a state of zeros). */
-__device__ __forceinline__ void part2_nucleation_bulk(const Inst& in, const int64_t o, const int k,
-                                                      const double* __restrict__ sm, const int S,
+/* Saturation over ice and p3_main_part2 of one level without hydrometeors in
+ * the FP32-bulk form, where ice nucleation is the only process that can have a
+ * rate: the same operations that hydro_level_bulk leaves once every other rate
+ * is +0 (a fifth of its FP64 instructions, which it spends on converting and
+ * updating a state of zeros). */
+__device__ __forceinline__ void nucleation_level_bulk(const Inst& in, const int col, const int k,
                                                       const KParams<float>& kp, const float dtf, const float inv_dtf,
-                                                      bool& hydro) {
+                                                      bool& hydro, uint32_t& err) {
   const RuntimeDev& rt = kp.rt;
   const bool predictNc = in.predictNc != 0, prescribedCCN = in.prescribedCCN != 0;
-  const double T = sm[A_TATM * S + k], qvssi = sm[A_QVSSI * S + k];
+  const int64_t o = int64_t(col) * in.ld + k;
+  const double T = scr_at(in, S_TATM, col)[k];
+  State s;
+  s.qc = s.nc = s.qr = s.nr = s.qm = s.bm = 0.0;
+  s.qv = in.qv[o];
+  const double ep_inv_p = C::ep_2 * rcp_newton1(dmax_c(in.pres[o], 1.e-3));
+  const double qvsi = __dmul_rn(svp_tabulated(rt.svp_tab, T, true, err), ep_inv_p);
+  const double qvssi = f2d(float(s.qv) / float(qvsi) - 1.0f);
   if (!(dlt(T, C::Tmelt - 14.0) && dge(qvssi, 0.04))) return;
-  const float T_r = float(T), inv_rho = 1.0f / reinterpret_cast<const float*>(&sm[A_RHO * S])[k];
+  const float T_r = float(T), inv_rho = 1.0f / scr_f(in, S_RHO, col)[k];
   const float activated = (predictNc && !prescribedCCN) ? float(in.ni_activated[o]) : 0.0f; /* read in that case only */
   Rates<float> r;
   r.zero();
   ice_nucleation<float>(T_r, inv_rho, 0.0f, activated, qvssi, inv_dtf, predictNc, prescribedCCN, r, rt);
   if (r.ni_nucleat_tend == 0.0f && r.qv2qi_nucleat_tend == 0.0f) return;
-  State s;
-  s.qc = s.nc = s.qr = s.nr = s.qm = s.bm = 0.0;
-  s.qv = in.qv[o];
   s.th = in.th[o];
   const double cld_i = in.cld_frac_i[o], inv_exner = in.inv_exner[o];
-  const double qvsi = sm[A_QVSI * S + k];
   ice_supersat_conservation_bulk(r, cld_i, s.qv, qvsi, float(qvsi), T_r, dtf);
   const float dni = r.ni_nucleat_tend * dtf;
   s.qi = f2d(r.qv2qi_nucleat_tend * dtf);
@@ -675,34 +736,52 @@ __device__ __forceinline__ double svp_liquid(double t, double logt) {
 __device__ __forceinline__ double svp_ice(double t, double logt) {
   return m_exp(9.550426 - m_div(5723.265, t) + (3.53068 * logt) - (0.00728332 * t));
 }
-/* p3_main_part2 of one level with a hydrometeor in the FP64 form
- * (p3_main_part2_impl.hpp, same order of processes).  Each library function
- * (a pow holds the FP64 pipe for 1,500 cycles) is evaluated once and only
- * where a process reads it: the cube root of the Schmidt number and the
- * ventilation term serve melting, wet growth, relaxation and rain
- * evaporation; the viscosity terms need rain or ice, rhofaci ice, acn cloud
- * and ice, and logn0r rain and ice. */
-__device__ __forceinline__ void part2_level_f64(const Inst& in, const int64_t o, const int k, double* __restrict__ sm,
-                                                const int S, const KParams<double>& kp, const Tabs<double>& tb,
-                                                const double dt, const double inv_dt, bool& hydro, uint32_t& err) {
+/* Saturation, the rest of p3_main_part1 and p3_main_part2 of one level with a
+ * hydrometeor in the FP64 form (p3_main_part2_impl.hpp, same order of
+ * processes).  Each library function (a pow holds the FP64 pipe for 1,500
+ * cycles) is evaluated once and only where a process reads it: the cube root of
+ * the Schmidt number and the ventilation term serve melting, wet growth,
+ * relaxation and rain evaporation; the viscosity terms need rain or ice, rhofaci
+ * ice, acn cloud and ice, and logn0r rain and ice. */
+__device__ __forceinline__ void hydro_level_f64(const Inst& in, const int col, const int k, const KParams<double>& kp,
+                                                const Tabs<double>& tb, const double dt, const double inv_dt,
+                                                bool& hydro, uint32_t& err) {
   const RuntimeDev& rt = kp.rt;
   const bool predictNc = in.predictNc != 0, prescribedCCN = in.prescribedCCN != 0;
   const bool do_ice = rt.do_ice_production != 0;
+  const int64_t o = int64_t(col) * in.ld + k;
+  const double rho = scr_at(in, S_RHO, col)[k];
+  double T = scr_at(in, S_TATM, col)[k];
   State s;
-  s.qc = in.qc[o]; s.nc = in.nc[o]; s.qr = in.qr[o]; s.nr = in.nr[o];
-  s.qi = in.qi[o]; s.qm = in.qm[o]; s.ni = in.ni[o]; s.bm = in.bm[o];
-  s.qv = in.qv[o]; s.th = in.th[o];
-  const double T = sm[A_TATM * S + k];
-  const double qvssi = sm[A_QVSSI * S + k];
-  if (dlt(s.qc, C::QSMALL) && dlt(s.qr, C::QSMALL) && dlt(s.qi, C::QSMALL) && dlt(T, C::T_zerodegc) &&
-      dlt_neg(qvssi, -0.05))
-    return;
-
-  const double pres = in.pres[o];
-  const double cld_i = in.cld_frac_i[o], cld_l = in.cld_frac_l[o], cld_r = in.cld_frac_r[o];
+  load_state(in, o, s);
   const double inv_exner = in.inv_exner[o];
-  const double qvsl = sm[A_QVSL * S + k], qvsi = sm[A_QVSI * S + k];
-  const double rho = sm[A_RHO * S + k];
+  const double pres = in.pres[o];
+  double qvsl, qvsi;
+  {
+    const double p = vmax(pres, 1.e-3);
+    const double logt = m_log(T);
+    qvsl = m_div(C::ep_2 * svp_liquid(T, logt), p);
+    qvsi = T < C::Tmelt ? m_div(C::ep_2 * svp_ice(T, logt), p) : qvsl;
+  }
+  const double qvssi = m_div(s.qv, qvsi) - 1;
+  const double T_before = T;
+  const bool th_changed = part1_thresholds(s, T, inv_exner, qvssi, [&](double nc) {
+    if (prescribedCCN)
+      return vmax(nc, m_div(rt.spa_ccn_to_nc_factor * in.nccn[o], m_div(1.0, in.cld_frac_l[o])));
+    if (predictNc) return dmax0(nc + in.nc_nuceat_tend[o] * dt);
+    return __dmul_rn(C::NCCNST, m_div(1.0, rho));
+  });
+  if (th_changed) {
+    T = __dmul_rn(s.th, m_div(1.0, inv_exner));
+    scr_at(in, S_TATM, col)[k] = T;
+  }
+  if (dlt(s.qc, C::QSMALL) && dlt(s.qr, C::QSMALL) && dlt(s.qi, C::QSMALL) && dlt(T, C::T_zerodegc) &&
+      dlt_neg(qvssi, -0.05)) {
+    store_state(in, o, s);
+    return;
+  }
+
+  const double cld_i = in.cld_frac_i[o], cld_l = in.cld_frac_l[o], cld_r = in.cld_frac_r[o];
   const double inv_rho = m_div(1.0, rho);
   Incld inc;
   calc_incloud(s.qc, s.qr, s.qi, s.qm, s.nc, s.nr, s.ni, s.bm, m_div(1.0, cld_l), m_div(1.0, cld_i),
@@ -795,10 +874,10 @@ __device__ __forceinline__ void part2_level_f64(const Inst& in, const int64_t o,
       epsi_tot = epsi_tot + epsi;
     }
     if (has_c && has_i) {
-      /* acn from the viscosity, which is part1's unless part1 changed the
-       * temperature (it then left acn with the sign bit set) */
-      const double a = sm[A_ACN * S + k];
-      const double acn = dneg(a) ? -a : m_div(C::gravit * C::RHO_H2O, 18.0 * v.mu);
+      /* acn is that of the temperature before part1's changes, and v.mu that
+       * viscosity wherever part1 changed none */
+      const double dum = th_changed ? m_div(1.496e-6 * m_pow(T_before, 1.5), T_before + 120.0) : v.mu;
+      const double acn = m_div(C::gravit * C::RHO_H2O, 18.0 * dum);
       rho_qm_cloud = calc_rime_density<double>(T, rhofaci, tv_fallspd, acn, lamc, mu_c, qc_r, r.qc2qi_collect_tend);
     }
     if (do_ice && (has_c || has_r) && T <= C::T_rainfrz) {
@@ -848,30 +927,30 @@ __device__ __forceinline__ void part2_level_f64(const Inst& in, const int64_t o,
   double ni_incld = m_div(s.ni, cld_i);
   impose_max_total_ni(ni_incld, rt.max_total_ni, inv_rho);
   s.ni = ni_incld * cld_i;
-  in.qc[o] = s.qc; in.nc[o] = s.nc; in.qr[o] = s.qr; in.nr[o] = s.nr;
-  in.qi[o] = s.qi; in.qm[o] = s.qm; in.ni[o] = s.ni; in.bm[o] = s.bm;
-  in.qv[o] = s.qv; in.th[o] = s.th;
+  store_state(in, o, s);
 }
 
-/* p3_main_part2 of one level without hydrometeors, where ice nucleation is
- * the only process that can have a rate: the same operations that
- * part2_level_f64 leaves once every other rate is +0 (its limiters do not
- * engage, its sums add zeros). */
-__device__ __forceinline__ void part2_nucleation_f64(const Inst& in, const int64_t o, const int k,
-                                                     const double* __restrict__ sm, const int S,
+/* Saturation over ice and p3_main_part2 of one level without hydrometeors,
+ * where ice nucleation is the only process that can have a rate: the same
+ * operations that hydro_level_f64 leaves once every other rate is +0 (its
+ * limiters do not engage, its sums add zeros). */
+__device__ __forceinline__ void nucleation_level_f64(const Inst& in, const int col, const int k,
                                                      const KParams<double>& kp, const double dt, const double inv_dt,
                                                      bool& hydro) {
   const RuntimeDev& rt = kp.rt;
-  const double T = sm[A_TATM * S + k], qvssi = sm[A_QVSSI * S + k], qvsi = sm[A_QVSI * S + k];
-  const double inv_rho = m_div(1.0, sm[A_RHO * S + k]);
+  const int64_t o = int64_t(col) * in.ld + k;
+  const double T = scr_at(in, S_TATM, col)[k];
+  State s;
+  s.qc = s.nc = s.qr = s.nr = s.qm = s.bm = 0.0;
+  s.qv = in.qv[o];
+  const double qvsi = m_div(C::ep_2 * svp_ice(T, m_log(T)), vmax(in.pres[o], 1.e-3));
+  const double qvssi = m_div(s.qv, qvsi) - 1;
+  const double inv_rho = m_div(1.0, scr_at(in, S_RHO, col)[k]);
   Rates<double> r;
   r.zero();
   ice_nucleation<double>(T, inv_rho, 0.0, in.ni_activated[o], qvssi, inv_dt, in.predictNc != 0, in.prescribedCCN != 0,
                          r, rt);
   if (!dnz(r.ni_nucleat_tend) && !dnz(r.qv2qi_nucleat_tend)) return;
-  State s;
-  s.qc = s.nc = s.qr = s.nr = s.qm = s.bm = 0.0;
-  s.qv = in.qv[o];
   s.th = in.th[o];
   const double cld_i = in.cld_frac_i[o], inv_exner = in.inv_exner[o];
   ice_supersat_conservation(r, cld_i, s.qv, qvsi, m_div(s.th, inv_exner), dt);
@@ -891,305 +970,64 @@ __device__ __forceinline__ void part2_nucleation_f64(const Inst& in, const int64
   in.th[o] = s.th;
 }
 
-/* K1 of one column in the FP64 form: p3_main_init, p3_main_part1,
- * p3_main_part2.
+/* K1 of `ncol` neighbouring columns of one instance: p3_main_init,
+ * p3_main_part1, p3_main_part2.  By one warp, or (WIDE) of one column by a CTA,
+ * whose warps share the levels of the first pass and then take the lists 32
+ * entries at a time.
  *
- * What bounds it: the FP64 pipe, through the library functions (pow 1,499
- * cycles of an SM, log 516, tanh 429, exp 274), whose bits ice sedimentation
- * carries into every later result, so they stay the library's.  They are
- * therefore evaluated only on the levels whose processes read them.  A first
- * pass over all levels does what part1 does without saturation (the fall-speed
- * factors, which only sedimentation reads on these levels, in fixed point)
- * and sorts the levels into three classes:
+ * What bounds it: the FP64 pipe; in the FP64 form through the library functions
+ * (pow 1,499 cycles of an SM, log 516, tanh 429, exp 274), whose bits ice
+ * sedimentation carries into every later result, so they stay the library's; in
+ * the FP32-bulk form through the state, residuals, saturation table and
+ * conversions.  A first pass over all levels does what part1 does without
+ * saturation (in the FP64 form the fall-speed factors, which only sedimentation
+ * reads from here, are in fixed point), writes the hand-over rows and sorts the
+ * levels into three classes:
  *   - with a hydrometeor: saturation, the rest of part1 and part2, on a list,
- *     so that a group's lanes hold LANES such levels and not the few of them
- *     among LANES consecutive ones;
- *   - without, cold, where the supersaturation over ice (in FP32, good to
- *     1e-4) is near the nucleation threshold or above, or so near the -0.05 of
- *     the early exit that FP32 cannot decide it: exact saturation over ice and
- *     nucleation, on a second list;
+ *     so that a warp's lanes hold 32 such levels and not the few of them among
+ *     32 consecutive ones;
+ *   - without, cold, where the FP32 supersaturation over ice does not exclude
+ *     nucleation: saturation over ice and nucleation, on a second list;
  *   - the rest: no process has a rate there.
- * At 21,600 x 128: 6.9 -> 3.4 ms, at 64 x 72: 325 -> 127 us, the state bit for
- * bit the same.  Of the 3.4 ms the FP64 pipe is busy 68 %; instruction fetch is
- * the largest stall besides it. */
-template <int LANES>
-__device__ void p3_part12_f64(const Inst& in, const int col, const KParams<double>& kp, const Tabs<double>& tb,
-                              double* __restrict__ sm, uint32_t& err) {
+ * The lists run over the pool of columns: a column's cloud fills a fraction of
+ * a warp (18 of 128 levels in a cloud of 1-4 km), and the FP64 pipe takes
+ * as long for one lane as for 32.  The same bits as with lists per column, where
+ * part1's remainder and part2 were separate passes over arrays in shared memory
+ * (FP64 16 lanes, FP32-bulk 32 lanes per column): 21,600 x 128 FP64 3.41 -> 2.35
+ * ms, FP32-bulk 0.468 -> 0.371; 345,600 x 128 FP32-bulk 8.43 -> 5.48 ms; 1,537 x
+ * 97 FP64 272 -> 242 us. */
+template <class TR, bool WIDE>
+__device__ void p3_part12(const Inst& in, const int col0, const int ncol, const KParams<TR>& kp, const Tabs<TR>& tb,
+                          uint16_t* __restrict__ list, PoolScratch* __restrict__ ps, uint32_t& err) {
+  constexpr bool kBulk = sizeof(TR) == sizeof(float);
   const RuntimeDev& rt = kp.rt;
-  const unsigned mask = group_mask<LANES>();
-  const int lane = threadIdx.x & (LANES - 1);
+  const unsigned lane = threadIdx.x & 31u;
+  const int tid = WIDE ? int(threadIdx.x) : int(lane), step = WIDE ? int(blockDim.x) : 32;
   const int nk = in.nlev;
-  const int S = kp.sm_stride;
-  const int64_t co = int64_t(col) * in.ld;
-  const int64_t ci = int64_t(col) * in.ld_int;
+  const int total = ncol * nk;
   const double dt = in.dt;
-  const double inv_dt = m_div(1.0, dt);
-  const bool predictNc = in.predictNc != 0, prescribedCCN = in.prescribedCCN != 0;
   const bool do_ice = rt.do_ice_production != 0;
-#define SMA(a, k) sm[(a)*S + (k)]
-  /* level lists: hydrometeor levels from the front, nucleation levels from
-   * position nk (2 nk 16-bit entries in one slot of S doubles) */
-  uint16_t* const list = reinterpret_cast<uint16_t*>(&SMA(A_LIST, 0));
-  __syncwarp(mask); /* every lane is done with the last column's arrays */
   int n_hyd = 0, n_nuc = 0;
-  const unsigned below = (1u << (threadIdx.x & 31u)) - 1u;
+  const unsigned below = (1u << lane) - 1u;
+  if constexpr (WIDE) {
+    __syncthreads(); /* every thread is done with the last column's lists */
+    if (tid == 0) ps->n_hyd = ps->n_nuc = ps->active = 0;
+    __syncthreads();
+  } else {
+    __syncwarp(); /* every lane is done with the last pool's lists */
+  }
 
   /* ---------------- p3_main_init, part1 without saturation ---------------- */
-  bool nucl = false, hydro = false;
-  for (int base = 0; base < nk; base += LANES) {
-    const int k = base + lane;
+  int c = 0, k = tid;
+  for (int base = 0; base < total; base += step) {
+    while (k >= nk && c < ncol) {
+      k -= nk;
+      ++c;
+    }
     bool is_hyd = false, is_nuc = false;
-    if (k < nk) {
-      const int64_t o = co + k;
-      const double inv_exner = in.inv_exner[o];
-      double th = in.th[o];
-      const double dz = in.dz[o];
-      double qv = dmax0(in.qv[o]);
-      const double pres = in.pres[o];
-      const double dpres = in.dpres[o];
-      const double qc = in.qc[o], qr = in.qr[o], qi = in.qi[o];
-
-      in.diag_eff_radius_qc[o] = 10.e-6;
-      in.diag_eff_radius_qi[o] = 25.e-6;
-      in.diag_eff_radius_qr[o] = 500.e-6;
-      in.rho_qi[o] = 0;
-      in.qv2qi_depos_tend[o] = 0;
-      in.precip_total_tend[o] = 0;
-      in.nevapr[o] = 0;
-      in.liq_ice_exchange[o] = 0;
-      in.vap_liq_exchange[o] = 0;
-      in.vap_ice_exchange[o] = 0;
-
-      const double exner = m_div(1.0, inv_exner);
-      double T = th * exner;
-      if (dbits(T) <= 0 || dbits(T) > kInfBits) err |= kErrNumeric;
-      const double rho = m_div(m_div(dpres, dz), C::gravit);
-      const double inv_rho = m_div(1.0, rho);
-      /* fall-speed factors; rhofaci is rhofacr times a constant */
-      const double rhofacr = pow_fix(C::RHO_1000MB * inv_rho, .54);
-      const double visc = m_div(1.496e-6 * (T * pow_fix(T, .5)), T + 120.0);
-      SMA(A_RHO, k) = rho;
-      SMA(A_RHOFACR, k) = rhofacr;
-      SMA(A_RHOFACI, k) = rhofacr * kRhofaciOverR;
-      SMA(A_ACN, k) = m_div(C::gravit * C::RHO_H2O, 18.0 * visc);
-
-      is_hyd = dge(qc, C::QSMALL) || dge(qr, C::QSMALL) || dge(qi, C::QSMALL);
-      if (is_hyd) {
-        in.qv[o] = qv;
-        SMA(A_TATM, k) = T;
-      } else {
-        if (dlt(T, C::T_zerodegc)) {
-          bool counts = false;
-          is_nuc = !dry_level_known(T, float(T), float(qv), float(dmax_c(pres, 1.e-3)), counts);
-          nucl = nucl || counts;
-          SMA(A_QVSSI, k) = qv; /* the vapour that the exact supersaturation is formed with */
-        }
-        /* a species below qsmall goes to vapour; a +0 moves nothing */
-        bool th_changed = false;
-        if (dnz(qc)) {
-          qv = qv + qc;
-          th = th - inv_exner * qc * C::LatVap * C::INV_CP;
-          th_changed = true;
-        }
-        if (dnz(qr)) {
-          qv = qv + qr;
-          th = th - inv_exner * qr * C::LatVap * C::INV_CP;
-          th_changed = true;
-        }
-        if (dnz(qi)) {
-          qv = qv + qi;
-          th = th - inv_exner * qi * (C::LatVap + C::LatIce) * C::INV_CP;
-          th_changed = true;
-        }
-        if (is_nuc) SMA(A_QVSI, k) = T; /* and the temperature */
-        if (th_changed) T = th * exner;
-        in.qc[o] = 0; in.nc[o] = 0; in.qr[o] = 0; in.nr[o] = 0;
-        in.qi[o] = 0; in.ni[o] = 0; in.qm[o] = 0; in.bm[o] = 0;
-        in.qv[o] = qv; in.th[o] = th;
-        SMA(A_TATM, k) = T;
-      }
-    }
-    const unsigned b_hyd = __ballot_sync(mask, is_hyd), b_nuc = __ballot_sync(mask, is_nuc);
-    if (is_hyd) list[n_hyd + __popc(b_hyd & below & mask)] = uint16_t(k);
-    if (is_nuc) list[nk + n_nuc + __popc(b_nuc & below & mask)] = uint16_t(k);
-    n_hyd += __popc(b_hyd & mask);
-    n_nuc += __popc(b_nuc & mask);
-  }
-  for (int k = lane; k <= nk; k += LANES) {
-    in.precip_liq_flux[ci + k] = 0;
-    in.precip_ice_flux[ci + k] = 0;
-  }
-  if (lane == 0) {
-    in.precip_liq_surf[col] = 0;
-    in.precip_ice_surf[col] = 0;
-  }
-  __syncwarp(mask);
-
-  /* ---------------- saturation over ice of the nucleation levels ---------------- */
-  for (int j = lane; j < n_nuc; j += LANES) {
-    const int k = list[nk + j];
-    const double T = SMA(A_QVSI, k);
-    const double qvsi = m_div(C::ep_2 * svp_ice(T, m_log(T)), vmax(in.pres[co + k], 1.e-3));
-    const double qvssi = m_div(SMA(A_QVSSI, k), qvsi) - 1;
-    SMA(A_QVSI, k) = qvsi;
-    SMA(A_QVSSI, k) = qvssi;
-    if (dge_neg(qvssi, -0.05)) nucl = true;
-  }
-  /* ---------------- the rest of part1 on the hydrometeor levels ---------------- */
-  for (int j = lane; j < n_hyd; j += LANES) {
-    const int k = list[j];
-    const int64_t o = co + k;
-    const double inv_exner = in.inv_exner[o];
-    const double exner = m_div(1.0, inv_exner);
-    double th = in.th[o], qv = in.qv[o], T = SMA(A_TATM, k);
-    double qc = in.qc[o], nc = in.nc[o], qr = in.qr[o], nr = in.nr[o];
-    double qi = in.qi[o], ni = in.ni[o], qm = in.qm[o], bm = in.bm[o];
-    const double p = vmax(in.pres[o], 1.e-3);
-    const bool cold = T < C::Tmelt;
-    const double logt = m_log(T);
-    const double qvsl = m_div(C::ep_2 * svp_liquid(T, logt), p);
-    const double qvsi = cold ? m_div(C::ep_2 * svp_ice(T, logt), p) : qvsl;
-    const double qvssi = m_div(qv, qvsi) - 1;
-    if (dlt(T, C::T_zerodegc) && dge_neg(qvssi, -0.05)) nucl = true;
-
-    /* A species below qsmall goes to vapour; a +0 moves nothing, so its FP64
-     * updates are skipped (bitwise the same result). */
-    const double T_before = T;
-    bool th_changed = false;
-    if (dlt(qc, C::QSMALL)) {
-      if (dnz(qc)) {
-        qv = qv + qc;
-        th = th - inv_exner * qc * C::LatVap * C::INV_CP;
-        th_changed = true;
-      }
-      qc = 0;
-      nc = 0;
-    } else {
-      hydro = true;
-      if (prescribedCCN) {
-        nc = vmax(nc, m_div(rt.spa_ccn_to_nc_factor * in.nccn[o], m_div(1.0, in.cld_frac_l[o])));
-      } else if (predictNc) {
-        nc = dmax0(nc + in.nc_nuceat_tend[o] * dt);
-      } else {
-        nc = C::NCCNST * m_div(1.0, SMA(A_RHO, k));
-      }
-    }
-    if (dlt(qr, C::QSMALL)) {
-      if (dnz(qr)) {
-        qv = qv + qr;
-        th = th - inv_exner * qr * C::LatVap * C::INV_CP;
-        th_changed = true;
-      }
-      qr = 0;
-      nr = 0;
-    } else {
-      hydro = true;
-    }
-    if (dlt(qi, C::QSMALL) || (dlt(qi, 1.e-8) && dlt_neg(qvssi, -0.1))) {
-      if (dnz(qi)) {
-        qv = qv + qi;
-        th = th - inv_exner * qi * (C::LatVap + C::LatIce) * C::INV_CP;
-        th_changed = true;
-      }
-      qi = 0; ni = 0; qm = 0; bm = 0;
-    } else {
-      hydro = true;
-    }
-    if (dge(qi, C::QSMALL) && dlt(qi, 1.e-8) && dge(T, C::T_zerodegc)) {
-      qr = qr + qi;
-      th = th - inv_exner * qi * C::LatIce * C::INV_CP;
-      th_changed = true;
-      qi = 0; ni = 0; qm = 0; bm = 0;
-    }
-    if (th_changed) {
-      T = th * exner;
-      if (dge(qc, C::QSMALL) && dge(qi, C::QSMALL)) {
-        /* part2 reads acn at the temperature before these changes */
-        const double dum = m_div(1.496e-6 * m_pow(T_before, 1.5), T_before + 120.0);
-        SMA(A_ACN, k) = -m_div(C::gravit * C::RHO_H2O, 18.0 * dum);
-      }
-    }
-    in.qc[o] = qc; in.nc[o] = nc; in.qr[o] = qr; in.nr[o] = nr;
-    in.qi[o] = qi; in.ni[o] = ni; in.qm[o] = qm; in.bm[o] = bm;
-    in.qv[o] = qv; in.th[o] = th;
-    SMA(A_TATM, k) = T;
-    SMA(A_QVSL, k) = qvsl;
-    SMA(A_QVSI, k) = qvsi;
-    SMA(A_QVSSI, k) = qvssi;
-  }
-  if (!group_any<LANES>(mask, nucl || hydro)) {
-    if (lane == 0) in.cflag[col] = 0;
-    return;
-  }
-
-  /* ---------------- p3_main_part2 ---------------- */
-  /* a lane owns the list positions it had above, so only its own stores are
-   * read back */
-  hydro = false;
-  for (int j = lane; j < n_hyd; j += LANES)
-    part2_level_f64(in, co + list[j], list[j], sm, S, kp, tb, dt, inv_dt, hydro, err);
-  if (do_ice) {
-    for (int j = lane; j < n_nuc; j += LANES)
-      part2_nucleation_f64(in, co + list[nk + j], list[nk + j], sm, S, kp, dt, inv_dt, hydro);
-  }
-  if (!group_any<LANES>(mask, hydro)) {
-    if (lane == 0) in.cflag[col] = 0;
-    return;
-  }
-  __syncwarp(mask);
-  for (int k = lane; k < nk; k += LANES) {
-    scr_at(in, S_TATM, col)[k] = SMA(A_TATM, k);
-    scr_at(in, S_RHO, col)[k] = SMA(A_RHO, k);
-    scr_at(in, S_RHOFACR, col)[k] = SMA(A_RHOFACR, k);
-    scr_at(in, S_RHOFACI, col)[k] = SMA(A_RHOFACI, k);
-    scr_at(in, S_ACN, col)[k] = m_fabs(SMA(A_ACN, k));
-  }
-  if (lane == 0) in.cflag[col] = 1;
-#undef SMA
-}
-
-/* K1 of one column in the FP32-bulk form: p3_main_init, p3_main_part1,
- * p3_main_part2.
- *
- * What bounds it: the FP64 pipe (state, residuals, saturation table,
- * conversions).  The levels are sorted as in p3_part12_f64: saturation, the
- * rest of part1 and part2 run on the listed levels only (those with a
- * hydrometeor first, then those where ice may nucleate), packed into the
- * group's lanes.  On the others the first pass needs 10 FP64 instructions, not
- * 32, and no table reads.  Bit for bit the same state; at 21,600 x 128 0.745 ->
- * 0.469 ms, at 345,600 x 128 with half the columns near saturation (their cold
- * levels nucleate) 11.4 -> 8.4 ms. */
-template <int LANES>
-__device__ void p3_part12_bulk(const Inst& in, const int col, const KParams<float>& kp, const Tabs<float>& tb,
-                               double* __restrict__ sm, uint32_t& err) {
-  const RuntimeDev& rt = kp.rt;
-  const unsigned mask = group_mask<LANES>();
-  const int lane = threadIdx.x & (LANES - 1);
-  const int nk = in.nlev;
-  const int S = kp.sm_stride;
-  const int64_t co = int64_t(col) * in.ld;
-  const int64_t ci = int64_t(col) * in.ld_int;
-  const double dt = in.dt;
-  const double inv_dt = 1 / dt;
-  const bool predictNc = in.predictNc != 0, prescribedCCN = in.prescribedCCN != 0;
-#define SMA(a, k) sm[(a)*S + (k)]
-  /* FP32-bulk: the float-valued slots (rho, fall-speed factors, acn) hold
-   * floats in the first half of their slot */
-#define SMF(a) reinterpret_cast<float*>(&sm[(a)*S])
-  /* level lists in the second half of the density's slot: hydrometeor levels
-   * from the front, nucleation levels from position nk (16-bit entries) */
-  uint16_t* const list = reinterpret_cast<uint16_t*>(SMF(A_RHO) + S);
-  __syncwarp(mask); /* every lane is done with the last column's arrays */
-  int n_hyd = 0, n_nuc = 0;
-  const unsigned below = (1u << (threadIdx.x & 31u)) - 1u;
-
-  /* ---------------- p3_main_init, part1 without saturation ---------------- */
-  bool nucl = false, hydro = false;
-  for (int base = 0; base < nk; base += LANES) {
-    const int k = base + lane;
-    bool is_hyd = false, is_nuc = false;
-    if (k < nk) {
-      const int64_t o = co + k;
+    if (c < ncol) {
+      const int col = col0 + c;
+      const int64_t o = int64_t(col) * in.ld + k;
       const double inv_exner = in.inv_exner[o];
       double th = in.th[o];
       const double dz = in.dz[o];
@@ -1208,186 +1046,139 @@ __device__ void p3_part12_bulk(const Inst& in, const int col, const KParams<floa
       in.vap_liq_exchange[o] = 0;
       in.vap_ice_exchange[o] = 0;
 
-      const double exner = rcp_newton1(inv_exner);
+      double exner;
+      if constexpr (kBulk) exner = rcp_newton1(inv_exner);
+      else exner = m_div(1.0, inv_exner);
       double T = th * exner;
       if (dbits(T) <= 0 || dbits(T) > kInfBits) err |= kErrNumeric;
-      /* rho and 1/rho only feed rates, fall speeds and fluxes (the
-       * sedimentation's FP64 coefficient is g / dpres), so they are FP32 and
-       * kept as floats in the shared slots and the hand-over */
-      const float rho_t = float(dpres) / (float(dz) * float(C::gravit));
-      const float inv_rho_t = 1.0f / rho_t;
-      const float tf = float(T);
-      const float dum = float(1.496e-6) * m_pow(tf, float(1.5)) / (tf + float(120));
-      SMF(A_RHO)[k] = rho_t;
-      SMF(A_RHOFACR)[k] = m_pow(float(C::RHO_1000MB) * inv_rho_t, float(.54));
-      SMF(A_RHOFACI)[k] = m_pow(float(C::RHO_600MB) * inv_rho_t, float(.54));
-      SMF(A_ACN)[k] = float(C::gravit) * float(C::RHO_H2O) / (float(18) * dum);
+      if constexpr (kBulk) {
+        /* rho and 1/rho only feed rates, fall speeds and fluxes (the
+         * sedimentation's FP64 coefficient is g / dpres), so they are FP32 */
+        const float rho_t = float(dpres) / (float(dz) * float(C::gravit));
+        const float inv_rho_t = 1.0f / rho_t;
+        const float tf = float(T);
+        const float dum = float(1.496e-6) * m_pow(tf, float(1.5)) / (tf + float(120));
+        scr_f(in, S_RHO, col)[k] = rho_t;
+        scr_f(in, S_RHOFACR, col)[k] = m_pow(float(C::RHO_1000MB) * inv_rho_t, float(.54));
+        scr_f(in, S_RHOFACI, col)[k] = m_pow(float(C::RHO_600MB) * inv_rho_t, float(.54));
+        scr_f(in, S_ACN, col)[k] = float(C::gravit) * float(C::RHO_H2O) / (float(18) * dum);
+      } else {
+        const double rho = m_div(m_div(dpres, dz), C::gravit);
+        const double inv_rho = m_div(1.0, rho);
+        /* rhofaci is rhofacr times a constant */
+        const double rhofacr = pow_fix(C::RHO_1000MB * inv_rho, .54);
+        const double visc = m_div(1.496e-6 * (T * pow_fix(T, .5)), T + 120.0);
+        scr_at(in, S_RHO, col)[k] = rho;
+        scr_at(in, S_RHOFACR, col)[k] = rhofacr;
+        scr_at(in, S_RHOFACI, col)[k] = rhofacr * kRhofaciOverR;
+        scr_at(in, S_ACN, col)[k] = m_div(C::gravit * C::RHO_H2O, 18.0 * visc);
+      }
 
       is_hyd = dge(qc, C::QSMALL) || dge(qr, C::QSMALL) || dge(qi, C::QSMALL);
-      if (is_hyd) {
-        in.qv[o] = qv;
-        SMA(A_TATM, k) = T;
-      } else {
-        if (dlt(T, C::T_zerodegc)) {
-          bool counts = false;
-          is_nuc = !dry_level_known(T, tf, float(qv), float(dmax_c(in.pres[o], 1.e-3)), counts);
-          nucl = nucl || counts;
-          SMA(A_QVSSI, k) = qv; /* the vapour and the temperature that the */
-          SMA(A_QVSI, k) = T;   /* exact supersaturation is formed with     */
+      if (!is_hyd) {
+        const bool traces = dnz(qc) || dnz(qr) || dnz(qi);
+        if (do_ice && dlt(T, C::T_zerodegc))
+          is_nuc = may_nucleate(T, float(T), float(qv), float(dmax_c(in.pres[o], 1.e-3)));
+        /* nucleation is decided before a trace of condensate goes to vapour:
+         * the general path does both */
+        is_hyd = is_nuc && traces;
+        is_nuc = is_nuc && !traces;
+        if (!is_hyd) {
+          if (traces) {
+            /* a species below qsmall goes to vapour; a +0 moves nothing */
+            if (dnz(qc)) {
+              qv = qv + qc;
+              th = th - inv_exner * qc * C::LatVap * C::INV_CP;
+            }
+            if (dnz(qr)) {
+              qv = qv + qr;
+              th = th - inv_exner * qr * C::LatVap * C::INV_CP;
+            }
+            if (dnz(qi)) {
+              qv = qv + qi;
+              th = th - inv_exner * qi * (C::LatVap + C::LatIce) * C::INV_CP;
+            }
+            T = th * exner;
+          }
+          in.qc[o] = 0; in.nc[o] = 0; in.qr[o] = 0; in.nr[o] = 0;
+          in.qi[o] = 0; in.ni[o] = 0; in.qm[o] = 0; in.bm[o] = 0;
+          in.th[o] = th;
         }
-        /* a species below qsmall goes to vapour; a +0 moves nothing */
-        bool th_changed = false;
-        if (dnz(qc)) {
-          qv = qv + qc;
-          th = th - inv_exner * qc * C::LatVap * C::INV_CP;
-          th_changed = true;
-        }
-        if (dnz(qr)) {
-          qv = qv + qr;
-          th = th - inv_exner * qr * C::LatVap * C::INV_CP;
-          th_changed = true;
-        }
-        if (dnz(qi)) {
-          qv = qv + qi;
-          th = th - inv_exner * qi * (C::LatVap + C::LatIce) * C::INV_CP;
-          th_changed = true;
-        }
-        if (th_changed) T = th * exner;
-        in.qc[o] = 0; in.nc[o] = 0; in.qr[o] = 0; in.nr[o] = 0;
-        in.qi[o] = 0; in.ni[o] = 0; in.qm[o] = 0; in.bm[o] = 0;
-        in.qv[o] = qv; in.th[o] = th;
-        SMA(A_TATM, k) = T;
       }
+      in.qv[o] = qv;
+      scr_at(in, S_TATM, col)[k] = T;
     }
-    const unsigned b_hyd = __ballot_sync(mask, is_hyd) & mask, b_nuc = __ballot_sync(mask, is_nuc) & mask;
-    if (is_hyd) list[n_hyd + __popc(b_hyd & below)] = uint16_t(k);
-    if (is_nuc) list[nk + n_nuc + __popc(b_nuc & below)] = uint16_t(k);
+    const unsigned b_hyd = __ballot_sync(0xffffffffu, is_hyd), b_nuc = __ballot_sync(0xffffffffu, is_nuc);
+    const uint16_t entry = uint16_t((c << kPoolLevelBits) | k);
+    if constexpr (WIDE) {
+      if (lane == 0) {
+        n_hyd = b_hyd ? int(atomicAdd(&ps->n_hyd, __popc(b_hyd))) : 0;
+        n_nuc = b_nuc ? int(atomicAdd(&ps->n_nuc, __popc(b_nuc))) : 0;
+      }
+      n_hyd = __shfl_sync(0xffffffffu, n_hyd, 0);
+      n_nuc = __shfl_sync(0xffffffffu, n_nuc, 0);
+    }
+    if (is_hyd) list[n_hyd + __popc(b_hyd & below)] = entry;
+    if (is_nuc) list[total - 1 - n_nuc - __popc(b_nuc & below)] = entry;
     n_hyd += __popc(b_hyd);
     n_nuc += __popc(b_nuc);
+    k += step;
   }
-  for (int k = lane; k <= nk; k += LANES) {
-    in.precip_liq_flux[ci + k] = 0;
-    in.precip_ice_flux[ci + k] = 0;
+  for (c = 0; c < ncol; ++c) {
+    const int64_t ci = int64_t(col0 + c) * in.ld_int;
+    for (k = tid; k <= nk; k += step) {
+      in.precip_liq_flux[ci + k] = 0;
+      in.precip_ice_flux[ci + k] = 0;
+    }
   }
-  if (lane == 0) {
-    in.precip_liq_surf[col] = 0;
-    in.precip_ice_surf[col] = 0;
+  if (tid < ncol) {
+    in.precip_liq_surf[col0 + tid] = 0;
+    in.precip_ice_surf[col0 + tid] = 0;
   }
-  __syncwarp(mask);
-
-  /* ---------------- saturation, the rest of part1 on the listed levels ---------------- */
-  const int n_list = n_hyd + n_nuc;
-  for (int j = lane; j < n_list; j += LANES) {
-    const bool hyd = j < n_hyd;
-    const int k = list[hyd ? j : nk + j - n_hyd];
-    const int64_t o = co + k;
-    /* one Newton reciprocal of the pressure, times ep_2, shared by both
-     * saturation ratios (and kept for part2's melting departure and
-     * supersaturation limiter); the supersaturation ratio (threshold and rate
-     * input) in FP32 */
-    const double ep_inv_p = C::ep_2 * rcp_newton1(dmax_c(in.pres[o], 1.e-3));
-    SMA(A_EPINVP, k) = ep_inv_p;
-    double T = hyd ? SMA(A_TATM, k) : SMA(A_QVSI, k);
-    double qv = hyd ? in.qv[o] : SMA(A_QVSSI, k);
-    const double qvsi = svp_tabulated(rt.svp_tab, T, true, err) * ep_inv_p;
-    const double qvssi = f2d(float(qv) / float(qvsi) - 1.0f);
-    SMA(A_QVSI, k) = qvsi;
-    SMA(A_QVSSI, k) = qvssi;
-    if (dlt(T, C::T_zerodegc) && dge_neg(qvssi, -0.05)) nucl = true;
-    if (!hyd) continue;
-    SMA(A_QVSL, k) = svp_tabulated(rt.svp_tab, T, false, err) * ep_inv_p;
-    const double inv_exner = in.inv_exner[o];
-    double th = in.th[o];
-    double qc = in.qc[o], nc = in.nc[o], qr = in.qr[o], nr = in.nr[o];
-    double qi = in.qi[o], ni = in.ni[o], qm = in.qm[o], bm = in.bm[o];
-
-    /* A species below qsmall goes to vapour; a +0 moves nothing, so its FP64
-     * updates are skipped (bitwise the same result). */
-    bool th_changed = false;
-    if (dlt(qc, C::QSMALL)) {
-      if (dnz(qc)) {
-        qv = qv + qc;
-        th = th - inv_exner * qc * C::LatVap * C::INV_CP;
-        th_changed = true;
-      }
-      qc = 0;
-      nc = 0;
-    } else {
-      hydro = true;
-      if (prescribedCCN) {
-        nc = vmax(nc, rt.spa_ccn_to_nc_factor * in.nccn[o] * in.cld_frac_l[o]);
-      } else if (predictNc) {
-        nc = dmax0(nc + in.nc_nuceat_tend[o] * dt);
-      } else {
-        nc = C::NCCNST * f2d(1.0f / SMF(A_RHO)[k]);
-      }
-    }
-    if (dlt(qr, C::QSMALL)) {
-      if (dnz(qr)) {
-        qv = qv + qr;
-        th = th - inv_exner * qr * C::LatVap * C::INV_CP;
-        th_changed = true;
-      }
-      qr = 0;
-      nr = 0;
-    } else {
-      hydro = true;
-    }
-    if (dlt(qi, C::QSMALL) || (dlt(qi, 1.e-8) && dlt_neg(qvssi, -0.1))) {
-      if (dnz(qi)) {
-        qv = qv + qi;
-        th = th - inv_exner * qi * (C::LatVap + C::LatIce) * C::INV_CP;
-        th_changed = true;
-      }
-      qi = 0; ni = 0; qm = 0; bm = 0;
-    } else {
-      hydro = true;
-    }
-    if (dge(qi, C::QSMALL) && dlt(qi, 1.e-8) && dge(T, C::T_zerodegc)) {
-      qr = qr + qi;
-      th = th - inv_exner * qi * C::LatIce * C::INV_CP;
-      th_changed = true;
-      qi = 0; ni = 0; qm = 0; bm = 0;
-    }
-    if (th_changed) SMA(A_TATM, k) = th * rcp_newton1(inv_exner);
-    in.qc[o] = qc; in.nc[o] = nc; in.qr[o] = qr; in.nr[o] = nr;
-    in.qi[o] = qi; in.ni[o] = ni; in.qm[o] = qm; in.bm[o] = bm;
-    in.qv[o] = qv; in.th[o] = th;
-  }
-  if (!group_any<LANES>(mask, nucl || hydro)) {
-    if (lane == 0) in.cflag[col] = 0;
-    return;
+  /* the lists, and the rows other lanes wrote */
+  if constexpr (WIDE) {
+    __syncthreads();
+    n_hyd = int(ps->n_hyd);
+    n_nuc = int(ps->n_nuc);
+  } else {
+    __syncwarp();
   }
 
-  /* ---------------- p3_main_part2 ---------------- */
-  /* a lane owns the list positions it had above, so only its own stores are
-   * read back */
-  hydro = false;
-  const float dtf = float(dt), inv_dtf = float(inv_dt);
-  for (int j = lane; j < n_list; j += LANES) {
-    if (j < n_hyd) {
-      const int k = list[j];
-      part2_level_bulk(in, co + k, k, sm, S, kp, tb, dtf, inv_dtf, hydro, err);
-    } else if (rt.do_ice_production != 0) {
-      const int k = list[nk + j - n_hyd];
-      part2_nucleation_bulk(in, co + k, k, sm, S, kp, dtf, inv_dtf, hydro);
+  /* ---------------- saturation, the rest of part1, part2 ---------------- */
+  uint32_t active = 0; /* columns with a hydrometeor after part2 */
+  /* a CTA's warps take one list or the other, a warp goes from the first to the second */
+  const int n_pad = WIDE ? (n_hyd + 31) & ~31 : n_hyd;
+  if constexpr (kBulk) {
+    const float dtf = float(dt), inv_dtf = float(1 / dt);
+    for (int j = tid; j < n_pad + n_nuc; j += step) {
+      if (WIDE && j >= n_hyd && j < n_pad) continue;
+      const int e = list[j < n_hyd ? j : total - 1 - (j - n_pad)];
+      const int ce = e >> kPoolLevelBits, ke = e & ((1 << kPoolLevelBits) - 1);
+      bool hydro = false;
+      if (j < n_hyd) hydro_level_bulk(in, col0 + ce, ke, kp, tb, dtf, inv_dtf, hydro, err);
+      else nucleation_level_bulk(in, col0 + ce, ke, kp, dtf, inv_dtf, hydro, err);
+      active |= uint32_t(hydro) << ce;
+    }
+  } else {
+    const double inv_dt = m_div(1.0, dt);
+    for (int j = tid; j < n_pad + n_nuc; j += step) {
+      if (WIDE && j >= n_hyd && j < n_pad) continue;
+      const int e = list[j < n_hyd ? j : total - 1 - (j - n_pad)];
+      const int ce = e >> kPoolLevelBits, ke = e & ((1 << kPoolLevelBits) - 1);
+      bool hydro = false;
+      if (j < n_hyd) hydro_level_f64(in, col0 + ce, ke, kp, tb, dt, inv_dt, hydro, err);
+      else nucleation_level_f64(in, col0 + ce, ke, kp, dt, inv_dt, hydro);
+      active |= uint32_t(hydro) << ce;
     }
   }
-  if (!group_any<LANES>(mask, hydro)) {
-    if (lane == 0) in.cflag[col] = 0;
-    return;
+  active = __reduce_or_sync(0xffffffffu, active);
+  if constexpr (WIDE) {
+    if (lane == 0 && active) atomicOr(&ps->active, active);
+    __syncthreads();
+    if (tid == 0) in.cflag[col0] = int(ps->active);
+  } else {
+    if (int(lane) < ncol) in.cflag[col0 + lane] = (active >> lane) & 1u;
   }
-  __syncwarp(mask);
-  for (int k = lane; k < nk; k += LANES) {
-    scr_at(in, S_TATM, col)[k] = SMA(A_TATM, k);
-    scr_f(in, S_RHO, col)[k] = SMF(A_RHO)[k];
-    scr_f(in, S_RHOFACR, col)[k] = SMF(A_RHOFACR)[k];
-    scr_f(in, S_RHOFACI, col)[k] = SMF(A_RHOFACI)[k];
-    scr_f(in, S_ACN, col)[k] = SMF(A_ACN)[k];
-  }
-  if (lane == 0) in.cflag[col] = 1;
-#undef SMA
-#undef SMF
 }
 
 /* K2 (FP64 form): cloud, rain and ice sedimentation of one column that went
@@ -1414,7 +1205,7 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
   if (in.cflag[col] == 0) return;
   const RuntimeDev& rt = kp.rt;
   const FixTables* const ft = &kFixTables;
-  const unsigned mask = group_mask<LANES>();
+  const unsigned mask = 0xffffffffu;
   const int lane = threadIdx.x & (LANES - 1);
   const int nk = in.nlev;
   const int S = kp.sm_stride;
@@ -1424,7 +1215,7 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
   const double inv_dt = m_div(1.0, dt);
   const bool predictNc = in.predictNc != 0;
   const int kbot = nk - 1;
-  constexpr int kWarp = LANES < 32 ? LANES : 32; /* lanes that shuffle with one another */
+  constexpr int kWarp = 32; /* lanes that shuffle with one another */
   double* const FR = sm + B_FR * S;   /* fall-speed factor of the species times rho */
   double* const CF = sm + B_CF * S;   /* 1 / (dz rho) */
   double* const QS = sm + B_QS * S;   /* QSMALL times the species' cloud fraction */
@@ -1758,7 +1549,7 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
                             double* __restrict__ sm, GroupScratch* gs, uint32_t& err) {
   if (in.cflag[col] == 0) return;
   const RuntimeDev& rt = kp.rt;
-  const unsigned mask = group_mask<LANES>();
+  const unsigned mask = 0xffffffffu;
   const int lane = threadIdx.x & (LANES - 1);
   const int nk = in.nlev;
   const int S = kp.sm_stride;
@@ -1768,7 +1559,7 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
   const double inv_dt = 1 / dt;
   const bool predictNc = in.predictNc != 0;
   const int kbot = nk - 1;
-  constexpr int kWarp = LANES < 32 ? LANES : 32; /* lanes that shuffle with one another */
+  constexpr int kWarp = 32; /* lanes that shuffle with one another */
 #define SMA(a, k) sm[(a)*S + (k)]
   /* kSedBulkSlots slots of S doubles; two float arrays share a slot.  The
    * density is read from the hand-over row (a float per level, L1-resident
@@ -2444,31 +2235,24 @@ __device__ __forceinline__ unsigned char* setup_tables(const KParams<TR>& kp, bo
   return smem_raw;
 }
 
-/* Runs f(w) for the work items of this column group.  With a counter, a warp
- * takes the next 32/LANES items whenever it has finished its last ones, so a
- * warp that drew cheap columns takes more of them and no SM idles behind the
- * slowest column list (a static stride gives every warp a fixed share, and an
- * even stride gives it columns of one parity only).  Without one, groups
- * stride the list. */
-template <int LANES, class F>
+/* Runs f(w) for the work items of this warp.  With a counter, a warp takes the
+ * next item whenever it has finished its last one, so a warp that drew cheap
+ * columns takes more of them and no SM idles behind the slowest column list (a
+ * static stride gives every warp a fixed share, and an even stride gives it
+ * columns of one parity only).  Without one, warps stride the list. */
+template <class F>
 __device__ __forceinline__ void for_each_work(uint32_t* ctr, int nwork, int groups_per_block, F&& f) {
   if (ctr) {
-    const int lane = threadIdx.x & 31;
-    const int nthr = min(32, int(blockDim.x) - int(threadIdx.x & ~31u));
-    const unsigned wmask = nthr == 32 ? 0xffffffffu : ((1u << nthr) - 1u);
-    const uint32_t per_warp = uint32_t(nthr / LANES);
-    const uint32_t g_in_warp = uint32_t(lane / LANES);
     for (;;) {
-      uint32_t base = 0;
-      if (lane == 0) base = atomicAdd(ctr, per_warp);
-      base = __shfl_sync(wmask, base, 0);
-      if (base >= uint32_t(nwork)) break;
-      const uint32_t w = base + g_in_warp;
-      if (w < uint32_t(nwork)) f(int(w));
+      uint32_t w = 0;
+      if ((threadIdx.x & 31) == 0) w = atomicAdd(ctr, 1u);
+      w = __shfl_sync(0xffffffffu, w, 0);
+      if (w >= uint32_t(nwork)) break;
+      f(int(w));
     }
   } else {
     const int groups_total = gridDim.x * groups_per_block;
-    for (int w = blockIdx.x * groups_per_block + int(threadIdx.x) / LANES; w < nwork; w += groups_total) f(w);
+    for (int w = blockIdx.x * groups_per_block + int(threadIdx.x >> 5); w < nwork; w += groups_total) f(w);
   }
 }
 
@@ -2484,10 +2268,28 @@ __device__ __forceinline__ const Inst& work_inst(const Inst& inst0, const KParam
   return inst0;
 }
 
+/* Pool i of a launch's work items: sizes go down from pool_cols to 1, halved
+ * whenever the pools of a size are used up (pool_end), so that the last pools
+ * are small and every warp ends at about the same time. */
+template <class TR>
+__device__ __forceinline__ void pool_range(const KParams<TR>& kp, const int i, int& w0, int& w1) {
+  int first = 0, size = kp.pool_cols;
+  w0 = 0;
+#pragma unroll
+  for (int t = 0; t < kPoolTiers - 1; ++t) {
+    if (i < kp.pool_end[t] || size == 1) break;
+    w0 += (kp.pool_end[t] - first) * size;
+    first = kp.pool_end[t];
+    size >>= 1;
+  }
+  w0 += (i - first) * size;
+  w1 = min(w0 + size, kp.nwork);
+}
+
 /* The FP32-bulk instantiation is held to 128 registers (two CTAs of 256
  * threads per SM; a few dozen bytes spill), which measured 25 % faster than 176
  * registers at one CTA per SM. */
-template <class TR, int LANES>
+template <class TR>
 __global__ void __launch_bounds__(256, sizeof(TR) == sizeof(float) ? 2 : 1)
     p3_part12_kernel(const Inst inst0, const KParams<TR> kp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -2498,17 +2300,37 @@ __global__ void __launch_bounds__(256, sizeof(TR) == sizeof(float) ? 2 : 1)
     if (threadIdx.x == 0) atomicOr(kp.err, err);
     return;
   }
-  const int g_in_block = threadIdx.x / LANES;
-  double* sm = reinterpret_cast<double*>(base) + size_t(g_in_block) * A_NARR * kp.sm_stride;
-  for_each_work<LANES>(kp.wctr ? kp.wctr + 0 : nullptr, kp.nwork, kp.groups_per_block, [&](int w) {
-    int col;
-    const Inst& in = work_inst(inst0, kp, w, col);
-    if constexpr (sizeof(TR) == sizeof(double)) {
-      p3_part12_f64<LANES>(in, col, kp, tb, sm, err);
-    } else {
-      p3_part12_bulk<LANES>(in, col, kp, tb, sm, err);
+  uint16_t* const list =
+      reinterpret_cast<uint16_t*>(base) + size_t(threadIdx.x >> 5) * pool_list_entries(kp.pool_cols, kp.nlev_max);
+  for_each_work(kp.wctr ? kp.wctr + 0 : nullptr, kp.npools, kp.groups_per_block, [&](int i) {
+    int w0, w1;
+    pool_range(kp, i, w0, w1);
+    while (w0 < w1) { /* a pool's run of columns of one instance */
+      int col;
+      const Inst& in = work_inst(inst0, kp, w0, col);
+      const int n = kp.work ? min(w1 - w0, in.ncol - col) : w1 - w0;
+      p3_part12<TR, false>(in, col, n, kp, tb, list, nullptr, err);
+      w0 += n;
     }
   });
+  if (err) atomicOr(kp.err, err);
+}
+
+/* K1 with a CTA per column, where a call has fewer columns than the GPU has
+ * room for such CTAs: its time is then the latency of one column. */
+template <class TR>
+__global__ void __launch_bounds__(kPart12WideThreads, sizeof(TR) == sizeof(float) ? 4 : 2)
+    p3_part12_wide_kernel(const Inst inst0, const KParams<TR> kp) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ PoolScratch ps;
+  uint32_t err = 0;
+  Tabs<TR> tb;
+  setup_tables<TR>(kp, false, smem_raw, tb, err);
+  for (int w = blockIdx.x; w < kp.nwork; w += gridDim.x) {
+    int col;
+    const Inst& in = work_inst(inst0, kp, w, col);
+    p3_part12<TR, true>(in, col, 1, kp, tb, reinterpret_cast<uint16_t*>(smem_raw), &ps, err);
+  }
   if (err) atomicOr(kp.err, err);
 }
 
@@ -2523,7 +2345,7 @@ __global__ void __maxnreg__(96) p3_sed_kernel(const Inst inst0, const KParams<TR
   setup_tables<TR>(kp, false, smem_raw, tb, err);
   const int g_in_block = threadIdx.x / LANES;
   double* sm = reinterpret_cast<double*>(smem_raw) + size_t(g_in_block) * sed_slots<TR>() * kp.sm_stride;
-  for_each_work<LANES>(kp.wctr ? kp.wctr + 1 : nullptr, kp.nwork, kp.groups_per_block, [&](int w) {
+  for_each_work(kp.wctr ? kp.wctr + 1 : nullptr, kp.nwork, kp.groups_per_block, [&](int w) {
     int col;
     const Inst& in = work_inst(inst0, kp, w, col);
     p3_sed<TR, LANES>(in, col, kp, tb, sm, nullptr, err);
@@ -2602,7 +2424,7 @@ __global__ void __maxnreg__(96) p3_sed_bulk_kernel(const Inst inst0, const KPara
   }
   const int g_in_block = threadIdx.x / LANES;
   double* sm = reinterpret_cast<double*>(columns) + size_t(g_in_block) * kSedBulkSlots * kp.sm_stride;
-  for_each_work<LANES>(kp.wctr ? kp.wctr + 1 : nullptr, kp.nwork, kp.groups_per_block, [&](int w) {
+  for_each_work(kp.wctr ? kp.wctr + 1 : nullptr, kp.nwork, kp.groups_per_block, [&](int w) {
     int col;
     const Inst& in = work_inst(inst0, kp, w, col);
     p3_sed_bulk<LANES>(in, col, kp, tb, sm, nullptr, err);
@@ -2636,7 +2458,7 @@ __global__ void __launch_bounds__(256) p3_part3_kernel(const Inst inst0, const K
   Tabs<TR> tb;
   setup_tables<TR>(kp, false, smem_raw, tb, err);
   const int split = kp.part3_split;
-  for_each_work<LANES>(kp.wctr ? kp.wctr + 2 : nullptr, kp.nwork * split, kp.groups_per_block, [&](int w) {
+  for_each_work(kp.wctr ? kp.wctr + 2 : nullptr, kp.nwork * split, kp.groups_per_block, [&](int w) {
     const int item = split == 1 ? w : w / split;
     int col;
     const Inst& in = work_inst(inst0, kp, item, col);

@@ -1,8 +1,16 @@
-/* Sedimentation with a CTA per column: rate type float.  At most one column an
- * SM: the three species at once, in 128 threads each. */
+/* Part1+2 and sedimentation with a CTA per column: rate type float.  Sedimentation
+ * of at most one column an SM: the three species at once, in 128 threads each. */
 #include "p3x_kernels_impl.cuh"
 
 namespace p3x {
+template <>
+cudaError_t launch_part12_wide<float>(const dev::Inst& inst0, const dev::KParams<float>& kp,
+                                        cudaStream_t stream) {
+  const size_t smem = dev::pool_list_entries(1, kp.nlev_max) * sizeof(uint16_t);
+  dev::p3_part12_wide_kernel<float><<<kp.nwork, dev::kPart12WideThreads, smem, stream>>>(inst0, kp);
+  return cudaGetLastError();
+}
+
 template <>
 cudaError_t launch_sed_wide<float>(const dev::Inst& inst0, const dev::KParams<float>& kp, int lanes, int num_sms,
                                 cudaStream_t stream) {

@@ -6,14 +6,14 @@
 namespace p3x {
 
 /* Persistent launch of one kernel: the grid is the number of CTAs that fit on
- * all SMs at once (capped by blocks_per_sm when given, and by the amount of
- * work); groups walk the work list with a grid stride.  The occupancy comes
+ * all SMs at once (capped by blocks_per_sm when given, and by what `groups`
+ * groups of work need); groups walk the work list with a grid stride.  The occupancy comes
  * from a per-device cache, so a launch makes no attribute or occupancy query
  * after the first one of its shape. */
 template <class TR, class Kern>
 cudaError_t launch_persistent(Kern kern, const dev::Inst& inst0, const dev::KParams<TR>& kp, int threads,
                               size_t smem, int blocks_per_sm, int num_sms, cudaStream_t stream,
-                              double grid_frac = 1.0, int split = 1) {
+                              double grid_frac, long long groups) {
   int per_sm = 0;
   cudaError_t e = kernel_occupancy(reinterpret_cast<const void*>(kern), threads, smem, &per_sm);
   if (e != cudaSuccess) return e;
@@ -25,21 +25,51 @@ cudaError_t launch_persistent(Kern kern, const dev::Inst& inst0, const dev::KPar
     const long long share = (long long)(double(grid) * grid_frac);
     grid = share > 0 ? share : 1;
   }
-  const long long need = ((long long)kp.nwork * split + kp.groups_per_block - 1) / kp.groups_per_block;
+  const long long need = (groups + kp.groups_per_block - 1) / kp.groups_per_block;
   if (need < grid) grid = need;
   if (grid <= 0) return cudaSuccess;
   kern<<<int(grid), threads, smem, stream>>>(inst0, kp);
   return cudaGetLastError();
 }
 
-template <class TR, int LANES>
+/* Pools of K1 (pool_range).  The largest hold what pool_columns allows and at
+ * most a warp's share of the call, or two columns where some warp has to take
+ * two anyway: at 21,600 x 128 FP64 2.33 ms with pools of 16 columns, 2.41 with 8,
+ * 3.38 with 1; at 345,600 x 128 FP32-bulk 5.42, 5.49 and 7.81 ms; at 21,600 x
+ * 128 FP32-bulk (a share of 8.9) 0.37 ms with 8, 0.58 with 16; at 5,400 x 72
+ * FP64 0.49 with 4, 0.80 with 1.  Pools of C columns end when C / 4 columns are
+ * left for each of the `warps` warps, and pools of half as many follow; not
+ * where the first are no more than the warps (4,864 x 97 FP64 509 us, with the
+ * smaller pools 562). */
+template <class TR>
+void plan_pools(dev::KParams<TR>& kp, int lanes, long long warps) {
+  int cols = pool_columns(kp.nlev_max, lanes);
+  while (cols > 2 && cols * warps > kp.nwork) cols /= 2;
+  if (kp.nwork <= warps) cols = 1;
+  kp.pool_cols = cols;
+  const bool one_round = cols * warps >= kp.nwork;
+  long long left = kp.nwork, n = 0;
+  int t = 0;
+  for (; cols > 1; cols /= 2) {
+    const long long keep = one_round ? 0 : warps * cols / 4;
+    const long long take = left > keep ? (left - keep + cols - 1) / cols : 0;
+    n += take;
+    left -= take * cols < left ? take * cols : left;
+    kp.pool_end[t++] = int(n);
+  }
+  n += left;
+  for (; t < dev::kPoolTiers - 1; ++t) kp.pool_end[t] = int(n);
+  kp.npools = int(n);
+}
+
+template <class TR>
 cudaError_t launch_p3_part(const dev::Inst& inst0, const dev::KParams<TR>& kp_in, const LaunchSpec& ls, int part,
                            int num_sms, cudaStream_t stream) {
+  constexpr int LANES = 32;
   dev::KParams<TR> kp = kp_in;
-  kp.groups_per_block = ls.groups_per_block;
+  const int threads = warp_threads(ls);
+  kp.groups_per_block = threads / 32;
   kp.staged = ls.staged;
-  const int threads = ls.groups_per_block * LANES;
-  if (threads <= 0 || threads > 256) return cudaErrorInvalidValue;
   cudaError_t e = cudaErrorInvalidValue;
   if (part == kPartK1) {
     if (kp.wctr) {
@@ -47,11 +77,29 @@ cudaError_t launch_p3_part(const dev::Inst& inst0, const dev::KParams<TR>& kp_in
       if (e != cudaSuccess) return e;
     }
     if (ls.marks) cudaEventRecord(ls.marks[0], stream);
-    e = launch_persistent<TR>(dev::p3_part12_kernel<TR, LANES>, inst0, kp, threads,
-                              p3_smem_bytes<TR>(ls, kp.sm_stride), ls.blocks_per_sm, num_sms, stream, ls.grid_frac);
+    if (!ls.staged && part12_wide_fits<TR>(kp, num_sms)) {
+      e = launch_part12_wide<TR>(inst0, kp, stream);
+    } else {
+      const auto kern = dev::p3_part12_kernel<TR>;
+      size_t smem = p3_smem_bytes<TR>(ls, kp.nlev_max);
+      int per_sm = 0;
+      e = kernel_occupancy(reinterpret_cast<const void*>(kern), threads, smem, &per_sm);
+      if (e != cudaSuccess) return e;
+      const long long warps = (long long)per_sm * num_sms * kp.groups_per_block;
+      plan_pools(kp, ls.lanes, warps);
+      /* Fewer pools than warps: CTAs of one warp spread them evenly over the SMs
+       * (912 x 97 FP64: CTAs of 4 warps 193 us, of 2 158). */
+      int cta = threads;
+      if (!ls.staged && kp.npools <= warps) {
+        smem /= kp.groups_per_block;
+        kp.groups_per_block = 1;
+        cta = 32;
+      }
+      e = launch_persistent<TR>(kern, inst0, kp, cta, smem, ls.blocks_per_sm, num_sms, stream, ls.grid_frac, kp.npools);
+    }
     if (e == cudaSuccess && ls.marks) cudaEventRecord(ls.marks[1], stream);
   } else if (part == kPartK2) {
-    if constexpr (LANES == 32) {
+    {
       const int wide = kp.wctr ? sed_wide_lanes(kp.nwork, kp.nlev_max, num_sms) : 0;
       if (wide) {
         e = launch_sed_wide<TR>(inst0, kp, wide, num_sms, stream);
@@ -62,19 +110,19 @@ cudaError_t launch_p3_part(const dev::Inst& inst0, const dev::KParams<TR>& kp_in
           const size_t smem = dev::sed_table_bytes() +
                               size_t(per_sm) * dev::kSedBulkSlots * size_t(kp.sm_stride) * sizeof(double);
           e = launch_persistent<TR>(dev::p3_sed_bulk_kernel<LANES, true>, inst0, kp, per_sm * LANES, smem, 0, num_sms,
-                                    stream, ls.grid_frac);
+                                    stream, ls.grid_frac, kp.nwork);
         } else {
           e = launch_persistent<TR>(dev::p3_sed_bulk_kernel<LANES, false>, inst0, kp, threads,
-                                    sed_smem_bytes<TR>(ls, kp.sm_stride), 0, num_sms, stream, ls.grid_frac);
+                                    sed_smem_bytes<TR>(ls, kp.sm_stride), 0, num_sms, stream, ls.grid_frac, kp.nwork);
         }
       } else {
         e = launch_persistent<TR>(dev::p3_sed_kernel<TR, LANES>, inst0, kp, threads,
-                                  sed_smem_bytes<TR>(ls, kp.sm_stride), 0, num_sms, stream, ls.grid_frac);
+                                  sed_smem_bytes<TR>(ls, kp.sm_stride), 0, num_sms, stream, ls.grid_frac, kp.nwork);
       }
       if (e == cudaSuccess && ls.marks) cudaEventRecord(ls.marks[2], stream);
     }
   } else if (part == kPartK3) {
-    if constexpr (LANES == 32) {
+    {
       /* Levels are independent here: where the columns leave warps idle, one
        * warp takes 32 levels of a column instead of all of them (64 x 72: FP64
        * 31 -> 16 us, FP32-bulk 16 -> 10 us). */
@@ -85,7 +133,8 @@ cudaError_t launch_p3_part(const dev::Inst& inst0, const dev::KParams<TR>& kp_in
       const int chunks = (kp.sm_stride - 1 + LANES - 1) / LANES;
       const long long groups = (long long)per_sm * num_sms * kp.groups_per_block;
       kp.part3_split = kp.wctr && (long long)kp.nwork * chunks <= groups ? chunks : 1;
-      e = launch_persistent<TR>(kern, inst0, kp, threads, 0, 0, num_sms, stream, ls.grid_frac, kp.part3_split);
+      e = launch_persistent<TR>(kern, inst0, kp, threads, 0, 0, num_sms, stream, ls.grid_frac,
+                                (long long)kp.nwork * kp.part3_split);
       if (e == cudaSuccess && ls.marks) cudaEventRecord(ls.marks[3], stream);
     }
   }

@@ -20,12 +20,26 @@ struct LaunchSpec {
   double grid_frac = 1.0;       /* share of the resident-CTA capacity the persistent grid takes */
 };
 
+/* Columns of K1's largest pools: as many as have kPoolLevels levels (16 columns
+ * of 128), 2 or 4 times as many at 16 or 8 lanes per column. */
+constexpr int kPoolLevels = 2048;
+inline int pool_columns(int nlev_max, int lanes) {
+  int cols = 1;
+  while (cols < dev::kPoolMaxCols && cols * 2 * nlev_max <= kPoolLevels) cols *= 2;
+  for (int l = 32; l > lanes && cols < dev::kPoolMaxCols; l /= 2) cols *= 2;
+  return cols;
+}
+
+/* Threads of a CTA: the configured columns x lanes in whole warps. */
+inline int warp_threads(const LaunchSpec& ls) { return (ls.groups_per_block * ls.lanes + 31) / 32 * 32; }
+
 /* Shared-memory bytes of one CTA of K1 (part1+part2; staged tables plus the
- * per-level arrays) and of K2 (sedimentation).  K3 uses none. */
+ * level lists) and of K2 (sedimentation).  K3 uses none. */
 template <class TR>
-inline size_t p3_smem_bytes(const LaunchSpec& ls, int sm_stride) {
+inline size_t p3_smem_bytes(const LaunchSpec& ls, int nlev_max) {
   const size_t tables = ls.staged ? dev::table_smem_bytes<TR>() : 0;
-  return tables + size_t(ls.groups_per_block) * dev::A_NARR * size_t(sm_stride) * sizeof(double);
+  return tables + size_t(warp_threads(ls) / 32) * dev::pool_list_entries(pool_columns(nlev_max, ls.lanes), nlev_max) *
+                      sizeof(uint16_t);
 }
 template <class TR>
 inline size_t sed_smem_bytes(const LaunchSpec& ls, int sm_stride) {
@@ -61,6 +75,17 @@ template <class TR>
 cudaError_t launch_sed_wide(const dev::Inst& inst0, const dev::KParams<TR>& kp, int lanes, int num_sms,
                             cudaStream_t stream);
 
+/* K1 with a CTA per column (p3x_k_dwide.cu, p3x_k_fwide.cu): where all those
+ * CTAs fit on the SMs at once, 2 an SM in the FP64 form, 4 in the FP32-bulk form.
+ * Measured, CTA per column against pools: 64 x 72 FP64 95 / 119 us, 304 x 128
+ * 101 / 182, 456 x 128 183 / 182; FP32-bulk 64 x 72 22 / 32, 304 x 128 24 / 43. */
+template <class TR>
+inline bool part12_wide_fits(const dev::KParams<TR>& kp, int num_sms) {
+  return kp.nwork <= (sizeof(TR) == sizeof(float) ? 4 : 2) * num_sms;
+}
+template <class TR>
+cudaError_t launch_part12_wide(const dev::Inst& inst0, const dev::KParams<TR>& kp, cudaStream_t stream);
+
 /* Columns of one CTA of the FP32-bulk sedimentation that keeps its tables in
  * shared memory, one CTA per SM: as many as fit beside the 20.8 KB of tables, 20
  * at most (96 registers a thread).  0 where that is fewer than 16. */
@@ -82,25 +107,13 @@ cudaError_t kernel_occupancy(const void* func, int threads, size_t smem, int* pe
  * (part3). */
 enum : int { kPartK1 = 1, kPartK2 = 2, kPartK3 = 4 };
 
-/* Persistent launch of one part for one lane count (defined in
- * p3x_kernels_impl.cuh, instantiated in p3x_k_*.cu; K2 and K3 only for 32
- * lanes).
+/* Persistent launch of one part (defined in p3x_kernels_impl.cuh, instantiated
+ * in p3x_k_d.cu and p3x_k_f.cu).
  * kp.nwork, kp.work, kp.insts and kp.sm_stride are set by the caller, and
  * every instance's scratch (Inst::scr, Inst::cflag) is bound. */
-template <class TR, int LANES>
+template <class TR>
 cudaError_t launch_p3_part(const dev::Inst& inst0, const dev::KParams<TR>& kp, const LaunchSpec& ls, int part,
                            int num_sms, cudaStream_t stream);
-
-template <class TR>
-inline cudaError_t launch_p3_part_lanes(const dev::Inst& inst0, const dev::KParams<TR>& kp, const LaunchSpec& ls,
-                                        int part, int num_sms, cudaStream_t stream) {
-  switch (ls.lanes) {
-    case 8: return launch_p3_part<TR, 8>(inst0, kp, ls, part, num_sms, stream);
-    case 16: return launch_p3_part<TR, 16>(inst0, kp, ls, part, num_sms, stream);
-    case 32: return launch_p3_part<TR, 32>(inst0, kp, ls, part, num_sms, stream);
-    default: return cudaErrorInvalidValue;
-  }
-}
 
 /* The column kernels of one step in order on one stream: all three (K1, K2,
  * K3) by default, or the subset `parts` (kPartK* bits).  K1 zeroes the work
@@ -110,17 +123,17 @@ inline cudaError_t launch_p3(const dev::Inst& inst0, const dev::KParams<TR>& kp,
                              int num_sms, cudaStream_t stream, int parts = kPartK1 | kPartK2 | kPartK3) {
   cudaError_t e = cudaSuccess;
   if (parts & kPartK1) {
-    e = launch_p3_part_lanes<TR>(inst0, kp, ls, kPartK1, num_sms, stream);
+    e = launch_p3_part<TR>(inst0, kp, ls, kPartK1, num_sms, stream);
     if (e != cudaSuccess) return e;
   } else if (kp.wctr) {
     e = cudaMemsetAsync(kp.wctr, 0, dev::kWorkCounters * sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
   }
   if (parts & kPartK2) {
-    e = launch_p3_part<TR, 32>(inst0, kp, sed_spec(ls), kPartK2, num_sms, stream);
+    e = launch_p3_part<TR>(inst0, kp, sed_spec(ls), kPartK2, num_sms, stream);
     if (e != cudaSuccess) return e;
   }
-  if (parts & kPartK3) e = launch_p3_part<TR, 32>(inst0, kp, sed_spec(ls), kPartK3, num_sms, stream);
+  if (parts & kPartK3) e = launch_p3_part<TR>(inst0, kp, sed_spec(ls), kPartK3, num_sms, stream);
   return e;
 }
 

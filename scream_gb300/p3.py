@@ -146,8 +146,8 @@ class P3Context:
     def set_launch_config(self, precision: int, lanes=None, columns_per_block=None, table_staging=None,
                           blocks_per_sm=None):
         """Launch configuration of a precision form; arguments left at None keep
-        their current value (defaults: FP64 16 lanes, FP32-bulk 32, both 4
-        columns per CTA, tables through L1)."""
+        their current value (defaults: 32 lanes, 4 columns per CTA, tables
+        through L1)."""
         cur = self.launch_config(precision)
         pick = lambda v, k: cur[k] if v is None else v  # noqa: E731
         cfg = L.LaunchConfig(pick(lanes, "lanes_per_column"), pick(columns_per_block, "columns_per_block"),
