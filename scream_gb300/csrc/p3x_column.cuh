@@ -160,6 +160,12 @@ __device__ __forceinline__ float* scr_f(const Inst& in, int f, int col) {
   return reinterpret_cast<float*>(scr_at(in, f, col));
 }
 
+/* a read where it stands */
+template <class T>
+__device__ __forceinline__ T read_now(const T* p) {
+  return *const_cast<const volatile T*>(p);
+}
+
 /* Launch-wide work counters of one step (K1, K2, K3, spare), zeroed on the
  * stream before K1.  They follow the hand-over doubles and the flags in an
  * instance's scratch. */
@@ -1031,7 +1037,8 @@ __device__ void p3_part12(const Inst& in, const int col0, const int ncol, const 
       const double inv_exner = in.inv_exner[o];
       double th = in.th[o];
       const double dz = in.dz[o];
-      double qv = dmax0(in.qv[o]);
+      const double qv_in = in.qv[o];
+      double qv = dmax0(qv_in);
       const double dpres = in.dpres[o];
       const double qc = in.qc[o], qr = in.qr[o], qi = in.qi[o];
 
@@ -1099,13 +1106,17 @@ __device__ void p3_part12(const Inst& in, const int col0, const int ncol, const 
               th = th - inv_exner * qi * (C::LatVap + C::LatIce) * C::INV_CP;
             }
             T = th * exner;
+            in.th[o] = th;
           }
-          in.qc[o] = 0; in.nc[o] = 0; in.qr[o] = 0; in.nr[o] = 0;
-          in.qi[o] = 0; in.ni[o] = 0; in.qm[o] = 0; in.bm[o] = 0;
-          in.th[o] = th;
+          /* what was read and keeps its bits is not written back: this pass is
+           * bound by its stores */
+          if (dbits(qc)) in.qc[o] = 0;
+          if (dbits(qr)) in.qr[o] = 0;
+          if (dbits(qi)) in.qi[o] = 0;
+          in.nc[o] = 0; in.nr[o] = 0; in.ni[o] = 0; in.qm[o] = 0; in.bm[o] = 0;
         }
       }
-      in.qv[o] = qv;
+      if (dbits(qv) != dbits(qv_in)) in.qv[o] = qv;
       scr_at(in, S_TATM, col)[k] = T;
     }
     const unsigned b_hyd = __ballot_sync(0xffffffffu, is_hyd), b_nuc = __ballot_sync(0xffffffffu, is_nuc);
@@ -1968,33 +1979,88 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
   const int nk = in.nlev;
   const int64_t co = int64_t(col) * in.ld;
   const bool do_ice = rt.do_ice_production != 0;
-  const double* const t_start = scr_at(in, S_TATM, col);
   constexpr bool kF64 = sizeof(TR) == sizeof(double);
+  const auto check = [&](const int64_t o, const int k) {
+    if (!kp.check) return;
+    /* check_values (p3_check_values_impl.hpp:26-81, called at
+     * p3_main_impl.hpp:316-323 with T = th exner): T must lie in
+     * (173, 323) K and qv in (0, 0.04); the reference traps only on T, and
+     * only when its debug abort is on.  Recorded, never trapped. */
+    const double qv = in.qv[o], T = in.th[o] * m_div(1.0, in.inv_exner[o]);
+    const unsigned long long key = check_key(inst_idx, col, k);
+    if (!(dgt(T, 173.0) && dlt(T, 323.0))) {
+      atomicAdd(&kp.check[kChkTCount], 1ull);
+      atomicMin(&kp.check[kChkTFirst], key);
+      if (kp.check_fail) err |= kErrRange;
+    }
+    if (!(dpos(qv) && dlt(qv, 0.04))) {
+      atomicAdd(&kp.check[kChkQvCount], 1ull);
+      atomicMin(&kp.check[kChkQvFirst], key);
+    }
+  };
   /* ---------------- phase 4: homogeneous freezing + p3_main_part3 ---------------- */
   for (int k = first + lane; k < nk; k += step) {
     const int64_t o = co + k;
+    /* Everything a level may need is read at once.  The volatile reads keep the
+     * compiler from moving them behind the hydrometeor test, which moves fewer
+     * bytes but waits for memory twice (FP32-bulk 345,600 x 128 1.85 ms against
+     * 1.64; with every output written back on every level 1.82). */
     State s;
     s.qc = in.qc[o]; s.nc = in.nc[o]; s.qr = in.qr[o]; s.nr = in.nr[o];
     s.qi = in.qi[o]; s.qm = in.qm[o]; s.ni = in.ni[o]; s.bm = in.bm[o];
-    s.qv = in.qv[o]; s.th = in.th[o];
-    const double inv_exner = in.inv_exner[o];
-    const double cld_l = in.cld_frac_l[o], cld_r = in.cld_frac_r[o], cld_i = in.cld_frac_i[o];
+    s.qv = read_now(in.qv + o);
+    s.th = read_now(in.th + o);
+    const double inv_exner = read_now(in.inv_exner + o);
+    const double cld_l = read_now(in.cld_frac_l + o), cld_r = read_now(in.cld_frac_r + o),
+                 cld_i = read_now(in.cld_frac_i + o);
+    const double t_start = read_now(scr_at(in, S_TATM, col) + k);
     /* rho: FP64 in the plain form, a float in the FP32-bulk hand-over */
     double rho = 0, inv_rho = 0;
     float rho_f = 0.f, inv_rho_f = 0.f;
-    if constexpr (kF64) {
-      rho = scr_at(in, S_RHO, col)[k];
-      inv_rho = m_div(1.0, rho);
-    } else {
-      rho_f = scr_f(in, S_RHO, col)[k];
-      inv_rho_f = 1.0f / rho_f;
+    if constexpr (kF64) rho = read_now(scr_at(in, S_RHO, col) + k);
+    else rho_f = read_now(scr_f(in, S_RHO, col) + k);
+    const double vap_in = read_now(in.vap_liq_exchange + o);
+    if (!(dge(s.qc, C::QSMALL) || dge(s.qr, C::QSMALL) || dge(s.qi, C::QSMALL))) {
+      /* no hydrometeor: what is left goes to vapour, and only what changes is
+       * written */
+      if (dnz(s.qc) || dnz(s.qr) || dnz(s.qi)) {
+        double qv = s.qv, th = s.th, vap_liq = vap_in;
+        if (dnz(s.qc)) {
+          qv = qv + s.qc;
+          th = th - inv_exner * s.qc * C::LatVap * C::INV_CP;
+          vap_liq = vap_liq - s.qc;
+        }
+        if (dnz(s.qr)) {
+          qv = qv + s.qr;
+          th = th - inv_exner * s.qr * C::LatVap * C::INV_CP;
+          vap_liq = vap_liq - s.qr;
+        }
+        if (dnz(s.qi)) {
+          qv = qv + s.qi;
+          th = th - inv_exner * s.qi * (C::LatVap + C::LatIce) * C::INV_CP;
+        }
+        in.qv[o] = qv;
+        in.th[o] = th;
+        in.vap_liq_exchange[o] = vap_liq;
+        in.qc[o] = 0; in.qr[o] = 0; in.qi[o] = 0;
+      }
+      if (dnz(s.nc)) in.nc[o] = 0;
+      if (dnz(s.nr)) in.nr[o] = 0;
+      if (dnz(s.ni)) in.ni[o] = 0;
+      if (dnz(s.qm)) in.qm[o] = 0;
+      if (dnz(s.bm)) in.bm[o] = 0;
+      in.rho_qi[o] = 0;
+      check(o, k);
+      continue;
     }
-    double vap_liq = in.vap_liq_exchange[o];
-    double eff_qc = in.diag_eff_radius_qc[o], eff_qr = in.diag_eff_radius_qr[o], eff_qi = in.diag_eff_radius_qi[o];
-    double rho_qi = 0;
+    if constexpr (kF64) inv_rho = m_div(1.0, rho);
+    else inv_rho_f = 1.0f / rho_f;
+    double vap_liq = vap_in;
+    double eff_qc = 0, eff_qr = 0, eff_qi = 0, rho_qi = 0; /* the first three are stored where formed */
+    bool has_c = false, has_r = false, has_i = false;
 
     /* homogeneous_freezing, p3/impl/p3_ice_sed_impl.hpp:207-270 */
-    if (do_ice && dlt(t_start[k], C::T_homogfrz)) {
+    if (do_ice && dlt(t_start, C::T_homogfrz)) {
       const double Qc_nuc = s.qc, Qr_nuc = s.qr;
       const double Nc_nuc = dmax_c(s.nc, C::NSMALL), Nr_nuc = dmax_c(s.nr, C::NSMALL);
       const bool qc_ge = dge(s.qc, C::QSMALL), qr_ge = dge(s.qr, C::QSMALL);
@@ -2027,6 +2093,7 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
         get_cloud_dsd2<TR>(TR(qc_incld), n_out, mu_c, TR(rho), lamc, [](TR x) { return cbrt_fix(x, &kFixTables); });
         apply_n_adjust(nc_incld, n_in, n_out);
         s.nc = nc_incld * cld_l;
+        has_c = true;
         eff_qc = double(m_div(TR(0.5) * (mu_c + TR(3)), lamc));
       } else {
         if (dnz(s.qc)) {
@@ -2047,6 +2114,7 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
         get_rain_dsd2<TR>(TR(qr_incld), n_out, mu_r, lamr, rt, [](TR x) { return cbrt_fix(x, &kFixTables); });
         apply_n_adjust(nr_incld, n_in, n_out);
         s.nr = nr_incld * cld_r;
+        has_r = true;
         eff_qr = double(m_div(TR(1.5), lamr));
       } else {
         if (dnz(s.qr)) {
@@ -2061,18 +2129,15 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
       {
         const bool qi_gt_small = dge(s.qi, C::QSMALL);
         s.ni = dmax_c(s.ni, C::NSMALL);
-        const double qi_incld = m_div(s.qi, cld_i);
-        double ni_incld = m_div(s.ni, cld_i);
-        double qm_incld = m_div(s.qm, cld_i);
-        double bm_incld = m_div(s.bm, cld_i);
-        double rhop = 0;
         if (qi_gt_small) {
-          rhop = calc_bulk_rho_rime(qi_incld, qm_incld, bm_incld, rt);
+          const double qi_incld = m_div(s.qi, cld_i);
+          double ni_incld = m_div(s.ni, cld_i);
+          double qm_incld = m_div(s.qm, cld_i);
+          double bm_incld = m_div(s.bm, cld_i);
+          const double rhop = calc_bulk_rho_rime(qi_incld, qm_incld, bm_incld, rt);
           s.qm = qm_incld * cld_i;
           s.bm = bm_incld * cld_i;
-        }
-        impose_max_total_ni(ni_incld, rt.max_total_ni, inv_rho);
-        if (qi_gt_small) {
+          impose_max_total_ni(ni_incld, rt.max_total_ni, inv_rho);
           /* table position, limits and values in fixed point (part3 0.87 ->
            * 0.37 ms at 21,600 x 128) */
           const IceCell cell = ice_cell(m_div(qi_incld, ni_incld), m_div(qm_incld, qi_incld), rhop, &kFixTables);
@@ -2081,16 +2146,16 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
           const int64_t hi = ice_cell_value(cf, cell), lo = ice_cell_value(cf + kCellCoefs, cell);
           if (fix_below_one(hi, sh.x)) ni_incld = d_from_fix(hi, sh.x) * ni_incld;
           if (!fix_below_one(lo, sh.y)) ni_incld = d_from_fix(lo, sh.y) * ni_incld;
+          has_i = true;
           eff_qi = d_from_fix(ice_cell_value(cf + 2 * kCellCoefs, cell), sh.z);
           rho_qi = d_from_fix(ice_cell_value(cf + 3 * kCellCoefs, cell), sh.w);
           if (cell.odd) ni_incld = eff_qi = rho_qi = d_from_bits(kNaNBits);
-        }
-        s.ni = ni_incld * cld_i;
-        if (dlt(s.qm, C::QSMALL) && qi_gt_small) {
-          s.qm = 0;
-          s.bm = 0;
-        }
-        if (!qi_gt_small) {
+          s.ni = ni_incld * cld_i;
+          if (dlt(s.qm, C::QSMALL)) {
+            s.qm = 0;
+            s.bm = 0;
+          }
+        } else {
           if (dnz(s.qi)) {
             s.qv = s.qv + s.qi;
             s.th = s.th - inv_exner * s.qi * (C::LatVap + C::LatIce) * C::INV_CP;
@@ -2108,6 +2173,7 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
         float n_out = n_in, mu_c, lamc;
         get_cloud_dsd2<float>(qc_f, n_out, mu_c, rho_f, lamc);
         if (n_out != n_in) s.nc = f2d_int(n_out) * cld_l;
+        has_c = true;
         eff_qc = f2d_int(0.5f * (mu_c + 3.0f) / lamc);
       } else {
         if (dnz(s.qc)) {
@@ -2125,6 +2191,7 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
         float n_out = n_in, mu_r = 0, lamr;
         get_rain_dsd2<float>(qr_f, n_out, mu_r, lamr, rt);
         if (n_out != n_in) s.nr = f2d_int(n_out) * cld_r;
+        has_r = true;
         eff_qr = f2d_int(1.5f / lamr);
       } else {
         if (dnz(s.qr)) {
@@ -2156,6 +2223,7 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
           apply_table_ice4<float>(tb, ti, 8, te); /* columns 5, 11, 8, 10 */
           ni_f = vmin(ni_f, ta[2] * ni_f);
           ni_f = vmax(ni_f, ta[3] * ni_f);
+          has_i = true;
           eff_qi = f2d_int(te[0]);
           rho_qi = f2d_int(te[1]);
           if (ni_f != ni0) s.ni = f2d_int(ni_f) * cld_i;
@@ -2174,31 +2242,13 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
     }
     if (dlt(s.qr, C::QSMALL)) s.nr = 0;
 
-    in.qc[o] = s.qc; in.nc[o] = s.nc; in.qr[o] = s.qr; in.nr[o] = s.nr;
-    in.qi[o] = s.qi; in.qm[o] = s.qm; in.ni[o] = s.ni; in.bm[o] = s.bm;
-    in.qv[o] = s.qv; in.th[o] = s.th;
+    store_state(in, o, s);
     in.vap_liq_exchange[o] = vap_liq;
-    in.diag_eff_radius_qc[o] = eff_qc;
-    in.diag_eff_radius_qr[o] = eff_qr;
-    in.diag_eff_radius_qi[o] = eff_qi;
+    if (has_c) in.diag_eff_radius_qc[o] = eff_qc;
+    if (has_r) in.diag_eff_radius_qr[o] = eff_qr;
+    if (has_i) in.diag_eff_radius_qi[o] = eff_qi;
     in.rho_qi[o] = rho_qi;
-    if (kp.check) {
-      /* check_values (p3_check_values_impl.hpp:26-81, called at
-       * p3_main_impl.hpp:316-323 with T = th exner): T must lie in
-       * (173, 323) K and qv in (0, 0.04); the reference traps only on T, and
-       * only when its debug abort is on.  Recorded, never trapped. */
-      const double T = s.th * m_div(1.0, inv_exner);
-      const unsigned long long key = check_key(inst_idx, col, k);
-      if (!(dgt(T, 173.0) && dlt(T, 323.0))) {
-        atomicAdd(&kp.check[kChkTCount], 1ull);
-        atomicMin(&kp.check[kChkTFirst], key);
-        if (kp.check_fail) err |= kErrRange;
-      }
-      if (!(dpos(s.qv) && dlt(s.qv, 0.04))) {
-        atomicAdd(&kp.check[kChkQvCount], 1ull);
-        atomicMin(&kp.check[kChkQvFirst], key);
-      }
-    }
+    check(o, k);
   }
 }
 
