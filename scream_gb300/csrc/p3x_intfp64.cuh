@@ -348,12 +348,15 @@ struct IceCell {
 constexpr int kCellI = 49, kCellR = 3, kCellD = 4, kIceCells = kCellI * kCellR * kCellD;
 /* log2_qn: log2(qi / ni), Q57; ratio: qm / qi in Q60, at most 1; rho52: rime
  * density in Q52, at most 1023 (beyond 900 the axis ends) */
-P3X_HD IceCell ice_cell_at(int64_t log2_qn, uint64_t ratio, uint64_t rho52) {
+P3X_HD FixAxis ice_size_at(int64_t log2_qn) {
   /* d log2(x) + c of the size axis less one, Q55 */
   constexpr int64_t kd = 5741805296813221454ll; /* 4.135985029041767 log10(2), Q62 */
   constexpr int64_t kc = 2285945404318149440ll;  /* 18 * 4.135985029041767 - 11, Q55 */
   const int64_t x1 = mulhi_s64(log2_qn, kd) + kc;
-  const FixAxis a1 = fix_axis(fix_clamp(x1, 0, 49ll << 55), 55, kCellI);
+  return fix_axis(fix_clamp(x1, 0, 49ll << 55), 55, kCellI);
+}
+P3X_HD IceCell ice_cell_at(int64_t log2_qn, uint64_t ratio, uint64_t rho52) {
+  const FixAxis a1 = ice_size_at(log2_qn);
   const FixAxis a4 = fix_axis(int64_t(3 * ratio), 60, kCellR);
   /* (rho - 50) 0.005 up to 650, 3 + (rho - 650) 0.004 above, Q58 */
   const bool low = rho52 <= (650ull << 52);
@@ -417,6 +420,15 @@ P3X_HD int64_t ice_cell_value(const int64_t* c, const IceCell& p) {
   for (int j = 0; j < kCellCoefs; ++j) k[j] = c[j];
 #endif
   return fix_trilinear(k, p.w1, p.w4, p.w5);
+}
+/* the same in cell {i of the size axis, 0, 0} with the rime and density weights 0 */
+P3X_HD int64_t ice_cell_value_unrimed(const int64_t* c, int64_t w1) {
+#ifdef __CUDA_ARCH__
+  const longlong2 v = __ldg(reinterpret_cast<const longlong2*>(c));
+  return mulhi_add(v.x, w1, v.y);
+#else
+  return mulhi_add(c[0], w1, c[1]);
+#endif
 }
 /* V 2^-s < 1 for V >= 0 */
 P3X_HD bool fix_below_one(int64_t V, int s) { return s >= 0 && (V >> (s < 63 ? s : 63)) == 0; }

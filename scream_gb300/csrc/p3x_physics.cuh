@@ -477,13 +477,17 @@ struct Table3 {
 
 /* lookup_ice, p3/impl/p3_table_ice_impl.hpp:80-138 */
 template <class TR>
+__device__ __forceinline__ void ice_size_axis(TR qi, TR ni, TR& dum1, int& dumi) {
+  dum1 = (m_log10(m_div(qi, ni)) + TR(18)) * TR(C::lookup_table_1a_dum1_c) - TR(10);
+  dumi = table_index(dum1, kIsize);
+  dum1 = vmin(dum1, TR(kIsize));
+  dum1 = vmax(dum1, TR(1.));
+  dumi = max(1, dumi);
+  dumi = min(kIsize - 1, dumi);
+}
+template <class TR>
 __device__ __forceinline__ void lookup_ice(TR qi, TR ni, TR qm, TR rhop, TableIce<TR>& tab) {
-  tab.dum1 = (m_log10(m_div(qi, ni)) + TR(18)) * TR(C::lookup_table_1a_dum1_c) - TR(10);
-  tab.dumi = table_index(tab.dum1, kIsize);
-  tab.dum1 = vmin(tab.dum1, TR(kIsize));
-  tab.dum1 = vmax(tab.dum1, TR(1.));
-  tab.dumi = max(1, tab.dumi);
-  tab.dumi = min(kIsize - 1, tab.dumi);
+  ice_size_axis<TR>(qi, ni, tab.dum1, tab.dumi);
   tab.dum4 = m_div(qm, qi) * TR(3) + TR(1);
   tab.dumii = table_index(tab.dum4, kRimsize);
   tab.dum4 = vmin(tab.dum4, TR(kRimsize));
@@ -578,6 +582,22 @@ __device__ __forceinline__ void ice_table4_f32(const float* ice, const TableIce<
   const float2 t2h = lerp2(lerp2(hi(b00), hi(b01), W1), lerp2(hi(b10), hi(b11), W1), W4);
   const float2 rl = lerp2(t1l, t2l, W5), rh = lerp2(t1h, t2h, W5);
   out[0] = rl.x; out[1] = rl.y; out[2] = rh.x; out[3] = rh.y;
+}
+/* lookup_ice and ice_table4_f32 of ice without rime: the rime and density axes
+ * are at their first points with zero weights, so the eight corners come down to
+ * two (the same value: a zero weight adds nothing). */
+template <int STRIDE>
+__device__ __forceinline__ void ice_table4_unrimed(const float* ice, float qi, float ni, int s0, float out[4]) {
+  float dum1;
+  int dumi;
+  ice_size_axis<float>(qi, ni, dum1, dumi);
+  dumi -= 1;
+  const float2 W1 = f2splat(dum1 - ival<float>(dumi) - 1.0f);
+  const float* const r = ice + dumi * STRIDE + s0;
+  const float4 a = *reinterpret_cast<const float4*>(r), b = *reinterpret_cast<const float4*>(r + STRIDE);
+  const float2 l = lerp2(make_float2(a.x, a.y), make_float2(b.x, b.y), W1);
+  const float2 h = lerp2(make_float2(a.z, a.w), make_float2(b.z, b.w), W1);
+  out[0] = l.x; out[1] = l.y; out[2] = h.x; out[3] = h.y;
 }
 template <>
 __device__ __forceinline__ void apply_table_ice4<float>(const Tabs<float>& t, const TableIce<float>& tab, int s0,
