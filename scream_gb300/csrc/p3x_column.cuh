@@ -1579,7 +1579,14 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
  * per field and level; both neighbours of a face read the same G, so the
  * column's mass telescopes exactly, and the surface precipitation is the
  * bottom face's G.  Where a limiter rewrites a level's state to x during the
- * walk, B_k is reset so that R_k = x at that moment. */
+ * walk, B_k is reset so that R_k = x at that moment.
+ *
+ * What bounds it: latency, at 20 warps an SM (issue 54 %, FP64 pipe 42 %).  The
+ * compiler keeps global reads behind the stores in front of them, which may
+ * alias, so each would wait for memory by itself; they are therefore grouped by
+ * hand: the density a chunk ahead in the flux walk, two chunks at a time where a
+ * species is read, all fields of a chunk at once where its state is rebuilt.
+ * 345,600 x 128 9.30 -> 8.00 ms, 21,600 x 128 822 -> 721 us. */
 template <int LANES, bool SPLIT = false>
 __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>& kp, const Tabs<float>& tb,
                             double* __restrict__ sm, GroupScratch* gs, uint32_t& err) {
@@ -1643,11 +1650,22 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
   if (SPLIT && lane < 3) gs->prt[lane] = 0;
   group_bounds<LANES, SPLIT>(mask, gs, top, bot);
   const int k_first = min(top[0], min(top[1], top[2]));
-  for (int k = k_first + lane; k < nk; k += LANES) {
-    const double coef = C::gravit * rcp_newton(in.dpres[co + k]);
-    INVDZf[k] = 1.0f / float(in.dz[co + k]);
-    COEF[k] = coef;
-    COEFf[k] = float(coef);
+  constexpr int kBatch = LANES > 32 ? 1 : 2; /* chunks read at once */
+  for (int k = k_first + lane; k < nk; k += kBatch * LANES) {
+    double dp[kBatch], dz[kBatch];
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      dp[i] = in.dpres[co + min(k + i * LANES, kbot)];
+      dz[i] = in.dz[co + min(k + i * LANES, kbot)];
+    }
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const int ki = min(k + i * LANES, kbot);
+      const double coef = C::gravit * rcp_newton(dp[i]);
+      INVDZf[ki] = 1.0f / float(dz[i]);
+      COEF[ki] = coef;
+      COEFf[ki] = float(coef);
+    }
   }
   double precip_liq_surf = 0, precip_ice_surf = 0;
 
@@ -1710,17 +1728,36 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
     int k_qxbot = bot[sp];
     if (k_qxbot < 0) return; /* species absent (group-uniform) */
     /* the walk and the rebuild read G one level above the top */
-    for (int k = max(k_qxtop - 1, 0) + lane; k < nk; k += LANES) {
-      G01[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (sp == 2) G23[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (k >= k_qxtop) {
-        R01[k] = make_float2(float(B0[co + k]), float(B1[co + k]));
-        CLDf[k] = float(cldp[co + k]);
-        FACf[k] = facp[k];
-        if (kDefer) late_vn[k] = kNotLate;
+    /* kBatch chunks are read before any is stored */
+    for (int k = max(k_qxtop - 1, 0) + lane; k < nk; k += kBatch * LANES) {
+      double b0[kBatch], b1[kBatch], b2[kBatch], b3[kBatch], cl[kBatch];
+      float fac[kBatch];
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) {
+        const int64_t o = co + min(k + i * LANES, kbot);
+        b0[i] = B0[o];
+        b1[i] = B1[o];
+        cl[i] = cldp[o];
+        fac[i] = facp[min(k + i * LANES, kbot)];
         if (sp == 2) {
-          R23[k] = make_float2(float(B2[co + k]), float(B3[co + k]));
-          late_vb[k] = kNotLate;
+          b2[i] = B2[o];
+          b3[i] = B3[o];
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) {
+        const int ki = k + i * LANES;
+        if (ki >= nk) break;
+        G01[ki] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (sp == 2) G23[ki] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ki < k_qxtop) continue;
+        R01[ki] = make_float2(float(b0[i]), float(b1[i]));
+        CLDf[ki] = float(cl[i]);
+        FACf[ki] = fac[i];
+        if (kDefer) late_vn[ki] = kNotLate;
+        if (sp == 2) {
+          R23[ki] = make_float2(float(b2[i]), float(b3[i]));
+          late_vb[ki] = kNotLate;
         }
       }
     }
@@ -1856,6 +1893,9 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
       if (k_qxbot < kbot && lane == (k_qxbot + 1 - k_qxtop) % LANES) {
         V12[k_qxbot + 1] = make_float2(0.f, 0.f); /* the cell receiving the leading edge has no fall speed */
       }
+      /* the density row has no slot and little L1 beside the shared memory: read a
+       * chunk ahead of its use */
+      float rho_next = RHOf[min(k_qxtop + lane, kbot)];
       const float Co_max = group_max_wide<LANES, SPLIT>(mask, gs, lmax) * dt_left;
       if (!(Co_max >= 0.0f) || Co_max > 2.0e9f) {
         err |= kErrNumeric;
@@ -1873,8 +1913,10 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
         const int k = base + lane;
         const bool act = k <= k_temp;
         float2 f01 = make_float2(0.f, 0.f), f23 = make_float2(0.f, 0.f);
+        const float rho = rho_next;
+        if (base + LANES <= k_temp) rho_next = RHOf[min(k + LANES, kbot)];
         if (act) {
-          const float2 rho2 = f2splat(RHOf[k]);
+          const float2 rho2 = f2splat(rho);
           const float2 v = V12[k];
           f01 = __fmul2_rn(__fmul2_rn(v, R01[k]), rho2);
           if (nfield < 2) f01.y = 0.f;
@@ -1946,30 +1988,41 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
     for (int base = k_qxtop; base <= k_qxbot; base += LANES) {
       const int k = base + lane;
       const bool act = k <= k_qxbot;
+      const int kc = min(k, kbot);
+      /* read at once: a field's store would hold up the next field's reads */
+      double B[4];
+      float late_n = kNotLate, late_b = kNotLate;
+#pragma unroll
+      for (int f = 0; f < nstate; ++f) B[f] = read_now(&Bf[f][co + kc]);
+      if (kDefer) late_n = read_now(&late_vn[kc]);
+      if (sp == 2) late_b = read_now(&late_vb[kc]);
+      bool rime = sp == 2;
+      if (sp == 2 && LANES == 32) {
+        const float4 g = G23[kc];
+        rime = __any_sync(mask, act && (g.x != 0.f || g.y != 0.f || __float_as_uint(late_b) != 0xffc0deadu)) ||
+               dnz(g_in[2]) || dnz(g_in[3]);
+      }
 #pragma unroll
       for (int f = 0; f < 4; ++f) {
-        if (f < nstate) {
+        if (f < nstate && (f < 2 || rime)) {
           const double g = act ? g_value(f, k) : 0.0;
           double gin = __shfl_up_sync(mask, g, 1, kWarp);
           if (lane == 0) gin = g_in[f];
           if (LANES > 32 && (lane & 31) == 0 && lane > 0 && act) gin = g_value(f, k - 1);
           if (act) {
-            double B = Bf[f][co + k];
-            if (kDefer && (f == 1 || f == 3)) {
-              const float v = f == 1 ? late_vn[k] : late_vb[k];
-              if (__float_as_uint(v) != 0xffc0deadu) {
-                const float2 g0 = make_float2(__int_as_float(__double2loint(B)), __int_as_float(__double2hiint(B)));
-                float2 gin0;
-                if (f == 1) {
-                  gin0 = make_float2(late_gh[k], late_gl[k]);
-                } else {
-                  gin0 = *reinterpret_cast<const float2*>(&in.rho_qi[co + k]);
-                  in.rho_qi[co + k] = 0;
-                }
-                B = reset_value(k, v, CLDf[k], dfloat_value(gin0), dfloat_value(g0));
+            const float v = f == 1 ? late_n : late_b;
+            if (kDefer && (f == 1 || f == 3) && __float_as_uint(v) != 0xffc0deadu) {
+              const float2 g0 = make_float2(__int_as_float(__double2loint(B[f])), __int_as_float(__double2hiint(B[f])));
+              float2 gin0;
+              if (f == 1) {
+                gin0 = make_float2(late_gh[k], late_gl[k]);
+              } else {
+                gin0 = *reinterpret_cast<const float2*>(&in.rho_qi[co + k]);
+                in.rho_qi[co + k] = 0;
               }
+              B[f] = reset_value(k, v, CLDf[k], dfloat_value(gin0), dfloat_value(g0));
             }
-            Bf[f][co + k] = B + COEF[k] * (gin - g);
+            Bf[f][co + k] = B[f] + COEF[k] * (gin - g);
           }
           g_in[f] = __shfl_sync(mask, g, kWarp - 1, kWarp);
         }
