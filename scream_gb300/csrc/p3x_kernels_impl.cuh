@@ -80,7 +80,7 @@ cudaError_t launch_p3_part(const dev::Inst& inst0, const dev::KParams<TR>& kp_in
     if (!ls.staged && part12_wide_fits<TR>(kp, num_sms)) {
       e = launch_part12_wide<TR>(inst0, kp, stream);
     } else {
-      const auto kern = dev::p3_part12_kernel<TR>;
+      const auto kern = kp.work ? dev::p3_part12_kernel<TR, true> : dev::p3_part12_kernel<TR, false>;
       size_t smem = p3_smem_bytes<TR>(ls, kp.nlev_max);
       int per_sm = 0;
       e = kernel_occupancy(reinterpret_cast<const void*>(kern), threads, smem, &per_sm);
