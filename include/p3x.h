@@ -128,9 +128,9 @@ typedef struct p3x_layout {
 
 /* Launch configuration (chosen by p3x_autotune or set by hand). */
 typedef struct p3x_launch_config {
-  int32_t lanes_per_column;  /* 8, 16 or 32: part1+2 pools 4, 2 or 1 times the */
-                             /*    default number of columns per warp;         */
-                             /*    sedimentation and part3 always run 32 lanes */
+  int32_t lanes_per_column;  /* 8, 16 or 32: a warp of part1+2 pools up to 4,  */
+                             /*    2 or 1 times 2,048 levels, 16 columns at    */
+                             /*    most; sedimentation and part3 always run 32 */
   int32_t columns_per_block; /* times lanes_per_column: threads of one CTA     */
   int32_t table_staging;     /* 0: tables read through L1/L2; 1: staged into   */
                              /*    shared memory by bulk copies (cp.async.bulk) */

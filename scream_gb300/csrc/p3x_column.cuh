@@ -2411,9 +2411,9 @@ __device__ __forceinline__ const Inst& work_inst(const Inst& inst0, const KParam
   return inst0;
 }
 
-/* Pool i of a launch's work items: sizes go down from pool_cols to 1, halved
- * whenever the pools of a size are used up (pool_end), so that the last pools
- * are small and every warp ends at about the same time. */
+/* Pool i of a launch's work items: pool_cols of them, and half as many whenever
+ * the pools of a size are used up (pool_end), so that the last pools of a call of
+ * several rounds are small and every warp ends at about the same time. */
 template <class TR>
 __device__ __forceinline__ void pool_range(const KParams<TR>& kp, const int i, int& w0, int& w1) {
   int first = 0, size = kp.pool_cols;

@@ -32,22 +32,26 @@ cudaError_t launch_persistent(Kern kern, const dev::Inst& inst0, const dev::KPar
   return cudaGetLastError();
 }
 
-/* Pools of K1 (pool_range).  The largest hold what pool_columns allows and at
- * most a warp's share of the call, or two columns where some warp has to take
- * two anyway: at 21,600 x 128 FP64 2.33 ms with pools of 16 columns, 2.41 with 8,
- * 3.38 with 1; at 345,600 x 128 FP32-bulk 5.42, 5.49 and 7.81 ms; at 21,600 x
- * 128 FP32-bulk (a share of 8.9) 0.37 ms with 8, 0.58 with 16; at 5,400 x 72
- * FP64 0.49 with 4, 0.80 with 1.  Pools of C columns end when C / 4 columns are
- * left for each of the `warps` warps, and pools of half as many follow; not
- * where the first are no more than the warps (4,864 x 97 FP64 509 us, with the
- * smaller pools 562). */
+/* Pools of K1 (pool_range).  A call of at most pool_columns columns for each of
+ * the `warps` warps gives every warp one pool of its share: against pools that
+ * get smaller towards the end 2,600 x 72 FP64 271 us / 356, 5,400 x 72 474 / 504,
+ * 16,000 x 128 1.86 ms / 1.99, FP32-bulk 16,000 x 128 262 us / 288.  A larger call
+ * takes pools of C = pool_columns columns until C / 4 columns are left for each
+ * warp, and then pools of half as many, and so on (21,600 x 128 FP64: C = 16 2.33
+ * ms, 8 2.41, 1 3.38; 345,600 x 128 FP32-bulk 5.42, 5.49 and 7.81 ms), and so does
+ * a work list, whose instances differ in depth. */
 template <class TR>
 void plan_pools(dev::KParams<TR>& kp, int lanes, long long warps) {
   int cols = pool_columns(kp.nlev_max, lanes);
-  while (cols > 2 && cols * warps > kp.nwork) cols /= 2;
-  if (kp.nwork <= warps) cols = 1;
+  const long long share = (kp.nwork + warps - 1) / warps;
+  const bool one_round = !kp.work && share <= cols;
+  if (one_round) {
+    cols = int(share);
+  } else {
+    while (cols > 2 && cols * warps > kp.nwork) cols /= 2;
+    if (kp.nwork <= warps) cols = 1;
+  }
   kp.pool_cols = cols;
-  const bool one_round = cols * warps >= kp.nwork;
   long long left = kp.nwork, n = 0;
   int t = 0;
   for (; cols > 1; cols /= 2) {
