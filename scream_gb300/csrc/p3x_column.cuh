@@ -511,8 +511,24 @@ __device__ __forceinline__ void hydro_level_bulk(const Inst& in, const int col, 
   const float cl = float(cld_l), ci = float(cld_i), cr = float(cld_r);
   const float icl = 1.0f / cl, ici = 1.0f / ci, icr = 1.0f / cr;
   /* FP32 shadows of the state (kept equal to float(s.x) where s.x changes) */
-  const float qc0 = float(s.qc), qr0 = float(s.qr), qi0 = float(s.qi), ni0 = float(s.ni);
-  float nc0 = float(s.nc), nr0 = float(s.nr), qm0 = float(s.qm), bm0 = float(s.bm);
+  /* part1 left a species below qsmall at zero */
+  float qc0 = 0, nc0 = 0, qr0 = 0, nr0 = 0, qi0 = 0, ni0 = 0, qm0 = 0, bm0 = 0;
+  if (dnz(s.qc) || dnz(s.nc)) {
+    qc0 = float(s.qc);
+    nc0 = float(s.nc);
+  }
+  if (dnz(s.qr) || dnz(s.nr)) {
+    qr0 = float(s.qr);
+    nr0 = float(s.nr);
+  }
+  if (dnz(s.qi) || dnz(s.ni)) {
+    qi0 = float(s.qi);
+    ni0 = float(s.ni);
+  }
+  if (dnz(s.qm) || dnz(s.bm)) {
+    qm0 = float(s.qm);
+    bm0 = float(s.bm);
+  }
   constexpr float QS = float(C::QSMALL);
 
   /* calculate_incloud_mixingratios (bm uses 1/cld_frac_l, p3_incloud_mixingratios_impl.hpp:49) */
@@ -666,13 +682,13 @@ __device__ __forceinline__ void hydro_level_bulk(const Inst& in, const int col, 
   update_prognostics_bulk(r, inv_exner, predictNc, prescribedCCN, wet, dtf, rho_qm_cloud, f2d(inv_rho), wlim, nlim,
                           r_lim, qi0, qm0, bm0, s);
 
-  in.qv2qi_depos_tend[o] = f2d(r.qv2qi_vapdep_tend - r.qi2qv_sublim_tend + r.qv2qi_nucleat_tend);
-  in.precip_total_tend[o] = f2d(r.qc2qr_accret_tend + r.qc2qr_autoconv_tend + r.qc2qr_ice_shed_tend +
+  in.qv2qi_depos_tend[o] = f2d_zero(r.qv2qi_vapdep_tend - r.qi2qv_sublim_tend + r.qv2qi_nucleat_tend);
+  in.precip_total_tend[o] = f2d_zero(r.qc2qr_accret_tend + r.qc2qr_autoconv_tend + r.qc2qr_ice_shed_tend +
                                 r.qc2qi_collect_tend);
-  in.nevapr[o] = f2d(r.qi2qv_sublim_tend + r.qr2qv_evap_tend);
-  in.vap_ice_exchange[o] = f2d(r.qv2qi_vapdep_tend - r.qi2qv_sublim_tend + r.qv2qi_nucleat_tend);
-  in.vap_liq_exchange[o] = f2d(-r.qr2qv_evap_tend);
-  in.liq_ice_exchange[o] = f2d(r.qc2qi_hetero_freeze_tend + r.qr2qi_immers_freeze_tend - r.qi2qr_melt_tend +
+  in.nevapr[o] = f2d_zero(r.qi2qv_sublim_tend + r.qr2qv_evap_tend);
+  in.vap_ice_exchange[o] = f2d_zero(r.qv2qi_vapdep_tend - r.qi2qv_sublim_tend + r.qv2qi_nucleat_tend);
+  in.vap_liq_exchange[o] = f2d_zero(-r.qr2qv_evap_tend);
+  in.liq_ice_exchange[o] = f2d_zero(r.qc2qi_hetero_freeze_tend + r.qr2qi_immers_freeze_tend - r.qi2qr_melt_tend +
                                r.qc2qi_berg_tend + r.qc2qi_collect_tend + r.qr2qi_collect_tend);
 
   hydro |= clip_to_vapour(s, inv_exner);

@@ -295,6 +295,13 @@ __device__ __forceinline__ double dmax_0x(double x) { return dpos(x) ? x : 0.0; 
  * intrinsics, so the compiler can neither contract nor reorder it.  One update
  * costs ~14 FP32 instructions, against one FP64 FMA that occupies the FP64
  * pipe for the issue time of ~64 FP32 instructions on this part. */
+/* float -> double that leaves the FP64 pipe alone where every lane's value is
+ * zero (+0 and -0 keep their sign) */
+__device__ __forceinline__ double f2d_zero(float x) {
+  double d = __hiloint2double(int(__float_as_uint(x)), 0);
+  if (x != 0.0f) d = f2d(x);
+  return d;
+}
 /* exact value as a double: |lo| <= ulp(hi)/2, so hi + lo spans <= 48 bits */
 __device__ __forceinline__ double dfloat_value(float2 g) { return f2d(g.x) + f2d(g.y); }
 
@@ -1523,21 +1530,35 @@ __device__ __forceinline__ void update_prognostics_bulk(const Rates<float>& r, d
    * cancelling terms (~1e10 /kg, FP32 spacing ~1e3) would otherwise leave a
    * residue of ~1e3 /kg in place of that value, and rain sedimentation turns
    * it into a different drop size and fall speed. */
-  const double Dqc = (wlim & 1) ? -s.qc : f2d(dqc);
-  const double Dqr = (wlim & 2) ? -s.qr + f2d((r_lim.qr2qv_evap_tend - r.qr2qv_evap_tend) * dtf) : f2d(dqr);
+  /* A change of zero (a species that is absent: its rates are +-0) is left out:
+   * an FP64 instruction takes its pipe as long for one lane as for 32, and
+   * neighbouring levels mostly hold the same species. */
+  double Dqc = 0, Dqr = 0;
+  if (dqc != 0.0f || (wlim & 1)) {
+    Dqc = (wlim & 1) ? -s.qc : f2d(dqc);
+    s.qc = s.qc + Dqc;
+  }
+  if (dqr != 0.0f || (wlim & 2)) {
+    Dqr = (wlim & 2) ? -s.qr + f2d((r_lim.qr2qv_evap_tend - r.qr2qv_evap_tend) * dtf) : f2d(dqr);
+    s.qr = s.qr + Dqr;
+  }
   const double Dqi = ((wlim & 4) && dge(s.qi, C::QSMALL))
                          ? -s.qi + f2d(((r.qv2qi_vapdep_tend - r_lim.qv2qi_vapdep_tend) +
                                         (r.qv2qi_nucleat_tend - r_lim.qv2qi_nucleat_tend) -
                                         (r.qi2qv_sublim_tend - r_lim.qi2qv_sublim_tend)) * dtf)
                          : f2d(dqi);
   s.qi = s.qi + Dqi;
-  s.qm = s.qm + f2d(dqm);
-  s.bm = s.bm + f2d(dbm);
-  s.ni = (nlim & 4) ? 0.0 : s.ni + f2d(dni);
+  if (dqm != 0.0f || dbm != 0.0f) {
+    s.qm = s.qm + f2d(dqm);
+    s.bm = s.bm + f2d(dbm);
+  }
+  if (nlim & 4) {
+    s.ni = 0.0;
+  } else if (dni != 0.0f) {
+    s.ni = s.ni + f2d(dni);
+  }
   if (dneg(s.qm)) { s.qm = 0; s.bm = 0; }
   if (log_wetgrowth) { s.qm = s.qi; s.bm = s.qm * C::INV_RHO_RIMEMAX; }
-  s.qc = s.qc + Dqc;
-  s.qr = s.qr + Dqr;
   s.qv = s.qv - (Dqc + Dqr + Dqi);
   /* Latent heating from the FP64 condensate changes.  The reference heats by
    * (Lv+Lf)/cp per vapour -> ice, Lf/cp per liquid -> ice and -Lv/cp per
@@ -1550,11 +1571,19 @@ __device__ __forceinline__ void update_prognostics_bulk(const Rates<float>& r, d
   if (predictNc || prescribedCCN) {
     float dnc = (-r.nc_accret_tend - r.nc2nr_autoconv_tend + r.nc_selfcollect_tend) * dtf;
     if (predictNc) dnc += (-r.nc_collect_tend - r.nc2ni_immers_freeze_tend) * dtf;
-    s.nc = ((nlim & 1) && predictNc) ? 0.0 : s.nc + f2d(dnc);
+    if ((nlim & 1) && predictNc) {
+      s.nc = 0.0;
+    } else if (dnc != 0.0f) {
+      s.nc = s.nc + f2d(dnc);
+    }
   } else {
     s.nc = C::NCCNST * inv_rho;
   }
-  s.nr = (nlim & 2) ? f2d((r.ncautr - r.nc2nr_autoconv_tend) * dtf) : s.nr + f2d(dnr);
+  if (nlim & 2) {
+    s.nr = f2d((r.ncautr - r.nc2nr_autoconv_tend) * dtf);
+  } else if (dnr != 0.0f) {
+    s.nr = s.nr + f2d(dnr);
+  }
 }
 
 }  // namespace dev
