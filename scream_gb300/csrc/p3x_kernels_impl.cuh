@@ -36,10 +36,13 @@ cudaError_t launch_persistent(Kern kern, const dev::Inst& inst0, const dev::KPar
  * the `warps` warps gives every warp one pool of its share: against pools that
  * get smaller towards the end 2,600 x 72 FP64 271 us / 356, 5,400 x 72 474 / 504,
  * 16,000 x 128 1.86 ms / 1.99, FP32-bulk 16,000 x 128 262 us / 288.  A larger call
- * takes pools of C = pool_columns columns until C / 4 columns are left for each
- * warp, and then pools of half as many, and so on (21,600 x 128 FP64: C = 16 2.33
- * ms, 8 2.41, 1 3.38; 345,600 x 128 FP32-bulk 5.42, 5.49 and 7.81 ms), and so does
- * a work list, whose instances differ in depth. */
+ * takes pools of C = pool_columns columns until C / 2 columns are left for each
+ * warp, and then pools of half as many, and so on, and so does a work list, whose
+ * instances differ in depth.  345,600 x 128 FP32-bulk: C = 16 4.86 ms, 8 4.92, 4
+ * 5.33; the last pools from C / 4 or C columns a warp on instead of C / 2: 86,400 x
+ * 128 FP32-bulk 1.34 and 1.32 ms against 1.30, after four steps (nearly every level
+ * with a hydrometeor) 3.14 and 3.06 against 3.04; 43,200 x 128 FP64 4.58 and 4.74
+ * against 4.53. */
 template <class TR>
 void plan_pools(dev::KParams<TR>& kp, int lanes, long long warps) {
   int cols = pool_columns(kp.nlev_max, lanes);
@@ -55,7 +58,7 @@ void plan_pools(dev::KParams<TR>& kp, int lanes, long long warps) {
   long long left = kp.nwork, n = 0;
   int t = 0;
   for (; cols > 1; cols /= 2) {
-    const long long keep = one_round ? 0 : warps * cols / 4;
+    const long long keep = one_round ? 0 : warps * cols / 2;
     const long long take = left > keep ? (left - keep + cols - 1) / cols : 0;
     n += take;
     left -= take * cols < left ? take * cols : left;
