@@ -233,9 +233,14 @@ int sm_stride_for(int nlev_max) {
   return (s + 1) & ~1;
 }
 
+/* Deepest columns of the FP64 form, 2,639 levels (the FP32-bulk form's shared
+ * memory ends at 2,903). */
+constexpr int kMaxStrideF64 = 2640;
+
 bool spec_fits(int precision, const LaunchSpec& ls, int stride) {
   if (ls.lanes != 8 && ls.lanes != 16 && ls.lanes != 32) return false;
   if (ls.groups_per_block <= 0 || ls.groups_per_block * ls.lanes > 256) return false;
+  if (precision == P3X_FP64 && stride > kMaxStrideF64) return false;
   const bool f32 = precision == P3X_FP32_BULK;
   const size_t k1 = f32 ? p3_smem_bytes<float>(ls, stride - 1) : p3_smem_bytes<double>(ls, stride - 1);
   const LaunchSpec ls2 = sed_spec(ls);

@@ -65,3 +65,17 @@ def test_pools_end_at_an_instance(gpu_ctx, precision):
         one = step(gpu_ctx, inps[i], precision)
         for k in one:
             np.testing.assert_array_equal(got[i][k], one[k], err_msg=f"{i} {k}")
+
+
+@pytest.mark.parametrize("precision,deepest", [(0, 2639), (1, 2903)])
+def test_deepest_columns(gpu_ctx, precision, deepest):
+    """The deepest accepted column gives the same bits alone and with others; a
+    deeper one is refused."""
+    import scream_gb300 as p3
+    inp = p3.generate_inputs(0, 8, 3, deepest)
+    whole = step(gpu_ctx, inp, precision)
+    one = step(gpu_ctx, rows(inp, 2, 3), precision)
+    for k, v in one.items():
+        np.testing.assert_array_equal(v, whole[k][2:3], err_msg=k)
+    with pytest.raises(p3.P3Error):
+        step(gpu_ctx, p3.generate_inputs(0, 8, 1, deepest + 1), precision)
