@@ -1018,9 +1018,9 @@ __device__ __forceinline__ void nucleation_level_f64(const Inst& in, const int c
  * a warp (18 of 128 levels in a cloud of 1-4 km), and the FP64 pipe takes
  * as long for one lane as for 32.  The same bits as with lists per column, where
  * part1's remainder and part2 were separate passes over arrays in shared memory
- * (FP64 16 lanes, FP32-bulk 32 lanes per column): 21,600 x 128 FP64 3.41 -> 2.35
- * ms, FP32-bulk 0.468 -> 0.371; 345,600 x 128 FP32-bulk 8.43 -> 5.48 ms; 1,537 x
- * 97 FP64 272 -> 242 us. */
+ * (FP64 16 lanes, FP32-bulk 32 lanes per column): 21,600 x 128 FP64 3.41 -> 2.36
+ * ms, FP32-bulk 0.468 -> 0.33; 345,600 x 128 FP32-bulk 8.43 -> 4.86 ms; 1,537 x
+ * 97 FP64 272 -> 239 us. */
 template <class TR, bool WIDE>
 __device__ void p3_part12(const Inst& in, const int col0, const int ncol, const KParams<TR>& kp, const Tabs<TR>& tb,
                           uint16_t* __restrict__ list, PoolScratch* __restrict__ ps, uint32_t& err) {
@@ -1226,8 +1226,10 @@ __device__ void p3_part12(const Inst& in, const int col0, const int ncol, const 
  * one product, one difference and one multiply-add per field, with 1 / (dz rho)
  * formed once per level and V rho kept instead of V.  At 21,600 x 128: 15.8 ms
  * with integer divisions alone, 2.7 ms in this form (3.6 ms with exact 64-bit
- * high products, rounded quotients and 100 registers); the results differ from
- * the reference's order of operations by rounding (1e-14 of a field's norm). */
+ * high products, rounded quotients and 100 registers), 2.5 ms with the rime left
+ * out where there is none; the FP64 pipe is 70 % busy then, the integer pipe 39 %.
+ * The results differ from the reference's order of operations by rounding (1e-14
+ * of a field's norm). */
 template <class TR, int LANES, bool SPLIT = false>
 __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, const Tabs<TR>& tb,
                        double* __restrict__ sm, GroupScratch* gs, uint32_t& err) {
@@ -2248,7 +2250,7 @@ __device__ void p3_part3(const Inst& in, const int col, const KParams<TR>& kp, c
           s.bm = bm_incld * cld_i;
           impose_max_total_ni(ni_incld, rt.max_total_ni, inv_rho);
           /* table position, limits and values in fixed point (part3 0.87 ->
-           * 0.37 ms at 21,600 x 128) */
+           * 0.37 ms at 21,600 x 128, now 0.28) */
           const IceCell cell = ice_cell(m_div(qi_incld, ni_incld), m_div(qm_incld, qi_incld), rhop, &kFixTables);
           const int64_t* const cf = kp.cell_part3 + size_t(cell.cell) * (kCellCols * kCellCoefs);
           const int4 sh = __ldg(reinterpret_cast<const int4*>(kp.cell_part3_shift) + cell.cell);

@@ -46,13 +46,11 @@ inline size_t sed_smem_bytes(const LaunchSpec& ls, int sm_stride) {
   return size_t(ls.groups_per_block) * dev::sed_slots<TR>() * size_t(sm_stride) * sizeof(double);
 }
 
-/* Launch shape of K2 and K3.  Sedimentation always runs 32 lanes per column,
- * whatever lane count K1 uses: its substeps walk the levels chunk by chunk, so a
- * narrower group only lengthens the walk (measured at 65,536 x 128 with 16
- * lanes: FP64 K2 +17 %, FP32-bulk K2 +95 %).  Part3 too: FP64 at 21,600 x 128
- * 344 us against 369 at 16 lanes, 1,537 x 97 39 against 55, 64 x 72 31 against
- * 43.  Columns per CTA as configured, at
- * most 8 (256 threads). */
+/* Launch shape of K2 and K3: always 32 lanes per column.  Sedimentation's
+ * substeps walk the levels chunk by chunk, so a narrower group only lengthens the
+ * walk (65,536 x 128 with 16 lanes: FP64 K2 +17 %, FP32-bulk K2 +95 %); part3 FP64
+ * at 21,600 x 128 took 344 us with 32 lanes, 369 with 16.  Columns per CTA as
+ * configured, at most 8 (256 threads). */
 inline LaunchSpec sed_spec(const LaunchSpec& ls) {
   LaunchSpec s = ls;
   s.lanes = 32;

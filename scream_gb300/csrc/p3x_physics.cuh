@@ -178,9 +178,10 @@ __device__ __forceinline__ double f2d_int(float x) {
 
 /* Float -> double where the instruction footprint limits the kernel more than
  * the FP64 pipe: the FP32-bulk part1+2 and sedimentation kernels are larger
- * than the SM's instruction cache (instruction fetch is part1+2's top stall at
- * 65,536 columns), and the hardware conversion is one instruction where
- * f2d_int inlines a dozen and a branch at each of some 80 call sites.  The
+ * than the SM's instruction cache, and the hardware conversion is one
+ * instruction where f2d_int inlines a dozen and a branch at each of some 80 call
+ * sites (sedimentation with f2d_int in its rebuild: 8.9 -> 9.6 ms at 345,600 x
+ * 128).  The
  * FP64-pipe-bound part3 keeps f2d_int.  Both are exact. */
 __device__ __forceinline__ double f2d(float x) { return double(x); }
 

@@ -88,7 +88,7 @@ constexpr int kMidOutputs = 10;             /* 7 per-level diagnostics + 3 histo
 constexpr int kBatchColumnCap = 1 << 18;    /* columns per dispatched work list */
 /* Latency policy (the default; p3x_server_set_latency_policy): small
  * requests must not wait behind large steps (an FP64 step of 65,536 x 128
- * takes ~130 ms alone).  A dispatch holds requests of one size kind (small:
+ * takes ~36 ms alone).  A dispatch holds requests of one size kind (small:
  * at most kSmallInstanceCl column-levels); a dispatch of more than
  * kLargeDispatchCl column-levels takes the policy's share of the
  * resident-CTA capacity, so every SM keeps room for other slots' launches;
