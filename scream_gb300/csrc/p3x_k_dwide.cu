@@ -6,7 +6,8 @@ namespace p3x {
 template <>
 cudaError_t launch_part12_wide<double>(const dev::Inst& inst0, const dev::KParams<double>& kp,
                                         cudaStream_t stream) {
-  const size_t smem = dev::pool_list_entries(1, kp.nlev_max) * sizeof(uint16_t);
+  const size_t smem = dev::pool_list_entries(1, kp.nlev_max) * sizeof(uint16_t) +
+                      dev::kPreFields * sizeof(double) * size_t(kp.nlev_max < dev::kPreLevels ? kp.nlev_max : dev::kPreLevels);
   dev::p3_part12_wide_kernel<double><<<kp.nwork, dev::kPart12WideThreads, smem, stream>>>(inst0, kp);
   return cudaGetLastError();
 }

@@ -75,8 +75,8 @@ cudaError_t launch_sed_wide(const dev::Inst& inst0, const dev::KParams<TR>& kp, 
 
 /* K1 with a CTA per column (p3x_k_dwide.cu, p3x_k_fwide.cu): where all those
  * CTAs fit on the SMs at once, 2 an SM in the FP64 form, 4 in the FP32-bulk form.
- * Measured, CTA per column against pools: 64 x 72 FP64 95 / 119 us, 304 x 128
- * 101 / 182, 456 x 128 183 / 182; FP32-bulk 64 x 72 22 / 32, 304 x 128 24 / 43. */
+ * Measured, CTA per column against pools: 64 x 72 FP64 88 / 119 us, 304 x 128
+ * 98 / 182, 456 x 128 183 / 182; FP32-bulk 64 x 72 22 / 32, 304 x 128 24 / 43. */
 template <class TR>
 inline bool part12_wide_fits(const dev::KParams<TR>& kp, int num_sms) {
   return kp.nwork <= (sizeof(TR) == sizeof(float) ? 4 : 2) * num_sms;

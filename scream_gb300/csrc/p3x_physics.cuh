@@ -823,11 +823,12 @@ template <class TR>
 struct PhysVars {
   TR mu, dv, sc, dqsdt, dqsidt, ab, abi, kap, eii;
 };
+/* t_1p5, t_1p81: those powers of the temperature */
 template <class TR>
-__device__ __forceinline__ void get_time_space_phys_variables(TR T_atm, TR pres, TR rho, TR qv_sat_l,
-                                                              TR qv_sat_i, PhysVars<TR>& v) {
-  v.mu = m_div(TR(1.496e-6) * m_pow(T_atm, TR(1.5)), T_atm + TR(120));
-  v.dv = m_div(TR(8.794e-5) * m_pow(T_atm, TR(1.81)), pres);
+__device__ __forceinline__ void get_time_space_phys_variables(TR T_atm, TR t_1p5, TR t_1p81, TR pres, TR rho,
+                                                              TR qv_sat_l, TR qv_sat_i, PhysVars<TR>& v) {
+  v.mu = m_div(TR(1.496e-6) * t_1p5, T_atm + TR(120));
+  v.dv = m_div(TR(8.794e-5) * t_1p81, pres);
   v.sc = m_div(v.mu, rho * v.dv);
   const TR dum = m_div(TR(1), TR(C::RV) * sq(T_atm));
   v.dqsdt = TR(C::LatVap) * qv_sat_l * dum;
