@@ -79,12 +79,13 @@ cudaError_t launch_p3_part(const dev::Inst& inst0, const dev::KParams<TR>& kp_in
   kp.staged = ls.staged;
   cudaError_t e = cudaErrorInvalidValue;
   if (part == kPartK1) {
-    if (kp.wctr) {
+    const bool wide = !ls.staged && part12_wide_fits<TR>(kp, num_sms); /* it zeroes the counters itself */
+    if (kp.wctr && !wide) {
       e = cudaMemsetAsync(kp.wctr, 0, dev::kWorkCounters * sizeof(uint32_t), stream);
       if (e != cudaSuccess) return e;
     }
     if (ls.marks) cudaEventRecord(ls.marks[0], stream);
-    if (!ls.staged && part12_wide_fits<TR>(kp, num_sms)) {
+    if (wide) {
       e = launch_part12_wide<TR>(inst0, kp, stream);
     } else {
       const auto kern = kp.work ? dev::p3_part12_kernel<TR, true> : dev::p3_part12_kernel<TR, false>;
