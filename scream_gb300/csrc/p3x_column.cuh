@@ -167,8 +167,8 @@ __device__ __forceinline__ T read_now(const T* p) {
 }
 
 /* Launch-wide work counters of one step (K1, K2, K3, spare), zeroed on the
- * stream before K1, or by a K1 that does not use them.  They follow the hand-over doubles and the flags in an
- * instance's scratch. */
+ * stream before K1, or by a K1 that does not use them.  They follow the
+ * hand-over doubles and the flags in an instance's scratch. */
 constexpr int kWorkCounters = 4;
 __host__ __device__ inline size_t work_counter_offset(int ncol, int64_t ld) {
   const size_t d = size_t(kScrFields) * size_t(ncol) * size_t(ld) * sizeof(double);
