@@ -271,7 +271,11 @@ constexpr double kRair = kRgas / 28.966, kCpair = 1.00464e3, kGravit = 9.80616;
 constexpr double kMincld = 0.0001, kQsmall = 1.0e-14;
 constexpr double kMucon = 5.3, kDcon = 25.e-6, kDeicon = 50.0;
 __device__ __forceinline__ double fmax_(double a, double b) { return a > b ? a : b; } /* Fortran max for these ranges */
-__device__ __forceinline__ double fmin_(double a, double b) { return a < b ? a : b; }
+/* the driver's max(0, x), max(c, x) and min(x, c), c > 0, by IEEE comparisons on
+ * the integer pipes: the maxima of a NaN are the NaN, the minimum is c */
+__device__ __forceinline__ double max0(double x) { return dev::ieee_neg(x) ? 0.0 : x; }
+__device__ __forceinline__ double max_c(double x, double c) { return dev::ieee_lt(x, c) ? c : x; }
+__device__ __forceinline__ double min_c(double x, double c) { return dev::ieee_lt(x, c) ? x : c; }
 }  // namespace eam
 
 /* Preparation of the P3 inputs (micro_p3_interface.F90:982-1047) and the
@@ -351,10 +355,10 @@ __global__ void eam_pre_kernel(EamPtrs p, int ncol, int nlev, int64_t ld, int64_
 
 /* Use of the P3 results (micro_p3_interface.F90:1182-1431).  The driver's
  * twenty divisions per level run on the integer pipes (ddiv_int, the same
- * doubles; the ten over dt share one reciprocal seed) and its threshold tests
- * compare bit patterns: 6.6 -> 1.3 ms at 65,536 x 128, where the ~4.7 GB it
- * moves take 0.7 ms; the FP64 multiplications and differences of its formulas
- * make up most of the rest. */
+ * doubles; the ten over dt share one reciprocal seed), and so do its threshold
+ * tests, as IEEE comparisons (false for a NaN): 6.6 -> 1.3 ms at 65,536 x 128,
+ * where the ~4.7 GB it moves take 0.7 ms; the FP64 multiplications and
+ * differences of its formulas make up most of the rest. */
 __global__ void eam_post_kernel(EamPtrs p, int ncol, int nlev, int64_t ld, int64_t ld_int, double dt) {
   const int col = int((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
@@ -372,7 +376,7 @@ __global__ void eam_post_kernel(EamPtrs p, int ncol, int nlev, int64_t ld, int64
     const double temp = dtemp + t;
     p.ptend_s[o] = dev::ddiv_int(eam::kCpair * (temp - t), dt);
 #pragma unroll
-    for (int s = 0; s < 9; ++s) p.ptend_q[s][o] = dev::ddiv_int(dev::dmax0(w[s]) - p.q[s][o], dt);
+    for (int s = 0; s < 9; ++s) p.ptend_q[s][o] = dev::ddiv_int(eam::max0(w[s]) - p.q[s][o], dt);
     p.t_prev[o] = temp;
     p.qv_prev[o] = w[0];
     const double cme = p.cmeliq[o];
@@ -381,9 +385,9 @@ __global__ void eam_post_kernel(EamPtrs p, int ncol, int nlev, int64_t ld, int64
     const double pmid = p.pmid[o];
     if (p.rho) p.rho[o] = dev::ddiv_int(pmid, eam::kRair * temp);
     const double cl = p.cld_l[o], ci = p.cld_i[o], cr = p.cld_r[o];
-    const double ci_d = dev::dmax_c(ci, eam::kMincld), cl_d = dev::dmax_c(cl, eam::kMincld), rt = 287.15 * t;
-    const double icimr = dev::dmin_c(dev::ddiv_int(p.q[5][o], ci_d), 0.005);
-    const double icwmr = dev::dmin_c(dev::ddiv_int(p.q[1][o], cl_d), 0.005);
+    const double ci_d = eam::max_c(ci, eam::kMincld), cl_d = eam::max_c(cl, eam::kMincld), rt = 287.15 * t;
+    const double icimr = eam::min_c(dev::ddiv_int(p.q[5][o], ci_d), 0.005);
+    const double icwmr = eam::min_c(dev::ddiv_int(p.q[1][o], cl_d), 0.005);
     const double icin = dev::ddiv_int(dev::ddiv_int(p.q[6][o], ci_d) * pmid, rt);
     const double icwn = dev::ddiv_int(dev::ddiv_int(p.q[2][o], cl_d) * pmid, rt);
     if (p.icimrst) p.icimrst[o] = icimr;
@@ -392,7 +396,7 @@ __global__ void eam_post_kernel(EamPtrs p, int ncol, int nlev, int64_t ld, int64
     if (p.icwnc) p.icwnc[o] = icwn;
     const double rel = p.eff_qc[o] * 1e6, rei = p.eff_qi[o] * 1e6;
     double dei = rei * 2.0, mu = 0.0, lambdac = 0.0;
-    if (dev::dlt(p.ast[o], 1.e-4)) {
+    if (dev::ieee_lt(p.ast[o], 1.e-4)) {
       mu = eam::kMucon;
       lambdac = (eam::kMucon + 1.0) / eam::kDcon;
       dei = eam::kDeicon;
@@ -404,9 +408,13 @@ __global__ void eam_post_kernel(EamPtrs p, int ncol, int nlev, int64_t ld, int64
     if (p.lambdac) p.lambdac[o] = lambdac;
     /* w: 1 cldliq, 2 numliq, 3 rain, 4 numrain, 5 cldice */
     const double tot = w[3] + w[5] + w[1];
-    if (p.nfice) p.nfice[o] = (dev::dgt(w[5], eam::kQsmall) && dev::dgt(tot, eam::kQsmall)) ? dev::dmin_c(dev::ddiv_int(w[5], tot), 1.0) : 0.0;
+    if (p.nfice)
+      p.nfice[o] = dev::ieee_gt(w[5], eam::kQsmall) && dev::ieee_gt(tot, eam::kQsmall)
+                       ? eam::min_c(dev::ddiv_int(w[5], tot), 1.0)
+                       : 0.0;
     cdnumc = cdnumc + dev::ddiv_int(w[2] * p.pdel[o], eam::kGravit);
-    const bool liq = dev::dgt(cl, 0.01) && dev::dgt(icwmr, 5.e-5), ice = dev::dgt(ci, 0.01) && dev::dgt(icimr, 1.e-6);
+    const bool liq = dev::ieee_gt(cl, 0.01) && dev::ieee_gt(icwmr, 5.e-5);
+    const bool ice = dev::ieee_gt(ci, 0.01) && dev::ieee_gt(icimr, 1.e-6);
     if (p.efcout) p.efcout[o] = liq ? rel * cl : 0.0;
     if (p.ncout) p.ncout[o] = liq ? icwn * cl : 0.0;
     if (p.freql) p.freql[o] = liq ? cl : 0.0;
@@ -415,7 +423,7 @@ __global__ void eam_post_kernel(EamPtrs p, int ncol, int nlev, int64_t ld, int64
     if (p.freqi) p.freqi[o] = ice ? ci : 0.0;
     const double reff = p.eff_qr[o];
     if (p.deff_rain) p.deff_rain[o] = reff * 2.0 * 1.e6;
-    const bool rain = dev::dge(w[3], 1.e-7);
+    const bool rain = dev::ieee_ge(w[3], 1.e-7);
     if (p.aqrain) p.aqrain[o] = rain ? w[3] * cr : 0.0;
     if (p.anrain) p.anrain[o] = rain ? w[4] * cr : 0.0;
     if (p.freqr) p.freqr[o] = rain ? cr : 0.0;

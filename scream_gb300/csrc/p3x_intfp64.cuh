@@ -55,6 +55,19 @@ P3X_HD double d_from_bits(uint64_t u) {
   return x;
 #endif
 }
+/* IEEE comparisons of any double x with a constant c > 0 on the integer pipes:
+ * the bit patterns as unsigned numbers are 0 to kInf for +0 to +infinity, 2^63
+ * to 2^63 + kInf for -0 to -infinity, and the NaNs of either sign lie behind
+ * those, so each test is one or two ranges (false for a NaN). */
+constexpr uint64_t kInfPattern = 0x7ff0000000000000ull, kSignPattern = 0x8000000000000000ull;
+P3X_HD bool ieee_gt(double x, double c) { return d_bits(x) - d_bits(c) - 1 < kInfPattern - d_bits(c); }
+P3X_HD bool ieee_ge(double x, double c) { return d_bits(x) - d_bits(c) <= kInfPattern - d_bits(c); }
+P3X_HD bool ieee_lt(double x, double c) {
+  return d_bits(x) < d_bits(c) || d_bits(x) - kSignPattern <= kInfPattern;
+}
+/* x < 0 */
+P3X_HD bool ieee_neg(double x) { return d_bits(x) - kSignPattern - 1 < kInfPattern; }
+
 P3X_HD int64_t mulhi_s64(int64_t a, int64_t b) {
 #ifdef __CUDA_ARCH__
   return __mul64hi(a, b);
