@@ -211,6 +211,13 @@ __device__ __forceinline__ int group_max_int(unsigned mask, int v) {
   return __reduce_max_sync(mask, v);
 }
 
+/* The lanes of a warp that hold the levels base to last, base + lane each (base
+ * <= last): the mask of a vote in a loop over those levels. */
+__device__ __forceinline__ unsigned chunk_mask(int base, int last) {
+  const int n = last - base + 1;
+  return n < 32 ? (1u << n) - 1u : 0xffffffffu;
+}
+
 /* A sedimentation group is a warp or several, LANES > 32 threads (at least
  * as many as the column has levels): the warps of a group exchange through this
  * shared scratch and meet at a barrier.  SPLIT: a CTA has three such groups,
@@ -1358,6 +1365,14 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
       for (int k = k_qxtop + lane; k <= k_qxbot; k += LANES) {
         const double qs = QS[k];
         double v1 = 0, v2 = 0;
+        /* Ice without rime in the whole chunk: no rime density, and two table
+         * corners instead of eight; below, its two fields' fluxes are left out as
+         * well.  Nucleated ice over the clouds is most of the walk: 21,600 x 128
+         * 2.66 -> 2.51 ms.  A warp of a wider group has one chunk and waits for the
+         * others', so it does not look. */
+        bool rime = true;
+        if constexpr (sp == 2 && LANES == kWarp)
+          rime = __any_sync(chunk_mask(k - lane, k_qxbot), dnz(R2[k]) || dnz(R3[k]));
         /* q: the mass field, limited in the first substep as the in-cloud
          * value is there; the field itself keeps its value */
         double q = R0[k], n = R1[k];
@@ -1416,13 +1431,6 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
             R1[k] = n;
           } else {
             double m = R2[k], b = R3[k];
-            /* Ice without rime in the whole chunk (the lanes that take part here):
-             * no rime density, and two table corners instead of eight; below, its
-             * two fields' fluxes are left out as well.  Nucleated ice over the
-             * clouds is most of the walk: 21,600 x 128 2.66 -> 2.48 ms.  A warp of
-             * a wider group has one chunk and waits for the others', so it does
-             * not look. */
-            const bool rime = LANES > 32 || __any_sync(__activemask(), dnz(m) || dnz(b));
             int64_t hi, lo, vm, vn;
             int4 sh;
             const int64_t size = log2_of(raw_quotient(q, n), ft);
@@ -1922,15 +1930,18 @@ __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>&
             qi_f = vmin(qi_f, float(C::incloud_limit));
             bm_f = vmin(bm_f, float(C::incloud_limit));
           }
-          if (qi_f > float(C::QSMALL)) {
+          const bool present = qi_f > float(C::QSMALL);
+          /* ice without rime in the whole chunk: no rime density, and two table
+           * corners instead of eight (with the fluxes below 345,600 x 128 10.04 ->
+           * 9.29 ms, 21,600 x 128 900 -> 822 us; a bit per chunk kept from substep
+           * to substep instead of the votes: 9.55 ms; the vote over all lanes ahead
+           * of the loop body 4 % slower) */
+          const bool rime = LANES > kWarp || __any_sync(chunk_mask(k - lane, k_qxbot),
+                                                        present && (r23.x != 0.f || r23.y != 0.f));
+          if (present) {
             const float ni_l = vmax(ni_f, float(C::NSMALL));
             float tv[4]; /* columns 0, 1, 6, 7, packed copy */
-            /* ice without rime in the whole chunk (the lanes that take part
-             * here): no rime density, and two table corners instead of eight
-             * (with the fluxes below 345,600 x 128 10.04 -> 9.29 ms, 21,600 x
-             * 128 900 -> 822 us; a bit per chunk kept from substep to substep
-             * instead of the votes: 9.55 ms) */
-            if (LANES > 32 || __any_sync(__activemask(), r23.x != 0.f || r23.y != 0.f)) {
+            if (rime) {
               const float rhop = calc_bulk_rho_rime<float>(qi_f, qm_f, bm_f, rt);
               if (qm_f != qm_plain) set_state(2, k, qm_f, cldf);
               if (bm_f != bm_plain) defer_state(3, k, bm_f, cldf);
