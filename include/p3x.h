@@ -134,7 +134,8 @@ typedef struct p3x_launch_config {
   int32_t columns_per_block; /* times lanes_per_column: threads of one CTA     */
   int32_t table_staging;     /* 0: tables read through L1/L2; 1: staged into   */
                              /*    shared memory by bulk copies (cp.async.bulk) */
-  int32_t blocks_per_sm;     /* persistent grid = blocks_per_sm x SM count (0 = auto) */
+  int32_t blocks_per_sm;     /* part1+2 keeps to blocks_per_sm x SM count CTAs */
+                             /*    (0: as many as fit; the others always so)   */
 } p3x_launch_config;
 
 typedef struct p3x_context p3x_context;

@@ -32,6 +32,7 @@
 #include <type_traits>
 
 #include "p3x_physics.cuh"
+#include "p3x_plan.hpp"
 
 namespace p3x {
 namespace dev {
@@ -60,9 +61,6 @@ struct WorkItem {
   int32_t inst, col;
 };
 
-/* K1: level lists of a pool of columns, entries (column of the pool, level) */
-constexpr int kPoolTiers = 5; /* pools of 16, 8, 4, 2, 1 columns */
-constexpr int kPoolMaxCols = 1 << (kPoolTiers - 1);
 constexpr int kPoolLevelBits = 12;
 constexpr int kPart12WideThreads = 128;
 /* what the warps of a CTA share where they work on one column */
@@ -2479,24 +2477,6 @@ __device__ __forceinline__ const Inst& work_inst(const Inst& inst0, const KParam
   }
   col = w;
   return inst0;
-}
-
-/* Pool i of a launch's work items: pool_cols of them, and half as many whenever
- * the pools of a size are used up (pool_end), so that the last pools of a call of
- * several rounds are small and every warp ends at about the same time. */
-template <class TR>
-__device__ __forceinline__ void pool_range(const KParams<TR>& kp, const int i, int& w0, int& w1) {
-  int first = 0, size = kp.pool_cols;
-  w0 = 0;
-#pragma unroll
-  for (int t = 0; t < kPoolTiers - 1; ++t) {
-    if (i < kp.pool_end[t] || size == 1) break;
-    w0 += (kp.pool_end[t] - first) * size;
-    first = kp.pool_end[t];
-    size >>= 1;
-  }
-  w0 += (i - first) * size;
-  w1 = min(w0 + size, kp.nwork);
 }
 
 /* BATCH: a work list of several instances, whose field pointers are read from

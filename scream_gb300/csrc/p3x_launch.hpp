@@ -15,20 +15,10 @@ struct LaunchSpec {
   int lanes;            /* 8, 16, 32 */
   int groups_per_block; /* columns per CTA */
   int staged;           /* tables in shared memory */
-  int blocks_per_sm;    /* 0: as many as fit */
+  int blocks_per_sm;    /* part1+2: CTAs an SM at most; 0: as many as fit */
   cudaEvent_t* marks = nullptr; /* optional: 4 events recorded around K1, K2, K3 */
   double grid_frac = 1.0;       /* share of the resident-CTA capacity the persistent grid takes */
 };
-
-/* Columns of K1's largest pools: as many as have kPoolLevels levels (16 columns
- * of 128), 2 or 4 times as many at 16 or 8 lanes per column. */
-constexpr int kPoolLevels = 2048;
-inline int pool_columns(int nlev_max, int lanes) {
-  int cols = 1;
-  while (cols < dev::kPoolMaxCols && cols * 2 * nlev_max <= kPoolLevels) cols *= 2;
-  for (int l = 32; l > lanes && cols < dev::kPoolMaxCols; l /= 2) cols *= 2;
-  return cols;
-}
 
 /* Threads of a CTA: the configured columns x lanes in whole warps. */
 inline int warp_threads(const LaunchSpec& ls) { return (ls.groups_per_block * ls.lanes + 31) / 32 * 32; }
@@ -73,14 +63,7 @@ template <class TR>
 cudaError_t launch_sed_wide(const dev::Inst& inst0, const dev::KParams<TR>& kp, int lanes, int num_sms,
                             cudaStream_t stream);
 
-/* K1 with a CTA per column (p3x_k_dwide.cu, p3x_k_fwide.cu): where all those
- * CTAs fit on the SMs at once, 2 an SM in the FP64 form, 4 in the FP32-bulk form.
- * Measured, CTA per column against pools: 64 x 72 FP64 88 / 119 us, 304 x 128
- * 98 / 182, 456 x 128 183 / 182; FP32-bulk 64 x 72 22 / 32, 304 x 128 24 / 43. */
-template <class TR>
-inline bool part12_wide_fits(const dev::KParams<TR>& kp, int num_sms) {
-  return kp.nwork <= (sizeof(TR) == sizeof(float) ? 4 : 2) * num_sms;
-}
+/* K1 with a CTA per column (part12_wide_fits). */
 template <class TR>
 cudaError_t launch_part12_wide(const dev::Inst& inst0, const dev::KParams<TR>& kp, cudaStream_t stream);
 
