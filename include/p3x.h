@@ -389,8 +389,10 @@ int p3x_main_stages(p3x_context* ctx, const p3x_runtime* rt, const p3x_prognosti
  * its FP32-pipe table indices with the hardware truncation (after the table
  * lookups' clamps), and checks its small-integer floats; for 2^32 doubles
  * covering every high word, compares its integer-pipe narrowing toward zero
- * with the hardware conversion; *mismatches receives the number of
- * disagreements (0 expected). */
+ * with the hardware conversion; compares the FP64 form's integer-pipe division
+ * with the hardware division, and its fixed-point logarithm, exponential, powers,
+ * cube root and table positions and values on the device with the same on the
+ * host; *mismatches receives the number of disagreements (0 expected). */
 int p3x_selftest(uint64_t* mismatches);
 
 /* Per-kernel timing of single-instance steps (no counterpart in the

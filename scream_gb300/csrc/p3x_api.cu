@@ -16,6 +16,7 @@
 
 #include "p3x.h"
 #include "p3x_fixtables.hpp"
+#include "p3x_fixtest.hpp"
 #include "p3x_internal.hpp"
 #include "p3x_launch.hpp"
 
@@ -854,14 +855,26 @@ int p3x_main_stages(p3x_context* ctx, const p3x_runtime* rt, const p3x_prognosti
 
 int p3x_selftest(uint64_t* mismatches) {
   if (!mismatches) return P3X_EINVAL;
+  const std::vector<int64_t> coef = fix_test_coefficients();
+  const std::vector<uint64_t> want = fix_test_words(coef);
+  std::vector<uint64_t> got(want.size());
   unsigned long long* d = nullptr;
-  P3X_CUDA(cudaMalloc(&d, sizeof(*d)));
-  cudaError_t e = cudaMemset(d, 0, sizeof(*d));
-  if (e == cudaSuccess) e = launch_selftest(d, nullptr);
+  int64_t* coef_d = nullptr;
+  uint64_t* words_d = nullptr;
   unsigned long long h = 0;
+  cudaError_t e = cudaMalloc(&d, sizeof(*d));
+  if (e == cudaSuccess) e = cudaMemset(d, 0, sizeof(*d));
+  if (e == cudaSuccess) e = launch_selftest(d, nullptr);
   if (e == cudaSuccess) e = cudaMemcpy(&h, d, sizeof(h), cudaMemcpyDeviceToHost);
-  cudaFree(d);
+  if (e == cudaSuccess) e = cudaMalloc(&coef_d, coef.size() * sizeof(int64_t));
+  if (e == cudaSuccess) e = cudaMalloc(&words_d, got.size() * sizeof(uint64_t));
+  if (e == cudaSuccess) e = cudaMemcpy(coef_d, coef.data(), coef.size() * sizeof(int64_t), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = launch_fix_selftest(coef_d, words_d, nullptr);
+  if (e == cudaSuccess) e = cudaMemcpy(got.data(), words_d, got.size() * sizeof(uint64_t), cudaMemcpyDeviceToHost);
+  for (void* p : {static_cast<void*>(d), static_cast<void*>(coef_d), static_cast<void*>(words_d)})
+    if (p) cudaFree(p);
   if (e != cudaSuccess) return cuda_status(e);
+  for (size_t i = 0; i < got.size(); ++i) h += got[i] != want[i];
   *mismatches = uint64_t(h);
   return P3X_OK;
 }

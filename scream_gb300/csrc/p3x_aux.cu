@@ -3,6 +3,7 @@
  * Fortran-layout entry point, and the FP64 column water / energy budgets
  * (share/property_checks/mass_and_energy_column_conservation_check.cpp:281-347).
  */
+#include "p3x_fixtest.hpp"
 #include "p3x_launch.hpp"
 
 namespace p3x {
@@ -483,8 +484,6 @@ cudaError_t launch_postamble(const dev::Inst* insts_d, const dev::WorkItem* work
   return cudaGetLastError();
 }
 
-/* Exhaustive check of the integer-pipe float -> double conversion against
- * the hardware conversion: every one of the 2^32 float bit patterns. */
 /* Every float bit pattern: the integer-pipe float -> double conversion
  * against the hardware one, and the FP32-pipe table index against the
  * hardware truncation after the callers' clamps ([1, hi - 1] and [1, hi]);
@@ -492,8 +491,9 @@ cudaError_t launch_postamble(const dev::Inst* insts_d, const dev::WorkItem* work
  * doubles covering every high word: the integer-pipe narrowing toward zero
  * against the hardware conversion; 2^24 hashed operand sets: the packed
  * double-float accumulation against the scalar one; 2^26 operand pairs: the
- * integer-pipe division against the FP64 division; every float in [1, 2]: the
- * reciprocal seed's error. */
+ * integer-pipe division against the FP64 division, and 2^26 unrounded quotients
+ * of significands against exact products; every float in [1, 2]: the reciprocal
+ * seed's error. */
 __global__ void f2d_selftest_kernel(unsigned long long* mismatches) {
   unsigned long long bad = 0;
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
@@ -565,8 +565,14 @@ __global__ void f2d_selftest_kernel(unsigned long long* mismatches) {
       }
       const uint64_t q = dev::d_bits(dev::ddiv_int(a, b)), want = dev::d_bits(a / b);
       if (q != want && !(isnan(a / b) && isnan(dev::d_from_bits(q)))) ++bad;
+      /* S = A / B 2^63 less under 2 units: 0 <= A 2^63 - S B < 2 B */
+      const uint64_t A = dev::d_sig(dev::d_bits(a)), B = dev::d_sig(dev::d_bits(b));
+      const unsigned __int128 num = static_cast<unsigned __int128>(A) << 63;
+      const unsigned __int128 got = static_cast<unsigned __int128>(dev::sig_quotient(A, B)) * B;
+      if (got > num || num - got >= 2 * B) ++bad;
     }
-    /* the reciprocal seed never exceeds 2^24 / b and falls short by < 4.1 */
+    /* the reciprocal seed falls short of 2^24 / f by 1 to 3 units (rounding b to
+     * f adds at most one) */
     if (i <= 0x800000u) {
       const double r = 16777216.0 / double(__uint_as_float(0x3f800000u + uint32_t(i)));
       const double short_by = r - double(dev::rcp_seed(0x3f800000u + uint32_t(i)));
@@ -594,6 +600,16 @@ cudaError_t saturation_at_melting(double* out) {
 
 cudaError_t launch_selftest(unsigned long long* mismatches_d, cudaStream_t st) {
   f2d_selftest_kernel<<<4096, 256, 0, st>>>(mismatches_d);
+  return cudaGetLastError();
+}
+
+__global__ void fix_selftest_kernel(const int64_t* __restrict__ coef, uint64_t* __restrict__ out) {
+  const int i = int(blockIdx.x * blockDim.x + threadIdx.x);
+  if (i < kFixTestRows) dev::fix_test_row(uint64_t(i), &dev::kFixTables, coef, out + size_t(i) * kFixTestWords);
+}
+
+cudaError_t launch_fix_selftest(const int64_t* coef_d, uint64_t* out_d, cudaStream_t st) {
+  fix_selftest_kernel<<<(kFixTestRows + 127) / 128, 128, 0, st>>>(coef_d, out_d);
   return cudaGetLastError();
 }
 

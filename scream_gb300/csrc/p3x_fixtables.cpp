@@ -6,6 +6,8 @@
 
 #include <cmath>
 
+#include "p3x_fixtest.hpp"
+
 namespace p3x {
 
 void build_ice_cells(const double* ice, const int cols[dev::kCellCols], std::vector<int64_t>& coef,
@@ -48,6 +50,20 @@ void build_ice_cells(const double* ice, const int cols[dev::kCellCols], std::vec
           for (int m = 0; m < dev::kCellCoefs; ++m)
             coef[cell * dev::kCellCoefs + m] = std::llroundl(std::ldexp(k[m], kWeights[m] + s));
         }
+}
+
+std::vector<int64_t> fix_test_coefficients() {
+  std::vector<int64_t> coef(size_t(kFixTestCells) * dev::kCellCoefs);
+  dev::FixTestHash next{1};
+  for (int64_t& c : coef) c = int64_t(next()) >> 4;
+  return coef;
+}
+
+std::vector<uint64_t> fix_test_words(const std::vector<int64_t>& coef) {
+  std::vector<uint64_t> out(size_t(kFixTestRows) * kFixTestWords);
+  for (int i = 0; i < kFixTestRows; ++i)
+    dev::fix_test_row(uint64_t(i), &dev::kFixTables, coef.data(), &out[size_t(i) * kFixTestWords]);
+  return out;
 }
 
 }  // namespace p3x

@@ -16,6 +16,11 @@ namespace p3x {
 void build_ice_cells(const double* ice, const int cols[dev::kCellCols], std::vector<int64_t>& coef,
                      std::vector<int32_t>& shift);
 
+/* The host's words of the fixed-point self-test (p3x_fixtest.hpp): kFixTestRows
+ * rows of kFixTestWords for these coefficients. */
+std::vector<int64_t> fix_test_coefficients();
+std::vector<uint64_t> fix_test_words(const std::vector<int64_t>& coef);
+
 }  // namespace p3x
 
 #endif

@@ -177,6 +177,8 @@ cudaError_t launch_eam(const EamPtrs& p, int ncol, int nlev, int64_t ld, int64_t
 cudaError_t saturation_at_melting(double* out);
 
 cudaError_t launch_selftest(unsigned long long* mismatches_d, cudaStream_t st);
+/* The device's words of the fixed-point self-test (p3x_fixtest.hpp). */
+cudaError_t launch_fix_selftest(const int64_t* coef_d, uint64_t* out_d, cudaStream_t st);
 
 /* Fields of the column mass / energy conservation check (device pointers;
  * per-level (ncol, ld), winds (ncol, 2, ld), per-column (ncol)). */
