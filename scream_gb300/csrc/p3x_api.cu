@@ -1555,8 +1555,7 @@ int p3x_batch_create(p3x_context* ctx, const p3x_runtime* rt, const p3x_instance
   P3X_CUDA(cudaMalloc(&b->insts_d, sizeof(dev::Inst) * n));
   P3X_CUDA(cudaMemcpy(b->insts_d, insts.data(), sizeof(dev::Inst) * n, cudaMemcpyHostToDevice));
   for (int p = 0; p < 2; ++p) {
-    /* deeper columns first, then interleave instances so that neighbouring
-     * work items belong to different instances */
+    /* deeper columns first; an instance's columns in a row, which part1+2 pools */
     std::vector<int> idx;
     for (int i = 0; i < n; ++i)
       if (insts[i].precision == p) idx.push_back(i);

@@ -124,8 +124,8 @@ cudaError_t launch_transpose_to_levels(const double* src, double* dst, int ncol,
 cudaError_t launch_transpose_to_columns(const double* src, double* dst, int ncol, int nlev, int64_t ld,
                                         cudaStream_t st);
 
-/* One step of a work list of (instance, column) items whose instances all
- * have the given precision: K1, K2, K3 with the context's launch
+/* One step of a work list of (instance, column) items, each column once and in
+ * any order (dev::WorkItem), whose instances all have the given precision: K1, K2, K3 with the context's launch
  * configuration for that precision (p3x_api.cu).  Every instance's scratch
  * must be bound.  wctr: dev::kWorkCounters device words used by no other
  * launch in flight (zeroed on the stream), or null for a static stride. */
