@@ -1656,7 +1656,7 @@ __device__ void p3_sed(const Inst& in, const int col, const KParams<TR>& kp, con
  * alias, so each would wait for memory by itself; they are therefore grouped by
  * hand: the density a chunk ahead in the flux walk, two chunks at a time where a
  * species is read, all fields of a chunk at once where its state is rebuilt.
- * 345,600 x 128 9.30 -> 8.00 ms, 21,600 x 128 822 -> 721 us. */
+ * 345,600 x 128 9.30 -> 8.05 ms, 21,600 x 128 822 -> 727 us. */
 template <int LANES, bool SPLIT = false>
 __device__ void p3_sed_bulk(const Inst& in, const int col, const KParams<float>& kp, const Tabs<float>& tb,
                             double* __restrict__ sm, GroupScratch* gs, uint32_t& err) {
